@@ -18,6 +18,11 @@
 // The products run on the warp-level tensor cores (mma.sync, bfloat16 with float sums). Everything that enters them is float: silu of
 // queries, keys and values (where asked for), powers of the decay, states, weighted scores; each operand is the sum of two bfloat16
 // terms (16 bits of mantissa), of whose four products three are taken. States and sums stay float.
+//
+// Queries and keys that are rotated by position on their way in (retention; in float, so that what enters the recurrence is never
+// rounded to 16 bits) take three terms (24 bits, a float's) and the six products above 2^-24 of them; values are then bfloat16
+// already and one term. What bounded the walk row by row was its chain, 160 to 270 us for portions of up to 1,000 rows, 12 heads of
+// 32 x 64, whatever their number of heads; in chunks the outputs, the longest of the three launches, take 17.5.
 #include <math.h>
 
 #include "common.cuh"
@@ -41,6 +46,8 @@ struct ChunkArgs {
   float* out; int out_stride;
   int n_heads, dim, vdim, dim16;   // dim16: dim to a multiple of 16
   int vec;                         // rows, heads and slices start on 16-byte boundaries and hold multiples of eight numbers
+  const float* inv_freq; int rot_half;   // of q and k the first 2 * rot_half dimensions turn, dimension i with i + rot_half, by the
+  const int32_t* positions;              // angle positions[row] * inv_freq[i] (rot_half 0: none do)
 };
 
 struct Tile { int entry, row0, rows; };   // entry -1: no such chunk
@@ -86,19 +93,40 @@ __device__ __forceinline__ float power(float decay, int n) {
   return out;
 }
 
-// A matrix in shared memory as two bfloat16 terms, rows `stride` numbers apart.
-struct Split { bf16* hi; bf16* lo; int stride; };
+// A matrix in shared memory as N bfloat16 terms, rows `stride` numbers apart.
+template <int N>
+struct Split { bf16* term[N]; int stride; };
 
-__device__ __forceinline__ void put2(const Split& m, int r, int c, float x, float y) {
-  const uint32_t head = pack_pair(x, y);
-  *reinterpret_cast<uint32_t*>(m.hi + r * m.stride + c) = head;
-  *reinterpret_cast<uint32_t*>(m.lo + r * m.stride + c) = pack_rest(x, y, head);
+template <int N>
+__device__ __forceinline__ void put2(const Split<N>& m, int r, int c, float x, float y) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const uint32_t head = pack_pair(x, y);
+    *reinterpret_cast<uint32_t*>(m.term[i] + r * m.stride + c) = head;
+    if (i + 1 < N) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&head));
+      x -= f.x;
+      y -= f.y;
+    }
+  }
 }
 
-// `rows` rows of `cols` numbers (zeros up to CHUNK rows and `padded` columns), silu, times `scale` and, with `powers`, times
+// cos and sin of a chunk's rows: [CHUNK][rot_half] each
+struct Turns { const float* cos; const float* sin; int half; };
+__device__ __forceinline__ Turns make_turns(const ChunkArgs& a, int row0, int rows, float* at) {
+  const int half = a.rot_half;
+  for (int i = threadIdx.x; i < rows * half; i += THREADS) {
+    const int r = i / half, d = i - r * half;
+    sincosf(float(a.positions[row0 + r]) * a.inv_freq[d], at + CHUNK * half + i, at + i);
+  }
+  return {at, at + CHUNK * half, half};
+}
+
+// `rows` rows of `cols` numbers (zeros up to CHUNK rows and `padded` columns), turned or silu, times `scale` and, with `powers`, times
 // powers[rows - 1 - row].
-__device__ __forceinline__ void stage(const Split& m, const bf16* src, long long stride, int rows, int cols, int padded, bool silu_in, float scale,
-                                      const float* powers, bool vec) {
+template <int N>
+__device__ __forceinline__ void stage(const Split<N>& m, const bf16* src, long long stride, int rows, int cols, int padded, bool silu_in, float scale,
+                                      const float* powers, bool vec, Turns turns = {nullptr, nullptr, 0}) {
   const int pieces = padded / 8;
   for (int i = threadIdx.x; i < CHUNK * pieces; i += THREADS) {
     const int r = i / pieces, c = (i - r * pieces) * 8;
@@ -120,6 +148,18 @@ __device__ __forceinline__ void stage(const Split& m, const bf16* src, long long
 #pragma unroll
         for (int u = 0; u < 8; ++u)
           if (c + u < cols) x[u] = to_float(p[u]);
+      }
+      if (turns.half > 0) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int d = c + u;
+          if (d < 2 * turns.half && d < cols) {   // the pair (u, v) becomes (u cos - v sin, v cos + u sin)
+            const bool low = d < turns.half;
+            const int pair = low ? d : d - turns.half, at = r * turns.half + pair;
+            const float other = to_float(src[r * stride + (low ? d + turns.half : pair)]);
+            x[u] = fmaf(x[u], turns.cos[at], other * (low ? -turns.sin[at] : turns.sin[at]));
+          }
+        }
       }
       const float factor = powers != nullptr ? scale * powers[rows - 1 - r] : scale;
 #pragma unroll
@@ -151,20 +191,32 @@ __device__ __forceinline__ void load_b_transposed(const bf16* m, int stride, int
   const int lane = threadIdx.x & 31;
   ldmatrix_x4_trans(smem_u32(m + (k + (lane & 15)) * stride + n + (lane >> 4) * 8), f[0], f[1], f[2], f[3]);
 }
-// (a_hi + a_lo)(b_hi + b_lo) without the product of the two small terms, for one tile of 8 columns
-__device__ __forceinline__ void mma_split(float (&c)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], uint32_t bh0, uint32_t bh1, uint32_t bl0, uint32_t bl1) {
-  mma_bf16(c, al[0], al[1], al[2], al[3], bh0, bh1);
-  mma_bf16(c, ah[0], ah[1], ah[2], ah[3], bl0, bl1);
-  mma_bf16(c, ah[0], ah[1], ah[2], ah[3], bh0, bh1);
+// (the sum of a's terms)(the sum of b's terms) for one tile of 8 columns, smallest products first; those below the last term of the longer
+// operand are left out
+template <int N, int M>
+__device__ __forceinline__ void mma_split(float (&c)[4], const uint32_t (&a)[N][4], const uint32_t (&b)[M][4], int half) {
+#pragma unroll
+  for (int order = (N > M ? N : M) - 1; order >= 0; --order)
+#pragma unroll
+    for (int i = N - 1; i >= 0; --i) {
+      const int j = order - i;
+      if (j >= 0 && j < M) mma_bf16(c, a[i][0], a[i][1], a[i][2], a[i][3], b[j < 0 || j >= M ? 0 : j][2 * half], b[j < 0 || j >= M ? 0 : j][2 * half + 1]);
+    }
 }
 
-__device__ __forceinline__ Split carve(uint8_t*& at, int rows, int stride) {
-  Split m = {reinterpret_cast<bf16*>(at), reinterpret_cast<bf16*>(at) + rows * stride, stride};
-  at += size_t(rows) * stride * 2 * sizeof(bf16);
+template <int N>
+__device__ __forceinline__ Split<N> carve(uint8_t*& at, int rows, int stride) {
+  Split<N> m;
+#pragma unroll
+  for (int i = 0; i < N; ++i) m.term[i] = reinterpret_cast<bf16*>(at) + size_t(i) * rows * stride;
+  m.stride = stride;
+  at += size_t(rows) * stride * N * sizeof(bf16);
   return m;
 }
 
+// N: terms of queries, keys, states and weighted scores; M: of values.
 // U of a chunk: [dim x COLS of the value columns]. Grid: chunks, heads, slices of the columns.
+template <int N, int M>
 __global__ void __launch_bounds__(THREADS)
 decay_chunk_sums_kernel(const ChunkArgs a) {
   pdl_launch_dependents();
@@ -177,25 +229,31 @@ decay_chunk_sums_kernel(const ChunkArgs a) {
   pdl_wait();
   if (tile.entry < 0) return;
   uint8_t* at = smem;
-  const Split k = carve(at, CHUNK, a.dim16 + 8), v = carve(at, CHUNK, COLS + 8);
+  const Split<N> k = carve<N>(at, CHUNK, a.dim16 + 8);
+  const Split<M> v = carve<M>(at, CHUNK, COLS + 8);
+  Turns turns = {nullptr, nullptr, 0};
+  if (a.rot_half > 0) {
+    turns = make_turns(a, tile.row0, tile.rows, reinterpret_cast<float*>(at));
+    __syncthreads();
+  }
   const int cols = min(COLS, a.vdim - col0);
-  stage(k, a.k + size_t(tile.row0) * a.k_stride + size_t(h) * a.dim, a.k_stride, tile.rows, a.dim, a.dim16, a.silu_in, a.k_scale, powers, a.vec);
+  stage(k, a.k + size_t(tile.row0) * a.k_stride + size_t(h) * a.dim, a.k_stride, tile.rows, a.dim, a.dim16, a.silu_in, a.k_scale, powers, a.vec, turns);
   stage(v, a.v + size_t(tile.row0) * a.v_stride + size_t(h) * a.vdim + col0, a.v_stride, tile.rows, cols, COLS, a.silu_in, 1.f, nullptr, a.vec);
   __syncthreads();
   float* sums = a.sums + (size_t(blockIdx.x) * a.n_heads + h) * a.dim * a.vdim + col0;
   for (int m0 = warp * 16; m0 < a.dim16; m0 += (THREADS / 32) * 16) {
     float acc[COLS / 8][4] = {};
     for (int j = 0; j < tile.rows; j += 16) {
-      uint32_t ah[4], al[4];
-      load_a_transposed(k.hi, k.stride, j, m0, ah);
-      load_a_transposed(k.lo, k.stride, j, m0, al);
+      uint32_t kf[N][4];
+#pragma unroll
+      for (int i = 0; i < N; ++i) load_a_transposed(k.term[i], k.stride, j, m0, kf[i]);
 #pragma unroll
       for (int n = 0; n < COLS; n += 16) {
-        uint32_t bh[4], bl[4];
-        load_b_transposed(v.hi, v.stride, j, n, bh);
-        load_b_transposed(v.lo, v.stride, j, n, bl);
-        mma_split(acc[n / 8], ah, al, bh[0], bh[1], bl[0], bl[1]);
-        mma_split(acc[n / 8 + 1], ah, al, bh[2], bh[3], bl[2], bl[3]);
+        uint32_t vf[M][4];
+#pragma unroll
+        for (int i = 0; i < M; ++i) load_b_transposed(v.term[i], v.stride, j, n, vf[i]);
+        mma_split(acc[n / 8], kf, vf, 0);
+        mma_split(acc[n / 8 + 1], kf, vf, 1);
       }
     }
 #pragma unroll
@@ -255,6 +313,7 @@ decay_chunk_states_kernel(const ChunkArgs a) {
 }
 
 // Outputs of a chunk. Grid: chunks, heads, slices of the columns. A warp has 16 of the chunk's rows.
+template <int N, int M>
 __global__ void __launch_bounds__(THREADS)
 decay_chunk_outputs_kernel(const ChunkArgs a) {
   pdl_launch_dependents();
@@ -267,10 +326,17 @@ decay_chunk_outputs_kernel(const ChunkArgs a) {
   pdl_wait();
   if (tile.entry < 0) return;
   uint8_t* at = smem;
-  const Split q = carve(at, CHUNK, a.dim16 + 8), k = carve(at, CHUNK, a.dim16 + 8), v = carve(at, CHUNK, COLS + 8), s = carve(at, a.dim16, COLS + 8);
+  const Split<N> q = carve<N>(at, CHUNK, a.dim16 + 8), k = carve<N>(at, CHUNK, a.dim16 + 8);
+  const Split<M> v = carve<M>(at, CHUNK, COLS + 8);
+  const Split<N> s = carve<N>(at, a.dim16, COLS + 8);
+  Turns turns = {nullptr, nullptr, 0};
+  if (a.rot_half > 0) {
+    turns = make_turns(a, tile.row0, tile.rows, reinterpret_cast<float*>(at));
+    __syncthreads();
+  }
   const int cols = min(COLS, a.vdim - col0);
-  stage(q, a.q + size_t(tile.row0) * a.q_stride + size_t(h) * a.dim, a.q_stride, tile.rows, a.dim, a.dim16, a.silu_in, 1.f, nullptr, a.vec);
-  stage(k, a.k + size_t(tile.row0) * a.k_stride + size_t(h) * a.dim, a.k_stride, tile.rows, a.dim, a.dim16, a.silu_in, a.k_scale, nullptr, a.vec);
+  stage(q, a.q + size_t(tile.row0) * a.q_stride + size_t(h) * a.dim, a.q_stride, tile.rows, a.dim, a.dim16, a.silu_in, 1.f, nullptr, a.vec, turns);
+  stage(k, a.k + size_t(tile.row0) * a.k_stride + size_t(h) * a.dim, a.k_stride, tile.rows, a.dim, a.dim16, a.silu_in, a.k_scale, nullptr, a.vec, turns);
   stage(v, a.v + size_t(tile.row0) * a.v_stride + size_t(h) * a.vdim + col0, a.v_stride, tile.rows, cols, COLS, a.silu_in, 1.f, nullptr, a.vec);
   const float* start = a.sums + (size_t(blockIdx.x) * a.n_heads + h) * a.dim * a.vdim + col0;
   for (int i = threadIdx.x; i < a.dim16 * (COLS / 2); i += THREADS) {
@@ -284,25 +350,25 @@ decay_chunk_outputs_kernel(const ChunkArgs a) {
   // what the chunk's first state gives, and the scores of the rows up to each row
   float acc[COLS / 8][4] = {}, p[CHUNK / 8][4] = {};
   for (int d = 0; d < a.dim16; d += 16) {
-    uint32_t ah[4], al[4];
-    load_a(q.hi, q.stride, i0, d, ah);
-    load_a(q.lo, q.stride, i0, d, al);
+    uint32_t qf[N][4];
+#pragma unroll
+    for (int i = 0; i < N; ++i) load_a(q.term[i], q.stride, i0, d, qf[i]);
 #pragma unroll
     for (int n = 0; n < COLS; n += 16) {
-      uint32_t bh[4], bl[4];
-      load_b_transposed(s.hi, s.stride, d, n, bh);
-      load_b_transposed(s.lo, s.stride, d, n, bl);
-      mma_split(acc[n / 8], ah, al, bh[0], bh[1], bl[0], bl[1]);
-      mma_split(acc[n / 8 + 1], ah, al, bh[2], bh[3], bl[2], bl[3]);
+      uint32_t sf[N][4];
+#pragma unroll
+      for (int i = 0; i < N; ++i) load_b_transposed(s.term[i], s.stride, d, n, sf[i]);
+      mma_split(acc[n / 8], qf, sf, 0);
+      mma_split(acc[n / 8 + 1], qf, sf, 1);
     }
 #pragma unroll
     for (int j = 0; j < CHUNK; j += 16) {
       if (j <= i0) {   // (later rows are seen by none of the warp's)
-        uint32_t bh[4], bl[4];
-        load_b(k.hi, k.stride, j, d, bh);
-        load_b(k.lo, k.stride, j, d, bl);
-        mma_split(p[j / 8], ah, al, bh[0], bh[1], bl[0], bl[1]);
-        mma_split(p[j / 8 + 1], ah, al, bh[2], bh[3], bl[2], bl[3]);
+        uint32_t kf[N][4];
+#pragma unroll
+        for (int i = 0; i < N; ++i) load_b(k.term[i], k.stride, j, d, kf[i]);
+        mma_split(p[j / 8], qf, kf, 0);
+        mma_split(p[j / 8 + 1], qf, kf, 1);
       }
     }
   }
@@ -318,25 +384,32 @@ decay_chunk_outputs_kernel(const ChunkArgs a) {
 #pragma unroll
   for (int j = 0; j < CHUNK; j += 16) {
     if (j > i0) break;
-    uint32_t ah[4], al[4];
+    uint32_t wf[N][4];
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       float* w = p[j / 8 + half];
       const int c = j + half * 8 + (lane & 3) * 2;
-      const float w0 = c <= r ? w[0] * powers[r - c] : 0.f, w1 = c + 1 <= r ? w[1] * powers[r - c - 1] : 0.f;
-      const float w2 = c <= r + 8 ? w[2] * powers[r + 8 - c] : 0.f, w3 = c + 1 <= r + 8 ? w[3] * powers[r + 7 - c] : 0.f;
-      ah[2 * half] = pack_pair(w0, w1);
-      al[2 * half] = pack_rest(w0, w1, ah[2 * half]);
-      ah[2 * half + 1] = pack_pair(w2, w3);
-      al[2 * half + 1] = pack_rest(w2, w3, ah[2 * half + 1]);
+      float w0 = c <= r ? w[0] * powers[r - c] : 0.f, w1 = c + 1 <= r ? w[1] * powers[r - c - 1] : 0.f;
+      float w2 = c <= r + 8 ? w[2] * powers[r + 8 - c] : 0.f, w3 = c + 1 <= r + 8 ? w[3] * powers[r + 7 - c] : 0.f;
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        wf[i][2 * half] = pack_pair(w0, w1);
+        wf[i][2 * half + 1] = pack_pair(w2, w3);
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wf[i][2 * half]));
+        const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wf[i][2 * half + 1]));
+        w0 -= f.x;
+        w1 -= f.y;
+        w2 -= g.x;
+        w3 -= g.y;
+      }
     }
 #pragma unroll
     for (int n = 0; n < COLS; n += 16) {
-      uint32_t bh[4], bl[4];
-      load_b_transposed(v.hi, v.stride, j, n, bh);
-      load_b_transposed(v.lo, v.stride, j, n, bl);
-      mma_split(acc[n / 8], ah, al, bh[0], bh[1], bl[0], bl[1]);
-      mma_split(acc[n / 8 + 1], ah, al, bh[2], bh[3], bl[2], bl[3]);
+      uint32_t vf[M][4];
+#pragma unroll
+      for (int i = 0; i < M; ++i) load_b_transposed(v.term[i], v.stride, j, n, vf[i]);
+      mma_split(acc[n / 8], wf, vf, 0);
+      mma_split(acc[n / 8 + 1], wf, vf, 1);
     }
   }
   float* out = a.out + size_t(h) * a.vdim + col0;
@@ -400,7 +473,16 @@ decay_step_kernel(const ChunkArgs a, int slice) {
     const bf16* q = a.q + size_t(t) * a.q_stride + size_t(h) * a.dim;
     const bf16* k = a.k + size_t(t) * a.k_stride + size_t(h) * a.dim;
     for (int i = threadIdx.x; i < a.dim; i += STEP_THREADS) {
-      const float x = to_float(q[i]), y = to_float(k[i]);
+      float x = to_float(q[i]), y = to_float(k[i]);
+      if (i < 2 * a.rot_half) {
+        const bool low = i < a.rot_half;
+        const int other = low ? i + a.rot_half : i - a.rot_half;
+        float sn, cs;
+        sincosf(float(a.positions[t]) * a.inv_freq[low ? i : other], &sn, &cs);
+        if (low) sn = -sn;
+        x = fmaf(x, cs, to_float(q[other]) * sn);
+        y = fmaf(y, cs, to_float(k[other]) * sn);
+      }
       qs[i] = a.silu_in ? silu(x) : x;
       ks[i] = (a.silu_in ? silu(y) : y) * a.k_scale;
     }
@@ -447,7 +529,30 @@ decay_step_kernel(const ChunkArgs a, int slice) {
   }
 }
 
-size_t split_bytes(int rows, int stride) { return size_t(rows) * stride * 2 * sizeof(bf16); }
+size_t split_bytes(int rows, int stride, int terms) { return size_t(rows) * stride * terms * sizeof(bf16); }
+
+template <int N, int M>
+int launch_chunks(const ChunkArgs& a, int n_tiles, cudaStream_t stream) {
+  const size_t rows_q = split_bytes(CHUNK, a.dim16 + 8, N), rows_v = split_bytes(CHUNK, COLS + 8, M), turns = size_t(2) * CHUNK * a.rot_half * sizeof(float);
+  const size_t smem_sums = rows_q + rows_v + turns, smem_out = 2 * rows_q + rows_v + split_bytes(a.dim16, COLS + 8, N) + turns;
+  constexpr size_t MOST = 226 * 1024;   // (beside the kernels' own few hundred bytes)
+  if (smem_out > MOST) return R2_UNSUPPORTED;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(decay_chunk_outputs_kernel<N, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(MOST));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_chunk_sums_kernel<N, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(MOST));
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return R2_UNSUPPORTED;
+    }
+    configured = true;
+  }
+  const dim3 grid(n_tiles, a.n_heads, (a.vdim + COLS - 1) / COLS);
+  r2_launch(decay_chunk_sums_kernel<N, M>, grid, dim3(THREADS), smem_sums, stream, a);
+  r2_launch(decay_chunk_states_kernel, dim3(a.n_entries, a.n_heads, (a.dim * a.vdim + 255) / 256), dim3(256), size_t(0), stream, a);
+  r2_launch(decay_chunk_outputs_kernel<N, M>, grid, dim3(THREADS), smem_out, stream, a);
+  return launch_status();
+}
 
 }  // namespace
 
@@ -456,12 +561,14 @@ extern "C" long long r2_decay_chunks_floats(int n_tiles, int n_heads, int dim, i
 
 // q, k [T, heads * dim], v [T, heads * vdim] bfloat16 (slices of a projection); decay float [heads]; silu_in: silu of all three on their
 // way in, k then times k_scale; state float [slots][heads][dim][vdim]; n_tiles at least the sum over entries of ceil(rows / 64); scratch
-// float (r2_decay_chunks_floats); out float [T, heads * vdim]. Three launches. R2_UNSUPPORTED: heads of more than 256 rows.
+// float (r2_decay_chunks_floats); out float [T, heads * vdim]. inv_freq float [rot_half] and positions [T] where q and k turn (then without
+// silu). Three launches. R2_UNSUPPORTED: heads of more than 256 rows (fewer, where they turn: what an SM's shared memory holds).
 extern "C" int r2_decay_chunks(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, const float* decay, float k_scale,
                                int silu_in, float* state, long long slot_stride, const int32_t* q_start, const int32_t* state_slot, const int32_t* fresh,
                                int n_entries, int n_tiles, float* scratch, long long scratch_floats, float* out, int out_stride, int n_heads, int dim,
-                               int vdim, cudaStream_t stream) {
+                               int vdim, const float* inv_freq, int rot_half, const int32_t* positions, cudaStream_t stream) {
   if (n_entries <= 0 || n_tiles <= 0) return R2_OK;
+  if (rot_half < 0 || 2 * rot_half > dim || (rot_half > 0 && (inv_freq == nullptr || positions == nullptr || silu_in))) return R2_BAD_SHAPE;
   if (n_heads < 1 || dim < 1 || vdim < 1 || scratch == nullptr || scratch_floats < r2_decay_chunks_floats(n_tiles, n_heads, dim, vdim)) return R2_BAD_SHAPE;
   if (dim > MAX_DIM || n_heads > 65535 || n_tiles > (1 << 20)) return R2_UNSUPPORTED;
   ChunkArgs a = {};
@@ -471,31 +578,17 @@ extern "C" int r2_decay_chunks(const void* q, int q_stride, const void* k, int k
   a.n_heads = n_heads; a.dim = dim; a.vdim = vdim; a.dim16 = (dim + 15) / 16 * 16;
   a.vec = dim % 8 == 0 && vdim % 8 == 0 && q_stride % 8 == 0 && k_stride % 8 == 0 && v_stride % 8 == 0 &&
           !((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15);
-  const size_t rows_q = split_bytes(CHUNK, a.dim16 + 8), rows_v = split_bytes(CHUNK, COLS + 8);
-  const size_t smem_sums = rows_q + rows_v, smem_out = 2 * rows_q + rows_v + split_bytes(a.dim16, COLS + 8);
-  static bool configured = false;
-  if (!configured) {
-    const int most = int(2 * split_bytes(CHUNK, MAX_DIM + 8) + split_bytes(CHUNK, COLS + 8) + split_bytes(MAX_DIM, COLS + 8));
-    cudaError_t e = cudaFuncSetAttribute(decay_chunk_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_chunk_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return R2_UNSUPPORTED;
-    }
-    configured = true;
-  }
-  const dim3 grid(n_tiles, n_heads, (vdim + COLS - 1) / COLS);
-  r2_launch(decay_chunk_sums_kernel, grid, dim3(THREADS), smem_sums, stream, a);
-  r2_launch(decay_chunk_states_kernel, dim3(n_entries, n_heads, (dim * vdim + 255) / 256), dim3(256), size_t(0), stream, a);
-  r2_launch(decay_chunk_outputs_kernel, grid, dim3(THREADS), smem_out, stream, a);
-  return launch_status();
+  a.inv_freq = inv_freq; a.rot_half = rot_half; a.positions = positions;
+  return rot_half > 0 ? launch_chunks<3, 1>(a, n_tiles, stream) : launch_chunks<2, 2>(a, n_tiles, stream);
 }
 
 // The same for batches in which (nearly) every entry is one row: one launch, no scratch.
 extern "C" int r2_decay_step(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, const float* decay, float k_scale,
                              int silu_in, float* state, long long slot_stride, const int32_t* q_start, const int32_t* state_slot, const int32_t* fresh,
-                             int n_entries, float* out, int out_stride, int n_heads, int dim, int vdim, int n_sms, cudaStream_t stream) {
+                             int n_entries, float* out, int out_stride, int n_heads, int dim, int vdim, int n_sms, const float* inv_freq, int rot_half,
+                             const int32_t* positions, cudaStream_t stream) {
   if (n_entries <= 0) return R2_OK;
+  if (rot_half < 0 || 2 * rot_half > dim || (rot_half > 0 && (inv_freq == nullptr || positions == nullptr || silu_in))) return R2_BAD_SHAPE;
   if (n_heads < 1 || dim < 1 || vdim < 1 || n_sms < 1) return R2_BAD_SHAPE;
   if (dim > MAX_DIM || n_heads > 65535) return R2_UNSUPPORTED;
   ChunkArgs a = {};
@@ -503,6 +596,7 @@ extern "C" int r2_decay_step(const void* q, int q_stride, const void* k, int k_s
   a.decay = decay; a.k_scale = k_scale; a.silu_in = silu_in; a.state = state; a.slot_stride = slot_stride;
   a.q_start = q_start; a.state_slot = state_slot; a.fresh = fresh; a.n_entries = n_entries; a.out = out; a.out_stride = out_stride;
   a.n_heads = n_heads; a.dim = dim; a.vdim = vdim;
+  a.inv_freq = inv_freq; a.rot_half = rot_half; a.positions = positions;
   // as many columns a CTA as leave twice as many CTAs as the GPU has SMs
   int slice = 64;
   while (slice > 16 && (long long)n_entries * n_heads * ((vdim + slice - 1) / slice) < 2ll * n_sms) slice /= 2;

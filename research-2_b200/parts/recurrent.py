@@ -87,8 +87,9 @@ class Retention:
 
     (rotation: of each head the first rot_dims dimensions, dimension i with i + rot_dims / 2, by the angle position *
     rot_freqs[i]). Each head's o is divided by its root mean square (no gain), the heads are concatenated, multiplied by
-    silu(W_g h) and projected by W_o. The rotation happens inside the recurrence's kernel, in float32: what enters the
-    recurrence is the projections' values and nothing rounded after them.
+    silu(W_g h) and projected by W_o. The rotation happens inside the recurrence's kernels, in float32: what enters the
+    recurrence is the projections' values and nothing rounded after them. Prompts in bfloat16 go in chunks of 64 rows on the tensor cores,
+    float32 operands as three bfloat16 terms; decoded tokens, and everything in float32, row by row.
 
     params: n_heads, head_dim, v_head_dim, decay (one number per head), rot_dims, rot_freqs, norm_eps.
     weights (stored [out, in], no biases): w_q, w_k [H head_dim, D], w_v, w_gate [H v_head_dim, D], w_out [D, H v_head_dim]."""
@@ -126,7 +127,7 @@ class Retention:
         a, b = self.qk_width, 2 * self.qk_width
         o = ops.retention_scan(proj[:, :a], proj[:, a:b], proj[:, b: b + self.v_width], self.decay, self.head_dim ** -0.5, self.freqs,
                                self.rot_dims, ctx.positions, state, ctx.q_start, ctx.state_slot, ctx.fresh, self.n_heads, self.head_dim,
-                               self.v_head_dim)
+                               self.v_head_dim, n_tiles=ctx.n_attention_tiles)
         return ops.group_norm_gated(o, proj[:, b + self.v_width:], None, self.n_heads, self.norm_eps, "silu_after", proj.dtype)
 
     def mix(self, h, ctx, cache=None, state=None, writes_cache: bool = True):
