@@ -74,7 +74,7 @@ using namespace r2ptx;
 constexpr int JOIN_BYTES = (HD + 2) * BM * 4;
 
 template <int SPLIT, bool X>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 2)  // (tensor memory holds two CTAs' scores and outputs)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                   const __grid_constant__ CUtensorMap map_v, const Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -338,96 +338,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     // and the store's completion pass under one another instead of one after the other. `fetch` always
     // issues its loads (past the last tile: of a buffer that exists), so that the registers are defined on
     // one path only and nothing the compiler adds reads them before the wait at the end of the loop's body.
-    uint32_t s0[32], s1[32];
-    auto fetch = [&](int it) {
-      if (it < n_mine && ok && !mbar_wait(s_ready_a + uint32_t(it & 1) * 8u, uint32_t(it >> 1) & 1u)) {
-        if (lane == 0) atomicMax(p.error_flag, R2_ERR_TIMEOUT_ATTN);
-        ok = false;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t at = lane_base + uint32_t(it & 1) * 64u;
-      tmem_load32(at, s0);
-      tmem_load32(at + 32u, s1);
-    };
-    fetch(0);
-    tmem_load_wait(s0);
-    tmem_tie(s1);
-    for (int it = 0; it < n_mine; ++it) {
-      const int j0 = j_of(it);
-      const uint32_t s_at = lane_base + uint32_t(it & 1) * 64u;
-      // mask in float: causal and window. Key c of the tile is seen if lo_c <= c <= hi (plain predicate
-      // logic on two registers: written with && and || over the position this loop took 1,300 cycles a tile).
-      const int hi = pos - j0;
-      const int lo_c = p.window > 0 ? pos - p.window + 1 - j0 : 0;
-      const int kf = keep - j0;   // (X) keys of the tile below it are kept first keys; without them it is <= 0
-      if (hi < BN - 1 || (lo_c > 0 && kf < BN)) {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const bool seen_a = (c <= hi) & ((c >= lo_c) | (X && c < kf));
-          const bool seen_b = (c + 32 <= hi) & ((c + 32 >= lo_c) | (X && c + 32 < kf));
-          s0[c] = seen_a ? s0[c] : __float_as_uint(-INFINITY);
-          s1[c] = seen_b ? s1[c] : __float_as_uint(-INFINITY);
-        }
-      }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains: the maximum's latency, not its count, is what costs
-#pragma unroll
-      for (int c = 0; c < 32; ++c) mx4[c & 3] = max3(mx4[c & 3], __uint_as_float(s0[c]), __uint_as_float(s1[c]));
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      // The maximum in use moves only when this tile's exceeds it by more than the step.
-      const float m_tile = mx * scale2;
-      const bool grow = m_tile > m_run + RESCALE_STEP || (m_run == -INFINITY && m_tile > -INFINITY);
-      const float m_new = grow ? m_tile : m_run;
-      const float base = m_new == -INFINITY ? 0.f : m_new;  // a row that has seen no key yet
-      const float corr = grow ? fast_exp2(m_run - base) : 1.f;
-      float sum_a = 0.f, sum_b = 0.f;
-      uint32_t pk[32];  // the row of P, two bfloat16 to a word: keys 2w and 2w + 1
-      uint32_t pr[X ? 32 : 1];  // (X) what the rounding left of each weight, as a second row of bfloat16
-#pragma unroll
-      for (int w = 0; w < 16; ++w) {
-        const float a0 = fast_exp2(fmaf(__uint_as_float(s0[2 * w]), scale2, -base));
-        const float a1 = fast_exp2(fmaf(__uint_as_float(s0[2 * w + 1]), scale2, -base));
-        const float b0 = fast_exp2(fmaf(__uint_as_float(s1[2 * w]), scale2, -base));
-        const float b1 = fast_exp2(fmaf(__uint_as_float(s1[2 * w + 1]), scale2, -base));
-        sum_a += a0 + a1;
-        sum_b += b0 + b1;
-        pk[w] = pack_bf16(a0, a1);
-        pk[16 + w] = pack_bf16(b0, b1);
-        if (X) {
-          const float2 ha = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[w]));
-          const float2 hb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[16 + w]));
-          pr[w] = pack_bf16(a0 - ha.x, a1 - ha.y);
-          pr[16 + w] = pack_bf16(b0 - hb.x, b1 - hb.y);
-        }
-      }
-      l_run = l_run * corr + (sum_a + sum_b);
-      m_run = m_new;
-      if (it > 0 && __any_sync(0xffffffffu, grow)) {
-        // O times the correction, once the product of the previous tile has completed (the warp
-        // decides together: every lane's tensor-memory access is one instruction)
-        if (ok && !mbar_wait(pv_done_a, uint32_t(it - 1) & 1u)) {
-          if (lane == 0) atomicMax(p.error_flag, R2_ERR_TIMEOUT_ATTN);
-          ok = false;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int part = 0; part < 2; ++part) {
-          uint32_t o[32];
-          tmem_load32(lane_base + 128u + uint32_t(part * 32), o);
-          tmem_load_wait(o);
-#pragma unroll
-          for (int c = 0; c < 32; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * corr);
-          tmem_store32(lane_base + 128u + uint32_t(part * 32), o);
-        }
-      }
-      tmem_store32(s_at, pk);  // over the scores this thread has read
-      if constexpr (X) {
-        if (p.split_p) tmem_store32(s_at + 32u, pr);   // the other half of the same buffer, which this thread has read too
-      }
-      fetch(it + 1);           // (the registers of the scores are free)
+    // Keys of a tile outside those that any row may see were not copied, or hold whatever
+    // their slots held: their p is 0, but the product multiplies, so their value rows must
+    // be finite. They are set to zero (the stage has landed: its scores exist).
+    auto zero_unseen = [&](int it, int j0) {
       if ((j0 < lo && j0 + BN > keep) || j0 + BN - 1 > pmax) {
-        // Keys of this tile outside those that any row may see were not copied, or hold whatever
-        // their slots held: their p is 0, but the product multiplies, so their value rows must
-        // be finite. They are set to zero (the stage has landed: its scores exist).
         const int j = j0 + row;
         if (row < BN && ((j < lo && j >= keep) || j > pmax)) {
           const uint32_t dst = smem_u32(v_s) + uint32_t((it % STAGES) * KV_BYTES + row * 128);
@@ -436,12 +351,115 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the zeroed rows are read by the tensor core
       }
-      tmem_store_wait();
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_ready_a + uint32_t(it & 1) * 8u);
-      tmem_load_wait(s0);  // the next tile's scores
+    };
+    if (q * 32 >= rows_here) {
+      // None of this warp's rows exist (a decoded token beside prompts is one row of a tile): it keeps the other warps' pace and leaves
+      // P as it finds it. What the products make of that stays in the accumulator rows of its own lanes, which nobody stores; the
+      // exponentials that it does not take are the ones that the rows that exist wait for (two CTAs share an SM's 16 a cycle).
+      for (int it = 0; it < n_mine; ++it) {
+        if (ok && !mbar_wait(s_ready_a + uint32_t(it & 1) * 8u, uint32_t(it >> 1) & 1u)) {
+          if (lane == 0) atomicMax(p.error_flag, R2_ERR_TIMEOUT_ATTN);
+          ok = false;
+        }
+        zero_unseen(it, j_of(it));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_ready_a + uint32_t(it & 1) * 8u);
+      }
+    } else {
+      uint32_t s0[32], s1[32];
+      auto fetch = [&](int it) {
+        if (it < n_mine && ok && !mbar_wait(s_ready_a + uint32_t(it & 1) * 8u, uint32_t(it >> 1) & 1u)) {
+          if (lane == 0) atomicMax(p.error_flag, R2_ERR_TIMEOUT_ATTN);
+          ok = false;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t at = lane_base + uint32_t(it & 1) * 64u;
+        tmem_load32(at, s0);
+        tmem_load32(at + 32u, s1);
+      };
+      fetch(0);
+      tmem_load_wait(s0);
       tmem_tie(s1);
+      for (int it = 0; it < n_mine; ++it) {
+        const int j0 = j_of(it);
+        const uint32_t s_at = lane_base + uint32_t(it & 1) * 64u;
+        // mask in float: causal and window. Key c of the tile is seen if lo_c <= c <= hi (plain predicate
+        // logic on two registers: written with && and || over the position this loop took 1,300 cycles a tile).
+        const int hi = pos - j0;
+        const int lo_c = p.window > 0 ? pos - p.window + 1 - j0 : 0;
+        const int kf = keep - j0;   // (X) keys of the tile below it are kept first keys; without them it is <= 0
+        if (hi < BN - 1 || (lo_c > 0 && kf < BN)) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            const bool seen_a = (c <= hi) & ((c >= lo_c) | (X && c < kf));
+            const bool seen_b = (c + 32 <= hi) & ((c + 32 >= lo_c) | (X && c + 32 < kf));
+            s0[c] = seen_a ? s0[c] : __float_as_uint(-INFINITY);
+            s1[c] = seen_b ? s1[c] : __float_as_uint(-INFINITY);
+          }
+        }
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains: the maximum's latency, not its count, is what costs
+#pragma unroll
+        for (int c = 0; c < 32; ++c) mx4[c & 3] = max3(mx4[c & 3], __uint_as_float(s0[c]), __uint_as_float(s1[c]));
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+        // The maximum in use moves only when this tile's exceeds it by more than the step.
+        const float m_tile = mx * scale2;
+        const bool grow = m_tile > m_run + RESCALE_STEP || (m_run == -INFINITY && m_tile > -INFINITY);
+        const float m_new = grow ? m_tile : m_run;
+        const float base = m_new == -INFINITY ? 0.f : m_new;  // a row that has seen no key yet
+        const float corr = grow ? fast_exp2(m_run - base) : 1.f;
+        float sum_a = 0.f, sum_b = 0.f;
+        uint32_t pk[32];  // the row of P, two bfloat16 to a word: keys 2w and 2w + 1
+        uint32_t pr[X ? 32 : 1];  // (X) what the rounding left of each weight, as a second row of bfloat16
+#pragma unroll
+        for (int w = 0; w < 16; ++w) {
+          const float a0 = fast_exp2(fmaf(__uint_as_float(s0[2 * w]), scale2, -base));
+          const float a1 = fast_exp2(fmaf(__uint_as_float(s0[2 * w + 1]), scale2, -base));
+          const float b0 = fast_exp2(fmaf(__uint_as_float(s1[2 * w]), scale2, -base));
+          const float b1 = fast_exp2(fmaf(__uint_as_float(s1[2 * w + 1]), scale2, -base));
+          sum_a += a0 + a1;
+          sum_b += b0 + b1;
+          pk[w] = pack_bf16(a0, a1);
+          pk[16 + w] = pack_bf16(b0, b1);
+          if (X) {
+            const float2 ha = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[w]));
+            const float2 hb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[16 + w]));
+            pr[w] = pack_bf16(a0 - ha.x, a1 - ha.y);
+            pr[16 + w] = pack_bf16(b0 - hb.x, b1 - hb.y);
+          }
+        }
+        l_run = l_run * corr + (sum_a + sum_b);
+        m_run = m_new;
+        if (it > 0 && __any_sync(0xffffffffu, grow)) {
+          // O times the correction, once the product of the previous tile has completed (the warp
+          // decides together: every lane's tensor-memory access is one instruction)
+          if (ok && !mbar_wait(pv_done_a, uint32_t(it - 1) & 1u)) {
+            if (lane == 0) atomicMax(p.error_flag, R2_ERR_TIMEOUT_ATTN);
+            ok = false;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int part = 0; part < 2; ++part) {
+            uint32_t o[32];
+            tmem_load32(lane_base + 128u + uint32_t(part * 32), o);
+            tmem_load_wait(o);
+#pragma unroll
+            for (int c = 0; c < 32; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * corr);
+            tmem_store32(lane_base + 128u + uint32_t(part * 32), o);
+          }
+        }
+        tmem_store32(s_at, pk);  // over the scores this thread has read
+        if constexpr (X) {
+          if (p.split_p) tmem_store32(s_at + 32u, pr);   // the other half of the same buffer, which this thread has read too
+        }
+        fetch(it + 1);           // (the registers of the scores are free)
+        zero_unseen(it, j0);
+        tmem_store_wait();
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_ready_a + uint32_t(it & 1) * 8u);
+        tmem_load_wait(s0);  // the next tile's scores
+        tmem_tie(s1);
+      }
     }
     // this CTA's last product has completed
     if (ok && n_mine > 0 && !mbar_wait(o_done_a, 0)) {
@@ -651,7 +669,11 @@ extern "C" int r2_attention_prefill_tc(const void* q, int q_row_stride, int n_ro
     // better trade (one CTA's softmax under the other's products); with fewer than two per SM the step waits
     // for the CTA with the most keys, which then should have an SM to itself: the CTA asks for more than half
     // an SM's shared memory, and the ones that do not fit at first start as the short ones end.
-    const size_t smem = busy <= 2L * n_sms ? size_t(120) * 1024 : smem_one;
+    // Not so where most entries are single decoded tokens beside a portion: three of four softmax warps of their tiles have no rows and
+    // leave the units to the others, and one after the other on an SM they wait for each other's chains (24.2 us a launch
+    // of 16 heads, 512 rows of a prompt and 15 decoded ones with contexts up to 780, 14.6 with two to an SM).
+    const bool sparse = long(n_rows) < long(BM) * n_entries;
+    const size_t smem = busy <= 2L * n_sms && !sparse ? size_t(120) * 1024 : smem_one;
     if (extras) r2_launch(prefill_tc_kernel<1, true>, dim3(n_heads, n_tiles), dim3(THREADS), smem, stream, mq, mk, mv, p);
     else r2_launch(prefill_tc_kernel<1, false>, dim3(n_heads, n_tiles), dim3(THREADS), smem, stream, mq, mk, mv, p);
   }
