@@ -352,25 +352,44 @@ causal_conv_kernel(const T* __restrict__ in, int in_stride, T* __restrict__ out,
                    long long conv_state_off, const int32_t* __restrict__ row_entry, const int32_t* __restrict__ q_start,
                    const int32_t* __restrict__ state_slot, const int32_t* __restrict__ fresh) {
   pdl_launch_dependents();
-  pdl_wait();
+  // (the batch's arrays and the weights are no kernel's output: what is looked up in them does not wait for the kernel before this one)
   const int t = blockIdx.x;
   const int e = row_entry[t];
+  const int l = e < 0 ? 0 : t - q_start[e];
+  const bool is_fresh = e < 0 || fresh[e] != 0;
+  const float* cs = state + (e < 0 ? 0 : size_t(state_slot[e])) * slot_stride + conv_state_off;
+  const int c_first = blockIdx.y * blockDim.x + threadIdx.x;
+  float first_tap[4], first_bias = 0.f;   // of this thread's first channel
+  const bool four = n_taps <= 4;
+  if (four && c_first < channels) {
+#pragma unroll
+    for (int d = 0; d < 4; ++d) first_tap[d] = d < n_taps ? taps[size_t(c_first) * n_taps + d] : 0.f;
+    first_bias = bias != nullptr ? bias[c_first] : 0.f;
+  }
+  pdl_wait();
   T* o = out + size_t(t) * out_stride;
   if (e < 0) {  // a pad row
-    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < channels; c += gridDim.y * blockDim.x) o[c] = from_float<T>(0.f);
+    for (int c = c_first; c < channels; c += gridDim.y * blockDim.x) o[c] = from_float<T>(0.f);
     return;
   }
-  const int l = t - q_start[e];
-  const bool is_fresh = fresh[e] != 0;
-  const float* cs = state + size_t(state_slot[e]) * slot_stride + conv_state_off;
-  for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < channels; c += gridDim.y * blockDim.x) {
-    float acc = bias != nullptr ? bias[c] : 0.f;
-    for (int d = 0; d < n_taps; ++d) {
-      const int src = l - (n_taps - 1) + d;
-      float val = 0.f;
-      if (src >= 0) val = to_float(in[size_t(t - (n_taps - 1) + d) * in_stride + c]);
-      else if (!is_fresh) val = cs[size_t(n_taps - 1 + src) * channels + c];
-      acc = fmaf(taps[size_t(c) * n_taps + d], val, acc);
+  auto input = [&](int c, int d) {
+    const int src = l - (n_taps - 1) + d;
+    if (src >= 0) return to_float(in[size_t(t - (n_taps - 1) + d) * in_stride + c]);
+    return is_fresh ? 0.f : cs[size_t(n_taps - 1 + src) * channels + c];
+  };
+  for (int c = c_first; c < channels; c += gridDim.y * blockDim.x) {
+    float acc;
+    if (four) {   // all inputs asked for at once
+      float val[4];
+#pragma unroll
+      for (int d = 0; d < 4; ++d) val[d] = d < n_taps ? input(c, d) : 0.f;
+      acc = c == c_first ? first_bias : bias != nullptr ? bias[c] : 0.f;
+#pragma unroll
+      for (int d = 0; d < 4; ++d)
+        if (d < n_taps) acc = fmaf(c == c_first ? first_tap[d] : taps[size_t(c) * n_taps + d], val[d], acc);
+    } else {
+      acc = bias != nullptr ? bias[c] : 0.f;
+      for (int d = 0; d < n_taps; ++d) acc = fmaf(taps[size_t(c) * n_taps + d], input(c, d), acc);
     }
     o[c] = from_float<T>(acc / (1.f + expf(-acc)));
   }
@@ -535,7 +554,9 @@ extern "C" int r2_causal_conv(const void* in, int in_stride, void* out, int out_
                               int n_rows, int dtype, cudaStream_t stream) {
   if (n_rows <= 0) return R2_OK;
   if (n_taps < 1 || channels < 1) return R2_BAD_SHAPE;
-  dim3 grid(n_rows, (channels + 1023) / 1024);
+  // a channel a thread for few rows, whose time is the chain of their loads; four for many
+  const int per_cta = n_rows <= 64 ? 256 : 1024;
+  dim3 grid(n_rows, (channels + per_cta - 1) / per_cta);
   if (dtype == R2_F32) {
     r2_launch(causal_conv_kernel<float>, grid, dim3(256), size_t(0), stream, (const float*)in, in_stride, (float*)out, out_stride,
               taps, bias, n_taps, channels, state, slot_stride, conv_state_off, row_entry, q_start, state_slot, fresh);

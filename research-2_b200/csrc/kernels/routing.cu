@@ -23,49 +23,112 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "small_products.cuh"
 
 namespace {
 
 constexpr int MAX_EXPERTS = 1024;
 
-template <typename T>
-__global__ void __launch_bounds__(256)
+// four neighbouring products into four sums: the order in which a sum's terms are added is the same wherever this is used
+__device__ __forceinline__ void add_quad(float (&sum)[4], const float4 x, const float4 w) {
+  sum[0] = fmaf(x.x, w.x, sum[0]);
+  sum[1] = fmaf(x.y, w.y, sum[1]);
+  sum[2] = fmaf(x.z, w.z, sum[2]);
+  sum[3] = fmaf(x.w, w.w, sum[3]);
+}
+
+// A warp has one output, for `rows_per_cta` rows one after the other; a CTA eight outputs. What bounds a few rows is one round trip after
+// another, so the output's weights are asked for in 16-byte pieces before the kernel before this one has ended (weights are no kernel's
+// output) and stay in registers (width up to 128 SMALL_AHEAD; what lies beyond is read again a row), and a row comes straight from memory,
+// all pieces at once: 4 rows x 768 x 24 take 2.3 us (7.0 with a CTA a row, three outputs a warp after the row's way through shared
+// memory). QUADS: rows of h and w start on boundaries of four numbers and hold a multiple of four.
+constexpr int SMALL_AHEAD = 8, SMALL_WARPS = 8;
+template <typename T, bool QUADS>
+__global__ void __launch_bounds__(SMALL_WARPS * 32)
 small_linear_kernel(const T* __restrict__ h, int h_stride, const float* __restrict__ w, const float* __restrict__ bias,
-                    float* __restrict__ out, int out_stride, int n_out, int width) {
+                    float* __restrict__ out, int out_stride, int n_out, int width, int n_rows, int rows_per_cta) {
   pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, n = blockIdx.y * SMALL_WARPS + (threadIdx.x >> 5);
+  const float* wr = w + size_t(n < n_out ? n : 0) * width;
+  float4 ahead[QUADS ? SMALL_AHEAD : 1];
+  if (QUADS) {
+#pragma unroll
+    for (int i = 0; i < (QUADS ? SMALL_AHEAD : 1); ++i) {
+      const int k = 4 * lane + 128 * i;
+      ahead[i] = k < width ? load4(wr + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  const float b = bias != nullptr && n < n_out ? bias[n] : 0.f;
   pdl_wait();
-  extern __shared__ float row[];
-  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-  const T* hr = h + size_t(t) * h_stride;
-  for (int k = threadIdx.x; k < width; k += blockDim.x) row[k] = to_float(hr[k]);
-  __syncthreads();
-  for (int n = warp; n < n_out; n += n_warps) {
-    const float* wr = w + size_t(n) * width;
+  if (n >= n_out) return;
+  const int t0 = blockIdx.x * rows_per_cta, t1 = min(n_rows, t0 + rows_per_cta);
+  for (int t = t0; t < t1; ++t) {
+    const T* hr = h + size_t(t) * h_stride;
     float acc = 0.f;
-    for (int k = lane; k < width; k += 32) acc = fmaf(row[k], wr[k], acc);
+    if (QUADS) {
+      float4 x[SMALL_AHEAD];
+#pragma unroll
+      for (int i = 0; i < SMALL_AHEAD; ++i) {
+        const int k = 4 * lane + 128 * i;
+        x[i] = k < width ? load4(hr + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < (QUADS ? SMALL_AHEAD : 1); ++i) add_quad(sum, x[i], ahead[i]);
+#pragma unroll 4
+      for (int k = 4 * lane + 128 * SMALL_AHEAD; k < width; k += 128) add_quad(sum, load4(hr + k), load4(wr + k));
+      acc = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+    } else {
+#pragma unroll 8
+      for (int k = lane; k < width; k += 32) acc = fmaf(to_float(hr[k]), wr[k], acc);
+    }
     acc = warp_sum(acc);
-    if (lane == 0) out[size_t(t) * out_stride + n] = acc + (bias != nullptr ? bias[n] : 0.f);
+    if (lane == 0) out[size_t(t) * out_stride + n] = acc + b;
   }
 }
 
+constexpr int TOP_K_AHEAD = 8;
 template <typename T>
 __global__ void __launch_bounds__(256)
 route_top_k_kernel(const T* __restrict__ h, int h_stride, const float* __restrict__ w, const float* __restrict__ bias,
                    float* __restrict__ dense, int32_t* __restrict__ chosen, float* __restrict__ chosen_weight,
-                   int n_experts, int top, int width) {
+                   int n_experts, int top, int width, int quads) {
   pdl_launch_dependents();
-  pdl_wait();
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) float smem[];
   float* row = smem;             // [width]
   float* logit = smem + width;   // [n_experts]
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+  // with `quads` (rows of w in whole 16-byte pieces) the first pieces of the warp's first output are asked for before the kernel before
+  // this one has ended
+  float4 ahead[TOP_K_AHEAD];
+  if (quads && warp < n_experts) {
+#pragma unroll
+    for (int i = 0; i < TOP_K_AHEAD; ++i) {
+      const int k = 4 * lane + 128 * i;
+      ahead[i] = k < width ? load4(w + size_t(warp) * width + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  pdl_wait();
   const T* hr = h + size_t(t) * h_stride;
   for (int k = threadIdx.x; k < width; k += blockDim.x) row[k] = to_float(hr[k]);
   __syncthreads();
   for (int n = warp; n < n_experts; n += n_warps) {
     const float* wr = w + size_t(n) * width;
     float acc = 0.f;
-    for (int k = lane; k < width; k += 32) acc = fmaf(row[k], wr[k], acc);
+    if (quads) {
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < TOP_K_AHEAD; ++i) {
+        const int k = 4 * lane + 128 * i;
+        if (k < width) add_quad(sum, load4(row + k), n == warp ? ahead[i] : load4(wr + k));
+      }
+#pragma unroll 4
+      for (int k = 4 * lane + 128 * TOP_K_AHEAD; k < width; k += 128) add_quad(sum, load4(row + k), load4(wr + k));
+      acc = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+    } else {
+#pragma unroll 8
+      for (int k = lane; k < width; k += 32) acc = fmaf(row[k], wr[k], acc);
+    }
     acc = warp_sum(acc);
     if (lane == 0) logit[n] = acc + (bias != nullptr ? bias[n] : 0.f);
   }
@@ -244,14 +307,6 @@ __device__ __forceinline__ float choose_experts(const RouteArgs& a, const RouteR
   float share = 0.f;
   for (int n = a.n_experts - a.n_identity + lane; n < a.n_experts; n += 32) share += r.given[n];
   return warp_sum(share);
-}
-
-// four neighbouring products into four sums: the order in which a logit's terms are added is the same in both forms below
-__device__ __forceinline__ void add_quad(float (&sum)[4], const float4 x, const float4 w) {
-  sum[0] = fmaf(x.x, w.x, sum[0]);
-  sum[1] = fmaf(x.y, w.y, sum[1]);
-  sum[2] = fmaf(x.z, w.z, sum[2]);
-  sum[3] = fmaf(x.w, w.w, sum[3]);
 }
 
 // A CTA a row. A warp has an output at a time; with `quads` its row of w comes as 16-byte pieces, the first ROUTE_AHEAD of them asked for
@@ -439,16 +494,18 @@ extern "C" int r2_small_linear(const void* h, int h_stride, const float* w, cons
                                int n_rows, int n_out, int width, int dtype, cudaStream_t stream) {
   if (n_rows <= 0 || n_out <= 0) return R2_OK;
   if (width < 1) return R2_BAD_SHAPE;
-  const size_t smem = sizeof(float) * width;
-  if (smem > 48 * 1024) return R2_UNSUPPORTED;
-  const int threads = n_out >= 8 ? 256 : 32 * n_out;
-  if (dtype == R2_F32) {
-    r2_launch(small_linear_kernel<float>, dim3(n_rows), dim3(threads), smem, stream, (const float*)h, h_stride, w, bias, out, out_stride, n_out, width);
-  } else if (dtype == R2_BF16) {
-    r2_launch(small_linear_kernel<bf16>, dim3(n_rows), dim3(threads), smem, stream, (const bf16*)h, h_stride, w, bias, out, out_stride, n_out, width);
-  } else {
-    return R2_BAD_DTYPE;
-  }
+  if (sizeof(float) * size_t(width) > 48 * 1024) return R2_UNSUPPORTED;
+  if (dtype != R2_F32 && dtype != R2_BF16) return R2_BAD_DTYPE;
+  const size_t four = dtype == R2_F32 ? 16 : 8;   // bytes of four numbers of h
+  const bool quads = width % 4 == 0 && h_stride % 4 == 0 && reinterpret_cast<uintptr_t>(h) % four == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0;
+  // many rows: eight to a CTA, whose warps then read their weights once for them (an output's sum is the same either way)
+  const int rows_per_cta = n_rows > 256 ? 8 : 1;
+  const dim3 grid((n_rows + rows_per_cta - 1) / rows_per_cta, (n_out + SMALL_WARPS - 1) / SMALL_WARPS);
+  auto go = [&](auto kernel, auto zero) {
+    r2_launch(kernel, grid, dim3(SMALL_WARPS * 32), size_t(0), stream, (const decltype(zero)*)h, h_stride, w, bias, out, out_stride, n_out, width, n_rows, rows_per_cta);
+  };
+  if (dtype == R2_F32) quads ? go(small_linear_kernel<float, true>, 0.f) : go(small_linear_kernel<float, false>, 0.f);
+  else quads ? go(small_linear_kernel<bf16, true>, bf16()) : go(small_linear_kernel<bf16, false>, bf16());
   return launch_status();
 }
 
@@ -458,10 +515,11 @@ extern "C" int r2_route_top_k(const void* h, int h_stride, const float* w, const
   if (width < 1 || n_experts < 1 || n_experts > MAX_EXPERTS || top < 1 || top > n_experts) return R2_BAD_SHAPE;
   const size_t smem = sizeof(float) * (size_t(width) + n_experts);
   if (smem > 48 * 1024) return R2_UNSUPPORTED;
+  const int quads = width % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0;
   if (dtype == R2_F32) {
-    r2_launch(route_top_k_kernel<float>, dim3(n_rows), dim3(256), smem, stream, (const float*)h, h_stride, w, bias, dense, chosen, chosen_weight, n_experts, top, width);
+    r2_launch(route_top_k_kernel<float>, dim3(n_rows), dim3(256), smem, stream, (const float*)h, h_stride, w, bias, dense, chosen, chosen_weight, n_experts, top, width, quads);
   } else if (dtype == R2_BF16) {
-    r2_launch(route_top_k_kernel<bf16>, dim3(n_rows), dim3(256), smem, stream, (const bf16*)h, h_stride, w, bias, dense, chosen, chosen_weight, n_experts, top, width);
+    r2_launch(route_top_k_kernel<bf16>, dim3(n_rows), dim3(256), smem, stream, (const bf16*)h, h_stride, w, bias, dense, chosen, chosen_weight, n_experts, top, width, quads);
   } else {
     return R2_BAD_DTYPE;
   }

@@ -1,0 +1,46 @@
+"""Kernels whose time at a few rows is a chain of loads: the weights they ask for ahead, what lies beyond those, rows one by one and many."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def ops():
+    from research_2_b200.kernels import ops as o
+
+    return o
+
+
+# widths inside and beyond the 1,024 numbers kept in registers, and one that is no multiple of four; outputs around a CTA's eight
+@pytest.mark.parametrize("width,n_out", [(768, 24), (1024, 7), (1600, 9), (770, 8), (36, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_small_linear_rows_do_not_depend_on_their_number(width, n_out, dtype):
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(width)
+    h = torch.randn(300, width, generator=gen, device=DEV).to(dtype)
+    w, b = torch.randn(n_out, width, generator=gen, device=DEV), torch.randn(n_out, generator=gen, device=DEV)
+    many = o.small_linear(h, w, b)
+    for n in (1, 5, 256):
+        assert torch.equal(o.small_linear(h[:n], w, b), many[:n])
+    want = h.double() @ w.double().T + b.double()
+    # a lane adds width / 128 terms to each of four sums, the warp's 32 meet in five steps: far fewer roundings than terms
+    bound = (width / 128 + 16) * 2.0 ** -24 * (h.double().abs() @ w.double().abs().T + b.double().abs())
+    assert ((many.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("width", [768, 1600, 770])
+def test_router_logits_beyond_what_is_asked_for_ahead(width):
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(width)
+    h = torch.randn(9, width, generator=gen, device=DEV).bfloat16()
+    w, b = torch.randn(20, width, generator=gen, device=DEV), torch.randn(20, generator=gen, device=DEV)
+    dense, chosen, weight = o.route_top_k(h, w, b, 3)
+    z = h.double() @ w.double().T + b.double()
+    best = z.topk(3, dim=1)
+    assert torch.equal(chosen.long(), best.indices)
+    torch.testing.assert_close(weight.double(), torch.softmax(best.values, dim=1), atol=1e-4, rtol=1e-4)
+    assert torch.equal(dense.gather(1, chosen.long()), weight)
