@@ -62,7 +62,25 @@ struct DecodeParams {
   const int32_t* slot_mapping;
   bf16* k_cache_w; bf16* v_cache_w;
   int* counters;  // [rows, n_kv_heads], zero between launches; null: a separate merge kernel follows
+  // The slices of a (row, kv head) are the CTAs of a cluster, which merge their results out of one another's shared memory: no
+  // scratch, no counters. (Through global memory the merge is four round trips one after the other: results, fence, counter, results.)
+  int clustered;
 };
+
+constexpr int MAX_CLUSTER = 8;
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The float at the same shared-memory place of another CTA of the cluster.
+__device__ __forceinline__ float remote_float(const float* mine, int rank) {
+  uint32_t addr, there = uint32_t(__cvta_generic_to_shared(mine));
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(there), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
@@ -122,6 +140,7 @@ decode_kernel(const DecodeParams p) {
   __shared__ float q_s[G][HD];
   __shared__ float red_o[WARPS][G][HD];
   __shared__ float red_m[WARPS][G], red_l[WARPS][G];
+  __shared__ float cta_m[G], cta_l[G];   // (clustered) of this CTA's slice
   __shared__ int is_last_s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slice = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
@@ -498,6 +517,12 @@ decode_kernel(const DecodeParams p) {
       p.out[size_t(t) * p.out_row_stride + size_t(h0 + g) * HD + d] = __float2bfloat16_rn(finish(
           o, lsum, mx, X ? p.sink : 0, gate, (X && p.sinks != nullptr) ? p.sinks[h0 + g] : 0.f,
           (X && p.head_gate != nullptr) ? p.head_gate + size_t(t) * p.head_gate_stride + h0 + g : nullptr, X == 2 ? p.out_scale : 1.f));
+    } else if (p.clustered) {
+      red_o[0][g][d] = o;   // (this thread alone has read the place)
+      if (d == 0) {
+        cta_m[g] = mx;
+        cta_l[g] = lsum;
+      }
     } else {
       size_t at = (size_t(t) * p.n_heads + h0 + g) * p.n_slices + slice;
       p.part_o[at * HD + d] = o;
@@ -506,6 +531,41 @@ decode_kernel(const DecodeParams p) {
         p.part_ml[at * 2 + 1] = lsum;
       }
     }
+  }
+  if (p.clustered) {
+    // the cluster's CTAs share the outputs; the slices are added in slice order
+    cluster_barrier();
+    for (int i = slice * WARPS * 32 + threadIdx.x; i < G * HD; i += p.n_slices * WARPS * 32) {
+      const int g = i / HD, d = i % HD;
+      float ms[MAX_CLUSTER], ls[MAX_CLUSTER], os[MAX_CLUSTER];
+#pragma unroll
+      for (int s = 0; s < MAX_CLUSTER; ++s) {
+        const bool there = s < p.n_slices;
+        ms[s] = there ? remote_float(&cta_m[g], s) : -INFINITY;
+        ls[s] = there ? remote_float(&cta_l[g], s) : 0.f;
+        os[s] = there ? remote_float(&red_o[0][g][d], s) : 0.f;
+      }
+      float mx = -INFINITY;
+#pragma unroll
+      for (int s = 0; s < MAX_CLUSTER; ++s) mx = fmaxf(mx, ms[s]);
+      float o = 0.f, lsum = 0.f;
+      if (mx > -INFINITY) {
+#pragma unroll
+        for (int s = 0; s < MAX_CLUSTER; ++s) {
+          const float c = __expf(ms[s] - mx);
+          if (s < p.n_slices) {
+            o += c * os[s];
+            lsum += c * ls[s];
+          }
+        }
+      }
+      const bf16* gate = (X && p.gate != nullptr) ? p.gate + size_t(t) * p.gate_row_stride + size_t(h0 + g) * HD + d : nullptr;
+      p.out[size_t(t) * p.out_row_stride + size_t(h0 + g) * HD + d] = __float2bfloat16_rn(finish(
+          o, lsum, mx, X ? p.sink : 0, gate, (X && p.sinks != nullptr) ? p.sinks[h0 + g] : 0.f,
+          (X && p.head_gate != nullptr) ? p.head_gate + size_t(t) * p.head_gate_stride + h0 + g : nullptr, X == 2 ? p.out_scale : 1.f));
+    }
+    cluster_barrier();   // the others read this CTA's shared memory until here
+    return;
   }
   if (p.n_slices > 1 && p.counters != nullptr) {
     // the slice that arrives last merges all of them, in slice order
@@ -589,6 +649,23 @@ template <int G, bool MMA, int X>
 int launch_form(const DecodeParams& p, int n_rows, cudaStream_t stream) {
   dim3 grid(p.n_slices, p.n_kv_heads, n_rows);
   if (!configure_smem<G, MMA, X>()) return R2_UNSUPPORTED;
+  if (p.clustered) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = dim3(WARPS * 32);
+    config.dynamicSmemBytes = TILE_SMEM;
+    config.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(p.n_slices);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attr;
+    config.numAttrs = (g_r2_pdl && !t_r2_plain_order) ? 2 : 1;
+    cudaLaunchKernelEx(&config, decode_kernel<G, MMA, X>, p);
+    return launch_status();
+  }
   r2_launch(decode_kernel<G, MMA, X>, dim3(grid), dim3(WARPS * 32), size_t(TILE_SMEM), stream, p);
   return launch_status();
 }
@@ -635,7 +712,7 @@ extern "C" int r2_attention_decode(const void* q, int q_row_stride, void* out, i
   p.part_o = scratch;
   p.part_ml = scratch != nullptr ? scratch + (long long)n_rows * n_heads * n_slices * HD : nullptr;
   p.k_new = nullptr; p.v_new = nullptr; p.new_row_stride = 0; p.slot_mapping = nullptr;
-  p.k_cache_w = nullptr; p.v_cache_w = nullptr; p.counters = nullptr;
+  p.k_cache_w = nullptr; p.v_cache_w = nullptr; p.counters = nullptr; p.clustered = 0;
   int status;
   switch (n_heads / n_kv_heads) {
     case 1: status = launch<1>(p, n_rows, stream); break;
@@ -669,7 +746,8 @@ int launch_fused(const DecodeParams& p, int n_rows, cudaStream_t stream) {
 // One launch for a decode-only batch: the new tokens' keys and values (k_new, v_new:
 // [rows, n_kv_heads * HD] with row stride new_row_stride) are written to their cache slots by
 // the kernel itself, and the slices of a (row, kv head) are merged by whichever of their CTAs
-// finishes last, so there is neither a separate cache-write kernel nor a merge kernel.
+// finishes last (up to eight slices are a cluster and merge through its shared memory), so there is neither a separate cache-write
+// kernel nor a merge kernel.
 // `scratch` as for r2_attention_decode; `counters` holds n_rows * n_kv_heads ints that are
 // zero before the call and zero again after it. `keep_first`, `sink`, `gate` and `split_p`: see DecodeParams.
 // `chunk`, `dist_bias`, `bias_len` and `out_scale` (0, null, 0 and 1: none of them) likewise.
@@ -709,6 +787,7 @@ extern "C" int r2_attention_decode_fused_biased(const void* q, int q_row_stride,
   p.slot_mapping = slot_mapping;
   p.k_cache_w = (bf16*)k_cache; p.v_cache_w = (bf16*)v_cache;
   p.counters = n_slices > 1 ? counters : nullptr;
+  p.clustered = n_slices > 1 && n_slices <= MAX_CLUSTER;
   switch (n_heads / n_kv_heads) {
     case 1: return launch_fused<1>(p, n_rows, stream);
     case 2: return launch_fused<2>(p, n_rows, stream);

@@ -245,10 +245,11 @@ def decode_slices(n_rows: int, n_kv_heads: int, max_context: int, device="cuda:0
     """Slices of the keys per (row, kv head) in decode attention: as many as keep every CTA
     resident at once (four to an SM is what every head size's kernel reaches; a second wave of
     CTAs costs more than the slices gain: 8 rows x 12 heads took 8.4 us with 6 slices, 10.3 us with
-    8), never less than 128 keys a slice."""
+    8), about 128 keys a slice at least: a tile of 32 for each of its warps (a window of 256 beside four kept
+    keys takes three slices, with two a warp had two tiles one after the other)."""
     ctas = max(1, n_rows * n_kv_heads)
     want = max(1, 4 * sm_count(device) // ctas)
-    most = max(1, max_context // 128)
+    most = max(1, -(-max_context // 128))
     return max(1, min(want, most, 32))
 
 

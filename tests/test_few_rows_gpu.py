@@ -5,6 +5,8 @@ from __future__ import annotations
 import pytest
 import torch
 
+from tests.test_kernels_gpu import PagedCase
+
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
@@ -44,3 +46,15 @@ def test_router_logits_beyond_what_is_asked_for_ahead(width):
     assert torch.equal(chosen.long(), best.indices)
     torch.testing.assert_close(weight.double(), torch.softmax(best.values, dim=1), atol=1e-4, rtol=1e-4)
     assert torch.equal(dense.gather(1, chosen.long()), weight)
+
+
+# slices that are a cluster (up to eight) and more of them than that; contexts from one key to several tiles a warp
+@pytest.mark.parametrize("max_context", [129, 260, 1024, 1030, 4096])
+@pytest.mark.parametrize("window", [0, 40])
+def test_slices_of_decode_attention_meet_in_their_cluster(max_context, window):
+    case = PagedCase([(c, 1) for c in (0, 31, 128, 500, 1000)], 4, 2, 64, 16, torch.bfloat16, seed=max_context)
+    got = case.run_fused(0.125, window, max_context).float().cpu()
+    torch.testing.assert_close(got, case.plain(0.125, window), atol=2e-2, rtol=2e-2)
+    one = PagedCase([(c, 1) for c in (0, 31, 128, 500, 1000)], 4, 2, 64, 16, torch.bfloat16, seed=max_context).run_fused(0.125, window, 100).float().cpu()
+    # the same rounding of every weight to bfloat16 against another maximum, and the output's own: two roundings of 2^-9
+    torch.testing.assert_close(got, one, atol=2.0 ** -7, rtol=2.0 ** -7)
