@@ -355,6 +355,16 @@ __device__ __forceinline__ uint4 ld_shared16(uint32_t addr) {
   return v;
 }
 
+// 32 columns of this warp's lanes, written and complete.
+__device__ __forceinline__ void tmem_store32(uint32_t taddr, const float (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n\t"
+      "tcgen05.wait::st.sync.aligned;"
+      ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]),
+        "f"(v[16]), "f"(v[17]), "f"(v[18]), "f"(v[19]), "f"(v[20]), "f"(v[21]), "f"(v[22]), "f"(v[23]), "f"(v[24]), "f"(v[25]), "f"(v[26]), "f"(v[27]), "f"(v[28]), "f"(v[29]), "f"(v[30]), "f"(v[31])
+      : "memory");
+}
+
 // The same load without its wait: several may be in flight before one tmem_wait().
 __device__ __forceinline__ void tmem_load32_issue(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -374,6 +384,9 @@ __device__ __forceinline__ void tmem_tie(uint32_t (&r)[32]) {
 constexpr int STAGING_ROW = 36;                       // words per staged row: 32 and four of padding (rows stay 16-byte aligned)
 constexpr int STAGING_WORDS = 32 * STAGING_ROW;       // per epilogue warp
 constexpr int BIAS_SLOTS = 256;                       // floats: the widest tile
+// Token-major split-K: a tile's columns go back to the CTAs of its cluster in groups of 32, group g to rank g % splits.
+constexpr int SHARE_COLS = 32;
+constexpr uint32_t SHARE_BYTES = uint32_t(BM) * SHARE_COLS * 4;   // a group's partial sums, [column][row]
 
 // The epilogue of a 32-row slab of a token-major tile over the tile's columns [c_begin, c_end)
 // (one warp; lane = accumulator row). The accumulator comes out of tensor memory one row per
@@ -386,12 +399,15 @@ constexpr int BIAS_SLOTS = 256;                       // floats: the widest tile
 // instruction every six cycles, so the count of instructions per element is what is kept small.
 // `bias_s` holds the tile's bias (zeros without one), 16-byte aligned. bfloat16 output without a
 // residual moves 64 columns a group as packed pairs; everything else 32 columns as floats.
+// `x`: the residual of the group at hand, `x_here` where the caller asked for the first group's while the products ran (the fast path's
+// conditions hold); the next group's is on its way while this one's rows are written.
 // `slab` is the warp's 32 x STAGING_ROW words of shared memory, as a shared-space address.
 // ROUTED: values are multiplied by their token's weight for their block of features (a form of its own: the other products' epilogues stay
 // as short as they are).
 template <bool ROUTED>
 __device__ __forceinline__ void finish_tile_rows(const GemmParams& p, uint32_t lane_addr, uint32_t slab, const float* bias_s,
-                                                 int row0, int col0, int c_begin, int c_end, int lane, bool have_acc) {
+                                                 int row0, int col0, int c_begin, int c_end, int lane, bool have_acc,
+                                                 float4 (&x)[8], bool x_here) {
   const int rows = min(32, p.a_total - row0);        // rows of this slab that exist
   const int sub = lane >> 3, piece = lane & 7;       // step (2): the row within four, the 16-byte piece of it
   // the weights of this lane's row for the 32 columns from c on, which lie in at most two blocks: the first one's, the second one's,
@@ -561,9 +577,9 @@ __device__ __forceinline__ void finish_tile_rows(const GemmParams& p, uint32_t l
     const int col = col0 + c0 + 4 * piece;                                     // this lane's four columns
     if (inside && vec_ok && c0 + 32 <= c_end && !p.out_is_bf16) {
       // the common case, free of per-element conditions
-      float4 x[8];
-      if (p.residual != nullptr) {
-        const float* src = p.residual + size_t(row0 + sub) * p.ldr + col;
+      const float* src = p.residual + size_t(row0 + sub) * p.ldr + col;
+      if (x_here) {
+      } else if (p.residual != nullptr) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(src + size_t(4 * i) * p.ldr);
       } else {
@@ -587,12 +603,17 @@ __device__ __forceinline__ void finish_tile_rows(const GemmParams& p, uint32_t l
         *reinterpret_cast<float4*>(d + size_t(4 * i) * p.ldo) =
             make_float4(__uint_as_float(w.x) + x[i].x, __uint_as_float(w.y) + x[i].y, __uint_as_float(w.z) + x[i].z, __uint_as_float(w.w) + x[i].w);
       }
+      x_here = p.residual != nullptr && c0 + 64 <= c_end;
+      if (x_here) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(src + 32 + size_t(4 * i) * p.ldr);
+      }
       __syncwarp();
       continue;
     }
     const int n_cols = min(4, min(c_end - (c0 + 4 * piece), p.b_total - col));
     const bool whole = n_cols == 4 && vec_ok;
-    float4 x[8];  // the residual of this lane's columns, its eight rows of the slab, in flight during step (1)
+    // the residual of this lane's columns, its eight rows of the slab, in flight during step (1)
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int r = 4 * i + sub;
@@ -654,7 +675,9 @@ __device__ __forceinline__ void finish_tile_rows(const GemmParams& p, uint32_t l
 // A_MN / B_MN: the operand's tile in shared memory is MN-major (rows of 64 MN-elements, one row
 // per k) instead of K-major (rows of 64 k-elements, one row per MN index).
 // TRANSPOSED: the a side is the features and the b side the tokens.
-template <bool A_MN, bool B_MN, bool TRANSPOSED, bool FUSED_LN = false, bool ROUTED = false>
+// SHARED: the token-major form whose cluster shares a tile's K (a kernel of its own: as a branch of the plain form it cost that one
+// 1 to 2 % of a prompt's step).
+template <bool A_MN, bool B_MN, bool TRANSPOSED, bool FUSED_LN = false, bool ROUTED = false, bool SHARED = false>
 __global__ void __launch_bounds__(THREADS, (TRANSPOSED && !FUSED_LN) ? 1 : 2)  // token-major tiles run two CTAs to an SM, and so does the form with the norm inside (the logits' 393 CTAs)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -673,7 +696,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   uint64_t* partials_ready = tokens_ready + 1;  // leader: the other CTAs' partial sums have landed (counted in bytes)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(partials_ready + 1);
   // partial sums of the other CTAs of the cluster, [rank - 1][column][row], used in the leader only
-  // (feature-major form); the token-major form keeps the tile's bias in the same place
+  // (feature-major form); the token-major form keeps the tile's bias in the same place, and after it the groups of partial sums that
+  // it receives: [sender][own group][column][row]
   float* reduce = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(tmem_slot + 4) + 15) & ~uintptr_t(15));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -697,7 +721,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     mbar_init(acc_ready, 1);
     mbar_init(tokens_ready, 4);  // one arrival per epilogue warp
     mbar_init(partials_ready, 1);
-    if (p.splits > 1 && rank == 0) {
+    if (SHARED && p.splits > 1) {
+      // every other CTA sends the groups of columns that this one finishes
+      mbar_expect_tx(smem_u32(partials_ready), uint32_t(p.splits - 1) * uint32_t((p.bn / SHARE_COLS - int(rank) + p.splits - 1) / p.splits) * SHARE_BYTES);
+    }
+    if (TRANSPOSED && p.splits > 1 && rank == 0) {
       // every other CTA sends its whole tile of partial sums, rows padded
       mbar_expect_tx(smem_u32(partials_ready), uint32_t(p.splits - 1) * BM * (uint32_t(live_cols) + 4u) * 4u);
     }
@@ -843,7 +871,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 
   // ---- epilogue: warps 2..5, each on the 32 accumulator lanes it may read ------------------
-  bool acc_ok = true;
+  bool acc_ok = true, res_here = false;
+  float4 res_first[8];                    // token-major epilogue: the residual of the warp's first 32 columns
   float bias_ahead = 0.f, res_ahead[32];  // feature-major epilogue: the lane's bias, and its residual for the first 32 tokens
 #pragma unroll
   for (int j = 0; j < 32; ++j) res_ahead[j] = 0.f;
@@ -896,13 +925,55 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
     }
+    if constexpr (!TRANSPOSED) {
+      // the residual of the first 32 columns that this warp finishes, while the products run
+      const int c = SHARED ? int(rank) * SHARE_COLS : 0, last = SHARED ? c + SHARE_COLS : p.bn;
+      res_here = p.residual != nullptr && !p.out_is_bf16 && a0 + q * 32 + 32 <= p.a_total && b0 + last <= p.b_total && p.bn >= SHARE_COLS &&
+                 (p.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 && (p.ldr & 3) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 15) == 0;
+      if (res_here) {
+        const float* src = p.residual + size_t(a0 + q * 32 + (lane >> 3)) * p.ldr + b0 + c + 4 * (lane & 7);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) res_first[i] = *reinterpret_cast<const float4*>(src + size_t(4 * i) * p.ldr);
+      }
+    }
     bool ok = n_kb <= 0 || mbar_wait(acc_ready, 0);
     cta_stamp(p, 4);
     if (!ok) atomicMax(p.error_flag, R2_ERR_TIMEOUT_ACC);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t lane_addr = tmem_base + (uint32_t(q * 32) << 16);
     acc_ok = ok;
-    if (p.splits > 1 && rank != 0) {
+    if constexpr (SHARED) {
+      // This slice's partial sums of the groups that other CTAs finish, laid out over the operand tiles (every product of this
+      // CTA has completed) as [group][column][row], so that a warp's stores and the receiver's loads are whole rows of banks; a
+      // group travels as one bulk copy whose bytes the receiver's barrier counts.
+      for (int g = 0; g < p.bn / SHARE_COLS; ++g) {
+        if (g % p.splits == int(rank)) continue;
+        uint32_t r[32];
+        if (ok && n_kb > 0) {
+          tmem_load32(lane_addr + uint32_t(g * SHARE_COLS), r);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) r[j] = 0u;
+        }
+        uint32_t* to = reinterpret_cast<uint32_t*>(a_tiles + size_t(g) * SHARE_BYTES) + q * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) to[j * BM] = r[j];
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes, read by the bulk copies
+      asm volatile("bar.sync 1, 128;" ::: "memory");               // the four epilogue warps
+      if (warp == 2 && lane < p.bn / SHARE_COLS && lane % p.splits != int(rank)) {
+        const uint32_t to = uint32_t(lane % p.splits), owned = uint32_t((p.bn / SHARE_COLS - int(to) + p.splits - 1) / p.splits);
+        const uint32_t sender = rank < to ? rank : rank - 1;
+        uint32_t remote, remote_bar;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(reduce + BIAS_SLOTS)), "r"(to));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_bar) : "r"(smem_u32(partials_ready)), "r"(to));
+        asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(remote + (sender * owned + uint32_t(lane / p.splits)) * SHARE_BYTES), "r"(smem_u32(a_tiles) + uint32_t(lane) * SHARE_BYTES),
+                     "r"(SHARE_BYTES), "r"(remote_bar)
+                     : "memory");
+      }
+    }
+    if (TRANSPOSED && p.splits > 1 && rank != 0) {
       // This slice's partial sums go to the leader's shared memory as [rank - 1][row][column] with
       // rows padded by 16 bytes (the leader's 16-byte reads of 32 rows then fall on different
       // banks): they are laid out in this CTA's own (otherwise unused) copy of the buffer first,
@@ -937,14 +1008,55 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     }
   }
-  if (p.splits > 1 && warp >= 2 && rank == 0 && acc_ok) {
+  if constexpr (SHARED) {
+    if (warp >= 2) {
+      const int q = warp & 3;
+      const uint32_t lane_addr = tmem_base + (uint32_t(q * 32) << 16);
+      const bool landed = mbar_wait(partials_ready, 0);   // (also after an error: the others' copies must not outlive this CTA)
+      if (!landed) atomicMax(p.error_flag, R2_ERR_TIMEOUT_ACC);
+      acc_ok = acc_ok && landed;
+      const int owned = (p.bn / SHARE_COLS - int(rank) + p.splits - 1) / p.splits;
+      const uint32_t* got = reinterpret_cast<const uint32_t*>(reduce + BIAS_SLOTS) + q * 32 + lane;
+      if (acc_ok) {
+        for (int i = 0; i < owned; ++i) {
+          // own sums out of tensor memory, the slices' added in rank order (the same bits every run), the total back into it
+          const uint32_t at = lane_addr + uint32_t((int(rank) + i * p.splits) * SHARE_COLS);
+          uint32_t own[32];
+          tmem_load32(at, own);
+          float v[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = 0.f;
+          for (int z = 0; z < p.splits; ++z) {
+            if (z == int(rank)) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(own[j]);
+            } else {
+              const uint32_t* part = got + ((z < int(rank) ? z : z - 1) * owned + i) * (SHARE_COLS * BM);
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(part[j * BM]);
+            }
+          }
+          tmem_store32(at, v);
+        }
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");   // the received sums have been read: their place serves as the warps' slabs
+      if (acc_ok && a0 + q * 32 < p.a_total) {
+        const uint32_t slab = smem_u32(reduce + BIAS_SLOTS) + uint32_t(q * STAGING_WORDS) * 4u;
+        for (int i = 0; i < owned; ++i) {
+          const int c = (int(rank) + i * p.splits) * SHARE_COLS;
+          finish_tile_rows<ROUTED>(p, lane_addr, slab, reduce, a0 + q * 32, b0, c, c + SHARE_COLS, lane, true, res_first, i == 0 && res_here);
+        }
+      }
+    }
+  }
+  if (TRANSPOSED && p.splits > 1 && warp >= 2 && rank == 0 && acc_ok) {
     // the other CTAs' partial sums have landed in this CTA's shared memory
     if (!mbar_wait(partials_ready, 0)) {
       atomicMax(p.error_flag, R2_ERR_TIMEOUT_ACC);
       acc_ok = false;
     }
   }
-  if (warp >= 2 && rank == 0) {
+  if (warp >= 2 && rank == 0 && !SHARED) {
     const int q = warp & 3;
     const int a = a0 + q * 32 + lane;
     const uint32_t lane_addr = tmem_base + (uint32_t(q * 32) << 16);
@@ -952,7 +1064,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if constexpr (!TRANSPOSED) {
       // every product has completed: the first tiles' shared memory serves as the warps' slabs
       if (ok && a0 + q * 32 < p.a_total) {
-        finish_tile_rows<ROUTED>(p, lane_addr, smem_u32(a_tiles) + uint32_t(q * STAGING_WORDS) * 4u, reduce, a0 + q * 32, b0, 0, p.bn, lane, n_kb > 0);
+        finish_tile_rows<ROUTED>(p, lane_addr, smem_u32(a_tiles) + uint32_t(q * STAGING_WORDS) * 4u, reduce, a0 + q * 32, b0, 0, p.bn, lane, n_kb > 0,
+                                 res_first, res_here);
       }
     } else if (ok) {
       const bool a_ok = a < p.a_total;
@@ -1286,7 +1399,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (ok && a0 + q * 32 < p.a_total) {
         const uint32_t lane_addr = tmem_base + buf * uint32_t(p.bn) + (uint32_t(q * 32) << 16);
-        finish_tile_rows<ROUTED>(p, lane_addr, slab, bias_s, a0 + q * 32, b_tile0, side * half, (side + 1) * half, lane, true);
+        float4 residual[8];
+        finish_tile_rows<ROUTED>(p, lane_addr, slab, bias_s, a0 + q * 32, b_tile0, side * half, (side + 1) * half, lane, true, residual, false);
       }
       // this warp has read the accumulator: the leader may overwrite it with the tile after next
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1314,9 +1428,12 @@ bool make_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer
   return r2::encode_bf16_map(map, base, 2, dims, strides, box);
 }
 
-template <bool A_MN, bool B_MN, bool TRANSPOSED, bool FUSED_LN = false, bool ROUTED = false>
+template <bool A_MN, bool B_MN, bool TRANSPOSED, bool FUSED_LN = false, bool ROUTED = false, bool SHARED = false>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, dim3 grid, size_t smem, cudaStream_t stream) {
-  auto kernel = gemm_tc_kernel<A_MN, B_MN, TRANSPOSED, FUSED_LN, ROUTED>;
+  if constexpr (!TRANSPOSED && !SHARED) {
+    if (p.splits > 1) return launch<A_MN, B_MN, TRANSPOSED, FUSED_LN, ROUTED, true>(ma, mb, p, grid, smem, stream);
+  }
+  auto kernel = gemm_tc_kernel<A_MN, B_MN, TRANSPOSED, FUSED_LN, ROUTED, SHARED>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -1387,7 +1504,47 @@ int max_resident_clusters(int size) {
   return cached[size];
 }
 
-Plan make_plan(int m, int n, int k, int w_is_nk, bool fused_ln = false) {
+// Which form many tokens take. 0: a tile a CTA, nothing else; 1: pairs of CTAs, and clusters that share K, where they are the faster
+// form; 2: pairs wherever they can run (r2_gemm_tc_set_pair; tests compare the forms).
+int g_pair_form = 1;
+
+// Tile width and shares of K of a token-major product, by a model of its time in nanoseconds. A k-block of 64 is bound by the SM's
+// shared memory (TMA writes it, the tensor core reads it: 48, 64 and 80 KB at 64, 128 and 192 columns): measured 200, 225 and
+// 252 ns with one CTA on an SM, 140 and 175 a CTA with two; what no k-block hides (launch, first loads, epilogue) 4.3, 5.2 and 6.5 us. Sharing
+// K over a cluster costs 3.8 us (3.0 with 64 columns). Measured against a 128-column tile a CTA, which was the only form (us): 512 x 1,024 x 1,024
+// 8.7 and now 6.9, 512 x 4,096 x 1,024 19.8 and 12.2, 1,024 x 768 x 768 7.8 and 6.4, 200 x 768 x 2,304 6.7 and 5.4, 512 x 6,400 x 1,600 29.6 and
+// 19.1, 2,048 x 6,400 x 1,600 (144 tiles of 192 columns in one wave instead of 208) 48.6 and 38.7. (Tiles of 256 columns are never the best.)
+void choose_tiles(int m, int n, int n_kb, bool share, bool whole_groups, int* bn_out, int* splits_out) {
+  static const int WIDTHS[3] = {64, 128, 192}, K_BLOCK[3] = {200, 225, 252}, K_BLOCK_TWO[2] = {140, 175}, FIXED[3] = {4300, 5200, 6500};
+  const int sms = n_sms(), row_tiles = (m + BM - 1) / BM;
+  long best = -1;
+  for (int i = 0; i < 3; ++i) {
+    const int bn = WIDTHS[i];
+    if (bn > 128 && (n < bn || whole_groups)) break;
+    const int tiles = row_tiles * ((n + bn - 1) / bn), per_sm = (tiles + sms - 1) / sms;
+    if (bn > 128 && per_sm > 1) continue;   // (two of them on an SM have no room for stages)
+    // inside a step two to an SM gain while few SMs have two (192 tiles: q/k/v of 512 x 1,024 9.2 us from 10.1; 256: 10.3 from 9.7)
+    if (bn == 64 && per_sm > 1 && 3 * tiles > 4 * sms) continue;
+    const long cost = FIXED[i] + (per_sm == 1 ? long(n_kb) * K_BLOCK[i] : long(n_kb) * per_sm * K_BLOCK_TWO[i] + ((per_sm + 1) / 2 - 1) * 3000L);
+    if (best < 0 || cost < best) {
+      best = cost;
+      *bn_out = bn;
+      *splits_out = 1;
+    }
+    for (int s = 2; share && bn <= 128 && s <= bn / SHARE_COLS && tiles * s <= sms; ++s) {
+      const int per = (n_kb + s - 1) / s;
+      if ((n_kb + per - 1) / per != s || tiles > max_resident_clusters(s)) continue;
+      const long shared = FIXED[i] + long(per) * K_BLOCK[i] + (bn == 64 ? 3000 : 3800);
+      if (shared < best) {
+        best = shared;
+        *bn_out = bn;
+        *splits_out = s;
+      }
+    }
+  }
+}
+
+Plan make_plan(int m, int n, int k, int w_is_nk, bool fused_ln = false, bool whole_groups = false) {
   Plan pl;
   pl.swapped = m <= 64;
   pl.a_total = pl.swapped ? n : m;
@@ -1402,8 +1559,10 @@ Plan make_plan(int m, int n, int k, int w_is_nk, bool fused_ln = false) {
   } else {
     pl.bn = pl.b_total > 64 ? 128 : 64;                   // MN-major boxes are 64 features wide
   }
-  const int tiles = ((pl.a_total + BM - 1) / BM) * ((pl.b_total + pl.bn - 1) / pl.bn);
   pl.n_kb = (k + BK - 1) / BK;
+  int shares = 1;
+  if (!pl.swapped && pl.b_total >= 128) choose_tiles(m, n, pl.n_kb, g_pair_form == 1, whole_groups, &pl.bn, &shares);
+  const int tiles = ((pl.a_total + BM - 1) / BM) * ((pl.b_total + pl.bn - 1) / pl.bn);
   // A CTA streams its K range at well under 100 GB/s, so a product with few tiles uses the CTAs
   // of a cluster (at most 8) on one tile, each with a share of K; the leader's shared memory
   // must hold the others' partial tiles.
@@ -1422,10 +1581,13 @@ Plan make_plan(int m, int n, int k, int w_is_nk, bool fused_ln = false) {
     if (s < 1) s = 1;
     pl.splits = s;
   }
+  if (!pl.swapped) pl.splits = shares;   // (the CTAs of a cluster share K and, afterwards, the tile's columns)
   pl.kb_per_split = (pl.n_kb + pl.splits - 1) / pl.splits;
+  size_t share = !pl.swapped && pl.splits > 1 ? size_t(pl.splits - 1) * ((pl.bn / SHARE_COLS + pl.splits - 1) / pl.splits) * SHARE_BYTES : 0;   // received
+  if (share > 0 && share < 4 * size_t(STAGING_WORDS) * 4) share = 4 * size_t(STAGING_WORDS) * 4;   // (its place serves as the epilogue's slabs)
   const size_t a_bytes = BM * BK * 2, b_stride = (size_t(pl.bn) * BK * 2 + 1023) & ~size_t(1023);
   const size_t fixed = 1024 + (2 * MAX_STAGES + 3) * 8 + 32 +
-                       (pl.swapped ? size_t(pl.splits - 1) * (pl.bn + 4) * BM * 4 : size_t(BIAS_SLOTS) * 4);  // partial sums, or the bias
+                       (pl.swapped ? size_t(pl.splits - 1) * (pl.bn + 4) * BM * 4 : size_t(BIAS_SLOTS) * 4 + share);  // partial sums, or the bias and them
   // with more tiles than SMs, leave room for two CTAs on an SM: one's epilogue under the other's loads
   const size_t budget = (tiles * pl.splits > n_sms() ? 113 * 1024 : 227 * 1024) - fixed;
   if (fused_ln) {
@@ -1443,7 +1605,8 @@ Plan make_plan(int m, int n, int k, int w_is_nk, bool fused_ln = false) {
   if (stages > pl.kb_per_split) stages = pl.kb_per_split;
   if (stages < 1) stages = 1;
   // the token-major epilogue lays its four slabs over the tiles: a short K keeps stages it does not fill
-  while (!pl.swapped && size_t(stages) * (a_bytes + b_stride) < 4 * size_t(STAGING_WORDS) * 4) ++stages;
+  // (with a shared K: the groups to be sent)
+  while (!pl.swapped && size_t(stages) * (a_bytes + b_stride) < (share > 0 ? size_t(pl.bn / SHARE_COLS) * SHARE_BYTES : 4 * size_t(STAGING_WORDS) * 4)) ++stages;
   pl.stages = stages;
   pl.smem = fixed + size_t(stages) * (a_bytes + b_stride);
   return pl;
@@ -1565,8 +1728,6 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& 
 long long* g_cta_stamps = nullptr;  // (r2_gemm_tc_set_cta_stamps)
 int g_cta_stamps_cap = 0, g_last_grid = 0;
 
-int g_pair_form = 1;  // 0: never, 1: where it is the faster form, 2: wherever it can run (r2_gemm_tc_set_pair; tests compare the forms)
-
 }  // namespace
 
 // Profiling: launches from now on leave six times per CTA in `buffer` ([cap][6] int64 on the device; null: off).
@@ -1624,7 +1785,7 @@ int gemm_tc_run(const void* x, int lda, const void* w, int ldw, int w_is_nk, con
   if (error_flag == nullptr) return R2_BAD_SHAPE;
   if (lda % 8 != 0 || ldw % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15)) return R2_UNSUPPORTED;
   if (k % 8 != 0 || (!w_is_nk && n % 8 != 0)) return R2_UNSUPPORTED;
-  const Plan pl = make_plan(m, n, k, w_is_nk, fused_ln);
+  const Plan pl = make_plan(m, n, k, w_is_nk, fused_ln, group_n > 0);
   if (pl.stages < 1) return R2_UNSUPPORTED;
   GemmParams p;
   p.ln_x = ln_x;

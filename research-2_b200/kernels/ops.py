@@ -303,7 +303,8 @@ def use_kv_in_epilogue(on: bool) -> bool:
 def use_pair_gemm(mode):
     """The two-CTA persistent form (tcgen05.mma.cta_group::2, 256-row tiles) of the tensor-core
     product: False never, True where it is the faster form (many tiles per SM), "always" wherever
-    it can run (192 rows and 128 columns or more; tests compare it with the single-CTA form).
+    it can run (192 rows and 128 columns or more; tests compare it with the single-CTA form). Only
+    with True do the CTAs of a cluster share K where there are few tiles.
     Returns the previous setting in the same terms."""
     names = {0: False, 1: True, 2: "always"}
     code = {False: 0, True: 1, "always": 2}[mode]
