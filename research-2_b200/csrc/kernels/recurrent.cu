@@ -21,12 +21,14 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "scan_pieces.cuh"
 
 namespace {
 
 // Rows whose vectors are staged at a time: 32 (16 where a thread has 32 rows of a column in registers); 4 for launches in
 // which every entry is a single decoded row (less shared memory: more CTAs to an SM).
 constexpr int MAX_TILE = 32, SMALL_TILE = 4;
+constexpr int SCAN_THREADS = 64;  // of a CTA that walks a prompt's rows, while there are slices (scan_shape)
 constexpr int NORM_COPIES = 8;  // copies of a matrix memory's normaliser and maximum: one per slice of the columns at most
 
 constexpr int MODE_MLSTM = 0, MODE_SSD = 1, MODE_DECAY = 2;
@@ -58,12 +60,13 @@ struct ScanArgs {
   float* out; int out_stride;            // [T, heads * cols] float
   int heads_per_group, rows, cols, G, cv;
   int single_rows;                       // a hint: no entry has more than one row (a decode step)
+  int pieces;                            // every row of every operand starts on a 16-byte boundary: tiles are copied ahead
   // state space: the convolution's last inputs, renewed by the entry's CTAs together
   const void* conv_in; int conv_in_stride; int conv_channels, conv_taps; long long conv_state_off;
 };
 
 template <typename T, int RPT, int MODE, int TILE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 1)
 outer_scan_kernel(const ScanArgs a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -105,12 +108,19 @@ outer_scan_kernel(const ScanArgs a) {
       }
   }
 
-  float S[RPT], nrm[RPT], m = 0.f;
+  uint64_t S[RPT / 2], nrm[RPT / 2];   // in twos: rows g * RPT + 2 r and the one after it
+  float m = 0.f;
 #pragma unroll
-  for (int r = 0; r < RPT; ++r) {
-    const int i = g * RPT + r;
-    S[r] = (!is_fresh && i < rows && j < cols) ? head_state[size_t(i) * cols + j] : 0.f;
-    nrm[r] = (MODE == MODE_MLSTM && !is_fresh && i < rows) ? norm_state[size_t(blockIdx.z) * (rows + 1) + i] : 0.f;
+  for (int r = 0; r < RPT / 2; ++r) {
+    float s2[2], n2[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = g * RPT + 2 * r + u;
+      s2[u] = (!is_fresh && i < rows && j < cols) ? head_state[size_t(i) * cols + j] : 0.f;
+      n2[u] = (MODE == MODE_MLSTM && !is_fresh && i < rows) ? norm_state[size_t(blockIdx.z) * (rows + 1) + i] : 0.f;
+    }
+    S[r] = pair_of(s2[0], s2[1]);
+    nrm[r] = pair_of(n2[0], n2[1]);
   }
   if (MODE == MODE_MLSTM && !is_fresh) m = norm_state[size_t(blockIdx.z) * (rows + 1) + rows];
 
@@ -119,56 +129,104 @@ outer_scan_kernel(const ScanArgs a) {
   const T* value = static_cast<const T*>(a.value) + size_t(h) * cols + size_t(blockIdx.z) * cv;
   const float skip = MODE == MODE_SSD ? a.skip[h] : 0.f;
 
-  for (int t0 = row0; t0 < row1; t0 += TILE) {
-    const int nt = row1 - t0 < TILE ? row1 - t0 : TILE;
-    __syncthreads();  // the last rows' vectors have been used
-    // (loads in batches of eight before their stores: a loop of load-then-store would wait for every load in turn)
-    for (int base = 0; base < nt * padded; base += 8 * blockDim.x) {
-      float tr[8], tw[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int idx = base + u * blockDim.x + tid;
-        const int tt = idx / padded, i = idx - tt * padded;
-        const bool live = idx < nt * padded && i < rows;
-        const size_t row = size_t(t0 + tt);
-        tr[u] = live ? to_float(read[row * a.read_stride + i]) : 0.f;
-        tw[u] = live ? to_float(write[row * a.write_stride + i]) : 0.f;
-        if (MODE == MODE_DECAY && live && i < 2 * a.rot_half) {
-          // the pair (u, v) = (x[i], x[i + half]) becomes (u cos - v sin, v cos + u sin); position and angle are float
-          const bool low = i < a.rot_half;
-          const int other = low ? i + a.rot_half : i - a.rot_half;
-          float sn, cs;
-          sincosf(float(a.positions[row]) * a.inv_freq[low ? i : other], &sn, &cs);
-          if (low) sn = -sn;
-          tr[u] = fmaf(tr[u], cs, to_float(read[row * a.read_stride + other]) * sn);
-          tw[u] = fmaf(tw[u], cs, to_float(write[row * a.write_stride + other]) * sn);
-        }
-        if (MODE == MODE_DECAY && a.silu_in) {
-          tr[u] = silu(tr[u]);
-          tw[u] = silu(tw[u]);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int idx = base + u * blockDim.x + tid;
-        if (idx < nt * padded) {
-          rs[idx] = tr[u] * a.read_scale;
-          ws[idx] = MODE == MODE_DECAY ? tw[u] * a.write_scale : tw[u];
-        }
-      }
+  // A prompt's rows come a tile ahead: as they are stored, by asynchronous copies, next to the float vectors of the tile in use; the
+  // gates in a register of the thread that turns them into factors. (Fetched when their tile began, every tile of 32 rows first
+  // waited for memory: see the figures at the launch.)
+  constexpr bool AHEAD = TILE > SMALL_TILE && MODE != MODE_DECAY;
+  constexpr int PER = 16 / int(sizeof(T));
+  const bool ahead = AHEAD && a.pieces != 0;
+  const int copy_cols = max(0, min(cv, cols - int(blockIdx.z) * cv)), raw_stage = TILE * (2 * rows + cv);
+  T* raw = reinterpret_cast<T*>(g2 + TILE);   // two stages of [TILE][rows] r, [TILE][rows] w, [TILE][cv] v
+  const PieceWalk of_vectors(rows / PER), of_values(copy_cols / PER);
+  float gate_a = 0.f, gate_b = 0.f;
+  auto gates_of = [&](int t) {
+    if (tid < TILE && t + tid < row1) {
+      const float* gr = a.gates + size_t(t + tid) * a.gates_stride;
+      gate_a = gr[h];
+      if (MODE == MODE_MLSTM) gate_b = gr[gridDim.y + h];
     }
-    for (int base = 0; base < nt * cv; base += 4 * blockDim.x) {
-      float tv[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int idx = base + u * blockDim.x + tid;
-        const int tt = idx / cv, c = idx - tt * cv;
-        tv[u] = (idx < nt * cv && blockIdx.z * cv + c < cols) ? to_float(value[size_t(t0 + tt) * a.value_stride + c]) : 0.f;
+  };
+  auto issue = [&](int t, int stage) {
+    T* to = raw + stage * raw_stage;
+    const int n = min(TILE, row1 - t);
+    stage_rows<T>(to, rows, read + size_t(t) * a.read_stride, a.read_stride, of_vectors, n, true);
+    stage_rows<T>(to + TILE * rows, rows, write + size_t(t) * a.write_stride, a.write_stride, of_vectors, n, true);
+    if (copy_cols > 0) stage_rows<T>(to + 2 * TILE * rows, cv, value + size_t(t) * a.value_stride, a.value_stride, of_values, n, true);
+  };
+  if (ahead) {
+    for (int i = tid; i < TILE * (2 * padded + cv); i += blockDim.x) smem[i] = 0.f;   // (dimensions and columns beyond the head's)
+    issue(row0, 0);
+    gates_of(row0);
+  }
+  int stage = 0;
+  for (int t0 = row0; t0 < row1; t0 += TILE, stage ^= 1) {
+    const int nt = row1 - t0 < TILE ? row1 - t0 : TILE;
+    if (ahead) asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // the last rows' vectors have been used (and the copies of this tile's are there)
+    float now_a = gate_a, now_b = gate_b;
+    if (ahead) {
+      if (t0 + TILE < row1) {
+        issue(t0 + TILE, stage ^ 1);
+        gates_of(t0 + TILE);
       }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int idx = base + u * blockDim.x + tid;
-        if (idx < nt * cv) vs[idx] = (MODE == MODE_DECAY && a.silu_in) ? silu(tv[u]) : tv[u];
+      const T* from = raw + stage * raw_stage;
+      spread_rows<T>(rs, padded, from, rows, of_vectors, nt, a.read_scale);
+      spread_rows<T>(ws, padded, from + TILE * rows, rows, of_vectors, nt, 1.f);
+      if (copy_cols > 0) spread_rows<T>(vs, cv, from + 2 * TILE * rows, cv, of_values, nt, 1.f);
+    } else {
+      // (loads in batches of eight before their stores: a loop of load-then-store would wait for every load in turn)
+      for (int base = 0; base < nt * padded; base += 8 * blockDim.x) {
+        float tr[8], tw[8];
+  #pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int idx = base + u * blockDim.x + tid;
+          const int tt = idx / padded, i = idx - tt * padded;
+          const bool live = idx < nt * padded && i < rows;
+          const size_t row = size_t(t0 + tt);
+          tr[u] = live ? to_float(read[row * a.read_stride + i]) : 0.f;
+          tw[u] = live ? to_float(write[row * a.write_stride + i]) : 0.f;
+          if (MODE == MODE_DECAY && live && i < 2 * a.rot_half) {
+            // the pair (u, v) = (x[i], x[i + half]) becomes (u cos - v sin, v cos + u sin); position and angle are float
+            const bool low = i < a.rot_half;
+            const int other = low ? i + a.rot_half : i - a.rot_half;
+            float sn, cs;
+            sincosf(float(a.positions[row]) * a.inv_freq[low ? i : other], &sn, &cs);
+            if (low) sn = -sn;
+            tr[u] = fmaf(tr[u], cs, to_float(read[row * a.read_stride + other]) * sn);
+            tw[u] = fmaf(tw[u], cs, to_float(write[row * a.write_stride + other]) * sn);
+          }
+          if (MODE == MODE_DECAY && a.silu_in) {
+            tr[u] = silu(tr[u]);
+            tw[u] = silu(tw[u]);
+          }
+        }
+  #pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int idx = base + u * blockDim.x + tid;
+          if (idx < nt * padded) {
+            rs[idx] = tr[u] * a.read_scale;
+            ws[idx] = MODE == MODE_DECAY ? tw[u] * a.write_scale : tw[u];
+          }
+        }
+      }
+      for (int base = 0; base < nt * cv; base += 4 * blockDim.x) {
+        float tv[4];
+  #pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int idx = base + u * blockDim.x + tid;
+          const int tt = idx / cv, c = idx - tt * cv;
+          tv[u] = (idx < nt * cv && blockIdx.z * cv + c < cols) ? to_float(value[size_t(t0 + tt) * a.value_stride + c]) : 0.f;
+        }
+  #pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int idx = base + u * blockDim.x + tid;
+          if (idx < nt * cv) vs[idx] = (MODE == MODE_DECAY && a.silu_in) ? silu(tv[u]) : tv[u];
+        }
+      }
+      if (MODE != MODE_DECAY && tid < nt) {
+        const float* gr = a.gates + size_t(t0 + tid) * a.gates_stride;
+        now_a = gr[h];
+        if (MODE == MODE_MLSTM) now_b = gr[gridDim.y + h];
       }
     }
     if (MODE == MODE_DECAY) {
@@ -177,12 +235,11 @@ outer_scan_kernel(const ScanArgs a) {
         g1[tid] = a.decay[h];
       }
     } else if (tid < nt) {
-      const float* gr = a.gates + size_t(t0 + tid) * a.gates_stride;
       if (MODE == MODE_MLSTM) {
-        g0[tid] = soft_cap(gr[h], a.cap);
-        g1[tid] = log_sigmoid(soft_cap(gr[gridDim.y + h], a.cap));
+        g0[tid] = soft_cap(now_a, a.cap);
+        g1[tid] = log_sigmoid(soft_cap(now_b, a.cap));
       } else {
-        const float step = softplus(gr[h] + a.step_bias[h]);
+        const float step = softplus(now_a + a.step_bias[h]);
         g0[tid] = step;
         g1[tid] = expf(-expf(a.log_rate[h]) * step);
       }
@@ -221,72 +278,84 @@ outer_scan_kernel(const ScanArgs a) {
       __syncthreads();
       m = g2[nt - 1];
     }
-    float num[TILE], nq[TILE];
+    // a row: this lane's shares of S^T r and, with a normaliser, of n . r
+    auto walk = [&](int tt, float& acc_n) {
+      const float take = g0[tt], keep = g1[tt];
+      const float tv = take * vs[tt * cv + jl];
+      const uint64_t keep2 = pair_of(keep, keep), tv2 = pair_of(tv, tv), take2 = pair_of(take, take);
+      const float4* wr = reinterpret_cast<const float4*>(ws + tt * padded + g * RPT);
+      const float4* rr = reinterpret_cast<const float4*>(rs + tt * padded + g * RPT);
+      float acc = 0.f;
+      acc_n = 0.f;
 #pragma unroll
-    for (int tt = 0; tt < TILE; ++tt) {
-      if (tt >= nt) break;   // (a branch that every thread of the CTA takes alike: rows that are not there cost nothing)
-      num[tt] = 0.f;
-      nq[tt] = 0.f;
-      {
-        const float take = g0[tt], keep = g1[tt];
-        const float tv = take * vs[tt * cv + jl];
-        const float4* wr = reinterpret_cast<const float4*>(ws + tt * padded + g * RPT);
-        const float4* rr = reinterpret_cast<const float4*>(rs + tt * padded + g * RPT);
-        float acc = 0.f, acc_n = 0.f;
+      for (int r4 = 0; r4 < RPT / 4; ++r4) {
+        const float4 w4 = wr[r4], q4 = rr[r4];
+        const uint64_t w[2] = {pair_of(w4.x, w4.y), pair_of(w4.z, w4.w)};
+        const float q[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
-        for (int r4 = 0; r4 < RPT / 4; ++r4) {
-          const float4 w4 = wr[r4], q4 = rr[r4];
-          const float w[4] = {w4.x, w4.y, w4.z, w4.w}, q[4] = {q4.x, q4.y, q4.z, q4.w};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int r = r4 * 4 + u;
-            S[r] = fmaf(keep, S[r], w[u] * tv);
-            acc = fmaf(S[r], q[u], acc);
-            if (MODE == MODE_MLSTM) {
-              nrm[r] = fmaf(keep, nrm[r], take * w[u]);
-              acc_n = fmaf(nrm[r], q[u], acc_n);
-            }
+        for (int u = 0; u < 2; ++u) {
+          const int r = r4 * 2 + u;
+          S[r] = fma_pair(keep2, S[r], mul_pair(w[u], tv2));
+          const float2 s2 = both(S[r]);
+          acc = fmaf(s2.y, q[2 * u + 1], fmaf(s2.x, q[2 * u], acc));
+          if (MODE == MODE_MLSTM) {
+            nrm[r] = fma_pair(keep2, nrm[r], mul_pair(take2, w[u]));
+            const float2 n2 = both(nrm[r]);
+            acc_n = fmaf(n2.y, q[2 * u + 1], fmaf(n2.x, q[2 * u], acc_n));
           }
         }
-        num[tt] = acc;
-        nq[tt] = acc_n;
       }
-    }
-    // the sums over a column's rows, for all rows of the tile at once (the shuffles of different rows overlap)
+      return acc;
+    };
+    auto store = [&](int tt, float num, float nq) {
+      float y;
+      if (MODE == MODE_MLSTM) y = num / (fmaxf(fabsf(nq), expf(-g2[tt])) + 1e-6f);
+      else y = fmaf(skip, vs[tt * cv + jl], num);
+      a.out[size_t(t0 + tt) * a.out_stride + size_t(h) * cols + j] = y;
+    };
+    // four rows at a time: their sums are independent of each other, and their shuffles overlap
+    int tt = 0;
+    for (; TILE > SMALL_TILE && tt + 4 <= nt; tt += 4) {
+      float num[4], nq[4];
 #pragma unroll
-    for (int tt = 0; tt < TILE; ++tt) {
-      if (tt >= nt) break;
-      {
-        for (int o = G >> 1; o > 0; o >>= 1) {
-          num[tt] += __shfl_xor_sync(0xffffffffu, num[tt], o);
-          if (MODE == MODE_MLSTM) nq[tt] += __shfl_xor_sync(0xffffffffu, nq[tt], o);
+      for (int i = 0; i < 4; ++i) num[i] = walk(tt + i, nq[i]);
+      if (G >= 4) {
+        const float y = sums_of_four(num[0], num[1], num[2], num[3], g, G);
+        const float z = MODE == MODE_MLSTM ? sums_of_four(nq[0], nq[1], nq[2], nq[3], g, G) : 0.f;
+        if ((g & ((G >> 2) - 1)) == 0 && j < cols) store(tt + ((g & (G >> 1)) ? 2 : 0) + ((g & (G >> 2)) ? 1 : 0), y, z);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (G == 2) {
+            num[i] += __shfl_xor_sync(0xffffffffu, num[i], 1);
+            if (MODE == MODE_MLSTM) nq[i] += __shfl_xor_sync(0xffffffffu, nq[i], 1);
+          }
+          if (g == 0 && j < cols) store(tt + i, num[i], nq[i]);
         }
       }
     }
-    if (g == 0 && j < cols) {
-#pragma unroll
-      for (int tt = 0; tt < TILE; ++tt) {
-        if (tt >= nt) break;
-        {
-          float y;
-          if (MODE == MODE_MLSTM) y = num[tt] / (fmaxf(fabsf(nq[tt]), expf(-g2[tt])) + 1e-6f);
-          else y = fmaf(skip, vs[tt * cv + jl], num[tt]);
-          a.out[size_t(t0 + tt) * a.out_stride + size_t(h) * cols + j] = y;
-        }
+    for (; tt < nt; ++tt) {
+      float nq, num = walk(tt, nq);
+      for (int o = G >> 1; o > 0; o >>= 1) {
+        num += __shfl_xor_sync(0xffffffffu, num, o);
+        if (MODE == MODE_MLSTM) nq += __shfl_xor_sync(0xffffffffu, nq, o);
       }
+      if (g == 0 && j < cols) store(tt, num, nq);
     }
   }
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
     const int i = g * RPT + r;
-    if (i < rows && j < cols) head_state[size_t(i) * cols + j] = S[r];
+    const float2 s2 = both(S[r / 2]);
+    if (i < rows && j < cols) head_state[size_t(i) * cols + j] = (r & 1) ? s2.y : s2.x;
   }
   if (MODE == MODE_MLSTM && jl == 0) {
     for (int copy = blockIdx.z; copy < NORM_COPIES; copy += gridDim.z) {
 #pragma unroll
       for (int r = 0; r < RPT; ++r) {
         const int i = g * RPT + r;
-        if (i < rows) norm_state[size_t(copy) * (rows + 1) + i] = nrm[r];
+        const float2 n2 = both(nrm[r / 2]);
+        if (i < rows) norm_state[size_t(copy) * (rows + 1) + i] = (r & 1) ? n2.y : n2.x;
       }
       if (tid == 0) norm_state[size_t(copy) * (rows + 1) + rows] = m;
     }
@@ -295,22 +364,26 @@ outer_scan_kernel(const ScanArgs a) {
 
 // How a head's state is spread over threads: RPT rows of a column in a thread's registers, a column's rows over G
 // neighbouring lanes (a power of two up to 32), cv columns a CTA and the columns over 1, 2, 4 or 8 CTAs: as few as the
-// 256 threads of a CTA allow, and more while the launch has fewer CTAs than the GPU has SMs.
+// threads of a CTA allow, and more while the launch has fewer CTAs than the GPU has SMs. `wide`: 256 threads (decode steps, and the
+// walk with a fixed decay, whose tiles are not copied ahead: 16 entries of 64 rows 57 us, 87 with 64 threads). Prompts of the other two
+// take 64: of a batch's entries few are long, and those then have their columns over as many SMs as there are slices (900 rows beside
+// 7 decoded ones, 12 heads of 64 x 64, matrix memory: 311 us with 256 threads, 242; 16 entries of 64 rows 59 and 55).
 struct ScanShape { int rpt, G, threads, cv, splits; };
 
-ScanShape scan_shape(int rows, int cols, int pairs) {
+ScanShape scan_shape(int rows, int cols, int pairs, bool wide, int per_piece) {
   ScanShape s;
   s.rpt = 4;
   while (s.rpt < 32 && (rows + s.rpt - 1) / s.rpt > 4) s.rpt *= 2;
   s.G = 1;
   while (s.G * s.rpt < rows) s.G *= 2;
-  const int G = s.G > 32 ? 32 : s.G, per_warp = 32 / G;
+  const int G = s.G > 32 ? 32 : s.G;
+  const int granule = !wide && per_piece > 32 / G ? per_piece : 32 / G;   // columns: whole warps and, where rows are copied, whole pieces
   s.splits = 1;
   for (;;) {
-    s.cv = ((cols + s.splits - 1) / s.splits + per_warp - 1) / per_warp * per_warp;
+    s.cv = ((cols + s.splits - 1) / s.splits + granule - 1) / granule * granule;
     s.threads = s.cv * G;
     if (s.splits == NORM_COPIES) break;
-    const bool fits = s.threads <= 256, enough = pairs * s.splits >= 120 || s.threads <= 64;
+    const bool fits = s.threads <= (wide ? 256 : SCAN_THREADS), enough = pairs * s.splits >= 120 || s.threads <= 64;
     if (fits && enough) break;
     s.splits *= 2;
   }
@@ -320,15 +393,23 @@ ScanShape scan_shape(int rows, int cols, int pairs) {
 template <typename T, int MODE>
 int launch_scan(const ScanArgs& in, int n_entries, int n_heads, cudaStream_t stream) {
   ScanArgs a = in;
-  const ScanShape s = scan_shape(a.rows, a.cols, n_entries * n_heads);
+  const ScanShape s = scan_shape(a.rows, a.cols, n_entries * n_heads, a.single_rows != 0 || MODE == MODE_DECAY, 16 / int(sizeof(T)));
   const int rpt = s.rpt, G = s.G, threads = s.threads, splits = s.splits;
   if (G > 32 || threads > 256) return R2_UNSUPPORTED;
   a.G = G;
   a.cv = s.cv;
   const bool single_rows = a.single_rows != 0;
   const int tile = single_rows ? SMALL_TILE : (rpt <= 16 ? MAX_TILE : 16);
-  const size_t smem = sizeof(float) * (size_t(tile) * (2 * rpt * G + a.cv) + 3 * tile);
+  size_t smem = sizeof(float) * (size_t(tile) * (2 * rpt * G + a.cv) + 3 * tile);
   if (smem > 48 * 1024) return R2_UNSUPPORTED;
+  // Tiles are copied ahead where whole 16-byte pieces can be. With the rows' sums four at a time: 900 rows beside 7 decoded ones, 12
+  // heads, state space of 32 x 64 245 to 103 us, matrix memory of 64 x 64 477 to 242; what is left is a warp's issue and latencies
+  // (some 90 instructions a row, one warp to a scheduler).
+  const size_t raw = 2 * size_t(tile) * (2 * a.rows + a.cv) * sizeof(T);
+  auto on_pieces = [](const void* p, int stride) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && stride * sizeof(T) % 16 == 0; };
+  a.pieces = !single_rows && MODE != MODE_DECAY && smem + raw <= 48 * 1024 && a.rows * sizeof(T) % 16 == 0 && a.cols * sizeof(T) % 16 == 0 &&
+             a.cv * sizeof(T) % 16 == 0 && on_pieces(a.read, a.read_stride) && on_pieces(a.write, a.write_stride) && on_pieces(a.value, a.value_stride);
+  if (a.pieces) smem += raw;
   dim3 grid(n_entries, n_heads, splits);
 #define R2_SCAN(RPT_, TILE_) r2_launch(outer_scan_kernel<T, RPT_, MODE, TILE_>, grid, dim3(threads), smem, stream, a)
   switch (rpt) {

@@ -1,0 +1,125 @@
+"""The recurrences that walk row by row, at the edges of their tiles of rows and slices of columns: against a walk in 64 bits, and the
+same bits whether rows can be copied in 16-byte pieces or not and however an entry is cut."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+ROWS = [15, 16, 0, 33, 1, 64, 3, 97]   # of the entries: around tiles of 16 and 32 rows and groups of four
+
+
+def ops():
+    from research_2_b200.kernels import ops as o
+
+    return o
+
+
+def entries(rows):
+    start = torch.tensor([0] + rows).cumsum(0).int()
+    gen = torch.Generator().manual_seed(len(rows))
+    return start.to(DEV), torch.randperm(len(rows), generator=gen).int().to(DEV), torch.tensor([i % 2 for i in range(len(rows))]).int().to(DEV)
+
+
+def shifted(t, by):
+    """The same numbers as columns of a wider tensor, `by` columns in (one: no row starts on a 16-byte boundary)."""
+    wide = torch.zeros(t.shape[0], t.shape[1] + 8, dtype=t.dtype, device=t.device)
+    wide[:, by: by + t.shape[1]] = t
+    return wide[:, by: by + t.shape[1]]
+
+
+def walk64(kind, rows, start, slot, fresh, state, heads, dim, vdim, data):
+    out = torch.zeros(sum(rows), heads * vdim, dtype=torch.float64)
+    for e, n in enumerate(rows):
+        s = torch.zeros(heads, dim, vdim, dtype=torch.float64) if fresh[e] else state[slot[e]].clone()
+        for t in range(int(start[e]), int(start[e]) + n):
+            if kind == "delta":
+                q, k, v, num = (data[x][t] for x in ("q", "k", "v", "num"))
+                s = s * num[:, 0, None, None]
+                u = num[:, 1, None] * (v - torch.einsum("hij,hi->hj", s, k))
+                o = torch.einsum("hij,hi->hj", s, q) + num[:, 2, None] * u
+                s = s + k[:, :, None] * u[:, None, :]
+            elif kind == "mix":
+                kv = data["k"][t][:, :, None] * data["v"][t][:, None, :]
+                o = torch.einsum("hij,hi->hj", s + data["bonus"][:, :, None] * kv, data["r"][t])
+                s = data["w"][t][:, :, None] * s + kv
+            else:
+                step = torch.nn.functional.softplus(data["steps"][t] + data["bias"])
+                s = torch.exp(-torch.exp(data["rate"]) * step)[:, None, None] * s + step[:, None, None] * data["b"][t][None, :, None] * data["x"][t][:, None, :]
+                o = torch.einsum("hij,i->hj", s, data["c"][t]) + data["skip"][:, None] * data["x"][t]
+            out[t] = o.reshape(-1)
+    return out
+
+
+# heads of whole and of odd pieces, one to sixteen lanes a column, slices of one and of many columns
+@pytest.mark.parametrize("heads,dim,vdim", [(3, 64, 64), (2, 32, 40), (2, 20, 36), (3, 4, 8), (2, 8, 10), (1, 200, 24)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_walks_at_the_edges_of_their_tiles(heads, dim, vdim, dtype):
+    o, total = ops(), sum(ROWS)
+    gen = torch.Generator().manual_seed(dim)
+    rand = lambda *s: torch.randn(*s, generator=gen)
+    start, slot, fresh = entries(ROWS)
+    # (float32 sums of at most `dim` terms behind a decaying state: well below 1e-4 of values around one; the random walks here reach some ten)
+    close = lambda got, want: torch.testing.assert_close(got.double().cpu(), want, rtol=1e-4, atol=1e-4 * max(1.0, float(want.abs().max())))
+
+    # the delta rule, over prepared rows
+    d4 = -(-dim // 4) * 4
+    qk = torch.zeros(total, heads, 2, d4)
+    qk[..., :dim] = torch.nn.functional.normalize(rand(total, heads, 2, dim), dim=-1)
+    num = torch.zeros(total, heads, 4)
+    num[..., 0], num[..., 1], num[..., 2] = 0.8 + 0.2 * torch.rand(total, heads, generator=gen), torch.rand(total, heads, generator=gen), (qk[:, :, 0] * qk[:, :, 1]).sum(-1)
+    v, packed = rand(total, heads * vdim), rand(len(ROWS), heads * o.scan_state_floats(dim, vdim))
+    first = o.delta_scan(qk.to(DEV), v.to(DEV), num.to(DEV), dim, packed.clone().to(DEV), start, slot, fresh)
+    from_zero = [e for e in range(len(ROWS)) if fresh[e]]   # (a slot's pieces are the kernel's own order: states that begin at zero)
+    want = walk64("delta", ROWS, start.cpu(), slot.cpu(), torch.ones(len(ROWS)), None, heads, dim, vdim,
+                  {"q": qk[:, :, 0, :dim].double(), "k": qk[:, :, 1, :dim].double(), "v": v.double().view(total, heads, vdim), "num": num.double()})
+    for e in from_zero:
+        close(first[start[e]: start[e + 1]], want[int(start[e]): int(start[e + 1])])
+
+    # time mixing
+    r, k, x = (rand(total, heads * dim).to(dtype) for _ in range(3))
+    w, bonus, packed = 0.5 + 0.5 * torch.rand(total, heads * dim, generator=gen), rand(heads * dim), rand(len(ROWS), heads * o.scan_state_floats(dim, dim))
+    both = []
+    for by in (0, 1):
+        mine = packed.clone().to(DEV)
+        got = o.time_mix_scan(*(shifted(t.to(DEV), by) for t in (r, k, x, w)), bonus.to(DEV), mine, start, slot, fresh, heads, dim)
+        both.append((got, mine))
+    assert torch.equal(both[0][0], both[1][0]) and torch.equal(both[0][1], both[1][1])
+    view = lambda t: t.double().view(total, heads, dim)
+    want = walk64("mix", ROWS, start.cpu(), slot.cpu(), torch.ones(len(ROWS)), None, heads, dim, dim,
+                  {"r": view(r), "k": view(k), "v": view(x), "w": view(w), "bonus": bonus.double().view(heads, dim)})
+    for e in from_zero:
+        close(both[0][0][start[e]: start[e + 1]], want[int(start[e]): int(start[e + 1])])
+
+    # the state-space recurrence, whose slot is [heads][dim][vdim]
+    x, b, c = rand(total, heads * vdim).to(dtype), rand(total, dim).to(dtype), rand(total, dim).to(dtype)
+    steps, bias, rate, skip, state = rand(total, heads), rand(heads), rand(heads), rand(heads), rand(len(ROWS), heads * dim * vdim)
+    both = []
+    for by in (0, 1):
+        mine = state.clone().to(DEV)
+        got = o.ssd_scan(*(shifted(t.to(DEV), by) for t in (x, b, c)), steps.to(DEV), bias.to(DEV), rate.to(DEV), skip.to(DEV), mine, start, slot, fresh,
+                         heads, 1, dim, vdim)
+        both.append((got, mine))
+    assert torch.equal(both[0][0], both[1][0]) and torch.equal(both[0][1], both[1][1])
+    want = walk64("ssd", ROWS, start.cpu(), slot.cpu(), fresh.cpu(), state.double().view(-1, heads, dim, vdim), heads, dim, vdim,
+                  {"x": x.double().view(total, heads, vdim), "b": b.double(), "c": c.double(), "steps": steps.double(), "bias": bias.double(), "rate": rate.double(), "skip": skip.double()})
+    close(both[0][0], want)
+
+    # the matrix memory: pieces and elements alike, and a prompt in one step and in three
+    q, k, x, gates = rand(total, heads * dim).to(dtype), rand(total, heads * dim).to(dtype), rand(total, heads * vdim).to(dtype), rand(total, 2 * heads)
+    memory = rand(len(ROWS), heads * o.mlstm_state_floats(dim, vdim)).abs()
+    both = []
+    for by in (0, 1):
+        mine = memory.clone().to(DEV)
+        got = o.mlstm_scan(*(shifted(t.to(DEV), by) for t in (q, k, x)), gates.to(DEV), 15.0, dim ** -0.5, mine, start, slot, fresh, heads, dim, vdim)
+        both.append((got, mine))
+    assert torch.equal(both[0][0], both[1][0]) and torch.equal(both[0][1], both[1][1])
+    last = len(ROWS) - 1
+    row0, n, mine = int(start[last]), ROWS[last], memory.clone().to(DEV)
+    for begin, end in ((0, 1), (1, 40), (40, n)):
+        part = [t.to(DEV)[row0 + begin: row0 + end].contiguous() for t in (q, k, x, gates)]
+        got = o.mlstm_scan(*part, 15.0, dim ** -0.5, mine, torch.tensor([0, end - begin], dtype=torch.int32, device=DEV), slot[last:].contiguous(),
+                           torch.tensor([int(fresh[last]) if begin == 0 else 0], dtype=torch.int32, device=DEV), heads, dim, vdim)
+        assert torch.equal(got, both[0][0][row0 + begin: row0 + end])
