@@ -7,7 +7,7 @@
 // S is [rows x cols] per head, float, in the request's slot, stored in pieces of four rows: [rows / 4][cols][4]. A CTA owns one (entry, head, slice of the columns), takes the state from
 // the slot (or zeros for a sequence's first rows), walks the entry's rows in order and puts the state back. A thread keeps RPT
 // rows of one column in registers, a column's rows are spread over G neighbouring lanes in pieces of four. The rows' vectors come
-// through shared memory in tiles, copied asynchronously one tile ahead. The delta rule's write needs what the state returns for
+// through shared memory in tiles, copied asynchronously two tiles ahead. The delta rule's write needs what the state returns for
 // the row's key: S'^T k and S'^T q are summed side by side (o = S'^T q + (k . q) u), which leaves one round of shuffles a row on the
 // chain. How a head's state is spread over lanes depends on its sizes alone, so a row's result is the same bits however its
 // prompt was cut and whatever else is in the batch.
@@ -16,12 +16,19 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "scan_pieces.cuh"
 #include "small_products.cuh"
 
 namespace {
 
 constexpr int MODE_DELTA = 0, MODE_CHANNEL = 1;
-constexpr int SCAN_STAGES = 2;
+constexpr int SCAN_STAGES = 3, SCAN_TILE = 16;
+// Threads of a CTA that walks a prompt's rows, at most: of a batch's entries few are long, and their columns should be on many SMs. 900
+// rows beside 7 decoded ones, 12 heads of 64 x 64, delta rule and time mixing (us): 143 and 184 with 256 threads, 151 and 147 with 128,
+// 161 and 171 with 64; 16 entries of 64 rows 35 and 27, 30 and 27, 32 and 30. (221 and 209, 31 and 29 before the tiles of 16 rows, the two
+// floats an instruction and the sums of four rows at a time.) A row is some 85 instructions, a third of the time waits for the one
+// before it and a quarter for shuffles and shared memory.
+constexpr int SCAN_THREADS = 128;
 
 __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float silu(float x) { return x / (1.f + expf(-x)); }
@@ -42,26 +49,6 @@ struct StateScanArgs {
   // the last keep_rows input rows (of the convolution, of the mixes) are state too: renewed here, spread over the entry's CTAs
   const void* keep_in; int keep_in_stride, keep_width, keep_rows, keep_is_bf16; long long keep_off;
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
-
-// n elements of a row into shared memory, by the threads of the CTA from `first` on in steps of blockDim.x over (row, piece).
-template <typename T>
-__device__ __forceinline__ void stage_rows(T* dst, int dst_stride, const T* src, long long src_stride, int n, int n_rows, bool pieces) {
-  constexpr int PER = 16 / int(sizeof(T));
-  if (pieces) {
-    const int per_row = n / PER;
-    for (int i = threadIdx.x; i < per_row * n_rows; i += blockDim.x) {
-      const int r = i / per_row, c = (i - r * per_row) * PER;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + r * dst_stride + c)), "l"(src + r * src_stride + c) : "memory");
-    }
-  } else {
-    for (int i = threadIdx.x; i < n * n_rows; i += blockDim.x) {
-      const int r = i / n, c = i - r * n;
-      dst[r * dst_stride + c] = src[r * src_stride + c];
-    }
-  }
-}
 
 // The newest keep_rows input rows of an entry: this step's, and before them what the slot held. Channel c is one thread's: it reads
 // a place before it writes over it.
@@ -115,142 +102,166 @@ state_scan_kernel(const StateScanArgs a) {
   const T* read = static_cast<const T*>(a.read) + size_t(group) * a.read_group;
   const T* write = static_cast<const T*>(a.write) + size_t(group) * a.write_group;
   const T* value = static_cast<const T*>(a.value) + size_t(h) * cols + j0;
-  const int copy_cols = min(cv, cols - j0);
+  const int copy_cols = max(0, min(cv, cols - j0));
   __syncthreads();
+  const bool pieces = a.pieces != 0;
+  constexpr int PER = 16 / int(sizeof(T));
+  const PieceWalk of_vectors(pieces ? rows / PER : rows), of_values(pieces ? copy_cols / PER : copy_cols);
+  const PieceWalk of_numbers(MODE == MODE_CHANNEL ? (pieces ? rows / 4 : rows) : 1);
   auto stage_at = [&](int s) { return scan_smem + s * stage_bytes; };
   auto issue = [&](int t0, int s) {
     const int nt = min(tile, row1 - t0);
     T* rs = reinterpret_cast<T*>(stage_at(s));
-    const bool pieces = a.pieces != 0;
-    stage_rows<T>(rs, padded, read + size_t(t0) * a.read_stride, a.read_stride, rows, nt, pieces);
-    stage_rows<T>(rs + tile * padded, padded, write + size_t(t0) * a.write_stride, a.write_stride, rows, nt, pieces);
-    if (copy_cols > 0) stage_rows<T>(rs + 2 * tile * padded, cvp, value + size_t(t0) * a.value_stride, a.value_stride, copy_cols, nt, pieces);
+    stage_rows<T>(rs, padded, read + size_t(t0) * a.read_stride, a.read_stride, of_vectors, nt, pieces);
+    stage_rows<T>(rs + tile * padded, padded, write + size_t(t0) * a.write_stride, a.write_stride, of_vectors, nt, pieces);
+    if (copy_cols > 0) stage_rows<T>(rs + 2 * tile * padded, cvp, value + size_t(t0) * a.value_stride, a.value_stride, of_values, nt, pieces);
     float* fs = reinterpret_cast<float*>(rs + tile * (2 * padded + cvp));
     if (MODE == MODE_CHANNEL) {
-      stage_rows<float>(fs, padded, a.decay + size_t(t0) * a.decay_stride + size_t(h) * rows, a.decay_stride, rows, nt, pieces);
+      stage_rows<float>(fs, padded, a.decay + size_t(t0) * a.decay_stride + size_t(h) * rows, a.decay_stride, of_numbers, nt, pieces);
     } else {
-      stage_rows<float>(fs, 4, reinterpret_cast<const float*>(a.row_numbers + size_t(t0) * gridDim.y + h), 4 * (long long)gridDim.y, 4, nt, true);
+      stage_rows<float>(fs, 4, reinterpret_cast<const float*>(a.row_numbers + size_t(t0) * gridDim.y + h), 4 * (long long)gridDim.y, of_numbers, nt, true);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  issue(row0, 0);
+  // (a commit group for every stage, empty past the last row: the wait below counts them)
+#pragma unroll
+  for (int i = 0; i < SCAN_STAGES - 1; ++i) {
+    if (row0 + i * tile < row1) issue(row0 + i * tile, i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
 
-  // this thread's rows of its column: pieces of four, piece r4 starts at row (r4 * G + g) * 4
-  float S[RPT];
+  // this thread's rows of its column, in twos: pieces of four, piece r4 starts at row (r4 * G + g) * 4
+  uint64_t S[RPT / 2];
   const int n_pieces = (rows + 3) >> 2;
 #pragma unroll
   for (int r4 = 0; r4 < Q; ++r4) {
     const int piece = r4 * G + g;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (!is_fresh && piece < n_pieces && j < cols) v = load4(head_state + (size_t(piece) * cols + j) * 4);
-    S[r4 * 4] = v.x; S[r4 * 4 + 1] = v.y; S[r4 * 4 + 2] = v.z; S[r4 * 4 + 3] = v.w;
+    S[r4 * 2] = pair_of(v.x, v.y);
+    S[r4 * 2 + 1] = pair_of(v.z, v.w);
   }
-  float bonus[MODE == MODE_CHANNEL ? RPT : 1];
+  uint64_t bonus[MODE == MODE_CHANNEL ? RPT / 2 : 1];
   if (MODE == MODE_CHANNEL) {
 #pragma unroll
-    for (int r = 0; r < RPT; ++r) {
+    for (int r = 0; r < RPT; r += 2) {
       const int i = ((r >> 2) * G + g) * 4 + (r & 3);
-      bonus[r] = i < rows ? a.bonus[size_t(h) * rows + i] : 0.f;
+      bonus[r / 2] = pair_of(i < rows ? a.bonus[size_t(h) * rows + i] : 0.f, i + 1 < rows ? a.bonus[size_t(h) * rows + i + 1] : 0.f);
     }
   }
   float* out = a.out + size_t(h) * cols + j;
-  const bool writes = g == 0 && j < cols;
+  // four rows' sums at a time where a column has four lanes or more: which of the rows this lane's sum is, and whether it stores it
+  const int row_of_four = ((g & (G >> 1)) ? 2 : 0) + ((g & (G >> 2)) ? 1 : 0);
+  const bool writes = g == 0 && j < cols, writes_four = G >= 4 && (g & ((G >> 2) - 1)) == 0 && j < cols;
 
-  int s = 0;
-  for (int t0 = row0; t0 < row1; t0 += tile, s ^= 1) {
+  int s = 0, s_next = SCAN_STAGES - 1;
+  for (int t0 = row0; t0 < row1; t0 += tile) {
     const int nt = min(tile, row1 - t0);
-    if (t0 + tile < row1) {
-      issue(t0 + tile, s ^ 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
+    asm volatile("cp.async.wait_group %0;" ::"n"(SCAN_STAGES - 2) : "memory");
+    __syncthreads();  // the tile is there, and nobody reads the one before it any more
+    if (t0 + (SCAN_STAGES - 1) * tile < row1) issue(t0 + (SCAN_STAGES - 1) * tile, s_next);
+    asm volatile("cp.async.commit_group;" ::: "memory");
     const T* rs = reinterpret_cast<const T*>(stage_at(s));
     const T* ws = rs + tile * padded;
     const T* vs = rs + 2 * tile * padded;
     const float* fs = reinterpret_cast<const float*>(rs + tile * (2 * padded + cvp));
+    s = s + 1 == SCAN_STAGES ? 0 : s + 1;
+    s_next = s_next + 1 == SCAN_STAGES ? 0 : s_next + 1;
     if (MODE == MODE_DELTA) {
       // the next row's vectors are fetched before this row's sums are waited for
-      float4 k4[Q], q4[Q], kn[Q], qn[Q], num = load4(fs), num_n = num;
-      float v = to_float(vs[jl]), v_n = v;
-#pragma unroll
-      for (int r4 = 0; r4 < Q; ++r4) {
-        k4[r4] = load4(ws + (r4 * G + g) * 4);
-        q4[r4] = load4(rs + (r4 * G + g) * 4);
-      }
-#pragma unroll 2
-      for (int tt = 0; tt < nt; ++tt) {
-        const int next = tt + 1 < nt ? tt + 1 : tt;
-        num_n = load4(fs + next * 4);
-        v_n = to_float(vs[next * cvp + jl]);
+      struct RowData { uint64_t k[RPT / 2], q[RPT / 2]; float4 num; float v; };
+      auto fetch = [&](int tt, RowData& d) {
+        d.num = load4(fs + tt * 4);
+        d.v = to_float(vs[tt * cvp + jl]);
 #pragma unroll
         for (int r4 = 0; r4 < Q; ++r4) {
-          kn[r4] = load4(ws + next * padded + (r4 * G + g) * 4);
-          qn[r4] = load4(rs + next * padded + (r4 * G + g) * 4);
+          const float4 k4 = load4(ws + tt * padded + (r4 * G + g) * 4), q4 = load4(rs + tt * padded + (r4 * G + g) * 4);
+          d.k[r4 * 2] = pair_of(k4.x, k4.y);
+          d.k[r4 * 2 + 1] = pair_of(k4.z, k4.w);
+          d.q[r4 * 2] = pair_of(q4.x, q4.y);
+          d.q[r4 * 2 + 1] = pair_of(q4.z, q4.w);
         }
-        float ak[4] = {0.f, 0.f, 0.f, 0.f}, aq[4] = {0.f, 0.f, 0.f, 0.f};
+      };
+      // a row: the write u and this lane's share of S'^T q. The chain of rows is the decay, the sum for the key with its shuffles, u
+      // and the write; the sum for the query is nobody's wait.
+      auto walk = [&](const RowData& d, float& sq) {
+        const uint64_t decay = pair_of(d.num.x, d.num.x);
+        uint64_t ak[2] = {0ull, 0ull}, aq[2] = {0ull, 0ull};
 #pragma unroll
-        for (int r4 = 0; r4 < Q; ++r4) {
-          const float k[4] = {k4[r4].x, k4[r4].y, k4[r4].z, k4[r4].w}, q[4] = {q4[r4].x, q4[r4].y, q4[r4].z, q4[r4].w};
+        for (int r = 0; r < RPT / 2; ++r) {
+          S[r] = mul_pair(S[r], decay);
+          ak[r & 1] = fma_pair(S[r], d.k[r], ak[r & 1]);
+        }
+        const float2 k01 = both(ak[0]), k23 = both(ak[1]);
+        float sk = (k01.x + k01.y) + (k23.x + k23.y);
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            S[r4 * 4 + u] *= num.x;
-            ak[u] = fmaf(S[r4 * 4 + u], k[u], ak[u]);
-            aq[u] = fmaf(S[r4 * 4 + u], q[u], aq[u]);
+        for (int r = 0; r < RPT / 2; ++r) aq[r & 1] = fma_pair(S[r], d.q[r], aq[r & 1]);
+#pragma unroll
+        for (int o = G >> 1; o > 0; o >>= 1) sk += __shfl_xor_sync(0xffffffffu, sk, o);
+        const float2 q01 = both(aq[0]), q23 = both(aq[1]);
+        sq = (q01.x + q01.y) + (q23.x + q23.y);
+        const float u_row = d.num.y * (d.v - sk);
+        const uint64_t u2 = pair_of(u_row, u_row);
+#pragma unroll
+        for (int r = 0; r < RPT / 2; ++r) S[r] = fma_pair(u2, d.k[r], S[r]);
+        return u_row;
+      };
+      RowData d[2];
+      fetch(0, d[0]);
+      int tt = 0;
+      if (G >= 4) {
+        for (; tt + 4 <= nt; tt += 4) {
+          float sq[4], u_mine = 0.f, z_mine = 0.f;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            fetch(min(tt + i + 1, nt - 1), d[(i + 1) & 1]);
+            const float u_row = walk(d[i & 1], sq[i]);
+            if (row_of_four == i) {
+              u_mine = u_row;
+              z_mine = d[i & 1].num.z;
+            }
           }
+          const float y = sums_of_four(sq[0], sq[1], sq[2], sq[3], g, G);
+          if (writes_four) out[size_t(t0 + tt + row_of_four) * a.out_stride] = fmaf(z_mine, u_mine, y);
         }
-        float sk = (ak[0] + ak[1]) + (ak[2] + ak[3]), sq = (aq[0] + aq[1]) + (aq[2] + aq[3]);
-#pragma unroll
-        for (int o = G >> 1; o > 0; o >>= 1) {
-          sk += __shfl_xor_sync(0xffffffffu, sk, o);
-          sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        }
-        const float u_row = num.y * (v - sk);
-        if (writes) out[size_t(t0 + tt) * a.out_stride] = fmaf(num.z, u_row, sq);
-#pragma unroll
-        for (int r4 = 0; r4 < Q; ++r4) {
-          const float k[4] = {k4[r4].x, k4[r4].y, k4[r4].z, k4[r4].w};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) S[r4 * 4 + u] = fmaf(u_row, k[u], S[r4 * 4 + u]);
-          k4[r4] = kn[r4];
-          q4[r4] = qn[r4];
-        }
-        num = num_n;
-        v = v_n;
+      }
+      for (; tt < nt; ++tt) {
+        fetch(min(tt + 1, nt - 1), d[1]);
+        float sq;
+        const float u_row = walk(d[0], sq);
+        for (int o = G >> 1; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if (writes) out[size_t(t0 + tt) * a.out_stride] = fmaf(d[0].num.z, u_row, sq);
+        d[0] = d[1];
       }
     } else {
       auto one_row = [&](int tt) {   // -> this lane's share of the row's output
         const float v = to_float(vs[tt * cvp + jl]);
-        float acc[2] = {0.f, 0.f}, own[2] = {0.f, 0.f};
+        const uint64_t v2 = pair_of(v, v);
+        uint64_t acc = 0ull, own = 0ull;
 #pragma unroll
         for (int r4 = 0; r4 < Q; ++r4) {
           const int at = tt * padded + (r4 * G + g) * 4;
           const float4 q4 = load4(rs + at), k4 = load4(ws + at), w4 = load4(fs + at);
-          const float q[4] = {q4.x, q4.y, q4.z, q4.w}, k[4] = {k4.x, k4.y, k4.z, k4.w}, w[4] = {w4.x, w4.y, w4.z, w4.w};
+          const uint64_t q[2] = {pair_of(q4.x, q4.y), pair_of(q4.z, q4.w)}, k[2] = {pair_of(k4.x, k4.y), pair_of(k4.z, k4.w)};
+          const uint64_t w[2] = {pair_of(w4.x, w4.y), pair_of(w4.z, w4.w)};
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int r = r4 * 4 + u;
-            acc[u & 1] = fmaf(S[r], q[u], acc[u & 1]);            // the state before this row's write
-            own[u & 1] = fmaf(bonus[r] * k[u], q[u], own[u & 1]); // the row's own write, times its bonus
-            S[r] = fmaf(w[u], S[r], k[u] * v);
+          for (int u = 0; u < 2; ++u) {
+            const int r = r4 * 2 + u;
+            acc = fma_pair(S[r], q[u], acc);                          // the state before this row's write
+            own = fma_pair(mul_pair(bonus[r], k[u]), q[u], own);      // the row's own write, times its bonus
+            S[r] = fma_pair(w[u], S[r], mul_pair(k[u], v2));
           }
         }
-        return fmaf(own[0] + own[1], v, acc[0] + acc[1]);
+        const float2 a2 = both(acc), o2 = both(own);
+        return fmaf(o2.x + o2.y, v, a2.x + a2.y);
       };
       int tt = 0;
-      for (; tt + 4 <= nt; tt += 4) {   // four rows' sums over the lanes at a time: their shuffles overlap
-        float y[4];
+      if (G >= 4) {
+        for (; tt + 4 <= nt; tt += 4) {
+          float y[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) y[i] = one_row(tt + i);
-#pragma unroll
-        for (int o = G >> 1; o > 0; o >>= 1) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) y[i] += __shfl_xor_sync(0xffffffffu, y[i], o);
-        }
-        if (writes) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) out[size_t(t0 + tt + i) * a.out_stride] = y[i];
+          for (int i = 0; i < 4; ++i) y[i] = one_row(tt + i);
+          const float sum = sums_of_four(y[0], y[1], y[2], y[3], g, G);
+          if (writes_four) out[size_t(t0 + tt + row_of_four) * a.out_stride] = sum;
         }
       }
       for (; tt < nt; ++tt) {
@@ -259,13 +270,12 @@ state_scan_kernel(const StateScanArgs a) {
         if (writes) out[size_t(t0 + tt) * a.out_stride] = y;
       }
     }
-    __syncthreads();  // the stage may be filled again
   }
 #pragma unroll
   for (int r4 = 0; r4 < Q; ++r4) {
     const int piece = r4 * G + g;
-    if (piece < n_pieces && j < cols)
-      *reinterpret_cast<float4*>(head_state + (size_t(piece) * cols + j) * 4) = make_float4(S[r4 * 4], S[r4 * 4 + 1], S[r4 * 4 + 2], S[r4 * 4 + 3]);
+    const float2 lo = both(S[r4 * 2]), hi = both(S[r4 * 2 + 1]);
+    if (piece < n_pieces && j < cols) *reinterpret_cast<float4*>(head_state + (size_t(piece) * cols + j) * 4) = make_float4(lo.x, lo.y, hi.x, hi.y);
   }
 }
 
@@ -391,14 +401,15 @@ int launch_state_scan(const StateScanArgs& in, int n_entries, int n_heads, int s
     const int unit = splits == 1 ? per_warp : granule, want = (a.cols + splits - 1) / splits;
     a.cv = (want + unit - 1) / unit * unit;
     const long long ctas = (long long)n_entries * n_heads * ((a.cols + a.cv - 1) / a.cv);
-    if (a.cv * a.G <= 256 && (ctas >= n_sms || a.cv <= granule)) break;
+    if (a.cv * a.G <= 256 && a.cv <= granule) break;
+    if (a.cv * a.G <= (single_rows ? 256 : SCAN_THREADS) && ctas >= n_sms) break;
     if (splits > a.cols) return R2_UNSUPPORTED;
   }
   splits = (a.cols + a.cv - 1) / a.cv;
   const int threads = a.cv * a.G;
   const int padded = rpt * a.G, cvp = (a.cv + 7) & ~7;
   const size_t per_row = size_t(2 * padded + cvp) * sizeof(T) + size_t(MODE == MODE_CHANNEL ? padded : 4) * 4;
-  int tile = 32;
+  int tile = SCAN_TILE;
   while (tile > 1 && SCAN_STAGES * tile * per_row > 100 * 1024) tile /= 2;
   a.tile = tile;
   const size_t smem = SCAN_STAGES * tile * per_row;
