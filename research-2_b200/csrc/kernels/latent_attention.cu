@@ -214,13 +214,16 @@ struct HeadLinearParams {
   const bf16* gate; int gate_stride, gate_vec;   // may be null: outputs times sigmoid(gate), laid out like out (4-byte loads possible)
 };
 
+// WHOLE: both operands' rows are whole 16-byte pieces on their boundaries (the path that loads single numbers, unrolled beside the other,
+// took the registers that keep the loads in flight); GATED: there is a gate.
+template <bool WHOLE, bool GATED>
 __global__ void __launch_bounds__(128)
 head_linear_mma_kernel(const HeadLinearParams p) {
   using namespace r2ptx;
   pdl_launch_dependents();
-  pdl_wait();
   __shared__ __align__(16) bf16 a_s[HM_TILE][HM_PAD];
   __shared__ __align__(16) bf16 w_s[HM_TILE][HM_PAD];
+  __shared__ __align__(8) float gate_s[GATED ? HM_TILE : 1][HM_TILE + 2];   // sigmoid(gate)
   const int h = blockIdx.z, r0 = blockIdx.x * HM_TILE, c0 = blockIdx.y * HM_TILE;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bf16* ah = p.a + size_t(h) * p.a_head;
@@ -230,19 +233,75 @@ head_linear_mma_kernel(const HeadLinearParams p) {
 #pragma unroll
   for (int i = 0; i < HM_TILE / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   const bool warp_has_rows = r0 + warp * 16 < p.n_rows;
+  auto piece = [&](const bf16* row, int c, int len, bool vec) {
+    if constexpr (WHOLE) return c * 8 < len ? *reinterpret_cast<const uint4*>(row + c * 8) : zero4;
+    else return eight_of(row, c, len, vec);
+  };
+  // A few rows' time is the chain of their loads: the head's matrix (no kernel's output) is asked for before the wait on the kernel
+  // before this one, the gates before the products, and a piece of K while the one before it is multiplied.
+  constexpr int PIECES = HM_TILE * (HM_TILE / 8) / 128;   // of a thread: four of either operand
+  uint4 av[PIECES], wv[PIECES];
+  auto load_w = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+      const int idx = tid + 128 * i, r = idx / (HM_TILE / 8), c = idx % (HM_TILE / 8);
+      wv[i] = zero4;
+      if (p.w_is_nk) {   // r: a column of the output, its K numbers lie side by side
+        if (c0 + r < p.n_total && k0 < p.k_total) wv[i] = piece(wh + size_t(c0 + r) * p.k_total + k0, c, p.k_total - k0, p.w_vec != 0);
+      } else {           // r: one of the K, the output's columns lie side by side
+        if (k0 + r < p.k_total) wv[i] = piece(wh + size_t(k0 + r) * p.n_total + c0, c, p.n_total - c0, p.w_vec != 0);
+      }
+    }
+  };
+  auto load_a = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+      const int idx = tid + 128 * i, r = idx / (HM_TILE / 8), c = idx % (HM_TILE / 8);
+      av[i] = zero4;
+      if (r0 + r < p.n_rows && k0 < p.k_total) av[i] = piece(ah + size_t(r0 + r) * p.a_stride + k0, c, p.k_total - k0, p.a_vec != 0);
+    }
+  };
+  load_w(0);
+  pdl_wait();
+  load_a(0);
+  const int g = lane >> 2, tq = lane & 3;
+  // The gates: whole rows by all four warps, whatever the number of rows, and their sigmoids through shared memory (12 rows of 128 -> 64 in
+  // 12 heads: 7.8 us with a lane's own 32 at the end of the one warp that has rows, 5.7 now, 2.3 without gates).
+  constexpr int PAIRS = HM_TILE * HM_TILE / 2 / 128;   // of a thread
+  uint32_t gates[PAIRS];
+  if constexpr (GATED) {
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) {
+      const int idx = tid + 128 * i, r = r0 + idx / (HM_TILE / 2), n = c0 + 2 * (idx % (HM_TILE / 2));
+      gates[i] = 0u;
+      if (r < p.n_rows && n < p.n_total) {
+        const bf16* gr = p.gate + size_t(r) * p.gate_stride + size_t(h) * p.out_head + n;
+        if (p.gate_vec && n + 1 < p.n_total) gates[i] = *reinterpret_cast<const uint32_t*>(gr);
+        else gates[i] = uint32_t(__bfloat16_as_ushort(gr[0])) | (n + 1 < p.n_total ? uint32_t(__bfloat16_as_ushort(gr[1])) << 16 : 0u);
+      }
+    }
+  }
   for (int k0 = 0; k0 < p.k_total; k0 += HM_TILE) {
     __syncthreads();
-    for (int idx = tid; idx < HM_TILE * (HM_TILE / 8); idx += 128) {
-      const int r = idx / (HM_TILE / 8), c = idx % (HM_TILE / 8);
-      uint4 av = zero4, wv = zero4;
-      if (r0 + r < p.n_rows) av = eight_of(ah + size_t(r0 + r) * p.a_stride + k0, c, p.k_total - k0, p.a_vec != 0);
-      if (p.w_is_nk) {   // r: a column of the output, its K numbers lie side by side
-        if (c0 + r < p.n_total) wv = eight_of(wh + size_t(c0 + r) * p.k_total + k0, c, p.k_total - k0, p.w_vec != 0);
-      } else {           // r: one of the K, the output's columns lie side by side
-        if (k0 + r < p.k_total) wv = eight_of(wh + size_t(k0 + r) * p.n_total + c0, c, p.n_total - c0, p.w_vec != 0);
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+      const int idx = tid + 128 * i, r = idx / (HM_TILE / 8), c = idx % (HM_TILE / 8);
+      *reinterpret_cast<uint4*>(&a_s[r][c * 8]) = av[i];
+      *reinterpret_cast<uint4*>(&w_s[r][c * 8]) = wv[i];
+    }
+    if (k0 + HM_TILE < p.k_total) {
+      load_w(k0 + HM_TILE);
+      load_a(k0 + HM_TILE);
+    }
+    if (GATED && k0 == 0) {
+#pragma unroll
+      for (int i = 0; i < PAIRS; ++i) {
+        const int idx = tid + 128 * i, r = idx / (HM_TILE / 2), n = 2 * (idx % (HM_TILE / 2));
+        if (r0 + r < p.n_rows) {
+          const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gates[i]));
+          *reinterpret_cast<float2*>(&gate_s[r][n]) = make_float2(1.f / (1.f + __expf(-z.x)), 1.f / (1.f + __expf(-z.y)));
+        }
       }
-      *reinterpret_cast<uint4*>(&a_s[r][c * 8]) = av;
-      *reinterpret_cast<uint4*>(&w_s[r][c * 8]) = wv;
     }
     __syncthreads();
     if (!warp_has_rows) continue;
@@ -260,26 +319,19 @@ head_linear_mma_kernel(const HeadLinearParams p) {
       }
     }
   }
-  const int g = lane >> 2, tq = lane & 3;
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int r = r0 + warp * 16 + g + 8 * half;
     if (r >= p.n_rows) continue;
     bf16* dst = p.out + size_t(r) * p.out_stride + size_t(h) * p.out_head;
-    const bf16* gr = p.gate != nullptr ? p.gate + size_t(r) * p.gate_stride + size_t(h) * p.out_head : nullptr;
 #pragma unroll
     for (int nt = 0; nt < HM_TILE / 8; ++nt) {
       const int n = c0 + nt * 8 + 2 * tq;
       float y0 = acc[nt][2 * half], y1 = acc[nt][2 * half + 1];
-      if (gr != nullptr) {
-        if (p.gate_vec && n + 1 < p.n_total) {
-          const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(gr + n));
-          y0 *= 1.f / (1.f + __expf(-z.x));
-          y1 *= 1.f / (1.f + __expf(-z.y));
-        } else {
-          if (n < p.n_total) y0 *= 1.f / (1.f + __expf(-to_float(gr[n])));
-          if (n + 1 < p.n_total) y1 *= 1.f / (1.f + __expf(-to_float(gr[n + 1])));
-        }
+      if constexpr (GATED) {
+        const float2 z = *reinterpret_cast<const float2*>(&gate_s[r - r0][n - c0]);
+        y0 *= z.x;
+        y1 *= z.y;
       }
       if (p.out_vec && n + 1 < p.n_total) {
         *reinterpret_cast<__nv_bfloat162*>(dst + n) = __floats2bfloat162_rn(y0, y1);
@@ -583,32 +635,42 @@ latent_attention_kernel(const LatentAttnParams p) {
 }
 
 // A decode step's slices of one (token, head) meet: out = sum_s y_s 2^(top_s - top) / (sum_s l_s 2^(top_s - top) + the sink's term).
-// One CTA per (token, head); the slices are added in their order.
+// One CTA per (token, head); the slices are added in their order. The slices' maxima and sums are read once, side by side, and a thread
+// has eight slices' numbers in flight (16 slices of 128 numbers, 12 tokens x 12 heads: 12.3 us with one slice after the other, 5.1 now).
+constexpr int MAX_SLICES = 128;
 __global__ void __launch_bounds__(128)
 latent_merge_kernel(const float* __restrict__ parts, int n_slices, int kv_rank, int n_heads, const float* __restrict__ sinks,
                     bf16* __restrict__ out, int out_stride) {
   pdl_launch_dependents();
+  __shared__ float tops[MAX_SLICES], sums[MAX_SLICES];
+  const int e = blockIdx.x / n_heads, h = blockIdx.x - e * n_heads, len = kv_rank + 2;
+  const float sink = sinks != nullptr ? sinks[h] * 1.4426950408889634f : -INFINITY;
   pdl_wait();
-  const int e = blockIdx.x / n_heads, h = blockIdx.x - e * n_heads;
-  const float* mine = parts + size_t(blockIdx.x) * n_slices * (kv_rank + 2);
-  float top = -INFINITY;
-  for (int s = 0; s < n_slices; ++s) top = fmaxf(top, mine[s * (kv_rank + 2) + kv_rank]);
-  float sum = 0.f;
-  if (top != -INFINITY) {
-    for (int s = 0; s < n_slices; ++s) {
-      const float t = mine[s * (kv_rank + 2) + kv_rank];
-      if (t != -INFINITY) sum += mine[s * (kv_rank + 2) + kv_rank + 1] * exp2f(t - top);
-    }
-    if (sinks != nullptr) sum += exp2f(sinks[h] * 1.4426950408889634f - top);
+  const float* mine = parts + size_t(blockIdx.x) * n_slices * len;
+  if (threadIdx.x < n_slices) {
+    tops[threadIdx.x] = mine[size_t(threadIdx.x) * len + kv_rank];
+    sums[threadIdx.x] = mine[size_t(threadIdx.x) * len + kv_rank + 1];
   }
-  const float inv = sum > 0.f ? 1.f / sum : 0.f;
+  __syncthreads();
+  float top = -INFINITY;
+  for (int s = 0; s < n_slices; ++s) top = fmaxf(top, tops[s]);
+  __syncthreads();
+  if (threadIdx.x < n_slices) tops[threadIdx.x] = tops[threadIdx.x] != -INFINITY ? exp2f(tops[threadIdx.x] - top) : -1.f;   // from here on: shares, -1 for an empty slice
+  __syncthreads();
+  float sum = 0.f;
+  for (int s = 0; s < n_slices; ++s)
+    if (tops[s] != -1.f) sum += sums[s] * tops[s];
+  if (top != -INFINITY && sinks != nullptr) sum += exp2f(sink - top);
+  const float inv = top != -INFINITY && sum > 0.f ? 1.f / sum : 0.f;
   for (int d = threadIdx.x; d < kv_rank; d += blockDim.x) {
     float y = 0.f;
-    if (top != -INFINITY) {
-      for (int s = 0; s < n_slices; ++s) {
-        const float t = mine[s * (kv_rank + 2) + kv_rank];
-        if (t != -INFINITY) y += mine[s * (kv_rank + 2) + d] * exp2f(t - top);
-      }
+    for (int s0 = 0; s0 < n_slices; s0 += 8) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = s0 + u < n_slices && tops[s0 + u] != -1.f ? mine[size_t(s0 + u) * len + d] : 0.f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (s0 + u < n_slices && tops[s0 + u] != -1.f) y += v[u] * tops[s0 + u];
     }
     out[size_t(e) * out_stride + size_t(h) * kv_rank + d] = from_float<bf16>(y * inv);
   }
@@ -672,8 +734,11 @@ extern "C" int r2_head_linear(const void* a, int a_stride, int a_head, const voi
     p.a_vec = (uintptr_t(a) % 16 == 0 && a_stride % 8 == 0 && a_head % 8 == 0) ? 1 : 0;
     p.w_vec = (uintptr_t(w) % 16 == 0 && (w_is_nk ? k : n) % 8 == 0 && (size_t(k) * n) % 8 == 0) ? 1 : 0;
     p.out_vec = (uintptr_t(out) % 4 == 0 && out_stride % 2 == 0 && out_head % 2 == 0) ? 1 : 0;
-    r2_launch(head_linear_mma_kernel, dim3((n_rows + HM_TILE - 1) / HM_TILE, (n + HM_TILE - 1) / HM_TILE, n_heads), dim3(128), size_t(0),
-              stream, p);
+    const dim3 tiles((n_rows + HM_TILE - 1) / HM_TILE, (n + HM_TILE - 1) / HM_TILE, n_heads);
+    const bool whole = p.a_vec && p.w_vec && k % 8 == 0 && (w_is_nk || n % 8 == 0);
+    auto kernel = whole ? (gate != nullptr ? head_linear_mma_kernel<true, true> : head_linear_mma_kernel<true, false>)
+                        : (gate != nullptr ? head_linear_mma_kernel<false, true> : head_linear_mma_kernel<false, false>);
+    r2_launch(kernel, tiles, dim3(128), size_t(0), stream, p);
   } else {
     return R2_BAD_DTYPE;
   }
@@ -738,6 +803,7 @@ extern "C" int r2_latent_attention(const void* q, int q_stride, void* out, int o
   p.scale = scale; p.window = window; p.split_p = split_p; p.sinks = sinks;
   // a decode step's tokens may have their key tiles cut over several CTAs, which leave partial sums for a merge kernel
   if (!single_rows || n_slices < 2 || parts == nullptr || (long long)n_entries * n_heads * n_slices * (kv_rank + 2) > parts_floats) n_slices = 1;
+  if (n_slices > MAX_SLICES) n_slices = MAX_SLICES;
   p.n_slices = n_slices; p.parts = parts;
   p.q_vec = (uintptr_t(q) % 16 == 0 && q_stride % 8 == 0 && row % 8 == 0) ? 1 : 0;
   p.k_vec = (uintptr_t(cache) % 16 == 0 && page_stride % 8 == 0 && row % 8 == 0) ? 1 : 0;

@@ -48,6 +48,23 @@ def test_router_logits_beyond_what_is_asked_for_ahead(width):
     assert torch.equal(dense.gather(1, chosen.long()), weight)
 
 
+# one, two and three pieces of K; rows around a warp's 16 and the tile's 64; gates read in pairs or one by one
+@pytest.mark.parametrize("rows,k,n,offset", [(1, 64, 64, 0), (12, 128, 64, 0), (65, 136, 72, 0), (17, 128, 70, 1)])
+@pytest.mark.parametrize("w_is_nk", [False, True])
+def test_gated_products_per_head(rows, k, n, offset, w_is_nk):
+    o, heads = ops(), 3
+    gen = torch.Generator(device=DEV).manual_seed(rows + k)
+    a = torch.randn(rows, heads * k, generator=gen, device=DEV).bfloat16()
+    w = (torch.randn(heads * (n if w_is_nk else k), k if w_is_nk else n, generator=gen, device=DEV) * k ** -0.5).bfloat16()
+    gate = torch.randn(rows, heads * n + offset, generator=gen, device=DEV).bfloat16()[:, offset:]
+    out = torch.empty(rows, heads * n, dtype=torch.bfloat16, device=DEV)
+    o.head_linear(a, k, w, w_is_nk, out, n, heads, k, n, gate=gate)
+    wide = w.double().view(heads, -1, w.shape[1])
+    want = torch.einsum("thk,hkn->thn", a.double().view(rows, heads, k), wide.transpose(1, 2) if w_is_nk else wide).reshape(rows, -1)
+    want = want * torch.sigmoid(gate.double())
+    torch.testing.assert_close(out.double(), want, atol=2.0 ** -8, rtol=2.0 ** -8)
+
+
 # slices that are a cluster (up to eight) and more of them than that; contexts from one key to several tiles a warp
 @pytest.mark.parametrize("max_context", [129, 260, 1024, 1030, 4096])
 @pytest.mark.parametrize("window", [0, 40])
