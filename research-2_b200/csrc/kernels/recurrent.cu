@@ -479,40 +479,74 @@ causal_conv_kernel(const T* __restrict__ in, int in_stride, T* __restrict__ out,
 // ---- norm over groups of columns, with a gate ---------------------------------------------------
 // One warp per (row, group). gate_first 1: y <- y * silu(gate), then the group's RMS norm, times weight.
 // 0: the group's RMS norm, times weight, times sigmoid(gate). 2: the group's RMS norm, times weight, times silu(gate).
-// weight may be null: a gain of one.
+// weight may be null: a gain of one. A few rows' time is a chain of round trips, so a thread's first NORM_HELD columns stay in
+// registers: gains before the wait on the kernel before this one (weights are no kernel's output), values and gates at once;
+// what lies beyond is read twice.
+constexpr int NORM_HELD = 4;
+
+// what a column adds to the sum and what it is multiplied by besides the norm and the gain
+template <typename T>
+__device__ __forceinline__ void gated_value(float v, const T gate, int gate_first, float& value, float& factor) {
+  const float z = to_float(gate);
+  value = v;
+  factor = 1.f;
+  if (gate_first == 1) value = v * (z / (1.f + expf(-z)));
+  else factor = (gate_first == 2 ? z : 1.f) / (1.f + expf(-z));
+}
+
+// A group's columns by `threads` threads, this one the `me`-th; `sum` adds their shares up.
+template <typename T, typename F>
+__device__ __forceinline__ void norm_group(const float* yr, const T* gr, const float* wr, T* o, int group_size, float eps, int gate_first, int me, int threads, F sum) {
+  float value[NORM_HELD], factor[NORM_HELD], gain[NORM_HELD];
+#pragma unroll
+  for (int i = 0; i < NORM_HELD; ++i) gain[i] = wr != nullptr && me + i * threads < group_size ? wr[me + i * threads] : 1.f;
+  pdl_wait();
+  T gate[NORM_HELD];
+#pragma unroll
+  for (int i = 0; i < NORM_HELD; ++i) {
+    const int d = me + i * threads;
+    value[i] = d < group_size ? yr[d] : 0.f;
+    gate[i] = d < group_size ? gr[d] : from_float<T>(0.f);
+  }
+  float sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < NORM_HELD; ++i) {
+    gated_value(value[i], gate[i], gate_first, value[i], factor[i]);
+    if (me + i * threads < group_size) sq = fmaf(value[i], value[i], sq);
+  }
+  for (int d = me + NORM_HELD * threads; d < group_size; d += threads) {
+    float v, f;
+    gated_value(yr[d], gr[d], gate_first, v, f);
+    sq = fmaf(v, v, sq);
+  }
+  const float inv = 1.f / sqrtf(sum(sq) / float(group_size) + eps);
+  auto result = [&](float v, float f, float w) { return from_float<T>(gate_first == 1 ? v * inv * w : v * inv * w * f); };
+#pragma unroll
+  for (int i = 0; i < NORM_HELD; ++i)
+    if (me + i * threads < group_size) o[me + i * threads] = result(value[i], factor[i], gain[i]);
+  for (int d = me + NORM_HELD * threads; d < group_size; d += threads) {
+    float v, f;
+    gated_value(yr[d], gr[d], gate_first, v, f);
+    o[d] = result(v, f, wr != nullptr ? wr[d] : 1.f);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128)
 group_norm_gated_kernel(const float* __restrict__ y, int y_stride, const T* __restrict__ gate, int gate_stride,
                         const float* __restrict__ weight, T* __restrict__ out, int out_stride, int n_rows, int n_groups,
                         int group_size, float eps, int gate_first) {
   pdl_launch_dependents();
-  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long unit = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (unit >= (long long)n_rows * n_groups) return;
+  if (unit >= (long long)n_rows * n_groups) {
+    pdl_wait();
+    return;
+  }
   const int t = int(unit / n_groups), grp = int(unit % n_groups);
-  const float* yr = y + size_t(t) * y_stride + size_t(grp) * group_size;
-  const T* gr = gate + size_t(t) * gate_stride + size_t(grp) * group_size;
-  const float* wr = weight + size_t(grp) * group_size;
-  T* o = out + size_t(t) * out_stride + size_t(grp) * group_size;
-  float sq = 0.f;
-  for (int d = lane; d < group_size; d += 32) {
-    float v = yr[d];
-    if (gate_first == 1) {
-      const float z = to_float(gr[d]);
-      v *= z / (1.f + expf(-z));
-    }
-    sq = fmaf(v, v, sq);
-  }
-  const float inv = 1.f / sqrtf(warp_sum(sq) / float(group_size) + eps);
-  for (int d = lane; d < group_size; d += 32) {
-    float v = yr[d];
-    const float z = to_float(gr[d]);
-    const float gain = weight != nullptr ? wr[d] : 1.f;
-    if (gate_first == 1) v = v * (z / (1.f + expf(-z))) * inv * gain;
-    else v = v * inv * gain * ((gate_first == 2 ? z : 1.f) / (1.f + expf(-z)));
-    o[d] = from_float<T>(v);
-  }
+  norm_group(y + size_t(t) * y_stride + size_t(grp) * group_size, gate + size_t(t) * gate_stride + size_t(grp) * group_size,
+             weight != nullptr ? weight + size_t(grp) * group_size : nullptr, out + size_t(t) * out_stride + size_t(grp) * group_size, group_size, eps,
+             gate_first, lane, 32, [](float x) { return warp_sum(x); });
 }
 
 // The same with a CTA per (row, group), for groups of many columns.
@@ -522,31 +556,11 @@ group_norm_gated_block_kernel(const float* __restrict__ y, int y_stride, const T
                               const float* __restrict__ weight, T* __restrict__ out, int out_stride, int n_groups,
                               int group_size, float eps, int gate_first) {
   pdl_launch_dependents();
-  pdl_wait();
   __shared__ float scratch[33];
   const int t = blockIdx.x / n_groups, grp = blockIdx.x % n_groups;
-  const float* yr = y + size_t(t) * y_stride + size_t(grp) * group_size;
-  const T* gr = gate + size_t(t) * gate_stride + size_t(grp) * group_size;
-  const float* wr = weight + size_t(grp) * group_size;
-  T* o = out + size_t(t) * out_stride + size_t(grp) * group_size;
-  float sq = 0.f;
-  for (int d = threadIdx.x; d < group_size; d += blockDim.x) {
-    float v = yr[d];
-    if (gate_first == 1) {
-      const float z = to_float(gr[d]);
-      v *= z / (1.f + expf(-z));
-    }
-    sq = fmaf(v, v, sq);
-  }
-  const float inv = 1.f / sqrtf(block_sum(sq, scratch) / float(group_size) + eps);
-  for (int d = threadIdx.x; d < group_size; d += blockDim.x) {
-    float v = yr[d];
-    const float z = to_float(gr[d]);
-    const float gain = weight != nullptr ? wr[d] : 1.f;
-    if (gate_first == 1) v = v * (z / (1.f + expf(-z))) * inv * gain;
-    else v = v * inv * gain * ((gate_first == 2 ? z : 1.f) / (1.f + expf(-z)));
-    o[d] = from_float<T>(v);
-  }
+  norm_group(y + size_t(t) * y_stride + size_t(grp) * group_size, gate + size_t(t) * gate_stride + size_t(grp) * group_size,
+             weight != nullptr ? weight + size_t(grp) * group_size : nullptr, out + size_t(t) * out_stride + size_t(grp) * group_size, group_size, eps,
+             gate_first, int(threadIdx.x), int(blockDim.x), [&](float x) { return block_sum(x, scratch); });
 }
 
 }  // namespace

@@ -75,3 +75,22 @@ def test_slices_of_decode_attention_meet_in_their_cluster(max_context, window):
     one = PagedCase([(c, 1) for c in (0, 31, 128, 500, 1000)], 4, 2, 64, 16, torch.bfloat16, seed=max_context).run_fused(0.125, window, 100).float().cpu()
     # the same rounding of every weight to bfloat16 against another maximum, and the output's own: two roundings of 2^-9
     torch.testing.assert_close(got, one, atol=2.0 ** -7, rtol=2.0 ** -7)
+
+
+# groups inside and beyond the columns that a thread keeps: four of a warp's 32 lanes, four of a CTA's 256 threads
+@pytest.mark.parametrize("rows,groups,size", [(1, 3, 1), (5, 2, 64), (4, 3, 128), (3, 2, 130), (2, 1, 1024), (2, 2, 1030)])
+@pytest.mark.parametrize("order", [True, False, "silu_after"])
+def test_gated_norms_inside_and_beyond_what_is_kept(rows, groups, size, order):
+    o, eps = ops(), 1e-5
+    gen = torch.Generator(device=DEV).manual_seed(size)
+    y = torch.randn(rows, groups * size, generator=gen, device=DEV)
+    gate, w = torch.randn(rows, groups * size, generator=gen, device=DEV).bfloat16(), torch.randn(groups * size, generator=gen, device=DEV)
+    got = o.group_norm_gated(y, gate, w, groups, eps, order, torch.bfloat16)
+    z, v = gate.double(), y.double()
+    if order is True:
+        v = v * torch.nn.functional.silu(z)
+    v = v.view(rows, groups, size)
+    v = (v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + eps)).view(rows, -1) * w.double()
+    if order is not True:
+        v = v * (torch.nn.functional.silu(z) if order == "silu_after" else torch.sigmoid(z))
+    torch.testing.assert_close(got.double(), v, rtol=2.0 ** -8, atol=1e-6)   # one rounding to bfloat16, 2^-9, and float sums before it
