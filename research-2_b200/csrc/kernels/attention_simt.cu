@@ -154,8 +154,10 @@ attention_simt_kernel(const T* __restrict__ q, int q_row_stride, T* __restrict__
       if (bias != nullptr) s += bias[pos - j < bias_len ? pos - j : bias_len - 1];
     }
     const float m_new = fmaxf(m, warp_max(s));
-    const float corr = expf(m - m_new);  // exp(-inf) = 0 on the first tile
-    const float p = valid ? expf(s - m_new) : 0.f;
+    // (a warp whose keys so far all score -inf, a bias that forbids their distance, has nothing to measure by: its weights are 0, not NaN)
+    const float base = m_new == -INFINITY ? 0.f : m_new;
+    const float corr = expf(m - base);  // exp(-inf) = 0 on the first tile
+    const float p = valid ? expf(s - base) : 0.f;
     l = l * corr + warp_sum(p);
     m = m_new;
 #pragma unroll
@@ -194,6 +196,7 @@ attention_simt_kernel(const T* __restrict__ q, int q_row_stride, T* __restrict__
   const int used = n_tiles < WARPS ? n_tiles : WARPS;
   float top = has_sink ? sink_at : -INFINITY;
   for (int w = 0; w < used; ++w) top = fmaxf(top, max_s[w]);
+  if (top == -INFINITY) top = 0.f;   // no key and no sink: every share is 0
   float share[WARPS], total = has_sink ? expf(sink_at - top) : 0.f;
 #pragma unroll
   for (int w = 0; w < WARPS; ++w) {

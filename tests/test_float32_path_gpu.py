@@ -92,3 +92,40 @@ def test_attention_rows_do_not_depend_on_the_batch(head_dim, page, window):
         worst = max(worst, float((whole[i].double() - want).abs().max()))
     # scores up to about 5 carry a relative error of some head_dim / 4 roundings, which is the weights' too; outputs are of size one
     assert worst < 5 * (head_dim / 4 + 40) * 2.0 ** -24 * 4
+
+
+# a bias by distance that forbids all but the nearest keys: whole tiles of 32 keys score -inf, the first ones of most warps among them
+@pytest.mark.parametrize("near", [1, 20, 70])
+@pytest.mark.parametrize("with_sinks", [False, True])
+@pytest.mark.parametrize("dtype,decoded", [(torch.float32, False), (torch.bfloat16, False), (torch.float32, True), (torch.bfloat16, True)])
+def test_tiles_of_forbidden_keys_weigh_nothing(near, with_sinks, dtype, decoded):
+    from tests.test_kernels_gpu import PagedCase
+
+    heads, dim, scale = 4, 64, 0.125
+    entries = [(n - 1, 1) for n in (1, 33, 300, 700)] if decoded else [(0, 300), (250, 90), (0, 1)]
+    case = PagedCase(entries, heads, 2, dim, 16, dtype, seed=near)
+    gen = torch.Generator().manual_seed(near)
+    bias = torch.full((heads, near + 1), float("-inf"))
+    bias[:, :near] = torch.randn(heads, near, generator=gen)
+    sinks = torch.randn(heads, generator=gen) if with_sinks else None
+    want = []
+    for e, (start, rows) in enumerate(entries):
+        k, v = (x[e].double().repeat_interleave(2, dim=1) for x in (case.k_dense, case.v_dense))
+        back = torch.arange(start, start + rows)[:, None] - torch.arange(start + rows)[None]
+        s = torch.einsum("thd,jhd->htj", case.q[e].double(), k) * scale + bias.double()[:, back.clamp(0, near)]
+        s = s.masked_fill(back < 0, float("-inf"))
+        if with_sinks:
+            s = torch.cat([s, sinks.double()[:, None, None].expand(heads, rows, 1)], dim=2)
+        want.append(torch.einsum("htj,jhd->thd", torch.softmax(s, dim=2)[..., : start + rows], v).reshape(rows, -1))
+    want = torch.cat(want)
+    extras = dict(dist_bias=bias.to(DEV), sinks=None if sinks is None else sinks.to(DEV))
+    # float32: scores of size one over 64 numbers, a dozen roundings each; bfloat16: the output's rounding and the weights' (2^-9 each)
+    close = dict(atol=2e-5, rtol=2e-5) if dtype == torch.float32 else dict(atol=1.2e-2, rtol=1.2e-2)
+    o = ops()
+    old = o.use_fast_attention(False)   # the general kernel
+    try:
+        torch.testing.assert_close(case.run(scale, **extras).double().cpu(), want, **close)
+    finally:
+        o.use_fast_attention(old)
+    if dtype == torch.bfloat16:
+        torch.testing.assert_close(case.run(scale, q_start=case.q_start, n_tiles=case.n_tiles, **extras).double().cpu(), want, **close)
