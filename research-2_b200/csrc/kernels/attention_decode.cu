@@ -337,15 +337,17 @@ decode_kernel(const DecodeParams p) {
       mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 2));
       mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 1));
       mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 2));
-      const float m_a = fmaxf(m_run[0], mx_a), m_b = fmaxf(m_run[1], mx_b);  // finite: a tile has a key that is seen
-      const float corr_a = __expf(m_run[0] - m_a), corr_b = __expf(m_run[1] - m_b);
+      const float m_a = fmaxf(m_run[0], mx_a), m_b = fmaxf(m_run[1], mx_b);  // finite: a tile has a key that is seen ...
+      // ... unless a bias by distance forbids them all: such a tile's weights are 0, not NaN
+      const float base_a = X == 2 && m_a == -INFINITY ? 0.f : m_a, base_b = X == 2 && m_b == -INFINITY ? 0.f : m_b;
+      const float corr_a = __expf(m_run[0] - base_a), corr_b = __expf(m_run[1] - base_b);
       float sum_a = 0.f, sum_b = 0.f;
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          sc[nt][c] = __expf(sc[nt][c] - m_a);
-          sc[nt][2 + c] = __expf(sc[nt][2 + c] - m_b);
+          sc[nt][c] = __expf(sc[nt][c] - base_a);
+          sc[nt][2 + c] = __expf(sc[nt][2 + c] - base_b);
           sum_a += sc[nt][c];
           sum_b += sc[nt][2 + c];
         }
@@ -425,8 +427,9 @@ decode_kernel(const DecodeParams p) {
       if (X && p.softcap > 0.f && valid) sv = soft_cap(sv, p.softcap);
       if (X == 2 && p.dist_bias != nullptr && valid) sv += bias_at(g, v0 + lane);
       float m_new = fmaxf(m[g], warp_max(sv));
-      float corr = __expf(m[g] - m_new);
-      pr[g] = valid ? __expf(sv - m_new) : 0.f;
+      const float base = X == 2 && m_new == -INFINITY ? 0.f : m_new;   // (as in the other form)
+      float corr = __expf(m[g] - base);
+      pr[g] = valid ? __expf(sv - base) : 0.f;
       l[g] = l[g] * corr + warp_sum(pr[g]);
       m[g] = m_new;
 #pragma unroll

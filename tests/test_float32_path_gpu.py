@@ -129,3 +129,7 @@ def test_tiles_of_forbidden_keys_weigh_nothing(near, with_sinks, dtype, decoded)
         o.use_fast_attention(old)
     if dtype == torch.bfloat16:
         torch.testing.assert_close(case.run(scale, q_start=case.q_start, n_tiles=case.n_tiles, **extras).double().cpu(), want, **close)
+    if dtype == torch.bfloat16 and decoded:
+        got = o.decode_attention_fused(case.q_rows, case.k_new, case.v_new, case.slots, case.k_cache, case.v_cache, case.page_stride, case.page, case.n_pages,
+                                       case.tables, case.row_entry, case.positions, case.seq_lens, heads, 2, dim, scale, 0, 700, **extras)
+        torch.testing.assert_close(got.double().cpu(), want, **close)
