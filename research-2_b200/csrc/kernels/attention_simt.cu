@@ -91,11 +91,10 @@ attention_simt_kernel(const T* __restrict__ q, int q_row_stride, T* __restrict__
   __shared__ float max_s[WARPS], sum_s[WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x, h = blockIdx.y;
-  // (the batch's index arrays are no kernel's output: they are read before the wait on the previous kernel)
+  pdl_wait();               // the previous kernel's writes are visible from here on (the index arrays may be among them)
   const int e = row_entry[t];
   const int pos = e < 0 ? 0 : positions[t], seq_len = e < 0 ? 0 : seq_lens[e];
   T* o = out + size_t(t) * out_row_stride + size_t(h) * v_head_dim;
-  pdl_wait();               // the previous kernel's writes are visible from here on
   if (e < 0) {  // a pad row
     for (int d = threadIdx.x; d < v_head_dim; d += WARPS * 32) o[d] = from_float<T>(0.f);
     return;

@@ -118,6 +118,16 @@ __device__ __forceinline__ int page_offset(int j, int page_size, int shift) { re
 // visible. `pdl_launch_dependents()` lets the successor start its own prologue. Both are no-ops
 // for a kernel launched without the attribute.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// For kernels that read weights or a batch's index arrays ahead of their wait. FIXED: the caller says that no launch shortly before wrote
+// them (a model's weights, a step's batch). Without that word they may be the output of the kernel just before, and the wait comes
+// first. The choice is made at compile time and every path has one wait: with the first of two under a condition at run time, rows came
+// out as if the second had not been there.
+template <bool FIXED> __device__ __forceinline__ void pdl_wait_before_operands() {
+  if constexpr (!FIXED) pdl_wait();
+}
+template <bool FIXED> __device__ __forceinline__ void pdl_wait_after_operands() {
+  if constexpr (FIXED) pdl_wait();
+}
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 static int g_r2_pdl = 1;

@@ -216,17 +216,18 @@ __device__ __forceinline__ Split<N> carve(uint8_t*& at, int rows, int stride) {
 
 // N: terms of queries, keys, states and weighted scores; M: of values.
 // U of a chunk: [dim x COLS of the value columns]. Grid: chunks, heads, slices of the columns.
-template <int N, int M>
+template <int N, int M, bool FIXED>
 __global__ void __launch_bounds__(THREADS)
 decay_chunk_sums_kernel(const ChunkArgs a) {
   pdl_launch_dependents();
+  pdl_wait_before_operands<FIXED>();
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ float powers[CHUNK];
   const Tile tile = find_tile(a.q_start, a.n_entries, blockIdx.x);
   const int h = blockIdx.y, col0 = blockIdx.z * COLS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < CHUNK; i += THREADS) powers[i] = power(a.decay[h], i);
   __syncthreads();
-  pdl_wait();
+  pdl_wait_after_operands<FIXED>();
   if (tile.entry < 0) return;
   uint8_t* at = smem;
   const Split<N> k = carve<N>(at, CHUNK, a.dim16 + 8);
@@ -277,9 +278,11 @@ decay_chunk_sums_kernel(const ChunkArgs a) {
 }
 
 // The states at the chunks' starts, and the request's new one. Grid: entries, heads, pieces of the state.
+template <bool FIXED>
 __global__ void __launch_bounds__(256)
 decay_chunk_states_kernel(const ChunkArgs a) {
   pdl_launch_dependents();
+  pdl_wait_before_operands<FIXED>();
   __shared__ float scratch[33];
   const int e = blockIdx.x, h = blockIdx.y;
   const int row0 = a.q_start[e], rows = a.q_start[e + 1] - row0;
@@ -290,7 +293,7 @@ decay_chunk_states_kernel(const ChunkArgs a) {
   const int size = a.dim * a.vdim, i = blockIdx.z * blockDim.x + threadIdx.x;
   const float decay = a.decay[h];
   const float whole = power(decay, CHUNK), last = power(decay, rows - (rows - 1) / CHUNK * CHUNK);
-  pdl_wait();
+  pdl_wait_after_operands<FIXED>();
   if (rows <= 0 || i >= size) return;   // an entry without rows touches no slot
   float* slot = a.state + size_t(a.state_slot[e]) * a.slot_stride + size_t(h) * size + i;
   float s = is_fresh ? 0.f : *slot;
@@ -313,17 +316,18 @@ decay_chunk_states_kernel(const ChunkArgs a) {
 }
 
 // Outputs of a chunk. Grid: chunks, heads, slices of the columns. A warp has 16 of the chunk's rows.
-template <int N, int M>
+template <int N, int M, bool FIXED>
 __global__ void __launch_bounds__(THREADS)
 decay_chunk_outputs_kernel(const ChunkArgs a) {
   pdl_launch_dependents();
+  pdl_wait_before_operands<FIXED>();
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ float powers[CHUNK + 1];
   const Tile tile = find_tile(a.q_start, a.n_entries, blockIdx.x);
   const int h = blockIdx.y, col0 = blockIdx.z * COLS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i <= CHUNK; i += THREADS) powers[i] = power(a.decay[h], i);
   __syncthreads();
-  pdl_wait();
+  pdl_wait_after_operands<FIXED>();
   if (tile.entry < 0) return;
   uint8_t* at = smem;
   const Split<N> q = carve<N>(at, CHUNK, a.dim16 + 8), k = carve<N>(at, CHUNK, a.dim16 + 8);
@@ -435,10 +439,11 @@ decay_chunk_outputs_kernel(const ChunkArgs a) {
 // Decode steps. A CTA has one (entry, head, slice of the columns); a thread has V neighbouring columns of every row_groups-th row, and
 // the row groups' sums meet in shared memory, in order.
 constexpr int STEP_THREADS = 128, STEP_ROWS = 8;
-template <int V>
+template <int V, bool FIXED>
 __global__ void __launch_bounds__(STEP_THREADS)
 decay_step_kernel(const ChunkArgs a, int slice) {
   pdl_launch_dependents();
+  pdl_wait_before_operands<FIXED>();
   __shared__ float qs[MAX_DIM], ks[MAX_DIM], sums[STEP_THREADS][V];
   const int e = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * slice;
   const int row0 = a.q_start[e], row1 = a.q_start[e + 1];
@@ -448,7 +453,7 @@ decay_step_kernel(const ChunkArgs a, int slice) {
   const int g = threadIdx.x % groups, rg = threadIdx.x / groups, j = col0 + g * V;
   const bool mine = j < a.vdim;
   float* head_state = a.state + size_t(a.state_slot[e]) * a.slot_stride + size_t(h) * a.dim * a.vdim;
-  pdl_wait();
+  pdl_wait_after_operands<FIXED>();
   for (int t = row0; t < row1; ++t) {
     const bool zero = is_fresh && t == row0;
     float s[STEP_ROWS][V], v[V], acc[V] = {};
@@ -531,7 +536,7 @@ decay_step_kernel(const ChunkArgs a, int slice) {
 
 size_t split_bytes(int rows, int stride, int terms) { return size_t(rows) * stride * terms * sizeof(bf16); }
 
-template <int N, int M>
+template <int N, int M, bool FIXED>
 int launch_chunks(const ChunkArgs& a, int n_tiles, cudaStream_t stream) {
   const size_t rows_q = split_bytes(CHUNK, a.dim16 + 8, N), rows_v = split_bytes(CHUNK, COLS + 8, M), turns = size_t(2) * CHUNK * a.rot_half * sizeof(float);
   const size_t smem_sums = rows_q + rows_v + turns, smem_out = 2 * rows_q + rows_v + split_bytes(a.dim16, COLS + 8, N) + turns;
@@ -539,8 +544,8 @@ int launch_chunks(const ChunkArgs& a, int n_tiles, cudaStream_t stream) {
   if (smem_out > MOST) return R2_UNSUPPORTED;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(decay_chunk_outputs_kernel<N, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(MOST));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_chunk_sums_kernel<N, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(MOST));
+    cudaError_t e = cudaFuncSetAttribute(decay_chunk_outputs_kernel<N, M, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(MOST));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_chunk_sums_kernel<N, M, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(MOST));
     if (e != cudaSuccess) {
       cudaGetLastError();
       return R2_UNSUPPORTED;
@@ -548,9 +553,9 @@ int launch_chunks(const ChunkArgs& a, int n_tiles, cudaStream_t stream) {
     configured = true;
   }
   const dim3 grid(n_tiles, a.n_heads, (a.vdim + COLS - 1) / COLS);
-  r2_launch(decay_chunk_sums_kernel<N, M>, grid, dim3(THREADS), smem_sums, stream, a);
-  r2_launch(decay_chunk_states_kernel, dim3(a.n_entries, a.n_heads, (a.dim * a.vdim + 255) / 256), dim3(256), size_t(0), stream, a);
-  r2_launch(decay_chunk_outputs_kernel<N, M>, grid, dim3(THREADS), smem_out, stream, a);
+  r2_launch(decay_chunk_sums_kernel<N, M, FIXED>, grid, dim3(THREADS), smem_sums, stream, a);
+  r2_launch(decay_chunk_states_kernel<FIXED>, dim3(a.n_entries, a.n_heads, (a.dim * a.vdim + 255) / 256), dim3(256), size_t(0), stream, a);
+  r2_launch(decay_chunk_outputs_kernel<N, M, FIXED>, grid, dim3(THREADS), smem_out, stream, a);
   return launch_status();
 }
 
@@ -562,11 +567,12 @@ extern "C" long long r2_decay_chunks_floats(int n_tiles, int n_heads, int dim, i
 // q, k [T, heads * dim], v [T, heads * vdim] bfloat16 (slices of a projection); decay float [heads]; silu_in: silu of all three on their
 // way in, k then times k_scale; state float [slots][heads][dim][vdim]; n_tiles at least the sum over entries of ceil(rows / 64); scratch
 // float (r2_decay_chunks_floats); out float [T, heads * vdim]. inv_freq float [rot_half] and positions [T] where q and k turn (then without
-// silu). Three launches. R2_UNSUPPORTED: heads of more than 256 rows (fewer, where they turn: what an SM's shared memory holds).
+// silu). `fixed` (here and below): no launch shortly before writes the decays or the batch's arrays, which are then read ahead of the wait
+// for it. Three launches. R2_UNSUPPORTED: heads of more than 256 rows (fewer, where they turn: what an SM's shared memory holds).
 extern "C" int r2_decay_chunks(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, const float* decay, float k_scale,
                                int silu_in, float* state, long long slot_stride, const int32_t* q_start, const int32_t* state_slot, const int32_t* fresh,
                                int n_entries, int n_tiles, float* scratch, long long scratch_floats, float* out, int out_stride, int n_heads, int dim,
-                               int vdim, const float* inv_freq, int rot_half, const int32_t* positions, cudaStream_t stream) {
+                               int vdim, const float* inv_freq, int rot_half, const int32_t* positions, int fixed, cudaStream_t stream) {
   if (n_entries <= 0 || n_tiles <= 0) return R2_OK;
   if (rot_half < 0 || 2 * rot_half > dim || (rot_half > 0 && (inv_freq == nullptr || positions == nullptr || silu_in))) return R2_BAD_SHAPE;
   if (n_heads < 1 || dim < 1 || vdim < 1 || scratch == nullptr || scratch_floats < r2_decay_chunks_floats(n_tiles, n_heads, dim, vdim)) return R2_BAD_SHAPE;
@@ -579,14 +585,15 @@ extern "C" int r2_decay_chunks(const void* q, int q_stride, const void* k, int k
   a.vec = dim % 8 == 0 && vdim % 8 == 0 && q_stride % 8 == 0 && k_stride % 8 == 0 && v_stride % 8 == 0 &&
           !((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15);
   a.inv_freq = inv_freq; a.rot_half = rot_half; a.positions = positions;
-  return rot_half > 0 ? launch_chunks<3, 1>(a, n_tiles, stream) : launch_chunks<2, 2>(a, n_tiles, stream);
+  if (rot_half > 0) return fixed ? launch_chunks<3, 1, true>(a, n_tiles, stream) : launch_chunks<3, 1, false>(a, n_tiles, stream);
+  return fixed ? launch_chunks<2, 2, true>(a, n_tiles, stream) : launch_chunks<2, 2, false>(a, n_tiles, stream);
 }
 
 // The same for batches in which (nearly) every entry is one row: one launch, no scratch.
 extern "C" int r2_decay_step(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, const float* decay, float k_scale,
                              int silu_in, float* state, long long slot_stride, const int32_t* q_start, const int32_t* state_slot, const int32_t* fresh,
                              int n_entries, float* out, int out_stride, int n_heads, int dim, int vdim, int n_sms, const float* inv_freq, int rot_half,
-                             const int32_t* positions, cudaStream_t stream) {
+                             const int32_t* positions, int fixed, cudaStream_t stream) {
   if (n_entries <= 0) return R2_OK;
   if (rot_half < 0 || 2 * rot_half > dim || (rot_half > 0 && (inv_freq == nullptr || positions == nullptr || silu_in))) return R2_BAD_SHAPE;
   if (n_heads < 1 || dim < 1 || vdim < 1 || n_sms < 1) return R2_BAD_SHAPE;
@@ -602,7 +609,8 @@ extern "C" int r2_decay_step(const void* q, int q_stride, const void* k, int k_s
   while (slice > 16 && (long long)n_entries * n_heads * ((vdim + slice - 1) / slice) < 2ll * n_sms) slice /= 2;
   const dim3 grid(n_entries, n_heads, (vdim + slice - 1) / slice);
   const bool quads = vdim % 4 == 0 && slot_stride % 4 == 0 && !(reinterpret_cast<uintptr_t>(state) & 15);
-  if (quads) r2_launch(decay_step_kernel<4>, grid, dim3(STEP_THREADS), size_t(0), stream, a, slice);
-  else r2_launch(decay_step_kernel<1>, grid, dim3(STEP_THREADS), size_t(0), stream, a, slice);
+  auto go = [&](auto kernel) { r2_launch(kernel, grid, dim3(STEP_THREADS), size_t(0), stream, a, slice); };
+  if (quads) fixed ? go(decay_step_kernel<4, true>) : go(decay_step_kernel<4, false>);
+  else fixed ? go(decay_step_kernel<1, true>) : go(decay_step_kernel<1, false>);
   return launch_status();
 }

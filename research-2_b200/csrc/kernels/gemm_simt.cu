@@ -14,8 +14,8 @@
 //
 //   gemm_rows_kernel   few rows. What bounds it is the stream of weights, so it is laid out for loads in flight: a warp has one slice
 //                      of 32 columns, its lanes read 128-byte lines of 32 rows of it ahead of the multiply-adds (an [N, K] matrix
-//                      passes through shared memory to be turned; the first lines are asked for before the wait on the kernel
-//                      before), and the groups of a column block are spread over a thread-block cluster whose first CTA adds them up.
+//                      passes through shared memory to be turned), and the groups of a column block are spread over a
+//                      thread-block cluster whose first CTA adds them up.
 //   gemm_tile_kernel   many rows: tiles in shared memory, the next stage's loads in flight under this one's multiply-adds; a
 //                      thread keeps the current slice's sums, the group's and, where one CTA has them all, the total. With few
 //                      tiles the groups go to the CTAs of a cluster: a lone CTA of four warps on an SM waits on its own latencies
@@ -120,8 +120,8 @@ gemm_rows_kernel(const Product p, int n_slices, int per_cta, int n_blocks) {
     for (int u = 0; u < STEP; ++u, from += p.ldw) cur[u] = u < n_live ? to_float(*from) : 0.f;
   };
 
+  pdl_wait();               // the previous kernel's writes are visible from here on (`w` may be one of them: any caller's tensor)
   load(blockIdx.y * ROW_COLS, warp, 0);
-  pdl_wait();               // the previous kernel's writes are visible from here on
 #pragma unroll
   for (int r = 0; r < MR; ++r)
     for (int k = threadIdx.x; k < mine * len; k += ROW_WARPS * 32)

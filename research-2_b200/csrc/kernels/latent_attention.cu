@@ -23,6 +23,8 @@
 #include <limits.h>
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "mma_sync.cuh"
 #include "sm100_ptx.cuh"
@@ -216,11 +218,12 @@ struct HeadLinearParams {
 
 // WHOLE: both operands' rows are whole 16-byte pieces on their boundaries (the path that loads single numbers, unrolled beside the other,
 // took the registers that keep the loads in flight); GATED: there is a gate.
-template <bool WHOLE, bool GATED>
+template <bool WHOLE, bool GATED, bool FIXED>
 __global__ void __launch_bounds__(128)
 head_linear_mma_kernel(const HeadLinearParams p) {
   using namespace r2ptx;
   pdl_launch_dependents();
+  pdl_wait_before_operands<FIXED>();
   __shared__ __align__(16) bf16 a_s[HM_TILE][HM_PAD];
   __shared__ __align__(16) bf16 w_s[HM_TILE][HM_PAD];
   __shared__ __align__(8) float gate_s[GATED ? HM_TILE : 1][HM_TILE + 2];   // sigmoid(gate)
@@ -237,7 +240,7 @@ head_linear_mma_kernel(const HeadLinearParams p) {
     if constexpr (WHOLE) return c * 8 < len ? *reinterpret_cast<const uint4*>(row + c * 8) : zero4;
     else return eight_of(row, c, len, vec);
   };
-  // A few rows' time is the chain of their loads: the head's matrix (no kernel's output) is asked for before the wait on the kernel
+  // A few rows' time is the chain of their loads: the head's matrix (FIXED: no kernel's output) is asked for before the wait on the kernel
   // before this one, the gates before the products, and a piece of K while the one before it is multiplied.
   constexpr int PIECES = HM_TILE * (HM_TILE / 8) / 128;   // of a thread: four of either operand
   uint4 av[PIECES], wv[PIECES];
@@ -262,7 +265,7 @@ head_linear_mma_kernel(const HeadLinearParams p) {
     }
   };
   load_w(0);
-  pdl_wait();
+  pdl_wait_after_operands<FIXED>();
   load_a(0);
   const int g = lane >> 2, tq = lane & 3;
   // The gates: whole rows by all four warps, whatever the number of rows, and their sigmoids through shared memory (12 rows of 128 -> 64 in
@@ -644,8 +647,8 @@ latent_merge_kernel(const float* __restrict__ parts, int n_slices, int kv_rank, 
   pdl_launch_dependents();
   __shared__ float tops[MAX_SLICES], sums[MAX_SLICES];
   const int e = blockIdx.x / n_heads, h = blockIdx.x - e * n_heads, len = kv_rank + 2;
-  const float sink = sinks != nullptr ? sinks[h] * 1.4426950408889634f : -INFINITY;
   pdl_wait();
+  const float sink = sinks != nullptr ? sinks[h] * 1.4426950408889634f : -INFINITY;
   const float* mine = parts + size_t(blockIdx.x) * n_slices * len;
   if (threadIdx.x < n_slices) {
     tops[threadIdx.x] = mine[size_t(threadIdx.x) * len + kv_rank];
@@ -714,9 +717,10 @@ extern "C" int r2_latent_prepare(void* buf, int row_stride, int n_rows, int n_he
 // a [n_rows, ...] with row stride a_stride, head h's k numbers at a[t][h * a_head ..]; out likewise with out_stride and out_head;
 // w: n_heads matrices of k x n numbers one after the other, each [k][n] (w_is_nk 0) or [n][k] (1).
 // gate (may be null; rows of stride gate_stride, laid out like out): out *= sigmoid(gate), element by element.
+// `fixed`: no launch shortly before writes w, which is then read ahead of the wait for it.
 extern "C" int r2_head_linear(const void* a, int a_stride, int a_head, const void* w, int w_is_nk, void* out, int out_stride,
                               int out_head, int n_rows, int n_heads, int k, int n, const void* gate, int gate_stride, int dtype,
-                              cudaStream_t stream) {
+                              int fixed, cudaStream_t stream) {
   if (n_rows <= 0 || n_heads <= 0 || n <= 0) return R2_OK;
   if (k < 1 || n_heads > 65535) return R2_BAD_SHAPE;
   dim3 grid((n_rows + HL_ROWS - 1) / HL_ROWS, (n + HL_COLS - 1) / HL_COLS, n_heads);
@@ -736,9 +740,12 @@ extern "C" int r2_head_linear(const void* a, int a_stride, int a_head, const voi
     p.out_vec = (uintptr_t(out) % 4 == 0 && out_stride % 2 == 0 && out_head % 2 == 0) ? 1 : 0;
     const dim3 tiles((n_rows + HM_TILE - 1) / HM_TILE, (n + HM_TILE - 1) / HM_TILE, n_heads);
     const bool whole = p.a_vec && p.w_vec && k % 8 == 0 && (w_is_nk || n % 8 == 0);
-    auto kernel = whole ? (gate != nullptr ? head_linear_mma_kernel<true, true> : head_linear_mma_kernel<true, false>)
-                        : (gate != nullptr ? head_linear_mma_kernel<false, true> : head_linear_mma_kernel<false, false>);
-    r2_launch(kernel, tiles, dim3(128), size_t(0), stream, p);
+    auto go = [&](auto whole_pieces, auto is_fixed) {
+      constexpr bool WHOLE = decltype(whole_pieces)::value, FIXED = decltype(is_fixed)::value;
+      r2_launch(gate != nullptr ? head_linear_mma_kernel<WHOLE, true, FIXED> : head_linear_mma_kernel<WHOLE, false, FIXED>, tiles, dim3(128), size_t(0), stream, p);
+    };
+    if (whole) fixed ? go(std::true_type(), std::true_type()) : go(std::true_type(), std::false_type());
+    else fixed ? go(std::false_type(), std::true_type()) : go(std::false_type(), std::false_type());
   } else {
     return R2_BAD_DTYPE;
   }

@@ -20,6 +20,8 @@
 // state too), and the norm over groups of columns with a gate that follows both mixers.
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "scan_pieces.cuh"
 
@@ -426,14 +428,15 @@ int launch_scan(const ScanArgs& in, int n_entries, int n_heads, cudaStream_t str
 // out[t][c] = silu(bias[c] + sum_d taps[c][d] * in[t - (n_taps - 1) + d][c]); inputs before this step's first row
 // of an entry come from the request's slot (the inputs of its last n_taps - 1 positions), zeros before a sequence's
 // start. The slot is only read here; the recurrence's kernel, which runs after this one, renews it.
-template <typename T>
+template <typename T, bool FIXED>
 __global__ void __launch_bounds__(256)
 causal_conv_kernel(const T* __restrict__ in, int in_stride, T* __restrict__ out, int out_stride, const float* __restrict__ taps,
                    const float* __restrict__ bias, int n_taps, int channels, const float* __restrict__ state, long long slot_stride,
                    long long conv_state_off, const int32_t* __restrict__ row_entry, const int32_t* __restrict__ q_start,
                    const int32_t* __restrict__ state_slot, const int32_t* __restrict__ fresh) {
   pdl_launch_dependents();
-  // (the batch's arrays and the weights are no kernel's output: what is looked up in them does not wait for the kernel before this one)
+  // (FIXED: the batch's arrays and the weights are no kernel's output, and what is looked up in them does not wait for the kernel before)
+  pdl_wait_before_operands<FIXED>();
   const int t = blockIdx.x;
   const int e = row_entry[t];
   const int l = e < 0 ? 0 : t - q_start[e];
@@ -447,7 +450,7 @@ causal_conv_kernel(const T* __restrict__ in, int in_stride, T* __restrict__ out,
     for (int d = 0; d < 4; ++d) first_tap[d] = d < n_taps ? taps[size_t(c_first) * n_taps + d] : 0.f;
     first_bias = bias != nullptr ? bias[c_first] : 0.f;
   }
-  pdl_wait();
+  pdl_wait_after_operands<FIXED>();
   T* o = out + size_t(t) * out_stride;
   if (e < 0) {  // a pad row
     for (int c = c_first; c < channels; c += gridDim.y * blockDim.x) o[c] = from_float<T>(0.f);
@@ -480,7 +483,7 @@ causal_conv_kernel(const T* __restrict__ in, int in_stride, T* __restrict__ out,
 // One warp per (row, group). gate_first 1: y <- y * silu(gate), then the group's RMS norm, times weight.
 // 0: the group's RMS norm, times weight, times sigmoid(gate). 2: the group's RMS norm, times weight, times silu(gate).
 // weight may be null: a gain of one. A few rows' time is a chain of round trips, so a thread's first NORM_HELD columns stay in
-// registers: gains before the wait on the kernel before this one (weights are no kernel's output), values and gates at once;
+// registers: gains before the wait on the kernel before this one (FIXED: they are no kernel's output), values and gates at once;
 // what lies beyond is read twice.
 constexpr int NORM_HELD = 4;
 
@@ -495,12 +498,13 @@ __device__ __forceinline__ void gated_value(float v, const T gate, int gate_firs
 }
 
 // A group's columns by `threads` threads, this one the `me`-th; `sum` adds their shares up.
-template <typename T, typename F>
+template <bool FIXED, typename T, typename F>
 __device__ __forceinline__ void norm_group(const float* yr, const T* gr, const float* wr, T* o, int group_size, float eps, int gate_first, int me, int threads, F sum) {
+  pdl_wait_before_operands<FIXED>();
   float value[NORM_HELD], factor[NORM_HELD], gain[NORM_HELD];
 #pragma unroll
   for (int i = 0; i < NORM_HELD; ++i) gain[i] = wr != nullptr && me + i * threads < group_size ? wr[me + i * threads] : 1.f;
-  pdl_wait();
+  pdl_wait_after_operands<FIXED>();
   T gate[NORM_HELD];
 #pragma unroll
   for (int i = 0; i < NORM_HELD; ++i) {
@@ -531,7 +535,7 @@ __device__ __forceinline__ void norm_group(const float* yr, const T* gr, const f
   }
 }
 
-template <typename T>
+template <typename T, bool FIXED>
 __global__ void __launch_bounds__(128)
 group_norm_gated_kernel(const float* __restrict__ y, int y_stride, const T* __restrict__ gate, int gate_stride,
                         const float* __restrict__ weight, T* __restrict__ out, int out_stride, int n_rows, int n_groups,
@@ -544,13 +548,13 @@ group_norm_gated_kernel(const float* __restrict__ y, int y_stride, const T* __re
     return;
   }
   const int t = int(unit / n_groups), grp = int(unit % n_groups);
-  norm_group(y + size_t(t) * y_stride + size_t(grp) * group_size, gate + size_t(t) * gate_stride + size_t(grp) * group_size,
+  norm_group<FIXED>(y + size_t(t) * y_stride + size_t(grp) * group_size, gate + size_t(t) * gate_stride + size_t(grp) * group_size,
              weight != nullptr ? weight + size_t(grp) * group_size : nullptr, out + size_t(t) * out_stride + size_t(grp) * group_size, group_size, eps,
              gate_first, lane, 32, [](float x) { return warp_sum(x); });
 }
 
 // The same with a CTA per (row, group), for groups of many columns.
-template <typename T>
+template <typename T, bool FIXED>
 __global__ void __launch_bounds__(256)
 group_norm_gated_block_kernel(const float* __restrict__ y, int y_stride, const T* __restrict__ gate, int gate_stride,
                               const float* __restrict__ weight, T* __restrict__ out, int out_stride, int n_groups,
@@ -558,7 +562,7 @@ group_norm_gated_block_kernel(const float* __restrict__ y, int y_stride, const T
   pdl_launch_dependents();
   __shared__ float scratch[33];
   const int t = blockIdx.x / n_groups, grp = blockIdx.x % n_groups;
-  norm_group(y + size_t(t) * y_stride + size_t(grp) * group_size, gate + size_t(t) * gate_stride + size_t(grp) * group_size,
+  norm_group<FIXED>(y + size_t(t) * y_stride + size_t(grp) * group_size, gate + size_t(t) * gate_stride + size_t(grp) * group_size,
              weight != nullptr ? weight + size_t(grp) * group_size : nullptr, out + size_t(t) * out_stride + size_t(grp) * group_size, group_size, eps,
              gate_first, int(threadIdx.x), int(blockDim.x), [&](float x) { return block_sum(x, scratch); });
 }
@@ -643,54 +647,45 @@ extern "C" int r2_ssd_scan(const void* x, int x_stride, const void* b, int b_str
   return R2_BAD_DTYPE;
 }
 
+// `fixed` (here and in r2_group_norm_gated): no launch shortly before writes the weights or the batch's arrays, which are then read ahead
+// of the wait for it.
 extern "C" int r2_causal_conv(const void* in, int in_stride, void* out, int out_stride, const float* taps, const float* bias,
                               int n_taps, int channels, const float* state, long long slot_stride, long long conv_state_off,
                               const int32_t* row_entry, const int32_t* q_start, const int32_t* state_slot, const int32_t* fresh,
-                              int n_rows, int dtype, cudaStream_t stream) {
+                              int n_rows, int dtype, int fixed, cudaStream_t stream) {
   if (n_rows <= 0) return R2_OK;
   if (n_taps < 1 || channels < 1) return R2_BAD_SHAPE;
   // a channel a thread for few rows, whose time is the chain of their loads; four for many
   const int per_cta = n_rows <= 64 ? 256 : 1024;
-  dim3 grid(n_rows, (channels + per_cta - 1) / per_cta);
-  if (dtype == R2_F32) {
-    r2_launch(causal_conv_kernel<float>, grid, dim3(256), size_t(0), stream, (const float*)in, in_stride, (float*)out, out_stride,
+  if (dtype != R2_F32 && dtype != R2_BF16) return R2_BAD_DTYPE;
+  auto go = [&](auto kernel, auto zero) {
+    r2_launch(kernel, dim3(n_rows, (channels + per_cta - 1) / per_cta), dim3(256), size_t(0), stream, (const decltype(zero)*)in, in_stride, (decltype(zero)*)out, out_stride,
               taps, bias, n_taps, channels, state, slot_stride, conv_state_off, row_entry, q_start, state_slot, fresh);
-  } else if (dtype == R2_BF16) {
-    r2_launch(causal_conv_kernel<bf16>, grid, dim3(256), size_t(0), stream, (const bf16*)in, in_stride, (bf16*)out, out_stride,
-              taps, bias, n_taps, channels, state, slot_stride, conv_state_off, row_entry, q_start, state_slot, fresh);
-  } else {
-    return R2_BAD_DTYPE;
-  }
+  };
+  if (dtype == R2_F32) fixed ? go(causal_conv_kernel<float, true>, 0.f) : go(causal_conv_kernel<float, false>, 0.f);
+  else fixed ? go(causal_conv_kernel<bf16, true>, bf16()) : go(causal_conv_kernel<bf16, false>, bf16());
   return launch_status();
 }
 
 extern "C" int r2_group_norm_gated(const float* y, int y_stride, const void* gate, int gate_stride, const float* weight,
                                    void* out, int out_stride, int n_rows, int n_groups, int group_size, float eps,
-                                   int gate_first, int dtype, cudaStream_t stream) {
+                                   int gate_first, int dtype, int fixed, cudaStream_t stream) {
   if (n_rows <= 0) return R2_OK;
   if (n_groups < 1 || group_size < 1) return R2_BAD_SHAPE;
   const long long units = (long long)n_rows * n_groups;
-  if (group_size > 256) {
-    if (dtype == R2_F32) {
-      r2_launch(group_norm_gated_block_kernel<float>, dim3((unsigned)units), dim3(256), size_t(0), stream, y, y_stride, (const float*)gate,
-                gate_stride, weight, (float*)out, out_stride, n_groups, group_size, eps, gate_first);
-    } else if (dtype == R2_BF16) {
-      r2_launch(group_norm_gated_block_kernel<bf16>, dim3((unsigned)units), dim3(256), size_t(0), stream, y, y_stride, (const bf16*)gate,
-                gate_stride, weight, (bf16*)out, out_stride, n_groups, group_size, eps, gate_first);
-    } else {
-      return R2_BAD_DTYPE;
+  if (dtype != R2_F32 && dtype != R2_BF16) return R2_BAD_DTYPE;
+  auto pick = [&](auto zero, auto is_fixed) {
+    using T = decltype(zero);
+    constexpr bool FIXED = decltype(is_fixed)::value;
+    if (group_size > 256) {
+      r2_launch(group_norm_gated_block_kernel<T, FIXED>, dim3((unsigned)units), dim3(256), size_t(0), stream, y, y_stride, (const T*)gate, gate_stride, weight, (T*)out,
+                out_stride, n_groups, group_size, eps, gate_first);
+      return;
     }
-    return launch_status();
-  }
-  dim3 grid((unsigned)((units + 3) / 4));
-  if (dtype == R2_F32) {
-    r2_launch(group_norm_gated_kernel<float>, grid, dim3(128), size_t(0), stream, y, y_stride, (const float*)gate, gate_stride,
-              weight, (float*)out, out_stride, n_rows, n_groups, group_size, eps, gate_first);
-  } else if (dtype == R2_BF16) {
-    r2_launch(group_norm_gated_kernel<bf16>, grid, dim3(128), size_t(0), stream, y, y_stride, (const bf16*)gate, gate_stride,
-              weight, (bf16*)out, out_stride, n_rows, n_groups, group_size, eps, gate_first);
-  } else {
-    return R2_BAD_DTYPE;
-  }
+    r2_launch(group_norm_gated_kernel<T, FIXED>, dim3((unsigned)((units + 3) / 4)), dim3(128), size_t(0), stream, y, y_stride, (const T*)gate, gate_stride, weight, (T*)out,
+              out_stride, n_rows, n_groups, group_size, eps, gate_first);
+  };
+  if (dtype == R2_F32) fixed ? pick(0.f, std::true_type()) : pick(0.f, std::false_type());
+  else fixed ? pick(bf16(), std::true_type()) : pick(bf16(), std::false_type());
   return launch_status();
 }

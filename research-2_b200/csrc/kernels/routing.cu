@@ -38,16 +38,17 @@ __device__ __forceinline__ void add_quad(float (&sum)[4], const float4 x, const 
 }
 
 // A warp has one output, for `rows_per_cta` rows one after the other; a CTA eight outputs. What bounds a few rows is one round trip after
-// another, so the output's weights are asked for in 16-byte pieces before the kernel before this one has ended (weights are no kernel's
+// another, so the output's weights are asked for in 16-byte pieces before the kernel before this one has ended (FIXED: they are no kernel's
 // output) and stay in registers (width up to 128 SMALL_AHEAD; what lies beyond is read again a row), and a row comes straight from memory,
 // all pieces at once: 4 rows x 768 x 24 take 2.3 us (7.0 with a CTA a row, three outputs a warp after the row's way through shared
 // memory). QUADS: rows of h and w start on boundaries of four numbers and hold a multiple of four.
 constexpr int SMALL_AHEAD = 8, SMALL_WARPS = 8;
-template <typename T, bool QUADS>
+template <typename T, bool QUADS, bool FIXED>
 __global__ void __launch_bounds__(SMALL_WARPS * 32)
 small_linear_kernel(const T* __restrict__ h, int h_stride, const float* __restrict__ w, const float* __restrict__ bias,
                     float* __restrict__ out, int out_stride, int n_out, int width, int n_rows, int rows_per_cta) {
   pdl_launch_dependents();
+  pdl_wait_before_operands<FIXED>();
   const int lane = threadIdx.x & 31, n = blockIdx.y * SMALL_WARPS + (threadIdx.x >> 5);
   const float* wr = w + size_t(n < n_out ? n : 0) * width;
   float4 ahead[QUADS ? SMALL_AHEAD : 1];
@@ -59,7 +60,7 @@ small_linear_kernel(const T* __restrict__ h, int h_stride, const float* __restri
     }
   }
   const float b = bias != nullptr && n < n_out ? bias[n] : 0.f;
-  pdl_wait();
+  pdl_wait_after_operands<FIXED>();
   if (n >= n_out) return;
   const int t0 = blockIdx.x * rows_per_cta, t1 = min(n_rows, t0 + rows_per_cta);
   for (int t = t0; t < t1; ++t) {
@@ -88,18 +89,19 @@ small_linear_kernel(const T* __restrict__ h, int h_stride, const float* __restri
 }
 
 constexpr int TOP_K_AHEAD = 8;
-template <typename T>
+template <typename T, bool FIXED>
 __global__ void __launch_bounds__(256)
 route_top_k_kernel(const T* __restrict__ h, int h_stride, const float* __restrict__ w, const float* __restrict__ bias,
                    float* __restrict__ dense, int32_t* __restrict__ chosen, float* __restrict__ chosen_weight,
                    int n_experts, int top, int width, int quads) {
   pdl_launch_dependents();
+  pdl_wait_before_operands<FIXED>();
   extern __shared__ __align__(16) float smem[];
   float* row = smem;             // [width]
   float* logit = smem + width;   // [n_experts]
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
   // with `quads` (rows of w in whole 16-byte pieces) the first pieces of the warp's first output are asked for before the kernel before
-  // this one has ended
+  // this one has ended (FIXED: they are no kernel's output)
   float4 ahead[TOP_K_AHEAD];
   if (quads && warp < n_experts) {
 #pragma unroll
@@ -108,7 +110,7 @@ route_top_k_kernel(const T* __restrict__ h, int h_stride, const float* __restric
       ahead[i] = k < width ? load4(w + size_t(warp) * width + k) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
-  pdl_wait();
+  pdl_wait_after_operands<FIXED>();
   const T* hr = h + size_t(t) * h_stride;
   for (int k = threadIdx.x; k < width; k += blockDim.x) row[k] = to_float(hr[k]);
   __syncthreads();
@@ -490,8 +492,9 @@ expert_unit_kernel(const T* __restrict__ up, int in_stride, T* __restrict__ out,
 
 }  // namespace
 
+// `fixed` (here and in r2_route_top_k): no launch shortly before writes w or the bias, which are then read ahead of the wait for it.
 extern "C" int r2_small_linear(const void* h, int h_stride, const float* w, const float* bias, float* out, int out_stride,
-                               int n_rows, int n_out, int width, int dtype, cudaStream_t stream) {
+                               int n_rows, int n_out, int width, int dtype, int fixed, cudaStream_t stream) {
   if (n_rows <= 0 || n_out <= 0) return R2_OK;
   if (width < 1) return R2_BAD_SHAPE;
   if (sizeof(float) * size_t(width) > 48 * 1024) return R2_UNSUPPORTED;
@@ -504,25 +507,28 @@ extern "C" int r2_small_linear(const void* h, int h_stride, const float* w, cons
   auto go = [&](auto kernel, auto zero) {
     r2_launch(kernel, grid, dim3(SMALL_WARPS * 32), size_t(0), stream, (const decltype(zero)*)h, h_stride, w, bias, out, out_stride, n_out, width, n_rows, rows_per_cta);
   };
-  if (dtype == R2_F32) quads ? go(small_linear_kernel<float, true>, 0.f) : go(small_linear_kernel<float, false>, 0.f);
-  else quads ? go(small_linear_kernel<bf16, true>, bf16()) : go(small_linear_kernel<bf16, false>, bf16());
+  auto pick = [&](auto zero) {
+    using T = decltype(zero);
+    if (quads) fixed ? go(small_linear_kernel<T, true, true>, zero) : go(small_linear_kernel<T, true, false>, zero);
+    else fixed ? go(small_linear_kernel<T, false, true>, zero) : go(small_linear_kernel<T, false, false>, zero);
+  };
+  dtype == R2_F32 ? pick(0.f) : pick(bf16());
   return launch_status();
 }
 
 extern "C" int r2_route_top_k(const void* h, int h_stride, const float* w, const float* bias, float* dense, int32_t* chosen,
-                              float* chosen_weight, int n_rows, int n_experts, int top, int width, int dtype, cudaStream_t stream) {
+                              float* chosen_weight, int n_rows, int n_experts, int top, int width, int dtype, int fixed, cudaStream_t stream) {
   if (n_rows <= 0) return R2_OK;
   if (width < 1 || n_experts < 1 || n_experts > MAX_EXPERTS || top < 1 || top > n_experts) return R2_BAD_SHAPE;
   const size_t smem = sizeof(float) * (size_t(width) + n_experts);
   if (smem > 48 * 1024) return R2_UNSUPPORTED;
   const int quads = width % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0;
-  if (dtype == R2_F32) {
-    r2_launch(route_top_k_kernel<float>, dim3(n_rows), dim3(256), smem, stream, (const float*)h, h_stride, w, bias, dense, chosen, chosen_weight, n_experts, top, width, quads);
-  } else if (dtype == R2_BF16) {
-    r2_launch(route_top_k_kernel<bf16>, dim3(n_rows), dim3(256), smem, stream, (const bf16*)h, h_stride, w, bias, dense, chosen, chosen_weight, n_experts, top, width, quads);
-  } else {
-    return R2_BAD_DTYPE;
-  }
+  if (dtype != R2_F32 && dtype != R2_BF16) return R2_BAD_DTYPE;
+  auto go = [&](auto kernel, auto zero) {
+    r2_launch(kernel, dim3(n_rows), dim3(256), smem, stream, (const decltype(zero)*)h, h_stride, w, bias, dense, chosen, chosen_weight, n_experts, top, width, quads);
+  };
+  if (dtype == R2_F32) fixed ? go(route_top_k_kernel<float, true>, 0.f) : go(route_top_k_kernel<float, false>, 0.f);
+  else fixed ? go(route_top_k_kernel<bf16, true>, bf16()) : go(route_top_k_kernel<bf16, false>, bf16());
   return launch_status();
 }
 

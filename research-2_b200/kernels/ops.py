@@ -603,9 +603,11 @@ def stream_join(x: torch.Tensor, read: torch.Tensor, gain: torch.Tensor | None =
     return (streams if y is not None else x), u
 
 
-def small_linear(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
+def small_linear(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, out: torch.Tensor | None = None, *, fixed: bool = False) -> torch.Tensor:
     """h [T, K] (any compute dtype) times w [N, K] float32 (+ bias float32) -> float32 [T, N]: the few outputs per row
-    that must stay in 32-bit (gates of a recurrence, one gate per head, step sizes), each one warp's sum."""
+    that must stay in 32-bit (gates of a recurrence, one gate per head, step sizes), each one warp's sum.
+    `fixed`: w and bias are no output of the launches just before (a model's weights, a step's batch), so the kernel may read them ahead of
+    its wait for those."""
     _need(h, "h", dim=2)
     _need(w, "w", torch.float32, 2)
     if w.shape[1] != h.shape[1] or not w.is_contiguous():
@@ -617,15 +619,17 @@ def small_linear(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = N
     if out is None:
         out = torch.empty(h.shape[0], w.shape[0], dtype=torch.float32, device=h.device)
     status = _lib("routing").r2_small_linear(_p(h), _rows(h, "h"), _p(w), _p(bias), _p(out), _rows(out, "out"), h.shape[0],
-                                            w.shape[0], h.shape[1], dtype_code(h.dtype), _stream())
+                                            w.shape[0], h.shape[1], dtype_code(h.dtype), int(fixed), _stream())
     _check(status, "small_linear")
     return out
 
 
-def route_top_k(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, top: int):
+def route_top_k(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, top: int, *, fixed: bool = False):
     """Router: logits h @ w^T + bias in float32, the `top` largest per row (the lower index wins a tie), softmax over
     the chosen logits only. -> (dense float32 [T, experts]: a row's weights, zero for experts not chosen;
-    chosen int32 [T, top]; their weights float32 [T, top])."""
+    chosen int32 [T, top]; their weights float32 [T, top]).
+    `fixed`: w are no output of the launches just before (a model's weights, a step's batch), so the kernel may read them ahead of
+    its wait for those."""
     _need(h, "h", dim=2)
     _need(w, "w", torch.float32, 2)
     if w.shape[1] != h.shape[1] or not w.is_contiguous() or not 1 <= top <= w.shape[0]:
@@ -637,7 +641,7 @@ def route_top_k(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, top
     chosen = torch.empty(n, top, dtype=torch.int32, device=h.device)
     weight = torch.empty(n, top, dtype=torch.float32, device=h.device)
     status = _lib("routing").r2_route_top_k(_p(h), _rows(h, "h"), _p(w), _p(bias), _p(dense), _p(chosen), _p(weight), n, e, top,
-                                           h.shape[1], dtype_code(h.dtype), _stream())
+                                           h.shape[1], dtype_code(h.dtype), int(fixed), _stream())
     _check(status, "route_top_k")
     return dense, chosen, weight
 
@@ -821,14 +825,16 @@ def use_decay_chunks(on: bool) -> bool:
 def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, k_scale: float,
                    inv_freq: torch.Tensor | None, rot_dims: int, positions: torch.Tensor, state: torch.Tensor, q_start: torch.Tensor,
                    state_slot: torch.Tensor, fresh: torch.Tensor, n_heads: int, dim: int, vdim: int, silu: bool = False,
-                   n_tiles: int = 0) -> torch.Tensor:
+                   n_tiles: int = 0, *, fixed: bool = False) -> torch.Tensor:
     """Retention's recurrence S <- decay[h] S + k v^T, o = S^T q for every entry of a batch, from and to the entries' state
     slots. q, k [T, heads * dim], v [T, heads * vdim] (slices of a projection); the kernel rotates q and k by position on their
     way in (of each head the first rot_dims dimensions, i with i + rot_dims / 2, angle positions[t] * inv_freq[i], in float32)
     and multiplies k by k_scale after that. `silu`: q, k and v pass silu on their way in (float32, instead of a rotation).
     With `n_tiles` (the sum over entries of ceil(rows / 64) or more) bfloat16 batches of 64 rows and more run in chunks of 64 rows on the tensor
     cores (csrc/kernels/decay_chunks.cu; heads of up to 256 rows, not rotated and silu both) instead of row by row; there is a kernel for decode steps beside it. decay float32 [heads]; state float32 [slots, heads * dim * vdim].
-    -> float32 [T, heads * vdim], the heads' outputs before their norm."""
+    -> float32 [T, heads * vdim], the heads' outputs before their norm.
+    `fixed`: decay and the index arrays are no output of the launches just before (a model's weights, a step's batch), so the kernel may read them ahead of
+    its wait for those."""
     n = _entries(q_start, state_slot, fresh)
     for name, t, width in (("q", q, n_heads * dim), ("k", k, n_heads * dim), ("v", v, n_heads * vdim)):
         _need(t, name, q.dtype, 2)
@@ -849,7 +855,7 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
         status = _lib("decay_chunks").r2_decay_chunks(
             _p(q), _rows(q, "q"), _p(k), _rows(k, "k"), _p(v), _rows(v, "v"), _p(decay), C.c_float(k_scale), int(bool(silu)), _p(state),
             C.c_longlong(state.shape[1]), _p(q_start), _p(state_slot), _p(fresh), n, n_tiles, _p(scratch), C.c_longlong(scratch.numel()), _p(out),
-            _rows(out, "out"), n_heads, dim, vdim, _p(inv_freq if rot_dims else None), rot_dims // 2, _p(positions), _stream())
+            _rows(out, "out"), n_heads, dim, vdim, _p(inv_freq if rot_dims else None), rot_dims // 2, _p(positions), int(fixed), _stream())
         if status != -4:
             _check(status, "retention_scan (chunks)")
             count_launches(2)  # the sums, the states, the outputs
@@ -859,7 +865,7 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
         status = _lib("decay_chunks").r2_decay_step(
             _p(q), _rows(q, "q"), _p(k), _rows(k, "k"), _p(v), _rows(v, "v"), _p(decay), C.c_float(k_scale), int(bool(silu)), _p(state),
             C.c_longlong(state.shape[1]), _p(q_start), _p(state_slot), _p(fresh), n, _p(out), _rows(out, "out"), n_heads, dim, vdim, sm_count(q.device),
-            _p(inv_freq if rot_dims else None), rot_dims // 2, _p(positions), _stream())
+            _p(inv_freq if rot_dims else None), rot_dims // 2, _p(positions), int(fixed), _stream())
         if status != -4:
             _check(status, "retention_scan (step)")
             _used("decay_step")
@@ -919,11 +925,13 @@ def latent_prepare(buf: torch.Tensor, n_heads: int, q_head_dim: int, q_rot_off: 
 
 
 def head_linear(a: torch.Tensor, a_head: int, w: torch.Tensor, w_is_nk: bool, out: torch.Tensor, out_head: int, n_heads: int,
-                k: int, n: int, gate: torch.Tensor | None = None) -> torch.Tensor:
+                k: int, n: int, gate: torch.Tensor | None = None, *, fixed: bool = False) -> torch.Tensor:
     """One small product per head: out[t, h * out_head: h * out_head + n] = a[t, h * a_head: h * a_head + k] @ W[h], float32
     sums. `w` holds the heads' matrices one after the other: [n_heads * k, n] (each [k, n]; w_is_nk False) or [n_heads * n, k]
     (each [n, k], stored [out, in]; w_is_nk True). a and out are 2-D with contiguous rows and may be wider than the heads.
-    `gate` (laid out like out: head h's n numbers at gate[t, h * out_head:]) multiplies the outputs by its sigmoid."""
+    `gate` (laid out like out: head h's n numbers at gate[t, h * out_head:]) multiplies the outputs by its sigmoid.
+    `fixed`: the numbers of w are no output of the launches just before (a model's weights, a step's batch), so the kernel may read them ahead of
+    its wait for those."""
     _need(a, "a", dim=2)
     _need(w, "w", a.dtype, 2)
     _need(out, "out", a.dtype, 2)
@@ -938,7 +946,7 @@ def head_linear(a: torch.Tensor, a_head: int, w: torch.Tensor, w_is_nk: bool, ou
             raise KernelError(f"head_linear: gate {tuple(gate.shape)} does not fit {n_heads} heads of {n} at a distance of {out_head}")
         gate_stride = _rows(gate, "gate")
     status = _lib("latent_attention").r2_head_linear(_p(a), _rows(a, "a"), a_head, _p(w), int(w_is_nk), _p(out), _rows(out, "out"),
-                                                    out_head, a.shape[0], n_heads, k, n, _p(gate), gate_stride, dtype_code(a.dtype), _stream())
+                                                    out_head, a.shape[0], n_heads, k, n, _p(gate), gate_stride, dtype_code(a.dtype), int(fixed), _stream())
     _check(status, "head_linear")
     return out
 
@@ -986,11 +994,13 @@ def mlstm_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gates: torch.T
 
 
 def causal_conv(x: torch.Tensor, taps: torch.Tensor, bias: torch.Tensor | None, state: torch.Tensor, conv_state_off: int,
-                row_entry: torch.Tensor, q_start: torch.Tensor, state_slot: torch.Tensor, fresh: torch.Tensor) -> torch.Tensor:
+                row_entry: torch.Tensor, q_start: torch.Tensor, state_slot: torch.Tensor, fresh: torch.Tensor, *, fixed: bool = False) -> torch.Tensor:
     """silu of a causal convolution per channel: x [T, C] (a slice of a projection), taps float32 [C, n_taps] whose last
     column is the current token's. Inputs before an entry's first row come from the request's state slot (float32
     [slots, floats]; at `conv_state_off` the inputs of the last n_taps - 1 positions, [n_taps - 1, C]), zeros before a
-    sequence's start. The slot is read only: `ssd_scan` renews it. -> [T, C] in x's dtype."""
+    sequence's start. The slot is read only: `ssd_scan` renews it. -> [T, C] in x's dtype.
+    `fixed`: taps, bias and the index arrays are no output of the launches just before (a model's weights, a step's batch), so the kernel may read them ahead of
+    its wait for those."""
     _need(x, "x", dim=2)
     _need(taps, "taps", torch.float32, 2)
     _need(state, "state", torch.float32, 2)
@@ -1004,7 +1014,7 @@ def causal_conv(x: torch.Tensor, taps: torch.Tensor, bias: torch.Tensor | None, 
     out = torch.empty(x.shape[0], channels, dtype=x.dtype, device=x.device)
     status = _lib("recurrent").r2_causal_conv(
         _p(x), _rows(x, "x"), _p(out), _rows(out, "out"), _p(taps), _p(bias), n_taps, channels, _p(state), C.c_longlong(state.shape[1]),
-        C.c_longlong(conv_state_off), _p(row_entry), _p(q_start), _p(state_slot), _p(fresh), x.shape[0], dtype_code(x.dtype), _stream())
+        C.c_longlong(conv_state_off), _p(row_entry), _p(q_start), _p(state_slot), _p(fresh), x.shape[0], dtype_code(x.dtype), int(fixed), _stream())
     _check(status, "causal_conv")
     return out
 
@@ -1230,11 +1240,13 @@ def soft_cap(x: torch.Tensor, cap: float) -> torch.Tensor:
 
 
 def group_norm_gated(y: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor | None, n_groups: int, eps: float, gate_first,
-                     out_dtype: torch.dtype, out: torch.Tensor | None = None) -> torch.Tensor:
+                     out_dtype: torch.dtype, out: torch.Tensor | None = None, *, fixed: bool = False) -> torch.Tensor:
     """RMS norm of float32 rows y [T, C] in n_groups equal parts, each by its own root mean square, times weight [C], with
     a gate [T, C] (a slice of a projection, in out_dtype): `gate_first`: y * silu(gate) is what is normalised; else the
     normalised, weighted result is multiplied by sigmoid(gate), or, with gate_first "silu_after", by silu(gate). `weight` None:
-    a gain of one. -> [T, C] in out_dtype."""
+    a gain of one. -> [T, C] in out_dtype.
+    `fixed`: the gains are no output of the launches just before (a model's weights, a step's batch), so the kernel may read them ahead of
+    its wait for those."""
     _need(y, "y", torch.float32, 2)
     _need(gate, "gate", out_dtype, 2)
     if weight is not None:
@@ -1249,7 +1261,7 @@ def group_norm_gated(y: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor |
         raise KernelError(f"group_norm_gated: out {tuple(out.shape)} is not {tuple(y.shape)}")
     status = _lib("recurrent").r2_group_norm_gated(
         _p(y), _rows(y, "y"), _p(gate), _rows(gate, "gate"), _p(weight), _p(out), _rows(out, "out"), y.shape[0], n_groups,
-        y.shape[1] // n_groups, C.c_float(eps), 2 if gate_first == "silu_after" else int(bool(gate_first)), dtype_code(out_dtype), _stream())
+        y.shape[1] // n_groups, C.c_float(eps), 2 if gate_first == "silu_after" else int(bool(gate_first)), dtype_code(out_dtype), int(fixed), _stream())
     _check(status, "group_norm_gated")
     return out
 
@@ -1326,6 +1338,8 @@ def linear(a, w: torch.Tensor, bias: torch.Tensor | None = None, *, w_is_nk: boo
     """act(a @ w + bias) (+ residual). `w` is [K, N], or [N, K] with w_is_nk. `a` and `w`
     share a dtype; bias and residual are float32; a float32 residual makes a float32 result.
     `a` may be NormedRows: the LayerNorm then runs inside the product's kernel where it can.
+    In bfloat16 `w` must not come from this package's launches just before: the tensor-core kernels read a weight while those still
+    run (a synchronisation or a plain launch, such as a torch operation's, between them settles it). Float32 products take any `w`.
 
     With `kv` (a fused q/k/v product) the result is (out, written): where the tensor-core kernel
     takes the case (more than 64 bfloat16 rows), the key and value columns go straight into the

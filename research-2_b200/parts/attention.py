@@ -295,7 +295,7 @@ class RotaryWindowAttention:
         if writes_cache and not self.own_kv:
             raise ValueError("attention: a layer without keys and values of its own reads a cache member that another layer writes")
         proj = ops.linear(h, self.w_in, self.b_in, w_is_nk=True)
-        gate = ops.small_linear(h, self.w_gate, None) if self.w_gate is not None else None
+        gate = ops.small_linear(h, self.w_gate, None, fixed=True) if self.w_gate is not None else None
         at = self.q_width + self.k_width
         q, k, v = proj[:, : self.q_width], proj[:, self.q_width: at], proj[:, at:]
         fused_decode = ctx.decode_only and self.v_head_dim == self.head_dim
@@ -436,7 +436,7 @@ class LatentAttention:
             ops.latent_prepare(proj, H, self.q_head, d, self.rot_dim, self.rot_dims, self.kv_col, c, self.dkv_norm, self.norm_eps,
                                self.freqs, self.rot_magnitude, ctx.positions, q_out=queries, q_out_head_dim=self.row, q_out_off=c,
                                **to_cache)
-        ops.head_linear(q, self.q_head, self.w_uk, False, queries, self.row, H, d, c)
+        ops.head_linear(q, self.q_head, self.w_uk, False, queries, self.row, H, d, c, fixed=True)
         mixed = ops.paged_attention(
             queries, cache.k, cache.k, cache.page_stride, cache.page_size, cache.n_pages, ctx.block_tables[cache.group], ctx.row_entry,
             ctx.positions, ctx.seq_lens, H, 1, self.row, self.scale, self.window, decode_only=ctx.decode_only,
@@ -444,7 +444,7 @@ class LatentAttention:
             sinks=self.sinks)
         out = torch.empty(proj.shape[0], H * self.v_head_dim, dtype=proj.dtype, device=proj.device)
         gate = proj[:, self.kv_col + self.row:] if self.gated else None     # the gate's columns of the input product
-        ops.head_linear(mixed, c, self.w_uv, True, out, self.v_head_dim, H, c, self.v_head_dim, gate=gate)
+        ops.head_linear(mixed, c, self.w_uv, True, out, self.v_head_dim, H, c, self.v_head_dim, gate=gate, fixed=True)
         return out
 
     def mix(self, h, ctx, cache=None, state=None, writes_cache: bool = True):

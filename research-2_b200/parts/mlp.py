@@ -232,7 +232,7 @@ class RoutedExperts:
             if self.n_identity:
                 addend = carried[0]
         else:
-            route, _, _ = ops.route_top_k(h, self.router, self.router_b, self.top)
+            route, _, _ = ops.route_top_k(h, self.router, self.router_b, self.top, fixed=True)
         if not self.gated:
             return ops.routed_linear(h, self.w_gate_up, self.activation, route, self.expert_width), addend
         return ops.expert_act(ops.linear(h, self.w_gate_up, None, w_is_nk=True), self.activation, self.limit, self.alpha,

@@ -65,11 +65,11 @@ class MatrixMemory:
 
     def _inner(self, h, ctx, state):
         proj = ops.linear(h, self.w_in, None, w_is_nk=True)
-        gates = ops.small_linear(h, self.w_gates, self.b_gates)
+        gates = ops.small_linear(h, self.w_gates, self.b_gates, fixed=True)
         a, b = self.qk_width, 2 * self.qk_width
         o = ops.mlstm_scan(proj[:, :a], proj[:, a:b], proj[:, b: b + self.v_width], gates, self.gate_cap, self.head_dim ** -0.5,
                            state, ctx.q_start, ctx.state_slot, ctx.fresh, self.n_heads, self.head_dim, self.v_head_dim)
-        return ops.group_norm_gated(o, proj[:, b + self.v_width:], self.norm, self.n_heads, self.norm_eps, False, proj.dtype)
+        return ops.group_norm_gated(o, proj[:, b + self.v_width:], self.norm, self.n_heads, self.norm_eps, False, proj.dtype, fixed=True)
 
     def mix(self, h, ctx, cache=None, state=None, writes_cache: bool = True):
         return ops.linear(self._inner(h, ctx, state), self.w_out, None, w_is_nk=True, out_dtype=torch.float32)
@@ -127,8 +127,8 @@ class Retention:
         a, b = self.qk_width, 2 * self.qk_width
         o = ops.retention_scan(proj[:, :a], proj[:, a:b], proj[:, b: b + self.v_width], self.decay, self.head_dim ** -0.5, self.freqs,
                                self.rot_dims, ctx.positions, state, ctx.q_start, ctx.state_slot, ctx.fresh, self.n_heads, self.head_dim,
-                               self.v_head_dim, n_tiles=ctx.n_attention_tiles)
-        return ops.group_norm_gated(o, proj[:, b + self.v_width:], None, self.n_heads, self.norm_eps, "silu_after", proj.dtype)
+                               self.v_head_dim, n_tiles=ctx.n_attention_tiles, fixed=True)
+        return ops.group_norm_gated(o, proj[:, b + self.v_width:], None, self.n_heads, self.norm_eps, "silu_after", proj.dtype, fixed=True)
 
     def mix(self, h, ctx, cache=None, state=None, writes_cache: bool = True):
         return ops.linear(self._inner(h, ctx, state), self.w_out, None, w_is_nk=True, out_dtype=torch.float32)
@@ -190,8 +190,8 @@ class DecayAttention:
         a, b = self.qk_width, 2 * self.qk_width
         o = ops.retention_scan(proj[:, :a], proj[:, a:b], proj[:, b: b + self.inner_width], self.decay, 1.0, None, 0, ctx.positions, state,
                                ctx.q_start, ctx.state_slot, ctx.fresh, self.n_heads, self.head_dim, self.v_head_dim, silu=True,
-                               n_tiles=ctx.n_attention_tiles)
-        return ops.group_norm_gated(o, proj[:, b + self.inner_width:], self.norm, 1, self.norm_eps, False, proj.dtype, out=out)
+                               n_tiles=ctx.n_attention_tiles, fixed=True)
+        return ops.group_norm_gated(o, proj[:, b + self.inner_width:], self.norm, 1, self.norm_eps, False, proj.dtype, out=out, fixed=True)
 
     def mix(self, h, ctx, cache=None, state=None, writes_cache: bool = True):
         return ops.linear(self.inner(h, ctx, cache, state), self.w_out, None, w_is_nk=True, out_dtype=torch.float32)
@@ -248,15 +248,15 @@ class StateSpace:
 
     def _inner(self, h, ctx, state):
         proj = ops.linear(h, self.w_in, None, w_is_nk=True)
-        steps = ops.small_linear(h, self.w_steps, None)
+        steps = ops.small_linear(h, self.w_steps, None, fixed=True)
         z, xbc = proj[:, : self.inner], proj[:, self.inner:]
         mixed = ops.causal_conv(xbc, self.conv, self.conv_b, state, self.conv_state_off, ctx.row_entry, ctx.q_start,
-                                ctx.state_slot, ctx.fresh)
+                                ctx.state_slot, ctx.fresh, fixed=True)
         x, b = mixed[:, : self.inner], mixed[:, self.inner: self.inner + self.bc_width]
         y = ops.ssd_scan(x, b, mixed[:, self.inner + self.bc_width:], steps, self.dt_bias, self.a_log, self.d_skip, state,
                          ctx.q_start, ctx.state_slot, ctx.fresh, self.n_heads, self.n_groups, self.n_state, self.v_head_dim,
                          conv_in=xbc, conv_taps=self.conv_taps, conv_state_off=self.conv_state_off)
-        return ops.group_norm_gated(y, z, self.norm, self.norm_groups, self.norm_eps, True, proj.dtype)
+        return ops.group_norm_gated(y, z, self.norm, self.norm_groups, self.norm_eps, True, proj.dtype, fixed=True)
 
     def mix(self, h, ctx, cache=None, state=None, writes_cache: bool = True):
         return ops.linear(self._inner(h, ctx, state), self.w_out, None, w_is_nk=True, out_dtype=torch.float32)
@@ -323,7 +323,7 @@ class DeltaRule:
                                            ctx.state_slot, ctx.fresh)
         o = ops.delta_scan(qk, v, numbers, self.head_dim, state, ctx.q_start, ctx.state_slot, ctx.fresh, conv_in=raw, conv_taps=self.conv_taps,
                            conv_state_off=self.conv_state_off)
-        return ops.group_norm_gated(o, proj[:, self.channels:], self.norm, self.n_heads, self.norm_eps, "silu_after", proj.dtype)
+        return ops.group_norm_gated(o, proj[:, self.channels:], self.norm, self.n_heads, self.norm_eps, "silu_after", proj.dtype, fixed=True)
 
     def mix(self, h, ctx, cache=None, state=None, writes_cache: bool = True):
         return ops.linear(self._inner(h, ctx, state), self.w_out, None, w_is_nk=True, out_dtype=torch.float32)
@@ -387,7 +387,7 @@ class TimeMix:
         r, k, v, gate = (proj[:, i * self.group: i * self.group + self.inner_width] for i in range(4))
         o = ops.time_mix_scan(r, k, v, decay, self.bonus, state, ctx.q_start, ctx.state_slot, ctx.fresh, self.n_heads, self.head_dim,
                               row_in=h, row_state_off=self.row_state_off)
-        return ops.group_norm_gated(o, gate, self.norm, self.n_heads, self.norm_eps, "silu_after", proj.dtype, out=out)
+        return ops.group_norm_gated(o, gate, self.norm, self.n_heads, self.norm_eps, "silu_after", proj.dtype, out=out, fixed=True)
 
     def mix(self, h, ctx, cache=None, state=None, writes_cache: bool = True):
         return ops.linear(self.inner(h, ctx, cache, state), self.w_out, None, w_is_nk=True, out_dtype=torch.float32)

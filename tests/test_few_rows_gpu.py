@@ -94,3 +94,75 @@ def test_gated_norms_inside_and_beyond_what_is_kept(rows, groups, size, order):
     if order is not True:
         v = v * (torch.nn.functional.silu(z) if order == "silu_after" else torch.sigmoid(z))
     torch.testing.assert_close(got.double(), v, rtol=2.0 ** -8, atol=1e-6)   # one rounding to bfloat16, 2^-9, and float sums before it
+
+
+def made_just_before(rows, cols, consumer, dtype=torch.float32, size=1.0):
+    """consumer(w) right behind the launch that writes w [rows, cols] (a long one), and again once w has settled: the same bits."""
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(rows + cols)
+    a, b = (torch.randn(*s, generator=gen, device=DEV) for s in ((rows, 4096), (cols, 4096)))
+    for turn in range(10):
+        w = torch.full((rows, cols), float(turn), dtype=dtype, device=DEV)
+        if dtype == torch.bfloat16:
+            o.linear((a * (size / 64)).bfloat16(), b.bfloat16(), None, w_is_nk=True, out=w)
+        else:
+            o.linear(a * (size / 64), b, None, w_is_nk=True, out=w)
+        soon = consumer(w)
+        torch.cuda.synchronize()
+        late = consumer(w)
+        for x, y in zip(soon if isinstance(soon, tuple) else (soon,), late if isinstance(late, tuple) else (late,)):
+            assert torch.equal(x, y)
+
+
+def test_operands_that_the_launch_just_before_writes():
+    """Without the word that its weights are fixed, a kernel reads them only after the launch before it."""
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    h = torch.randn(4, 768, generator=gen, device=DEV)
+    made_just_before(768, 640, lambda w: o.linear(h, w))
+    made_just_before(640, 768, lambda w: o.linear(h, w, w_is_nk=True))
+    made_just_before(24, 768, lambda w: o.small_linear(h, w))
+    made_just_before(16, 768, lambda w: o.route_top_k(h, w, None, 2))
+    q, gate = torch.randn(4, 12 * 64, generator=gen, device=DEV).bfloat16(), torch.randn(4, 12 * 128, generator=gen, device=DEV).bfloat16()
+    made_just_before(12 * 64, 128, lambda w: o.head_linear(q, 64, w, False, torch.empty_like(gate), 128, 12, 64, 128, gate=gate), torch.bfloat16)
+    made_just_before(1, 768, lambda w: o.group_norm_gated(h, h, w[0], 12, 1e-5, True, torch.float32))
+    made_just_before(1, 768, lambda w: o.group_norm_gated(h, h, w[0], 1, 1e-5, False, torch.float32))
+    one = torch.arange(5, dtype=torch.int32, device=DEV)
+    old, new = torch.zeros_like(one), torch.ones_like(one)
+    state = torch.randn(4, 12 * 64 * 64, generator=gen, device=DEV)
+    made_just_before(768, 4, lambda w: o.causal_conv(h, w, None, state, 0, one[:4], one, one[:4], old))
+    # retention's decays: a decode step, and chunks of a prompt (fresh entries: the slots' contents are not read)
+    for n in (4, 100):
+        x = torch.randn(n, 12 * 64, generator=gen, device=DEV).bfloat16()
+        start = one if n == 4 else torch.tensor([0, n], dtype=torch.int32, device=DEV)
+        freq, positions = torch.rand(16, generator=gen, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV)
+        made_just_before(1, 12, lambda w: o.retention_scan(x, x, x, w[0], 0.125, freq, 32, positions, state, start, one, new, 12, 64, 64, n_tiles=2), size=0.2)
+
+
+def test_fixed_operands_change_no_bit():
+    """With that word weights and the batch's arrays are asked for ahead of the wait, in instances of their own."""
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    rand = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    one = torch.arange(9, dtype=torch.int32, device=DEV)
+    fresh = (one % 2).int()
+    for n in (3, 80):
+        h, start = rand(n, 768), one[: n + 1] if n == 3 else torch.tensor([0, n], dtype=torch.int32, device=DEV)
+        entry = one[:n] if n == 3 else torch.zeros(n, dtype=torch.int32, device=DEV)
+        w, taps, gain, state = rand(24, 768), rand(768, 4), rand(768), rand(8, 12 * 64 * 64)
+        q, gate, heads = rand(n, 768).bfloat16(), rand(n, 1536).bfloat16(), rand(768, 128).bfloat16()
+        freq, positions, decay = torch.rand(16, generator=gen, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV), torch.full((12,), 0.9, device=DEV)
+
+        def retention(fixed, silu):
+            mine = state.clone()
+            out = o.retention_scan(q, q, q, decay, 0.125, None if silu else freq, 0 if silu else 32, positions, mine, start, one, fresh, 12, 64, 64, silu, 2, fixed=fixed)
+            return torch.cat([out.reshape(-1), mine.reshape(-1)])
+
+        calls = [lambda f: o.small_linear(h, w, None, fixed=f), lambda f: o.small_linear(h[:, :766], w[:, :766].contiguous(), None, fixed=f),
+                 lambda f: o.route_top_k(h, w, None, 2, fixed=f)[0], lambda f: o.causal_conv(h, taps, gain, state, 0, entry, start, one, fresh, fixed=f),
+                 lambda f: o.head_linear(q, 64, heads, False, torch.empty_like(gate), 128, 12, 64, 128, fixed=f),
+                 lambda f: o.head_linear(q, 64, heads, False, torch.empty_like(gate), 128, 12, 64, 128, gate=gate, fixed=f),
+                 lambda f: retention(f, False), lambda f: retention(f, True)]
+        calls += [lambda f, g=g: o.group_norm_gated(h, h, gain, g, 1e-5, True, torch.float32, fixed=f) for g in (24, 12, 6, 1)]
+        for i, call in enumerate(calls):
+            assert torch.equal(call(True), call(False)), (n, i)
