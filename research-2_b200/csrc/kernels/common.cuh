@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 // Launcher status: 0 = launched; > 0 = a CUDA runtime error code; < 0 = refused before launch.
 #define R2_OK 0
 #define R2_BAD_DTYPE (-1)
@@ -151,6 +153,21 @@ static inline void r2_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
   config.attrs = attr;
   config.numAttrs = (g_r2_pdl && !t_r2_plain_order) ? 1 : 0;
   cudaLaunchKernelEx(&config, kernel, static_cast<Args&&>(args)...);  // a failure shows in launch_status()
+}
+
+// Dynamic shared memory beyond the default 48 KB, allowed once per kernel instance and device (an instance has a `done` of its own) and up
+// to the most that any of its launches asks for: the limit belongs to the function, so a launch that set it to its own size could lower
+// it between another thread's setting and launch, which would then be refused.
+template <typename... KArgs>
+static inline int allow_smem(void (*kernel)(KArgs...), size_t most, std::atomic<bool> (&done)[64]) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return int(e);
+  if (device < 64 && done[device].load(std::memory_order_acquire)) return R2_OK;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most));
+  if (e != cudaSuccess) return int(e);
+  if (device < 64) done[device].store(true, std::memory_order_release);
+  return R2_OK;
 }
 
 static inline int launch_status() {

@@ -404,6 +404,8 @@ int launch_clustered(void (*kernel)(KArgs...), dim3 grid, int threads, size_t sm
   return launch_status();
 }
 
+constexpr size_t MOST_SMEM = 227 * 1024;
+
 template <typename TA, typename TW, typename TO, bool W_IS_NK, int MR>
 int launch_rows(const Product& p, cudaStream_t stream) {
   const int len = slice_len(p.k_total), n_slices = (p.k_total + len - 1) / len, n_groups = (n_slices + GROUP - 1) / GROUP;
@@ -414,10 +416,8 @@ int launch_rows(const Product& p, cudaStream_t stream) {
   const int per_cta = ranks == 1 ? n_slices : GROUP;
   const size_t smem = sizeof(float) * (size_t(per_cta) * MR * ROW_COLS + size_t(MR) * per_cta * len + (W_IS_NK ? ROW_WARPS * 32 * 33 : 0));
   auto kernel = gemm_rows_kernel<TA, TW, TO, W_IS_NK, MR>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e != cudaSuccess) return int(e);
-  }
+  static std::atomic<bool> allowed[64];
+  if (int status = allow_smem(kernel, MOST_SMEM, allowed)) return status;
   int grid_y = blocks;
   if (ranks == 1) {   // as many CTAs as are resident: the rows are staged once, and a warp's next lines are on their way over a block's end
     const int resident = int(size_t(220) * 1024 / (smem + 1024));
@@ -432,11 +432,10 @@ int launch_tiles(const Product& p, bool vec, int n_groups, int ranks, cudaStream
   const dim3 grid((p.n_total + BN - 1) / BN, (p.m_total + BM - 1) / BM, ranks);
   constexpr bool FLOATS = sizeof(TA) == 4 && sizeof(TW) == 4;
   const size_t smem = sizeof(float) * (2 * BK * (BM + 4) + 2 * BK * (BN + 4) + 2 * BM * BN);
-  auto kernel = vec && FLOATS ? gemm_tile_kernel<TA, TW, TO, W_IS_NK, BM, BN, FLOATS> : gemm_tile_kernel<TA, TW, TO, W_IS_NK, BM, BN, false>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e != cudaSuccess) return int(e);
-  }
+  const bool pieces = vec && FLOATS;
+  auto kernel = pieces ? gemm_tile_kernel<TA, TW, TO, W_IS_NK, BM, BN, FLOATS> : gemm_tile_kernel<TA, TW, TO, W_IS_NK, BM, BN, false>;
+  static std::atomic<bool> allowed[2][64];
+  if (int status = allow_smem(kernel, MOST_SMEM, allowed[pieces])) return status;
   return launch_clustered(kernel, grid, BM * BN / 64, smem, 2, stream, p, (n_groups + ranks - 1) / ranks);
 }
 

@@ -133,3 +133,35 @@ def test_tiles_of_forbidden_keys_weigh_nothing(near, with_sinks, dtype, decoded)
         got = o.decode_attention_fused(case.q_rows, case.k_new, case.v_new, case.slots, case.k_cache, case.v_cache, case.page_stride, case.page, case.n_pages,
                                        case.tables, case.row_entry, case.positions, case.seq_lens, heads, 2, dim, scale, 0, 700, **extras)
         torch.testing.assert_close(got.double().cpu(), want, **close)
+
+
+def test_threads_with_products_of_different_sizes():
+    """Two host threads on streams of their own take turns on one kernel instance with different needs of shared memory: no launch is refused."""
+    import threading
+
+    o, failed = ops(), []
+    gen = torch.Generator(device=DEV).manual_seed(9)
+    sizes = [(8, 4096, 2600), (8, 1600, 2600)]   # (rows, K, N): eight rows of K floats are staged
+    operands = [(torch.randn(m, k, generator=gen, device=DEV), torch.randn(k, n, generator=gen, device=DEV)) for m, k, n in sizes]
+    want = [o.linear(a, w) for a, w in operands]
+    torch.cuda.synchronize()
+
+    def work(i):
+        stream = torch.cuda.Stream()
+        try:
+            with torch.cuda.stream(stream):
+                a, w = operands[i]
+                out = torch.empty_like(want[i])
+                for _ in range(1500):
+                    o.linear(a, w, out=out)
+            stream.synchronize()
+            assert torch.equal(out, want[i])
+        except Exception as ex:  # noqa: BLE001
+            failed.append(ex)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
