@@ -22,7 +22,7 @@
 // Queries and keys that are rotated by position on their way in (retention; in float, so that what enters the recurrence is never
 // rounded to 16 bits) take three terms (24 bits, a float's) and the six products above 2^-24 of them; values are then bfloat16
 // already and one term. What bounded the walk row by row was its chain, 160 to 270 us for portions of up to 1,000 rows, 12 heads of
-// 32 x 64, whatever their number of heads; in chunks the outputs, the longest of the three launches, take 17.5.
+// 32 x 64, whatever their number of heads; in chunks the three launches take 32 (700 and 324 rows; 235 row by row on the same GPU).
 #include <math.h>
 
 #include "common.cuh"
@@ -92,6 +92,18 @@ __device__ __forceinline__ float power(float decay, int n) {
     if (n & 1) out *= square;
   return out;
 }
+
+// The same to 48 bits: a float's rounding and what it leaves. (A factor's own error is the same at every chunk, so it adds up over a
+// state's memory where roundings cancel: by squaring in float, 900 rows of a decay of 1 - 2^-8 were off by four times the walk's error.)
+__device__ __forceinline__ float2 exact_power(float decay, int n) {
+  double out = 1.0, square = decay;
+  for (; n > 0; n >>= 1, square *= square)
+    if (n & 1) out *= square;
+  const float head = float(out);
+  return make_float2(head, float(out - double(head)));
+}
+template <int N>
+__device__ __forceinline__ float power_for(float decay, int n) { return N > 2 ? exact_power(decay, n).x : power(decay, n); }
 
 // A matrix in shared memory as N bfloat16 terms, rows `stride` numbers apart.
 template <int N>
@@ -192,15 +204,41 @@ __device__ __forceinline__ void load_b_transposed(const bf16* m, int stride, int
   ldmatrix_x4_trans(smem_u32(m + (k + (lane & 15)) * stride + n + (lane >> 4) * 8), f[0], f[1], f[2], f[3]);
 }
 // (the sum of a's terms)(the sum of b's terms) for one tile of 8 columns, smallest products first; those below the last term of the longer
-// operand are left out
+// operand are left out. The tensor core cuts its sums off instead of rounding them, a bias that grows with every step along K. Three
+// terms are there for a float's accuracy, so theirs keeps the large products' sums of 16 apart, added by rounding additions, and the
+// small products (2^-8 of them) in an accumulator of their own, `low`. (A prompt of 900 rows, 12 heads of 32 x 64, against 64 bits: the walk
+// row by row 2.3e-7, one accumulator for all and powers by squaring in float 6.1e-7, now 1.1e-7.)
 template <int N, int M>
-__device__ __forceinline__ void mma_split(float (&c)[4], const uint32_t (&a)[N][4], const uint32_t (&b)[M][4], int half) {
+__device__ __forceinline__ void mma_split(float (&c)[4], float (&low)[4], const uint32_t (&a)[N][4], const uint32_t (&b)[M][4], int half) {
 #pragma unroll
   for (int order = (N > M ? N : M) - 1; order >= 0; --order)
 #pragma unroll
     for (int i = N - 1; i >= 0; --i) {
       const int j = order - i;
-      if (j >= 0 && j < M) mma_bf16(c, a[i][0], a[i][1], a[i][2], a[i][3], b[j < 0 || j >= M ? 0 : j][2 * half], b[j < 0 || j >= M ? 0 : j][2 * half + 1]);
+      if (j < 0 || j >= M) continue;
+      const int at = j < 0 || j >= M ? 0 : j;
+      if (N == 2) {
+        mma_bf16(c, a[i][0], a[i][1], a[i][2], a[i][3], b[at][2 * half], b[at][2 * half + 1]);
+      } else if (order > 0) {
+        mma_bf16(low, a[i][0], a[i][1], a[i][2], a[i][3], b[at][2 * half], b[at][2 * half + 1]);
+      } else {
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_bf16(sum, a[i][0], a[i][1], a[i][2], a[i][3], b[at][2 * half], b[at][2 * half + 1]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) c[u] += sum[u];
+      }
+    }
+}
+// the small products' sums join the large ones'
+template <int N, int TILES>
+__device__ __forceinline__ void join(float (&c)[TILES][4], float (&low)[TILES][4]) {
+  if (N == 2) return;
+#pragma unroll
+  for (int t = 0; t < TILES; ++t)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      c[t][u] += low[t][u];
+      low[t][u] = 0.f;
     }
 }
 
@@ -225,7 +263,7 @@ decay_chunk_sums_kernel(const ChunkArgs a) {
   __shared__ float powers[CHUNK];
   const Tile tile = find_tile(a.q_start, a.n_entries, blockIdx.x);
   const int h = blockIdx.y, col0 = blockIdx.z * COLS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < CHUNK; i += THREADS) powers[i] = power(a.decay[h], i);
+  for (int i = threadIdx.x; i < CHUNK; i += THREADS) powers[i] = power_for<N>(a.decay[h], i);
   __syncthreads();
   pdl_wait_after_operands<FIXED>();
   if (tile.entry < 0) return;
@@ -243,7 +281,7 @@ decay_chunk_sums_kernel(const ChunkArgs a) {
   __syncthreads();
   float* sums = a.sums + (size_t(blockIdx.x) * a.n_heads + h) * a.dim * a.vdim + col0;
   for (int m0 = warp * 16; m0 < a.dim16; m0 += (THREADS / 32) * 16) {
-    float acc[COLS / 8][4] = {};
+    float acc[COLS / 8][4] = {}, acc_low[COLS / 8][4] = {};
     for (int j = 0; j < tile.rows; j += 16) {
       uint32_t kf[N][4];
 #pragma unroll
@@ -253,10 +291,11 @@ decay_chunk_sums_kernel(const ChunkArgs a) {
         uint32_t vf[M][4];
 #pragma unroll
         for (int i = 0; i < M; ++i) load_b_transposed(v.term[i], v.stride, j, n, vf[i]);
-        mma_split(acc[n / 8], kf, vf, 0);
-        mma_split(acc[n / 8 + 1], kf, vf, 1);
+        mma_split(acc[n / 8], acc_low[n / 8], kf, vf, 0);
+        mma_split(acc[n / 8 + 1], acc_low[n / 8 + 1], kf, vf, 1);
       }
     }
+    join<N>(acc, acc_low);
 #pragma unroll
     for (int t = 0; t < COLS / 8; ++t) {
       const int c = t * 8 + (lane & 3) * 2;
@@ -278,7 +317,7 @@ decay_chunk_sums_kernel(const ChunkArgs a) {
 }
 
 // The states at the chunks' starts, and the request's new one. Grid: entries, heads, pieces of the state.
-template <bool FIXED>
+template <int N, bool FIXED>
 __global__ void __launch_bounds__(256)
 decay_chunk_states_kernel(const ChunkArgs a) {
   pdl_launch_dependents();
@@ -292,7 +331,9 @@ decay_chunk_states_kernel(const ChunkArgs a) {
   const bool is_fresh = a.fresh[e] != 0;
   const int size = a.dim * a.vdim, i = blockIdx.z * blockDim.x + threadIdx.x;
   const float decay = a.decay[h];
-  const float whole = power(decay, CHUNK), last = power(decay, rows - (rows - 1) / CHUNK * CHUNK);
+  const int last_rows = rows - (rows - 1) / CHUNK * CHUNK;
+  const float2 whole = N > 2 ? exact_power(decay, CHUNK) : make_float2(power(decay, CHUNK), 0.f);
+  const float2 last = N > 2 ? exact_power(decay, last_rows) : make_float2(power(decay, last_rows), 0.f);
   pdl_wait_after_operands<FIXED>();
   if (rows <= 0 || i >= size) return;   // an entry without rows touches no slot
   float* slot = a.state + size_t(a.state_slot[e]) * a.slot_stride + size_t(h) * size + i;
@@ -308,7 +349,8 @@ decay_chunk_states_kernel(const ChunkArgs a) {
     for (int c = 0; c < 8; ++c) {
       if (base + c < n) {
         sums[(base + c) * step] = s;
-        s = fmaf(base + c == n - 1 ? last : whole, s, u[c]);
+        const float2 keep = base + c == n - 1 ? last : whole;
+        s = fmaf(keep.x, s, N > 2 ? fmaf(keep.y, s, u[c]) : u[c]);
       }
     }
   }
@@ -325,7 +367,7 @@ decay_chunk_outputs_kernel(const ChunkArgs a) {
   __shared__ float powers[CHUNK + 1];
   const Tile tile = find_tile(a.q_start, a.n_entries, blockIdx.x);
   const int h = blockIdx.y, col0 = blockIdx.z * COLS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i <= CHUNK; i += THREADS) powers[i] = power(a.decay[h], i);
+  for (int i = threadIdx.x; i <= CHUNK; i += THREADS) powers[i] = power_for<N>(a.decay[h], i);
   __syncthreads();
   pdl_wait_after_operands<FIXED>();
   if (tile.entry < 0) return;
@@ -352,7 +394,7 @@ decay_chunk_outputs_kernel(const ChunkArgs a) {
   const int i0 = warp * 16;
   if (i0 >= tile.rows) return;   // (no barrier follows)
   // what the chunk's first state gives, and the scores of the rows up to each row
-  float acc[COLS / 8][4] = {}, p[CHUNK / 8][4] = {};
+  float acc[COLS / 8][4] = {}, acc_low[COLS / 8][4] = {}, p[CHUNK / 8][4] = {}, p_low[CHUNK / 8][4] = {};
   for (int d = 0; d < a.dim16; d += 16) {
     uint32_t qf[N][4];
 #pragma unroll
@@ -362,8 +404,8 @@ decay_chunk_outputs_kernel(const ChunkArgs a) {
       uint32_t sf[N][4];
 #pragma unroll
       for (int i = 0; i < N; ++i) load_b_transposed(s.term[i], s.stride, d, n, sf[i]);
-      mma_split(acc[n / 8], qf, sf, 0);
-      mma_split(acc[n / 8 + 1], qf, sf, 1);
+      mma_split(acc[n / 8], acc_low[n / 8], qf, sf, 0);
+      mma_split(acc[n / 8 + 1], acc_low[n / 8 + 1], qf, sf, 1);
     }
 #pragma unroll
     for (int j = 0; j < CHUNK; j += 16) {
@@ -371,11 +413,13 @@ decay_chunk_outputs_kernel(const ChunkArgs a) {
         uint32_t kf[N][4];
 #pragma unroll
         for (int i = 0; i < N; ++i) load_b(k.term[i], k.stride, j, d, kf[i]);
-        mma_split(p[j / 8], qf, kf, 0);
-        mma_split(p[j / 8 + 1], qf, kf, 1);
+        mma_split(p[j / 8], p_low[j / 8], qf, kf, 0);
+        mma_split(p[j / 8 + 1], p_low[j / 8 + 1], qf, kf, 1);
       }
     }
   }
+  join<N>(acc, acc_low);
+  join<N>(p, p_low);
   const int r = i0 + (lane >> 2);   // this lane's rows: r and r + 8
   const float lead0 = powers[r + 1], lead1 = powers[r + 9];
 #pragma unroll
@@ -412,10 +456,11 @@ decay_chunk_outputs_kernel(const ChunkArgs a) {
       uint32_t vf[M][4];
 #pragma unroll
       for (int i = 0; i < M; ++i) load_b_transposed(v.term[i], v.stride, j, n, vf[i]);
-      mma_split(acc[n / 8], wf, vf, 0);
-      mma_split(acc[n / 8 + 1], wf, vf, 1);
+      mma_split(acc[n / 8], acc_low[n / 8], wf, vf, 0);
+      mma_split(acc[n / 8 + 1], acc_low[n / 8 + 1], wf, vf, 1);
     }
   }
+  join<N>(acc, acc_low);
   float* out = a.out + size_t(h) * a.vdim + col0;
   const bool pairs = (a.vdim & 1) == 0 && (a.out_stride & 1) == 0;
 #pragma unroll
@@ -554,7 +599,7 @@ int launch_chunks(const ChunkArgs& a, int n_tiles, cudaStream_t stream) {
   }
   const dim3 grid(n_tiles, a.n_heads, (a.vdim + COLS - 1) / COLS);
   r2_launch(decay_chunk_sums_kernel<N, M, FIXED>, grid, dim3(THREADS), smem_sums, stream, a);
-  r2_launch(decay_chunk_states_kernel<FIXED>, dim3(a.n_entries, a.n_heads, (a.dim * a.vdim + 255) / 256), dim3(256), size_t(0), stream, a);
+  r2_launch(decay_chunk_states_kernel<N, FIXED>, dim3(a.n_entries, a.n_heads, (a.dim * a.vdim + 255) / 256), dim3(256), size_t(0), stream, a);
   r2_launch(decay_chunk_outputs_kernel<N, M, FIXED>, grid, dim3(THREADS), smem_out, stream, a);
   return launch_status();
 }
