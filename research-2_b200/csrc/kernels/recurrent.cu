@@ -366,10 +366,7 @@ outer_scan_kernel(const ScanArgs a) {
 
 // How a head's state is spread over threads: RPT rows of a column in a thread's registers, a column's rows over G
 // neighbouring lanes (a power of two up to 32), cv columns a CTA and the columns over 1, 2, 4 or 8 CTAs: as few as the
-// threads of a CTA allow, and more while the launch has fewer CTAs than the GPU has SMs. `wide`: 256 threads (decode steps, and the
-// walk with a fixed decay, whose tiles are not copied ahead: 16 entries of 64 rows 57 us, 87 with 64 threads). Prompts of the other two
-// take 64: of a batch's entries few are long, and those then have their columns over as many SMs as there are slices (900 rows beside
-// 7 decoded ones, 12 heads of 64 x 64, matrix memory: 311 us with 256 threads, 242; 16 entries of 64 rows 59 and 55).
+// threads of a CTA allow, and more while the launch has fewer CTAs than the GPU has SMs. `wide`: 256 threads instead of SCAN_THREADS.
 struct ScanShape { int rpt, G, threads, cv, splits; };
 
 ScanShape scan_shape(int rows, int cols, int pairs, bool wide, int per_piece) {
@@ -392,28 +389,64 @@ ScanShape scan_shape(int rows, int cols, int pairs, bool wide, int per_piece) {
   return s;
 }
 
+// A walk's launch. Tiles are copied ahead (`pieces`) where whole 16-byte pieces can be (`aligned`: the operands' addresses and strides) and
+// two stages fit beside the floats. With the rows' sums four at a time: 900 rows beside 7 decoded ones, 12 heads, state space of 32 x 64
+// 245 to 103 us, matrix memory of 64 x 64 477 to 242; what is left is a warp's issue and latencies (some 90 instructions a row, one
+// warp to a scheduler).
+// Such prompts take 64 threads: of a batch's entries few are long, and those then have their columns over as many SMs as there are
+// slices (that matrix memory: 311 us with 256 threads, 242; 16 entries of 64 rows 59 and 55). A walk that stages a tile when it begins
+// takes 256, since every slice stages the vectors again (16 entries of 64 rows, the fixed decay: 57 us, 87 with 64 threads; matrix
+// memory of 64 x 64 in unaligned rows 59 and 75, state space 78 and 97), and so do decode steps.
+// The room for the copies is what two CTAs to an SM leave: in 48 KB only bfloat16 heads of up to 64 rows and 65 to 150, and float32
+// heads of up to 32, had it (900 rows beside 7 decoded ones, matrix memory: float32 64 x 64 391 us without copies, 250 with; bfloat16 200 x 64
+// 2,189 and 1,441).
+struct ScanPlan { ScanShape shape; int tile, pieces; size_t smem; };
+
+constexpr size_t SCAN_SMEM = 48 * 1024, AHEAD_SMEM = 100 * 1024;   // without and with tiles copied ahead (two such CTAs to an SM)
+
+ScanPlan scan_plan(int rows, int cols, int pairs, bool single_rows, bool fixed_decay, int elem, bool aligned) {
+  const int per_piece = 16 / elem;
+  ScanPlan p = {};
+  auto take = [&](bool wide) {
+    p.shape = scan_shape(rows, cols, pairs, wide, per_piece);
+    p.tile = single_rows ? SMALL_TILE : (p.shape.rpt <= 16 ? MAX_TILE : 16);
+    p.smem = sizeof(float) * (size_t(p.tile) * (2 * p.shape.rpt * p.shape.G + p.shape.cv) + 3 * p.tile);
+  };
+  if (!single_rows && !fixed_decay) {
+    take(false);
+    const size_t raw = 2 * size_t(p.tile) * (2 * rows + p.shape.cv) * elem;
+    p.pieces = aligned && p.smem <= SCAN_SMEM && p.smem + raw <= AHEAD_SMEM && rows % per_piece == 0 && cols % per_piece == 0 && p.shape.cv % per_piece == 0;
+    if (p.pieces) {
+      p.smem += raw;
+      return p;
+    }
+  }
+  take(true);
+  if (p.smem > SCAN_SMEM && !single_rows && !fixed_decay) take(false);   // (narrower slices may still fit)
+  return p;
+}
+
 template <typename T, int MODE>
 int launch_scan(const ScanArgs& in, int n_entries, int n_heads, cudaStream_t stream) {
   ScanArgs a = in;
-  const ScanShape s = scan_shape(a.rows, a.cols, n_entries * n_heads, a.single_rows != 0 || MODE == MODE_DECAY, 16 / int(sizeof(T)));
-  const int rpt = s.rpt, G = s.G, threads = s.threads, splits = s.splits;
-  if (G > 32 || threads > 256) return R2_UNSUPPORTED;
-  a.G = G;
-  a.cv = s.cv;
   const bool single_rows = a.single_rows != 0;
-  const int tile = single_rows ? SMALL_TILE : (rpt <= 16 ? MAX_TILE : 16);
-  size_t smem = sizeof(float) * (size_t(tile) * (2 * rpt * G + a.cv) + 3 * tile);
-  if (smem > 48 * 1024) return R2_UNSUPPORTED;
-  // Tiles are copied ahead where whole 16-byte pieces can be. With the rows' sums four at a time: 900 rows beside 7 decoded ones, 12
-  // heads, state space of 32 x 64 245 to 103 us, matrix memory of 64 x 64 477 to 242; what is left is a warp's issue and latencies
-  // (some 90 instructions a row, one warp to a scheduler).
-  const size_t raw = 2 * size_t(tile) * (2 * a.rows + a.cv) * sizeof(T);
   auto on_pieces = [](const void* p, int stride) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && stride * sizeof(T) % 16 == 0; };
-  a.pieces = !single_rows && MODE != MODE_DECAY && smem + raw <= 48 * 1024 && a.rows * sizeof(T) % 16 == 0 && a.cols * sizeof(T) % 16 == 0 &&
-             a.cv * sizeof(T) % 16 == 0 && on_pieces(a.read, a.read_stride) && on_pieces(a.write, a.write_stride) && on_pieces(a.value, a.value_stride);
-  if (a.pieces) smem += raw;
+  const bool aligned = on_pieces(a.read, a.read_stride) && on_pieces(a.write, a.write_stride) && on_pieces(a.value, a.value_stride);
+  const ScanPlan plan = scan_plan(a.rows, a.cols, n_entries * n_heads, single_rows, MODE == MODE_DECAY, int(sizeof(T)), aligned);
+  const int rpt = plan.shape.rpt, threads = plan.shape.threads, splits = plan.shape.splits;
+  const size_t smem = plan.smem;
+  if (plan.shape.G > 32 || threads > 256 || smem > (plan.pieces ? AHEAD_SMEM : SCAN_SMEM)) return R2_UNSUPPORTED;
+  a.G = plan.shape.G;
+  a.cv = plan.shape.cv;
+  a.pieces = plan.pieces;
   dim3 grid(n_entries, n_heads, splits);
-#define R2_SCAN(RPT_, TILE_) r2_launch(outer_scan_kernel<T, RPT_, MODE, TILE_>, grid, dim3(threads), smem, stream, a)
+#define R2_SCAN(RPT_, TILE_)                                                                        \
+  do {                                                                                              \
+    static std::atomic<bool> allowed[64];                                                           \
+    if (smem > SCAN_SMEM)                                                                           \
+      if (int status = allow_smem(outer_scan_kernel<T, RPT_, MODE, TILE_>, AHEAD_SMEM, allowed)) return status; \
+    r2_launch(outer_scan_kernel<T, RPT_, MODE, TILE_>, grid, dim3(threads), smem, stream, a);       \
+  } while (0)
   switch (rpt) {
     case 4: if (single_rows) R2_SCAN(4, SMALL_TILE); else R2_SCAN(4, MAX_TILE); break;
     case 8: if (single_rows) R2_SCAN(8, SMALL_TILE); else R2_SCAN(8, MAX_TILE); break;
@@ -595,6 +628,15 @@ extern "C" int r2_mlstm_scan(const void* q, int q_stride, const void* k, int k_s
   if (dtype == R2_F32) return launch_scan<float, MODE_MLSTM>(a, n_entries, n_heads, stream);
   if (dtype == R2_BF16) return launch_scan<bf16, MODE_MLSTM>(a, n_entries, n_heads, stream);
   return R2_BAD_DTYPE;
+}
+
+// The launch that a prompt's walk of the matrix memory or the state space takes (profiles, tests): threads of a CTA, slices of the columns,
+// and whether its tiles are copied ahead.
+extern "C" void r2_scan_plan(int rows, int cols, int n_entries, int n_heads, int dtype, int aligned, int* threads, int* splits, int* copied) {
+  const ScanPlan p = scan_plan(rows, cols, n_entries * n_heads, false, false, dtype == R2_F32 ? 4 : 2, aligned != 0);
+  *threads = p.shape.threads;
+  *splits = p.shape.splits;
+  *copied = p.pieces;
 }
 
 // Retention: S <- decay[h] S + k v^T, o = S^T q per head, with q and k rotated by position (the first rot_dims dimensions

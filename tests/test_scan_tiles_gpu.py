@@ -3,6 +3,8 @@ same bits whether rows can be copied in 16-byte pieces or not and however an ent
 
 from __future__ import annotations
 
+import ctypes as C
+
 import pytest
 import torch
 
@@ -51,6 +53,12 @@ def walk64(kind, rows, start, slot, fresh, state, heads, dim, vdim, data):
                 o = torch.einsum("hij,i->hj", s, data["c"][t]) + data["skip"][:, None] * data["x"][t]
             out[t] = o.reshape(-1)
     return out
+
+
+def scan_plan(dim, vdim, n, heads, dtype, aligned=True):
+    out = [C.c_int(0) for _ in range(3)]
+    ops()._lib("recurrent").r2_scan_plan(dim, vdim, n, heads, ops().dtype_code(dtype), int(aligned), *[C.byref(x) for x in out])
+    return out[0].value, out[1].value, bool(out[2].value)
 
 
 # heads of whole and of odd pieces, one to sixteen lanes a column, slices of one and of many columns
@@ -123,3 +131,19 @@ def test_walks_at_the_edges_of_their_tiles(heads, dim, vdim, dtype):
         got = o.mlstm_scan(*part, 15.0, dim ** -0.5, mine, torch.tensor([0, end - begin], dtype=torch.int32, device=DEV), slot[last:].contiguous(),
                            torch.tensor([int(fresh[last]) if begin == 0 else 0], dtype=torch.int32, device=DEV), heads, dim, vdim)
         assert torch.equal(got, both[0][0][row0 + begin: row0 + end])
+
+
+@pytest.mark.parametrize("dim,vdim,dtype,copied", [(64, 64, torch.bfloat16, True), (32, 64, torch.float32, True), (96, 40, torch.bfloat16, True), (128, 64, torch.bfloat16, True),
+                                                   (64, 64, torch.float32, True), (200, 64, torch.bfloat16, True), (128, 64, torch.float32, True),
+                                                   (20, 36, torch.bfloat16, False), (22, 64, torch.float32, False)])
+def test_only_walks_whose_tiles_are_copied_ahead_are_cut_into_narrow_slices(dim, vdim, dtype, copied):
+    """A slice stages a row's two vectors again: without the copies ahead 64 threads a CTA are slower than 256."""
+    threads, splits, ahead = scan_plan(dim, vdim, 16, 12, dtype)
+    assert ahead == copied
+    if copied:
+        assert threads <= 64 or splits == 8
+    lanes = 1   # of a column
+    while lanes * min(32, max(4, 1 << (-(-dim // 4) - 1).bit_length())) < dim:
+        lanes *= 2
+    for t, s, a in [(threads, splits, ahead)] * (not copied) + [scan_plan(dim, vdim, 16, 12, dtype, aligned=False)]:
+        assert not a and (s == 1 or -(-vdim // (s // 2)) * lanes > 256), (t, s)   # half as many slices would not fit a CTA
