@@ -49,7 +49,7 @@ small_linear_kernel(const T* __restrict__ h, int h_stride, const float* __restri
                     float* __restrict__ out, int out_stride, int n_out, int width, int n_rows, int rows_per_cta) {
   pdl_launch_dependents();
   pdl_wait_before_operands<FIXED>();
-  const int lane = threadIdx.x & 31, n = blockIdx.y * SMALL_WARPS + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, n = blockIdx.x * SMALL_WARPS + (threadIdx.x >> 5);
   const float* wr = w + size_t(n < n_out ? n : 0) * width;
   float4 ahead[QUADS ? SMALL_AHEAD : 1];
   if (QUADS) {
@@ -62,7 +62,7 @@ small_linear_kernel(const T* __restrict__ h, int h_stride, const float* __restri
   const float b = bias != nullptr && n < n_out ? bias[n] : 0.f;
   pdl_wait_after_operands<FIXED>();
   if (n >= n_out) return;
-  const int t0 = blockIdx.x * rows_per_cta, t1 = min(n_rows, t0 + rows_per_cta);
+  const int t0 = blockIdx.y * rows_per_cta, t1 = min(n_rows, t0 + rows_per_cta);
   for (int t = t0; t < t1; ++t) {
     const T* hr = h + size_t(t) * h_stride;
     float acc = 0.f;
@@ -502,8 +502,9 @@ extern "C" int r2_small_linear(const void* h, int h_stride, const float* w, cons
   const size_t four = dtype == R2_F32 ? 16 : 8;   // bytes of four numbers of h
   const bool quads = width % 4 == 0 && h_stride % 4 == 0 && reinterpret_cast<uintptr_t>(h) % four == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0;
   // many rows: eight to a CTA, whose warps then read their weights once for them (an output's sum is the same either way)
-  const int rows_per_cta = n_rows > 256 ? 8 : 1;
-  const dim3 grid((n_rows + rows_per_cta - 1) / rows_per_cta, (n_out + SMALL_WARPS - 1) / SMALL_WARPS);
+  // (and as many as keep the grid's second extent within 65,535)
+  const int rows_per_cta = n_rows > 65535 * 8 ? (n_rows + 65534) / 65535 : n_rows > 256 ? 8 : 1;
+  const dim3 grid((n_out + SMALL_WARPS - 1) / SMALL_WARPS, (n_rows + rows_per_cta - 1) / rows_per_cta);
   auto go = [&](auto kernel, auto zero) {
     r2_launch(kernel, grid, dim3(SMALL_WARPS * 32), size_t(0), stream, (const decltype(zero)*)h, h_stride, w, bias, out, out_stride, n_out, width, n_rows, rows_per_cta);
   };

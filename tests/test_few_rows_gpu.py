@@ -34,6 +34,17 @@ def test_small_linear_rows_do_not_depend_on_their_number(width, n_out, dtype):
     assert ((many.double() - want).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("rows,n_out", [(1, 8 * 65535 + 9), (8 * 65535 + 9, 1)])   # eight outputs or eight rows to a CTA: beyond a grid's second extent
+def test_small_linear_of_any_number_of_rows_and_outputs(rows, n_out):
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(rows)
+    h, w = torch.randn(rows, 4, generator=gen, device=DEV), torch.randn(n_out, 4, generator=gen, device=DEV)
+    got = o.small_linear(h, w)
+    # four products and their sum: 2^-22 of the terms' sizes
+    assert ((got.double() - h.double() @ w.double().T).abs() <= 2.0 ** -22 * (h.abs().double() @ w.abs().double().T)).all()
+
+
+
 @pytest.mark.parametrize("width", [768, 1600, 770])
 def test_router_logits_beyond_what_is_asked_for_ahead(width):
     o = ops()
