@@ -25,21 +25,42 @@ def plan_of(m, n, k, nk):
     return out[0].value, out[1].value
 
 
-# tile widths and numbers of shares; K shares of unequal length, a K tail, rows and features that end inside a tile, one k-block
-CASES = [((512, 1024, 1024), (64, 1)), ((512, 4096, 1024), (128, 4)), ((576, 6000, 1024), (128, 3)), ((65, 3080, 136), (128, 4)), ((130, 4096, 2048), (128, 4)), ((512, 6392, 1600), (128, 2)),
-         ((200, 2048, 520), (64, 2)), ((1024, 1600, 3200), (192, 1)), ((700, 2040, 4608), (192, 1)), ((2048, 64, 200), (64, 1))]
+# K shares of unequal length, a K tail, rows and features that end inside a tile, one k-block
+SHAPES = [(512, 1024, 1024), (512, 4096, 1024), (576, 6000, 1024), (65, 3080, 136), (130, 4096, 2048), (512, 6392, 1600), (200, 2048, 520), (1024, 1600, 3200), (700, 2040, 4608),
+          (2048, 64, 200)]
 
 
-@pytest.mark.parametrize("shape,plan", CASES)
+def shapes_by_plan(w_is_nk):
+    """A ragged shape for every (tile width, shares of K) that the plan gives anywhere on a grid of sizes, whatever its constants are."""
+    found = {}
+    for m in (65, 130, 200, 333, 576, 700, 1000, 2040):
+        for k in (200, 1032, 2040, 4096, 6392):
+            for n in (136, 520, 1032, 2056, 3208, 4616):
+                found.setdefault(plan_of(m, n, k, w_is_nk), (m, k, n))
+    return found
+
+
 @pytest.mark.parametrize("w_is_nk", [False, True])
-def test_tiles_and_shares_of_k(shape, plan, w_is_nk):
+def test_every_form_that_the_plan_knows(w_is_nk):
+    found = shapes_by_plan(w_is_nk)
+    assert {bn for bn, _ in found} >= {64, 128, 192} and {bn for bn, shares in found if shares > 1} >= {64, 128}, found
+    for shape in found.values():
+        check(shape, w_is_nk)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("w_is_nk", [False, True])
+def test_tiles_and_shares_of_k(shape, w_is_nk):
+    check(shape, w_is_nk)
+
+
+def check(shape, w_is_nk):
     o = ops()
     m, k, n = shape
     gen = torch.Generator(device=DEV).manual_seed(m + k + n)
     a = torch.randn(m, k, generator=gen, device=DEV).bfloat16()
     w = (torch.randn((n, k) if w_is_nk else (k, n), generator=gen, device=DEV) * k ** -0.5).bfloat16()
     bias, res = torch.randn(n, generator=gen, device=DEV), torch.randn(m, n, generator=gen, device=DEV)
-    assert plan_of(m, n, k, w_is_nk) == plan
 
     def run():
         return (o.linear(a, w, None, w_is_nk=w_is_nk, out_dtype=torch.float32), o.linear(a, w, bias, w_is_nk=w_is_nk, residual=res),
