@@ -5,9 +5,11 @@
 // keeps a running maximum and sum (online softmax) over its tiles (lane = key for the scores, lanes over the head dimension for
 // P.V), and the eight warps' parts are merged in warp order at the end. The walk depends only on the row's position, its window and
 // the head size, never on how the step was cut or batched, so a row's output is the same bits
-// whichever batch it came in. What bounds it is the latency of its loads: a key row is read in 16-byte pieces with all pieces of a
-// score in flight, a tile's value rows eight at a time, and eight warps share a row's keys (3 rows x 12 heads of 64, float, 200 keys:
-// 148 us with one warp a (row, head) and one number a load, 14 us now; 332 rows: 242 and 71 us). It also takes what the fast kernels leave out: a value head size that
+// whichever batch it came in. What bounds it is the latency of its loads: a key row is read in 16-byte pieces, eight of them in flight
+// (sixteen, a whole row, for float heads of up to 64), a tile's value rows sixteen at a time for heads of up to 64, eight for up
+// to 128 and one after the other beyond, where a lane's share of a row is eight numbers and more; and eight warps share a row's
+// keys (3 rows x 12 heads of 64, float, 200 keys: 148 us with one warp a (row, head) and one number a load, 14 us now; 332 rows: 242
+// and 71 us). It also takes what the fast kernels leave out: a value head size that
 // differs from the key's, a window that keeps a sequence's first keys, a sink in the softmax's
 // denominator, an output gate, chunks, a bias by distance, and values that are the first numbers of the key rows themselves (a
 // cache of latents: the value pointer is the key pointer and a value row is as long as a key row).
