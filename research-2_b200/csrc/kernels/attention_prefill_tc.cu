@@ -669,9 +669,11 @@ extern "C" int r2_attention_prefill_tc(const void* q, int q_row_stride, int n_ro
     // better trade (one CTA's softmax under the other's products); with fewer than two per SM the step waits
     // for the CTA with the most keys, which then should have an SM to itself: the CTA asks for more than half
     // an SM's shared memory, and the ones that do not fit at first start as the short ones end.
-    // Not so where most entries are single decoded tokens beside a portion: three of four softmax warps of their tiles have no rows and
-    // leave the units to the others, and one after the other on an SM they wait for each other's chains (24.2 us a launch
-    // of 16 heads, 512 rows of a prompt and 15 decoded ones with contexts up to 780, 14.6 with two to an SM).
+    // Not so where an entry has less than a tile's rows on average (decoded tokens beside a portion, short prompts): the softmax warps
+    // without rows leave the units to the others, and one after the other on an SM such CTAs wait for each other's chains (24.2 us a
+    // launch of 16 heads, 512 rows of a prompt and 15 decoded ones with contexts up to 780, 14.6 with two to an SM; whole passes without and
+    // with the rule: ten prompts of 100 rows at 355M 1.84 and 1.74 ms, with a sink and a gate 2.03 and 1.76, twenty of 50 at 124M 0.96
+    // and 0.90, forty of 25 at 355M the same).
     const bool sparse = long(n_rows) < long(BM) * n_entries;
     const size_t smem = busy <= 2L * n_sms && !sparse ? size_t(120) * 1024 : smem_one;
     if (extras) r2_launch(prefill_tc_kernel<1, true>, dim3(n_heads, n_tiles), dim3(THREADS), smem, stream, mq, mk, mv, p);
