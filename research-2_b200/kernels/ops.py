@@ -144,7 +144,7 @@ def _lib(source: str) -> C.CDLL:
 def build_all(head_dims=()) -> None:
     """Compile every kernel library that does not depend on a model, and the attention kernels
     for the given head sizes (a model compiles its own head size at first use otherwise)."""
-    for source in ("rowwise", "recurrent", "state_scan", "decay_chunks", "streams", "routing", "gemm_simt", "gemm_tc", "attention_simt", "attention_prefill_tc", "latent_attention",
+    for source in ("rowwise", "recurrent", "state_scan", "decay_chunks", "streams", "routing", "gemm_simt", "gemm_tc", "few_rows", "attention_simt", "attention_prefill_tc", "latent_attention",
                    "sampling", "wait_selftest"):
         _lib(source)
     kernel_library("sfu_probe")  # (profiling/sfu_probe.py: a measurement, no part of a step)
@@ -1266,6 +1266,18 @@ def group_norm_gated(y: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor |
     return out
 
 
+FEW_ROWS = 64   # the most rows that csrc/kernels/few_rows.cu takes
+_few_rows = os.environ.get("R2_FEW_ROWS", "1") != "0"
+
+
+def use_few_rows(on: bool) -> bool:
+    """Switch the products of few bfloat16 rows with matrices stored [out, in] (csrc/kernels/few_rows.cu) on or off; off, the tcgen05
+    kernel takes them. Returns the previous setting."""
+    global _few_rows
+    before, _few_rows = _few_rows, bool(on)
+    return before
+
+
 class NormedRows:
     """LayerNorm of float32 rows that has not been computed yet: `linear` may compute it inside
     its own kernel (few rows, bfloat16), or `materialize()` runs the LayerNorm kernel. With `beta`
@@ -1299,6 +1311,13 @@ def _linear_of_normed(a: NormedRows, w, bias, w_is_nk, act, residual, out_dtype,
     if out is None:
         out = torch.empty(m, n, dtype=out_dtype, device=a.device)
     ldr = _rows(residual, "residual") if residual is not None else 0
+    if w_is_nk and a.rows is None and _few_rows:
+        status = _lib("few_rows").r2_few_rows(
+            None, 0, _p(a.x), a.x.stride(0), _p(a.gamma), _p(a.beta), C.c_float(a.eps), int(a.beta is not None), _p(w), _rows(w, "w"), _p(bias),
+            _p(residual), ldr, _p(out), _rows(out, "out"), dtype_code(out.dtype), m, n, k, ACTIVATIONS[act], 0, _stream())
+        if status != -4:
+            _check(status, "linear (few rows, norm inside)")
+            return out
     ws = _workspace(a.device)
     status = _lib("gemm_tc").r2_gemm_tc(
         None, 0, _p(w), _rows(w, "w"), int(w_is_nk), _p(bias), _p(residual), ldr, _p(out), _rows(out, "out"), m, n, k,
@@ -1311,11 +1330,11 @@ def _linear_of_normed(a: NormedRows, w, bias, w_is_nk, act, residual, out_dtype,
 
 
 def mlp(h, w_in: torch.Tensor, b_in: torch.Tensor, act: str, w_out: torch.Tensor, b_out: torch.Tensor | None,
-        residual: torch.Tensor | None = None) -> torch.Tensor:
-    """act(h @ w_in + b_in) @ w_out + b_out (+ residual), both matrices stored [in, out]. `h` may be
+        residual: torch.Tensor | None = None, w_is_nk: bool = False) -> torch.Tensor:
+    """act(h @ w_in + b_in) @ w_out + b_out (+ residual), both matrices stored [in, out] ([out, in] with w_is_nk). `h` may be
     NormedRows (the LayerNorm then runs inside the first product's kernel where it can)."""
-    inner = linear(h, w_in, b_in, act=act)
-    return linear(inner, w_out, b_out, residual=residual)
+    inner = linear(h, w_in, b_in, w_is_nk=w_is_nk, act=act)
+    return linear(inner, w_out, b_out, w_is_nk=w_is_nk, residual=residual)
 
 
 class KvScatter(C.Structure):
@@ -1388,6 +1407,13 @@ def linear(a, w: torch.Tensor, bias: torch.Tensor | None = None, *, w_is_nk: boo
     if act not in ACTIVATIONS:
         raise KernelError(f"linear: unknown activation {act!r}; known: {sorted(k for k in ACTIVATIONS if k)}")
     if a.dtype == torch.bfloat16 and _tensor_core_gemm:
+        if w_is_nk and m <= FEW_ROWS and _few_rows:
+            status = _lib("few_rows").r2_few_rows(
+                _p(a), lda, None, 0, None, None, C.c_float(0.0), 0, _p(w), ldw, _p(bias), _p(residual), ldr, _p(out), _rows(out, "out"),
+                dtype_code(out.dtype), m, n, k, ACTIVATIONS[act], 0, _stream())
+            if status != -4:
+                _check(status, "linear (few rows)")
+                return out
         ws = _workspace(a.device)
         status = _lib("gemm_tc").r2_gemm_tc(
             _p(a), lda, _p(w), ldw, int(w_is_nk), _p(bias), _p(residual), ldr, _p(out), _rows(out, "out"), m, n, k,
@@ -1415,6 +1441,12 @@ def grouped_linear(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     flat = a.view(t, n * k)
     if a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and _tensor_core_gemm and n > 1:
         _need(w, "w", dim=2)
+        if t <= FEW_ROWS and _few_rows:
+            status = _lib("few_rows").r2_few_rows(_p(flat), n * k, None, 0, None, None, C.c_float(0.0), 0, _p(w), _rows(w, "w"), None, None, 0, _p(out), n * per,
+                                                  BF16, t, n * per, k, ACT_NONE, per, _stream())
+            if status != -4:
+                _check(status, "grouped_linear (few rows)")
+                return out
         status = _lib("gemm_tc").r2_gemm_tc_grouped(_p(flat), n * k, _p(w), _rows(w, "w"), _p(out), n * per, t, per, k, n, BF16,
                                                     _p(_workspace(a.device).error), _stream())
         if status != -4:
@@ -1712,15 +1744,14 @@ def use_resident_decode(on: bool) -> bool:
     return before
 
 
-_resident_rows = int(os.environ.get("R2_RESIDENT_ROWS", "16"))
+_resident_rows = int(os.environ.get("R2_RESIDENT_ROWS", "0"))
 
 
 def set_resident_decode_rows(n: int) -> int:
-    """The most rows of a decode-only batch that run as the resident kernel (it takes up to 64). The
-    default is 16: up to there it measured faster than the chain of kernels at GPT-2 124M sizes (0.39 against
-    0.46 ms a step of 8 rows, 0.46 against 0.54 at 12, 0.53 against 0.57 at 16), at 24 rows the same (0.62) and
-    beyond it slower (0.73 against 0.69 at 32, 1.07 against 0.88 at 64: every CTA reads all rows of a
-    product's input). Returns the previous value."""
+    """The most rows of a decode-only batch that run as the resident kernel (it takes up to 64). The default is
+    0: since products of few rows have a kernel of their own the chain of kernels is the faster form at every size measured
+    (0.22 against 0.35 ms a step of one row and 0.25 against 0.38 of 8 at GPT-2 124M sizes, 0.31 against 0.51 of 16; 0.52 against
+    0.85 of 8 rows at 355M, 1.83 against 2.40 at 1.5B). Returns the previous value."""
     global _resident_rows
     before, _resident_rows = _resident_rows, int(n)
     return before

@@ -15,7 +15,7 @@ import torch
 
 from ..kernels import ops
 from .base import MemberSpec, Runtime, register_mixer
-from .util import matrix, vector
+from .util import matrix, product_matrix, vector
 
 
 def _stacked_bias(parts: list, widths: list[int], rt: Runtime) -> torch.Tensor | None:
@@ -45,12 +45,14 @@ class PagedAttention:
             raise ValueError(f"attention: head sizes come in steps of 16 from 16 to 256, got {self.head_dim}")
         self.q_width = self.n_heads * self.head_dim
         self.kv_width = self.n_kv_heads * self.head_dim
-        self.w_qkv = matrix(weights["w_qkv"], rt)
+        shapes = tuple(weights["w_qkv"].shape), tuple(weights["w_out"].shape)
+        self.width, self.out_width = shapes[0][0], shapes[1][1]
+        self.w_qkv, self.w_is_nk = product_matrix(weights["w_qkv"], rt)
         self.b_qkv = vector(weights["b_qkv"], rt)
-        self.w_out = matrix(weights["w_out"], rt)
+        self.w_out, _ = product_matrix(weights["w_out"], rt)
         self.b_out = vector(weights["b_out"], rt)
-        if self.w_qkv.shape[1] != self.q_width + 2 * self.kv_width or self.w_out.shape[0] != self.q_width:
-            raise ValueError(f"attention: weights {tuple(self.w_qkv.shape)} / {tuple(self.w_out.shape)} do not fit "
+        if shapes[0][1] != self.q_width + 2 * self.kv_width or shapes[1][0] != self.q_width:
+            raise ValueError(f"attention: weights {shapes[0]} / {shapes[1]} do not fit "
                              f"{self.n_heads} heads, {self.n_kv_heads} kv heads of {self.head_dim}")
         self.rotary = None  # a positions part that changes q and k may be attached by the model
 
@@ -68,21 +70,21 @@ class PagedAttention:
 
     def resident_attention(self) -> dict | None:
         """For the one-kernel form of a decode step; None while a positions part rotates q and k."""
-        if self.rotary is not None or self.w_out.shape[1] != self.w_qkv.shape[0]:
+        if self.rotary is not None or self.out_width != self.width or not self.w_is_nk:
             return None
-        return {"w_qkv": self.w_qkv, "b_qkv": self.b_qkv, "w_out": self.w_out, "b_out": self.b_out, "n_heads": self.n_heads,
+        return {"w_qkv": self.w_qkv.t(), "b_qkv": self.b_qkv, "w_out": self.w_out.t(), "b_out": self.b_out, "n_heads": self.n_heads,
                 "n_kv_heads": self.n_kv_heads, "head_dim": self.head_dim, "scale": self.scale, "window": self.window,
-                "width": self.w_qkv.shape[0]}
+                "width": self.width}
 
     def forward(self, h, residual, ctx, cache, state=None, writes_cache: bool = True):
         in_cache = False
         if writes_cache and not ctx.decode_only and self.rotary is None:
             # keys and values leave the product's epilogue for their cache slots (where that kernel takes the shape)
-            qkv, in_cache = ops.linear(h, self.w_qkv, self.b_qkv, kv=ops.kv_scatter(
+            qkv, in_cache = ops.linear(h, self.w_qkv, self.b_qkv, w_is_nk=self.w_is_nk, kv=ops.kv_scatter(
                 ctx.slot_mapping[cache.group], cache.k, cache.v, cache.page_stride, cache.page_size, cache.n_pages,
                 self.q_width, self.kv_width, self.head_dim))
         else:
-            qkv = ops.linear(h, self.w_qkv, self.b_qkv)
+            qkv = ops.linear(h, self.w_qkv, self.b_qkv, w_is_nk=self.w_is_nk)
         q = qkv[:, : self.q_width]
         k = qkv[:, self.q_width: self.q_width + self.kv_width]
         v = qkv[:, self.q_width + self.kv_width:]
@@ -94,7 +96,7 @@ class PagedAttention:
                 cache.n_pages, ctx.block_tables[cache.group], ctx.row_entry, ctx.positions, ctx.seq_lens, self.n_heads,
                 self.n_kv_heads, self.head_dim, self.scale, self.window, ctx.max_context)
             if mixed is not None:
-                return ops.linear(mixed, self.w_out, self.b_out, residual=residual)
+                return ops.linear(mixed, self.w_out, self.b_out, w_is_nk=self.w_is_nk, residual=residual)
         if writes_cache and not in_cache:
             ops.kv_write(k, v, cache.k, cache.v, ctx.slot_mapping[cache.group], self.n_kv_heads, self.head_dim,
                          cache.page_size, cache.page_stride, cache.n_pages)
@@ -103,7 +105,7 @@ class PagedAttention:
             ctx.row_entry, ctx.positions, ctx.seq_lens, self.n_heads, self.n_kv_heads, self.head_dim, self.scale,
             self.window, decode_only=ctx.decode_only, max_context=ctx.max_context, q_start=ctx.q_start,
             n_tiles=ctx.n_attention_tiles)
-        return ops.linear(mixed, self.w_out, self.b_out, residual=residual)
+        return ops.linear(mixed, self.w_out, self.b_out, w_is_nk=self.w_is_nk, residual=residual)
 
 
 @register_mixer("qk_norm_attention")

@@ -8,7 +8,7 @@ import torch
 
 from ..kernels import ops
 from .base import Runtime, register_feed_forward
-from .util import matrix, vector
+from .util import matrix, product_matrix, vector
 
 
 @register_feed_forward("mlp")
@@ -20,12 +20,14 @@ class DenseMLP:
         self.activation = params["activation"]
         if self.activation not in ops.ACTIVATIONS or self.activation in (None, "none"):
             raise ValueError(f"mlp: unknown activation {self.activation!r}")
-        self.w_in = matrix(weights["w_in"], rt)
+        shapes = tuple(weights["w_in"].shape), tuple(weights["w_out"].shape)
+        if shapes[0] != shapes[1][::-1]:
+            raise ValueError(f"mlp: w_in {shapes[0]} and w_out {shapes[1]} do not fit")
+        self.width, self.inner = shapes[0]
+        self.w_in, self.w_is_nk = product_matrix(weights["w_in"], rt)
         self.b_in = vector(weights["b_in"], rt)
-        self.w_out = matrix(weights["w_out"], rt)
+        self.w_out, _ = product_matrix(weights["w_out"], rt)
         self.b_out = vector(weights["b_out"], rt)
-        if self.w_in.shape[1] != self.w_out.shape[0] or self.w_in.shape[0] != self.w_out.shape[1]:
-            raise ValueError(f"mlp: w_in {tuple(self.w_in.shape)} and w_out {tuple(self.w_out.shape)} do not fit")
 
     takes_lazy_norm = True  # the input goes straight into ops.linear
 
@@ -33,12 +35,14 @@ class DenseMLP:
         """The weight matrices in the order in which forward() uses them."""
         return [self.w_in, self.w_out]
 
-    def resident_mlp(self) -> dict:
-        return {"w_fc": self.w_in, "b_fc": self.b_in, "w_pr": self.w_out, "b_pr": self.b_out, "act": self.activation,
-                "width": self.w_in.shape[0], "inner": self.w_in.shape[1]}
+    def resident_mlp(self) -> dict | None:
+        if not self.w_is_nk:
+            return None
+        return {"w_fc": self.w_in.t(), "b_fc": self.b_in, "w_pr": self.w_out.t(), "b_pr": self.b_out, "act": self.activation,
+                "width": self.width, "inner": self.inner}
 
     def forward(self, h, residual, ctx):
-        return ops.mlp(h, self.w_in, self.b_in, self.activation, self.w_out, self.b_out, residual=residual)
+        return ops.mlp(h, self.w_in, self.b_in, self.activation, self.w_out, self.b_out, residual=residual, w_is_nk=self.w_is_nk)
 
 
 @register_feed_forward("gated_clamped")

@@ -177,3 +177,79 @@ def test_fixed_operands_change_no_bit():
         calls += [lambda f, g=g: o.group_norm_gated(h, h, gain, g, 1e-5, True, torch.float32, fixed=f) for g in (24, 12, 6, 1)]
         for i, call in enumerate(calls):
             assert torch.equal(call(True), call(False)), (n, i)
+
+
+def few_rows_case(m, n, k, seed=0):
+    gen = torch.Generator(device=DEV).manual_seed(seed + m + 7 * n + 31 * k)
+    a = torch.randn(m, k + 8, generator=gen, device=DEV).bfloat16()[:, :k]          # rows with a stride of their own
+    w = (torch.randn(n, k + 16, generator=gen, device=DEV) * k ** -0.5).bfloat16()[:, 8: k + 8]
+    return gen, a, w
+
+
+def sums_bound(a, w, k):
+    """float32 sums of k exact products: under two roundings a term and some that join the shares, each 2^-23 of the terms' sizes."""
+    return (k + 32) * 2.0 ** -23 * (a.double().abs() @ w.double().abs().T)
+
+
+# rows around the tiles of 8, 16 and 32; features and K around the rules that pick a split, no multiples of a tile, K beside blocks of 32
+@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("n,k", [(1, 8), (24, 40), (768, 768), (1184, 1000), (1185, 96), (2369, 256), (4737, 64), (2376, 1032), (8192, 32), (72, 2048), (65, 5128), (768, 3072)])
+def test_products_of_few_rows(m, n, k):
+    o = ops()
+    gen, a, w = few_rows_case(m, n, k)
+    bias, residual = torch.randn(n, generator=gen, device=DEV), torch.randn(m, n, generator=gen, device=DEV)
+    want = a.double() @ w.double().T
+    bound = sums_bound(a, w, k)
+    got = o.linear(a, w, bias, w_is_nk=True, residual=residual)
+    assert ((got.double() - (want + bias.double() + residual.double())).abs() <= bound + 2.0 ** -22 * (bias.abs() + residual.abs() + want.abs())).all()
+    out = torch.full((m, n + 3), 7.0, dtype=torch.bfloat16, device=DEV)
+    o.linear(a, w, None, w_is_nk=True, out=out[:, 1: n + 1])
+    assert ((out[:, 1: n + 1].double() - want).abs() <= bound + 2.0 ** -8 * want.abs()).all()
+    assert (out[:, 0] == 7.0).all() and (out[:, n + 1:] == 7.0).all()
+
+
+@pytest.mark.parametrize("act", ["gelu_new", "gelu"])
+def test_products_of_few_rows_with_an_activation(act):
+    o = ops()
+    gen, a, w = few_rows_case(5, 200, 768)
+    bias = torch.randn(200, generator=gen, device=DEV)
+    z = a.double() @ w.double().T + bias.double()
+    want = torch.nn.functional.gelu(z, approximate="tanh" if act == "gelu_new" else "none")
+    exact = o.linear(a, w, bias, w_is_nk=True, act=act, out_dtype=torch.float32)
+    torch.testing.assert_close(exact.double(), want, atol=2e-5, rtol=2e-5)
+    rounded = o.linear(a, w, bias, w_is_nk=True, act=act)
+    # the hardware's tanh is within 2^-11 of the value and the result is rounded to 2^-9
+    torch.testing.assert_close(rounded.double(), want, atol=2.0 ** -10, rtol=2.0 ** -8)
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("k", [64, 768, 1000, 1024])
+@pytest.mark.parametrize("centred", [True, False])
+def test_products_of_few_rows_with_a_norm(m, k, centred):
+    """Rows far from zero: the mean is 30 times the spread."""
+    o = ops()
+    n = 100
+    gen, _, w = few_rows_case(m, n, k)
+    x = torch.randn(m, k, generator=gen, device=DEV) + (30.0 if centred else 0.0)
+    gain, shift = 1.0 + 0.3 * torch.randn(k, generator=gen, device=DEV), torch.randn(k, generator=gen, device=DEV)
+    rows = x.double()
+    if centred:
+        normed = torch.nn.functional.layer_norm(rows, (k,), gain.double(), shift.double(), 1e-5)
+    else:
+        normed = rows * torch.rsqrt((rows * rows).mean(-1, keepdim=True) + 1e-5) * gain.double()
+    got = o.linear(o.NormedRows(x, gain, shift if centred else None, 1e-5, torch.bfloat16), w, None, w_is_nk=True, out_dtype=torch.float32)
+    # each normed value is rounded to bfloat16 once (2^-9 of it, independent signs: a root of the squares' sum, six of them)
+    bound = 6 * 2.0 ** -9 * ((normed ** 2) @ (w.double() ** 2).T).sqrt()
+    assert ((got.double() - normed @ w.double().T).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("t,groups,per,k", [(1, 4, 128, 64), (9, 3, 768, 768), (40, 2, 160, 40), (3, 2, 24, 64)])   # (the last: groups that are no multiple of a CTA's features)
+def test_products_of_few_rows_side_by_side(t, groups, per, k):
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(t)
+    a = torch.randn(t, groups, k, generator=gen, device=DEV).bfloat16()
+    w = torch.randn(groups * per, k, generator=gen, device=DEV).bfloat16()
+    got = o.grouped_linear(a, w).double().view(t, groups, per)
+    for s in range(groups):
+        want = a[:, s].double() @ w[s * per: (s + 1) * per].double().T
+        assert ((got[:, s] - want).abs() <= sums_bound(a[:, s], w[s * per: (s + 1) * per], k) + 2.0 ** -8 * want.abs()).all()
