@@ -253,3 +253,23 @@ def test_products_of_few_rows_side_by_side(t, groups, per, k):
     for s in range(groups):
         want = a[:, s].double() @ w[s * per: (s + 1) * per].double().T
         assert ((got[:, s] - want).abs() <= sums_bound(a[:, s], w[s * per: (s + 1) * per], k) + 2.0 ** -8 * want.abs()).all()
+
+
+# one warp to eight, rows that end inside a thread's eight values, the widest row in registers and the next one beyond
+@pytest.mark.parametrize("width", [4, 36, 256, 260, 768, 1600, 2048, 2052])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("gathered", [False, True])
+def test_norms_of_rows(width, dtype, gathered):
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(width)
+    x = torch.randn(37, width, generator=gen, device=DEV) + 20.0   # (a mean far beyond the spread)
+    gain, shift = torch.randn(width, generator=gen, device=DEV), torch.randn(width, generator=gen, device=DEV)
+    rows = torch.tensor([36, 0, 5, 5], dtype=torch.int32, device=DEV) if gathered else None
+    read = x[rows.long()].double() if gathered else x.double()
+    want = torch.nn.functional.layer_norm(read, (width,), gain.double(), shift.double(), 1e-5)
+    # the statistics' roundings grow with mean / spread (20): 2^-24 * 20 a value, some tens of them, beside the result's own rounding
+    bound = 2.0 ** -16 * (gain.abs().double() + 1.0) * (1.0 + want.abs()) + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0.0)
+    assert ((o.layer_norm(x, gain, shift, 1e-5, dtype, rows=rows).double() - want).abs() <= bound).all()
+    want = read * torch.rsqrt((read * read).mean(-1, keepdim=True) + 1e-5) * gain.double()
+    bound = 2.0 ** -20 * want.abs() + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0.0)
+    assert ((o.rms_norm(x, gain, 1e-5, dtype, rows=rows).double() - want).abs() <= bound).all()
