@@ -1,10 +1,12 @@
 // Decode attention over the paged cache, bfloat16 cache and queries, float arithmetic: rows
 // that are one new token each, the case whose time is the reading of the cache.
 //
-// A CTA takes one (row, kv head, slice of the keys). Its four warps walk the slice's 32-key
+// A CTA's warps (4, or 8 or 16 where the chip has room for all pairs; a part of them where a CTA takes several pairs) have one (row, kv head,
+// slice of the keys) and walk the slice's 32-key
 // tiles in turn: lane = key for q.k (each lane reads its key's row in 16-byte pieces), lanes
 // over the head dimension for p.v; all query heads that share the kv head ride along on the
-// same loads. Every warp keeps an online-softmax state; the warps' states are merged in
+// same loads. The cache's rows come from steps that have ended, so the first tiles are asked for while the product that makes q, k and v still
+// runs (`cache_settled`); only the query and the newest key and value are fetched after it. Every warp keeps an online-softmax state; the warps' states are merged in
 // shared memory. With one slice the CTA writes the output row; with several it leaves
 // (max, sum, unnormalised output) per slice in a scratch buffer and `merge` combines them.
 // The slicing depends on the row's own context length and on the number of slices only.
@@ -22,12 +24,14 @@
 namespace {
 
 constexpr int HD = HEAD_DIM;
-constexpr int WARPS = 4;
+constexpr int NARROW = 4, WIDE = HD <= 64 ? 16 : 8;   // warps of a CTA (see decode_kernel)
 constexpr int VECS = HD / 8;                 // 16-byte pieces of a key row
 constexpr int DPL = (HD + 63) / 64;          // pairs of head-dimension elements per lane in p.v
 constexpr int ROW_BYTES = HD * 2 + 16;       // a key's row in shared memory, padded against bank conflicts
-constexpr int NBUF = 1;                      // tiles in flight per warp; other warps' work hides the wait
-constexpr int TILE_SMEM = WARPS * NBUF * 2 * 32 * ROW_BYTES;
+constexpr int TILE_SMEM = 2 * 32 * ROW_BYTES;   // a tile's keys and values
+// Tiles in flight: one a warp (other warps' work hides the wait); in wide CTAs two for the first half of a pair's warps (24 tiles of an SM's
+// shared memory at head size 64): rows of 513 to 768 keys would pay a second round trip to memory for a few tiles more than warps.
+__host__ __device__ constexpr int tile_places(int warps) { return warps == NARROW ? warps : warps + warps / 2; }
 static_assert(HD % 16 == 0 && HD >= 16 && HD <= 256, "head sizes come in steps of 16 up to 256");
 
 struct DecodeParams {
@@ -37,7 +41,7 @@ struct DecodeParams {
   long long page_stride; int page_size; int page_shift; int n_pages;
   const int32_t* block_tables; int table_width;
   const int32_t* row_entry; const int32_t* positions; const int32_t* seq_lens;
-  int n_heads, n_kv_heads;
+  int n_rows, n_heads, n_kv_heads;
   float scale; int window;
   // With a window, the entry's first `keep_first` keys stay visible beside the window's. `sink` adds one
   // to every softmax's denominator (an extra exp(0) term). `gate` (may be null;
@@ -65,6 +69,11 @@ struct DecodeParams {
   // The slices of a (row, kv head) are the CTAs of a cluster, which merge their results out of one another's shared memory: no
   // scratch, no counters. (Through global memory the merge is four round trips one after the other: results, fence, counter, results.)
   int clustered;
+  // No launch shortly before wrote the cache's rows (they come from steps that have ended; the newest key and value come from k_new and
+  // v_new): the first tiles are asked for ahead of the wait.
+  int cache_settled;
+  int wide;         // CTAs of WIDE warps, else of NARROW
+  int pair_warps;   // warps that share a (row, kv head) pair's keys: a power of two, a CTA's at most
 };
 
 constexpr int MAX_CLUSTER = 8;
@@ -130,20 +139,30 @@ bool g_decode_mma = true;              // r2_attention_decode_set_mma (tests com
 // bandwidth with the scalar form).
 // X 1: the form with kept first keys, a sink, a gate and two-term weights; without it those parameters are not
 // read and the plain form compiles to what it was. X 2: chunks, a bias by distance and a factor on the output besides.
-template <int G, bool MMA, int X>
-__global__ void __launch_bounds__(WARPS * 32, (MMA && HD <= 64) ? 5 : 1)  // five CTAs to an SM is what the tiles' shared memory allows
+// WARPS: a CTA's warps take `pair_warps` each for the keys of one (row, kv head) pair, a tile of 32 at a time and all first tiles asked for
+// at once. WIDE CTAs, one to an SM, are for launches whose pairs all find room on the chip: there the time is a chain (hand-over, query,
+// a tile, merge), and what makes it short is that a pair's first 512 keys (head sizes up to 64) are one tile a warp, with no merge
+// between CTAs: clusters cost a launch 0.5 to 0.8 us even where a row is too short for their merge and 1 to 2.7 us where it is not. Inside a
+// step of 8 rows of GPT-2 124M (12 layers; 200 and 500 keys a row) CTAs of four warps in clusters of six take 272 and 285 us, wide ones 236 and 258.
+// NARROW CTAs, several to an SM, are for more pairs than that.
+template <int G, bool MMA, int X, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, (MMA && HD <= 64 && WARPS == NARROW) ? 5 : 1)  // five narrow CTAs to an SM is what the tiles' shared memory allows
 decode_kernel(const DecodeParams p) {
   pdl_launch_dependents();  // the next kernel may begin its prologue
   // The wait on the previous kernel comes further down: positions, context lengths and block
   // tables belong to the batch, which no kernel writes, so the chain of lookups that leads to the
   // first tile's addresses runs while the previous kernel (the product that makes q, k and v) ends.
-  __shared__ float q_s[G][HD];
-  __shared__ float red_o[WARPS][G][HD];
+  __shared__ float q_s[MMA ? 1 : WARPS / NARROW][G][HD];
   __shared__ float red_m[WARPS][G], red_l[WARPS][G];
   __shared__ float cta_m[G], cta_l[G];   // (clustered) of this CTA's slice
   __shared__ int is_last_s;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int slice = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
+  const int lane = threadIdx.x & 31;
+  const int pair_warps = WARPS == NARROW ? WARPS : p.pair_warps;
+  const int warp = (threadIdx.x >> 5) % pair_warps, first_warp = (threadIdx.x >> 5) - warp;   // within the pair's; the CTA's number of its first
+  const int pair_thread = warp * 32 + lane, pair_threads = pair_warps * 32;
+  const int slice = blockIdx.x, pair = (blockIdx.z * gridDim.y + blockIdx.y) * (WARPS / pair_warps) + first_warp / pair_warps;
+  const bool exists = pair < p.n_rows * p.n_kv_heads;
+  const int t = exists ? pair / p.n_kv_heads : 0, kvh = exists ? pair % p.n_kv_heads : 0;
   const int h0 = kvh * G;
   // Every row is an entry of its own, in order: row t is entry t. A pad row is an entry of no keys
   // (context length 0, position 0), which the code below turns into zeros without a branch of
@@ -165,9 +184,17 @@ decode_kernel(const DecodeParams p) {
     const int n = pos - key_at(v);
     return p.dist_bias[size_t(h0 + g) * p.bias_len + (n < p.bias_len ? n : p.bias_len - 1)];
   };
-  // this slice's keys: equal runs of whole 32-key tiles
-  const int tiles = (n_keys + 31) / 32;
-  const int tiles_per = (tiles + p.n_slices - 1) / p.n_slices;
+  // this slice's keys: equal runs of whole 32-key tiles, as many in a run as all warps take at a time. A short row has fewer runs than the
+  // launch has slices (their number goes by the longest context that a captured step may meet): the CTAs of the others leave at once where
+  // the slices of a row are a cluster, and a row of one run needs no merge.
+  const int tiles = exists ? (n_keys + 31) / 32 : 0;
+  int tiles_per = (tiles + p.n_slices - 1) / p.n_slices;
+  int n_slices = p.n_slices;
+  if (p.clustered) {
+    tiles_per = tiles_per > WARPS ? (tiles_per + WARPS - 1) / WARPS * WARPS : WARPS;   // (a CTA of a cluster has one pair)
+    n_slices = tiles > tiles_per ? (tiles + tiles_per - 1) / tiles_per : 1;
+    if (slice >= n_slices) return;
+  }
   const int tile_begin = slice * tiles_per;
   const int tile_end = min(tiles, tile_begin + tiles_per);
   const int32_t* table = p.block_tables + size_t(e) * p.table_width;
@@ -180,11 +207,11 @@ decode_kernel(const DecodeParams p) {
 #pragma unroll
     for (int i = 0; i < DPL; ++i) acc[g][i][0] = acc[g][i][1] = 0.f;
   }
-  // tensor-core form: this lane's rows are heads gq and gq + 8 of the group (those below G exist)
+  // tensor-core form: this lane's row is head gq of the group (those below G exist)
   constexpr int KS = MMA ? HD / 16 : 1, DT = MMA ? HD / 8 : 1;
   const int gq = lane >> 2, tq = lane & 3;
-  uint32_t qf[KS][4];
-  float o[DT][4], m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+  uint32_t qf[KS][2];
+  float o[DT][4], m_run = -INFINITY, l_run = 0.f;
 #pragma unroll
   for (int i = 0; i < DT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   const size_t head_off = size_t(kvh) * p.page_size * HD;
@@ -192,113 +219,116 @@ decode_kernel(const DecodeParams p) {
   // Tiles of 32 keys go through shared memory: every lane copies its own key's K row and V row
   // with 16-byte asynchronous copies, so a tile's 2 x 32 rows are all in flight at once, and
   // (for head sizes up to 128) the next tile is on its way while this one is used. The newest
-  // key's row comes from the projection's output (k_new, v_new), not from the cache.
+  // key's row comes from the projection's output (k_new, v_new), not from the cache: it is left out of the copies and put in its place
+  // once the tile has landed.
   extern __shared__ __align__(16) uint8_t tile_smem[];
-  uint8_t* my_smem = tile_smem + size_t(warp) * NBUF * 2 * 32 * ROW_BYTES;
+  // this warp's places for tiles: its own and, in the first half of a wide CTA's pair, one behind all warps'
+  const int depth = WARPS != NARROW && warp < pair_warps / 2 ? 2 : 1;
+  auto place = [&](int it) { return tile_smem + size_t(depth == 2 && (it & 1) ? WARPS + first_warp / 2 + warp : first_warp + warp) * TILE_SMEM; };
+  // the warps' results lie over their tiles, which have been used by then: [G][HD] floats
+  auto red_o = [&](int w) { return reinterpret_cast<float*>(tile_smem + size_t(first_warp + w) * TILE_SMEM); };
+  static_assert(G * HD * 4 <= TILE_SMEM, "a warp's result must fit its tiles");
   const int tile_of_new = (p.k_new != nullptr && pos == last) ? v_of_pos / 32 : -1;
 
-  // lane r finds row r's place: element offsets from k_cache / v_cache; -1 for a row past the last key
-  auto lookup = [&](int tile, long long& my_k, long long& my_v) {
+  // lane r finds row r's place: an element offset from k_cache and v_cache; -1 for a row past the last key
+  auto lookup = [&](int tile, long long& my_row) {
     const int v = tile * 32 + lane;
     const int j = key_at(v);
     if (v >= n_keys) {
-      my_k = my_v = -1;
-    } else if (tile == tile_of_new && v == v_of_pos) {
-      my_k = (p.k_new + size_t(t) * p.new_row_stride + size_t(kvh) * HD) - p.k_cache;
-      my_v = (p.v_new + size_t(t) * p.new_row_stride + size_t(kvh) * HD) - p.v_cache;
+      my_row = -1;
     } else {
       int page = table[page_index(j, p.page_size, p.page_shift)];
       page = (page < 0 || page >= p.n_pages) ? 0 : page;
-      my_k = my_v = (long long)(size_t(page) * p.page_stride + head_off + size_t(page_offset(j, p.page_size, p.page_shift)) * HD);
+      my_row = (long long)(size_t(page) * p.page_stride + head_off + size_t(page_offset(j, p.page_size, p.page_shift)) * HD);
     }
   };
   // then consecutive lanes copy consecutive 16-byte pieces of a row, then the next row: whole
   // lines per request
-  auto copy = [&](int tile, int buf, long long my_k, long long my_v) {
-    const int v0 = tile * 32;
-    const uint32_t kd = smem_u32(my_smem + (size_t(buf) * 2 + 0) * 32 * ROW_BYTES);
-    const uint32_t vd = smem_u32(my_smem + (size_t(buf) * 2 + 1) * 32 * ROW_BYTES);
+  auto copy = [&](int tile, uint8_t* to, long long my_row) {
+    const int new_row = tile == tile_of_new ? v_of_pos - tile * 32 : -1;
+    const uint32_t kd = smem_u32(to), vd = smem_u32(to + 32 * ROW_BYTES);
 #pragma unroll
     for (int i = 0; i < VECS; ++i) {
       const int f = lane + 32 * i;
       const int row = f / VECS, c = f % VECS;
-      const long long ko = __shfl_sync(0xffffffffu, my_k, row);
-      const long long vo = __shfl_sync(0xffffffffu, my_v, row);
-      const bool valid = ko >= 0 || (tile == tile_of_new && v0 + row == v_of_pos);
-      const int bytes = valid ? 16 : 0;  // 0 source bytes: zeros
-      const bf16* ksrc = valid ? p.k_cache + ko + c * 8 : p.k_cache;
-      const bf16* vsrc = valid ? p.v_cache + vo + c * 8 : p.v_cache;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kd + row * ROW_BYTES + c * 16), "l"(ksrc), "r"(bytes) : "memory");
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vd + row * ROW_BYTES + c * 16), "l"(vsrc), "r"(bytes) : "memory");
+      const long long from = __shfl_sync(0xffffffffu, my_row, row);
+      const int bytes = from >= 0 ? 16 : 0;  // 0 source bytes: zeros
+      const bf16* ksrc = from >= 0 ? p.k_cache + from + c * 8 : p.k_cache;
+      const bf16* vsrc = from >= 0 ? p.v_cache + from + c * 8 : p.v_cache;
+      if (row != new_row) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kd + row * ROW_BYTES + c * 16), "l"(ksrc), "r"(bytes) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vd + row * ROW_BYTES + c * 16), "l"(vsrc), "r"(bytes) : "memory");
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  auto issue = [&](int tile, int buf) {
-    long long my_k, my_v;
-    lookup(tile, my_k, my_v);
-    copy(tile, buf, my_k, my_v);
+  auto issue = [&](int tile, uint8_t* to) {
+    long long my_row;
+    lookup(tile, my_row);
+    copy(tile, to, my_row);
   };
 
-  // The first tile's addresses are found before the wait; its copies (one row of which may be the
-  // new key and value, which the previous kernel made) and the query's fetch come after it.
-  long long first_k = -1, first_v = -1;
-  if (tile_begin + warp < tile_end) lookup(tile_begin + warp, first_k, first_v);
+  // The first tiles' addresses are found before the wait, and their rows are asked for there where the cache is settled: then only the
+  // query and the newest key's and value's rows, which the previous kernel made, are fetched after it.
+  long long first_row = -1, second_row = -1;
+  const bool has_tile = tile_begin + warp < tile_end, has_second = depth == 2 && tile_begin + warp + pair_warps < tile_end;
+  const bool has_new = tile_of_new >= tile_begin && tile_of_new < tile_end && (tile_of_new - tile_begin) % pair_warps == warp;
+  int new_slot = -1;
+  if (has_tile) lookup(tile_begin + warp, first_row);
+  if (has_second) lookup(tile_begin + warp + pair_warps, second_row);
+  if (has_new) new_slot = p.slot_mapping[t];
+  auto first_copies = [&]() {
+    if (has_tile) copy(tile_begin + warp, place(0), first_row);
+    if (has_second) copy(tile_begin + warp + pair_warps, place(1), second_row);
+  };
+  if (p.cache_settled) first_copies();
   pdl_wait();  // the previous kernel's writes are visible from here on
-  if (tile_begin + warp < tile_end) copy(tile_begin + warp, 0, first_k, first_v);
+  if (!p.cache_settled) first_copies();
+  // the newest key's and value's rows, a 16-byte piece a lane: they go into their tile and, at the end, into the cache
+  constexpr int FRESH = (2 * VECS + 31) / 32;
+  uint4 fresh[FRESH];
+#pragma unroll
+  for (int i = 0; i < FRESH; ++i) {
+    const int f = lane + 32 * i;
+    fresh[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (has_new && f < 2 * VECS) {
+      fresh[i] = __ldcg(reinterpret_cast<const uint4*>((f < VECS ? p.k_new : p.v_new) + size_t(t) * p.new_row_stride + size_t(kvh) * HD) + f % VECS);
+    }
+  }
   if (MMA) {
     // the query heads straight into the lane's operand registers (unscaled: the scale goes on the scores)
     const bf16* qa = p.q + size_t(t) * p.q_row_stride + size_t(h0 + gq) * HD + 2 * tq;
-    const bf16* qb = qa + size_t(8) * HD;
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
       qf[ks][0] = gq < G ? *reinterpret_cast<const uint32_t*>(qa + ks * 16) : 0u;
-      qf[ks][1] = gq + 8 < G ? *reinterpret_cast<const uint32_t*>(qb + ks * 16) : 0u;
-      qf[ks][2] = gq < G ? *reinterpret_cast<const uint32_t*>(qa + ks * 16 + 8) : 0u;
-      qf[ks][3] = gq + 8 < G ? *reinterpret_cast<const uint32_t*>(qb + ks * 16 + 8) : 0u;
+      qf[ks][1] = gq < G ? *reinterpret_cast<const uint32_t*>(qa + ks * 16 + 8) : 0u;
     }
   } else {
-    for (int i = threadIdx.x; i < G * HD; i += WARPS * 32) {
+    for (int i = pair_thread; i < G * HD; i += pair_threads) {
       int g = i / HD, d = i % HD;
-      q_s[g][d] = __bfloat162float(p.q[size_t(t) * p.q_row_stride + size_t(h0 + g) * HD + d]) * p.scale;
+      q_s[first_warp / NARROW][g][d] = __bfloat162float(p.q[size_t(t) * p.q_row_stride + size_t(h0 + g) * HD + d]) * p.scale;
     }
     __syncthreads();
   }
   int it = 0;
-  for (int tile = tile_begin + warp; tile < tile_end; tile += WARPS, ++it) {
+  for (int tile = tile_begin + warp; tile < tile_end; tile += pair_warps, ++it) {
     const int v0 = tile * 32;
-    const int buf = NBUF == 2 ? (it & 1) : 0;
+    // this tile has landed, and the one after it may still be on its way
+    if (depth == 2 && tile + pair_warps < tile_end) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    uint8_t* k_tile = place(it);
+    uint8_t* v_tile = k_tile + 32 * ROW_BYTES;
     if (tile == tile_of_new) {
-      // the newest key lies in this tile: this warp also puts its key and value into the cache
-      const int slot = p.slot_mapping[t];
-      const int page = slot < 0 ? -1 : page_index(slot, p.page_size, p.page_shift);
-      if (page >= 0 && page < p.n_pages) {
-        const size_t dst = size_t(page) * p.page_stride + size_t(kvh) * p.page_size * HD + size_t(page_offset(slot, p.page_size, p.page_shift)) * HD;
-        const __nv_bfloat162* ks = reinterpret_cast<const __nv_bfloat162*>(p.k_new + size_t(t) * p.new_row_stride + size_t(kvh) * HD);
-        const __nv_bfloat162* vs = reinterpret_cast<const __nv_bfloat162*>(p.v_new + size_t(t) * p.new_row_stride + size_t(kvh) * HD);
-        __nv_bfloat162* kd = reinterpret_cast<__nv_bfloat162*>(p.k_cache_w + dst);
-        __nv_bfloat162* vd = reinterpret_cast<__nv_bfloat162*>(p.v_cache_w + dst);
-        for (int i = lane; i < HD / 2; i += 32) {
-          kd[i] = ks[i];
-          vd[i] = vs[i];
-        }
+#pragma unroll
+      for (int i = 0; i < FRESH; ++i) {
+        const int f = lane + 32 * i;
+        if (f < 2 * VECS) *reinterpret_cast<uint4*>((f < VECS ? k_tile : v_tile) + (v_of_pos - v0) * ROW_BYTES + f % VECS * 16) = fresh[i];
       }
-    }
-    if (NBUF == 2) {
-      if (tile + WARPS < tile_end) {
-        issue(tile + WARPS, buf ^ 1);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-      } else {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-      }
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncwarp();
-    const uint8_t* k_tile = my_smem + (size_t(buf) * 2 + 0) * 32 * ROW_BYTES;
-    const uint8_t* v_tile = my_smem + (size_t(buf) * 2 + 1) * 32 * ROW_BYTES;
     if (MMA) {
       const uint32_t kt = smem_u32(k_tile), vt = smem_u32(v_tile);
-      float sc[4][4];  // [8-key tile][row gq: 2 keys, row gq + 8: 2 keys]
+      float sc[4][4];  // [8-key tile][row gq: 2 keys, and two of the empty row gq + 8]
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
 #pragma unroll
@@ -308,95 +338,75 @@ decode_kernel(const DecodeParams p) {
           uint32_t b0, b1, b2, b3;
           const int key = np * 16 + (lane & 7) + 8 * (lane >> 4);
           ldmatrix_x4(kt + uint32_t(key * ROW_BYTES + (ks * 2 + ((lane >> 3) & 1)) * 16), b0, b1, b2, b3);
-          mma_bf16(sc[2 * np], qf[ks][0], qf[ks][1], qf[ks][2], qf[ks][3], b0, b1);
-          mma_bf16(sc[2 * np + 1], qf[ks][0], qf[ks][1], qf[ks][2], qf[ks][3], b2, b3);
+          mma_bf16(sc[2 * np], qf[ks][0], 0u, qf[ks][1], 0u, b0, b1);
+          mma_bf16(sc[2 * np + 1], qf[ks][0], 0u, qf[ks][1], 0u, b2, b3);
         }
       }
-      // scale, mask keys past the last one, online softmax over the lane's two rows (in float)
-      float mx_a = -INFINITY, mx_b = -INFINITY;
+      // scale, mask keys past the last one, online softmax over the lane's row (in float; a group has at most eight heads, so the operand's
+      // upper eight rows are zeros and their halves of the results are left alone)
+      float mx = -INFINITY;
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const bool seen = v0 + nt * 8 + 2 * tq + c < n_keys;
           sc[nt][c] = seen ? sc[nt][c] * p.scale : -INFINITY;
-          sc[nt][2 + c] = seen ? sc[nt][2 + c] * p.scale : -INFINITY;
-          if (X && p.softcap > 0.f) {
-            if (seen) sc[nt][c] = soft_cap(sc[nt][c], p.softcap);
-            if (seen) sc[nt][2 + c] = soft_cap(sc[nt][2 + c], p.softcap);
-          }
-          if (X == 2 && p.dist_bias != nullptr && seen) {
-            if (gq < G) sc[nt][c] += bias_at(gq, v0 + nt * 8 + 2 * tq + c);
-            if (gq + 8 < G) sc[nt][2 + c] += bias_at(gq + 8, v0 + nt * 8 + 2 * tq + c);
-          }
-          mx_a = fmaxf(mx_a, sc[nt][c]);
-          mx_b = fmaxf(mx_b, sc[nt][2 + c]);
+          if (X && p.softcap > 0.f && seen) sc[nt][c] = soft_cap(sc[nt][c], p.softcap);
+          if (X == 2 && p.dist_bias != nullptr && seen && gq < G) sc[nt][c] += bias_at(gq, v0 + nt * 8 + 2 * tq + c);
+          mx = fmaxf(mx, sc[nt][c]);
         }
       }
-      mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 1));
-      mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 2));
-      mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 1));
-      mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 2));
-      const float m_a = fmaxf(m_run[0], mx_a), m_b = fmaxf(m_run[1], mx_b);  // finite: a tile has a key that is seen ...
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      const float m_new = fmaxf(m_run, mx);  // finite: a tile has a key that is seen ...
       // ... unless a bias by distance forbids them all: such a tile's weights are 0, not NaN
-      const float base_a = X == 2 && m_a == -INFINITY ? 0.f : m_a, base_b = X == 2 && m_b == -INFINITY ? 0.f : m_b;
-      const float corr_a = __expf(m_run[0] - base_a), corr_b = __expf(m_run[1] - base_b);
-      float sum_a = 0.f, sum_b = 0.f;
+      const float base = X == 2 && m_new == -INFINITY ? 0.f : m_new;
+      const float corr = __expf(m_run - base);
+      float sum = 0.f;
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          sc[nt][c] = __expf(sc[nt][c] - base_a);
-          sc[nt][2 + c] = __expf(sc[nt][2 + c] - base_b);
-          sum_a += sc[nt][c];
-          sum_b += sc[nt][2 + c];
+          sc[nt][c] = __expf(sc[nt][c] - base);
+          sum += sc[nt][c];
         }
       }
-      sum_a += __shfl_xor_sync(0xffffffffu, sum_a, 1);
-      sum_a += __shfl_xor_sync(0xffffffffu, sum_a, 2);
-      sum_b += __shfl_xor_sync(0xffffffffu, sum_b, 1);
-      sum_b += __shfl_xor_sync(0xffffffffu, sum_b, 2);
-      l_run[0] = l_run[0] * corr_a + sum_a;
-      l_run[1] = l_run[1] * corr_b + sum_b;
-      m_run[0] = m_a;
-      m_run[1] = m_b;
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      l_run = l_run * corr + sum;
+      m_run = m_new;
+      if (it > 0) {
 #pragma unroll
-      for (int dt = 0; dt < DT; ++dt) {
-        o[dt][0] *= corr_a;
-        o[dt][1] *= corr_a;
-        o[dt][2] *= corr_b;
-        o[dt][3] *= corr_b;
+        for (int dt = 0; dt < DT; ++dt) {
+          o[dt][0] *= corr;
+          o[dt][1] *= corr;
+        }
       }
       // o += p . v, 16 keys at a time (rows past the last key are zeros in shared memory and p = 0)
 #pragma unroll
       for (int kk = 0; kk < 2; ++kk) {
-        const uint32_t a0 = pack_bf16(sc[2 * kk][0], sc[2 * kk][1]), a1 = pack_bf16(sc[2 * kk][2], sc[2 * kk][3]);
-        const uint32_t a2 = pack_bf16(sc[2 * kk + 1][0], sc[2 * kk + 1][1]), a3 = pack_bf16(sc[2 * kk + 1][2], sc[2 * kk + 1][3]);
+        const uint32_t a0 = pack_bf16(sc[2 * kk][0], sc[2 * kk][1]), a2 = pack_bf16(sc[2 * kk + 1][0], sc[2 * kk + 1][1]);
         // what the rounding to bfloat16 left of each weight, as a second bfloat16 operand
-        uint32_t r0 = 0, r1 = 0, r2 = 0, r3 = 0;
+        uint32_t r0 = 0, r2 = 0;
         if (X && p.split_p) {
-          r0 = pack_rest(sc[2 * kk][0], sc[2 * kk][1], a0); r1 = pack_rest(sc[2 * kk][2], sc[2 * kk][3], a1);
-          r2 = pack_rest(sc[2 * kk + 1][0], sc[2 * kk + 1][1], a2); r3 = pack_rest(sc[2 * kk + 1][2], sc[2 * kk + 1][3], a3);
+          r0 = pack_rest(sc[2 * kk][0], sc[2 * kk][1], a0);
+          r2 = pack_rest(sc[2 * kk + 1][0], sc[2 * kk + 1][1], a2);
         }
 #pragma unroll
         for (int dp = 0; dp < DT / 2; ++dp) {  // two 8-wide output tiles per ldmatrix
           uint32_t b0, b1, b2, b3;
           const int key = kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1);
           ldmatrix_x4_trans(vt + uint32_t(key * ROW_BYTES + (dp * 2 + (lane >> 4)) * 16), b0, b1, b2, b3);
-          mma_bf16(o[2 * dp], a0, a1, a2, a3, b0, b1);
-          mma_bf16(o[2 * dp + 1], a0, a1, a2, a3, b2, b3);
+          mma_bf16(o[2 * dp], a0, 0u, a2, 0u, b0, b1);
+          mma_bf16(o[2 * dp + 1], a0, 0u, a2, 0u, b2, b3);
           if (X && p.split_p) {
-            mma_bf16(o[2 * dp], r0, r1, r2, r3, b0, b1);
-            mma_bf16(o[2 * dp + 1], r0, r1, r2, r3, b2, b3);
+            mma_bf16(o[2 * dp], r0, 0u, r2, 0u, b0, b1);
+            mma_bf16(o[2 * dp + 1], r0, 0u, r2, 0u, b2, b3);
           }
         }
       }
-      if (NBUF == 1) {
-        __syncwarp();
-        if (tile + WARPS < tile_end) issue(tile + WARPS, 0);
-      } else {
-        __syncwarp();
-      }
+      __syncwarp();
+      if (tile + depth * pair_warps < tile_end) issue(tile + depth * pair_warps, k_tile);
       continue;
     }
     const bool valid = v0 + lane < n_keys;
@@ -414,8 +424,8 @@ decode_kernel(const DecodeParams p) {
           float2 kf = __bfloat1622float2(k2[u]);
 #pragma unroll
           for (int g = 0; g < G; ++g) {
-            s[g] = fmaf(q_s[g][c * 8 + 2 * u], kf.x, s[g]);
-            s[g] = fmaf(q_s[g][c * 8 + 2 * u + 1], kf.y, s[g]);
+            s[g] = fmaf(q_s[first_warp / NARROW][g][c * 8 + 2 * u], kf.x, s[g]);
+            s[g] = fmaf(q_s[first_warp / NARROW][g][c * 8 + 2 * u + 1], kf.y, s[g]);
           }
         }
       }
@@ -458,70 +468,72 @@ decode_kernel(const DecodeParams p) {
         }
       }
     }
-    if (NBUF == 1) {
-      __syncwarp();
-      if (tile + WARPS < tile_end) issue(tile + WARPS, 0);
-    } else {
-      __syncwarp();  // the buffer may be overwritten by the copy after next
-    }
+    __syncwarp();
+    if (tile + depth * pair_warps < tile_end) issue(tile + depth * pair_warps, k_tile);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-
-  // merge the four warps' states
-  if (MMA) {
+  if (has_new) {   // the newest key and value go into the cache
+    const int page = new_slot < 0 ? -1 : page_index(new_slot, p.page_size, p.page_shift);
+    if (page >= 0 && page < p.n_pages) {
+      const size_t dst = size_t(page) * p.page_stride + head_off + size_t(page_offset(new_slot, p.page_size, p.page_shift)) * HD;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int g = gq + 8 * half;
-      if (g < G) {
-        if (tq == 0) {
-          red_m[warp][g] = m_run[half];
-          red_l[warp][g] = l_run[half];
-        }
-#pragma unroll
-        for (int dt = 0; dt < DT; ++dt) {
-          red_o[warp][g][dt * 8 + 2 * tq] = o[dt][2 * half];
-          red_o[warp][g][dt * 8 + 2 * tq + 1] = o[dt][2 * half + 1];
-        }
+      for (int i = 0; i < FRESH; ++i) {
+        const int f = lane + 32 * i;
+        if (f < 2 * VECS) reinterpret_cast<uint4*>((f < VECS ? p.k_cache_w : p.v_cache_w) + dst)[f % VECS] = fresh[i];
       }
+    }
+  }
+
+  __syncwarp();
+  // merge the warps' states
+  if (MMA) {
+    if (gq < G) {
+      if (tq == 0) {
+        red_m[first_warp + warp][gq] = m_run;
+        red_l[first_warp + warp][gq] = l_run;
+      }
+#pragma unroll
+      for (int dt = 0; dt < DT; ++dt) *reinterpret_cast<float2*>(red_o(warp) + gq * HD + dt * 8 + 2 * tq) = make_float2(o[dt][0], o[dt][1]);
     }
   }
 #pragma unroll
   for (int g = 0; g < G && !MMA; ++g) {
     if (lane == 0) {
-      red_m[warp][g] = m[g];
-      red_l[warp][g] = l[g];
+      red_m[first_warp + warp][g] = m[g];
+      red_l[first_warp + warp][g] = l[g];
     }
 #pragma unroll
     for (int i = 0; i < DPL; ++i) {
       int d = 2 * (lane + 32 * i);
       if (HD % 64 == 0 || d < HD) {
-        red_o[warp][g][d] = acc[g][i][0];
-        red_o[warp][g][d + 1] = acc[g][i][1];
+        red_o(warp)[g * HD + d] = acc[g][i][0];
+        red_o(warp)[g * HD + d + 1] = acc[g][i][1];
       }
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < G * HD; i += WARPS * 32) {
+  // warps without a tile have nothing to add
+  const int used = min(pair_warps, max(tile_end - tile_begin, 0));
+  for (int i = pair_thread; exists && i < G * HD; i += pair_threads) {
     int g = i / HD, d = i % HD;
     float mx = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) mx = fmaxf(mx, red_m[w][g]);
+    for (int w = 0; w < used; ++w) mx = fmaxf(mx, red_m[first_warp + w][g]);
     float o = 0.f, lsum = 0.f;
     if (mx > -INFINITY) {
-#pragma unroll
-      for (int w = 0; w < WARPS; ++w) {
-        float c = __expf(red_m[w][g] - mx);
-        o += c * red_o[w][g][d];
-        lsum += c * red_l[w][g];
+#pragma unroll 4
+      for (int w = 0; w < used; ++w) {
+        float c = __expf(red_m[first_warp + w][g] - mx);
+        o += c * red_o(w)[g * HD + d];
+        lsum += c * red_l[first_warp + w][g];
       }
     }
-    if (p.n_slices == 1) {
+    if (n_slices == 1) {
       const bf16* gate = (X && p.gate != nullptr) ? p.gate + size_t(t) * p.gate_row_stride + size_t(h0 + g) * HD + d : nullptr;
       p.out[size_t(t) * p.out_row_stride + size_t(h0 + g) * HD + d] = __float2bfloat16_rn(finish(
           o, lsum, mx, X ? p.sink : 0, gate, (X && p.sinks != nullptr) ? p.sinks[h0 + g] : 0.f,
           (X && p.head_gate != nullptr) ? p.head_gate + size_t(t) * p.head_gate_stride + h0 + g : nullptr, X == 2 ? p.out_scale : 1.f));
     } else if (p.clustered) {
-      red_o[0][g][d] = o;   // (this thread alone has read the place)
+      red_o(0)[g * HD + d] = o;   // (this thread alone has read the place)
       if (d == 0) {
         cta_m[g] = mx;
         cta_l[g] = lsum;
@@ -536,17 +548,18 @@ decode_kernel(const DecodeParams p) {
     }
   }
   if (p.clustered) {
+    if (n_slices == 1) return;
     // the cluster's CTAs share the outputs; the slices are added in slice order
     cluster_barrier();
-    for (int i = slice * WARPS * 32 + threadIdx.x; i < G * HD; i += p.n_slices * WARPS * 32) {
+    for (int i = slice * WARPS * 32 + threadIdx.x; i < G * HD; i += n_slices * WARPS * 32) {
       const int g = i / HD, d = i % HD;
       float ms[MAX_CLUSTER], ls[MAX_CLUSTER], os[MAX_CLUSTER];
 #pragma unroll
       for (int s = 0; s < MAX_CLUSTER; ++s) {
-        const bool there = s < p.n_slices;
+        const bool there = s < n_slices;
         ms[s] = there ? remote_float(&cta_m[g], s) : -INFINITY;
         ls[s] = there ? remote_float(&cta_l[g], s) : 0.f;
-        os[s] = there ? remote_float(&red_o[0][g][d], s) : 0.f;
+        os[s] = there ? remote_float(red_o(0) + g * HD + d, s) : 0.f;
       }
       float mx = -INFINITY;
 #pragma unroll
@@ -556,7 +569,7 @@ decode_kernel(const DecodeParams p) {
 #pragma unroll
         for (int s = 0; s < MAX_CLUSTER; ++s) {
           const float c = __expf(ms[s] - mx);
-          if (s < p.n_slices) {
+          if (s < n_slices) {
             o += c * os[s];
             lsum += c * ls[s];
           }
@@ -631,7 +644,7 @@ __global__ void merge_kernel(const float* __restrict__ part_o, const float* __re
   }
 }
 
-template <int G, bool MMA, int X>
+template <int G, bool MMA, int X, int WARPS>
 bool configure_smem() {
   // once per kernel instance and device (function attributes belong to a device's context): room for
   // the tiles beyond the default 48 KB
@@ -640,23 +653,25 @@ bool configure_smem() {
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return false;
   bool& done = done_on[device];
   if (!done) {
-    if (cudaFuncSetAttribute(decode_kernel<G, MMA, X>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM) != cudaSuccess) return false;
+    if (cudaFuncSetAttribute(decode_kernel<G, MMA, X, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_places(WARPS) * TILE_SMEM) != cudaSuccess) return false;
     // the CTAs hide each other's waits: ask for the shared memory that lets as many as fit be resident
-    if (cudaFuncSetAttribute(decode_kernel<G, MMA, X>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess) return false;
+    if (cudaFuncSetAttribute(decode_kernel<G, MMA, X, WARPS>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess) return false;
     done = true;
   }
   return true;
 }
 
-template <int G, bool MMA, int X>
+template <int G, bool MMA, int X, int WARPS>
 int launch_form(const DecodeParams& p, int n_rows, cudaStream_t stream) {
+  const int at_once = WARPS / p.pair_warps;
   dim3 grid(p.n_slices, p.n_kv_heads, n_rows);
-  if (!configure_smem<G, MMA, X>()) return R2_UNSUPPORTED;
+  if (at_once > 1) grid = dim3(p.n_slices, (n_rows * p.n_kv_heads + at_once - 1) / at_once, 1);   // (the plan's launches of a few hundred pairs)
+  if (!configure_smem<G, MMA, X, WARPS>()) return R2_UNSUPPORTED;
   if (p.clustered) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = dim3(WARPS * 32);
-    config.dynamicSmemBytes = TILE_SMEM;
+    config.dynamicSmemBytes = tile_places(WARPS) * TILE_SMEM;
     config.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -666,19 +681,19 @@ int launch_form(const DecodeParams& p, int n_rows, cudaStream_t stream) {
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attr;
     config.numAttrs = (g_r2_pdl && !t_r2_plain_order) ? 2 : 1;
-    cudaLaunchKernelEx(&config, decode_kernel<G, MMA, X>, p);
+    cudaLaunchKernelEx(&config, decode_kernel<G, MMA, X, WARPS>, p);
     return launch_status();
   }
-  r2_launch(decode_kernel<G, MMA, X>, dim3(grid), dim3(WARPS * 32), size_t(TILE_SMEM), stream, p);
+  r2_launch(decode_kernel<G, MMA, X, WARPS>, dim3(grid), dim3(WARPS * 32), size_t(tile_places(WARPS) * TILE_SMEM), stream, p);
   return launch_status();
 }
 
 template <int G, int X = 0>
 int launch(const DecodeParams& p, int n_rows, cudaStream_t stream) {
   if constexpr (MMA_FITS) {
-    if (g_decode_mma) return launch_form<G, true, X>(p, n_rows, stream);
+    if (g_decode_mma) return p.wide ? launch_form<G, true, X, WIDE>(p, n_rows, stream) : launch_form<G, true, X, NARROW>(p, n_rows, stream);
   }
-  return launch_form<G, false, X>(p, n_rows, stream);
+  return launch_form<G, false, X, NARROW>(p, n_rows, stream);
 }
 
 }  // namespace
@@ -715,7 +730,7 @@ extern "C" int r2_attention_decode(const void* q, int q_row_stride, void* out, i
   p.part_o = scratch;
   p.part_ml = scratch != nullptr ? scratch + (long long)n_rows * n_heads * n_slices * HD : nullptr;
   p.k_new = nullptr; p.v_new = nullptr; p.new_row_stride = 0; p.slot_mapping = nullptr;
-  p.k_cache_w = nullptr; p.v_cache_w = nullptr; p.counters = nullptr; p.clustered = 0;
+  p.k_cache_w = nullptr; p.v_cache_w = nullptr; p.counters = nullptr; p.clustered = 0; p.cache_settled = 0; p.wide = 0; p.pair_warps = NARROW; p.n_rows = n_rows;
   int status;
   switch (n_heads / n_kv_heads) {
     case 1: status = launch<1>(p, n_rows, stream); break;
@@ -753,7 +768,8 @@ int launch_fused(const DecodeParams& p, int n_rows, cudaStream_t stream) {
 // kernel nor a merge kernel.
 // `scratch` as for r2_attention_decode; `counters` holds n_rows * n_kv_heads ints that are
 // zero before the call and zero again after it. `keep_first`, `sink`, `gate` and `split_p`: see DecodeParams.
-// `chunk`, `dist_bias`, `bias_len` and `out_scale` (0, null, 0 and 1: none of them) likewise.
+// `chunk`, `dist_bias`, `bias_len` and `out_scale` (0, null, 0 and 1: none of them) likewise. `cache_settled`: the caller says that no launch
+// shortly before wrote the cache's rows that the batch reads (those of steps that have ended).
 extern "C" int r2_attention_decode_fused_biased(const void* q, int q_row_stride, void* out, int out_row_stride, void* k_cache,
                                          void* v_cache, long long page_stride, int page_size, int n_pages,
                                          const int32_t* block_tables, int table_width, const int32_t* row_entry,
@@ -763,7 +779,7 @@ extern "C" int r2_attention_decode_fused_biased(const void* q, int q_row_stride,
                                          float* scratch, long long scratch_floats, int* counters, int n_counters,
                                          int keep_first, int sink, const void* gate, int gate_row_stride, int split_p,
                                          float softcap, const float* sinks, const float* head_gate, int head_gate_stride,
-                                         int chunk, const float* dist_bias, int bias_len, float out_scale, cudaStream_t stream) {
+                                         int chunk, const float* dist_bias, int bias_len, float out_scale, int cache_settled, int pair_warps, cudaStream_t stream) {
   if (n_rows <= 0) return R2_OK;
   if (keep_first < 0 || chunk < 0 || (chunk > 0 && window > 0) || (dist_bias != nullptr && bias_len < 1)) return R2_BAD_SHAPE;
   if (n_heads < 1 || n_kv_heads < 1 || n_heads % n_kv_heads != 0 || page_size < 1 || window < 0 || n_slices < 1) return R2_BAD_SHAPE;
@@ -791,6 +807,12 @@ extern "C" int r2_attention_decode_fused_biased(const void* q, int q_row_stride,
   p.k_cache_w = (bf16*)k_cache; p.v_cache_w = (bf16*)v_cache;
   p.counters = n_slices > 1 ? counters : nullptr;
   p.clustered = n_slices > 1 && n_slices <= MAX_CLUSTER;
+  p.n_rows = n_rows;
+  // the caller's plan (r2_attention_decode_plan); the scalar form has narrow CTAs alone
+  p.wide = MMA_FITS && g_decode_mma && pair_warps > NARROW;
+  p.pair_warps = p.wide ? pair_warps : NARROW;
+  if (p.wide && (pair_warps > WIDE || (pair_warps & (pair_warps - 1)) != 0 || (n_slices > 1 && (pair_warps != WIDE || !p.clustered)))) return R2_BAD_SHAPE;
+  p.cache_settled = cache_settled != 0 && k_new != nullptr;   // (without k_new the newest key is another layer's, written in this step)
   switch (n_heads / n_kv_heads) {
     case 1: return launch_fused<1>(p, n_rows, stream);
     case 2: return launch_fused<2>(p, n_rows, stream);
@@ -816,7 +838,7 @@ extern "C" int r2_attention_decode_fused(const void* q, int q_row_stride, void* 
   return r2_attention_decode_fused_biased(q, q_row_stride, out, out_row_stride, k_cache, v_cache, page_stride, page_size, n_pages,
                                           block_tables, table_width, row_entry, positions, seq_lens, n_rows, n_heads, n_kv_heads, scale,
                                           window, n_slices, k_new, v_new, new_row_stride, slot_mapping, scratch, scratch_floats, counters,
-                                          n_counters, keep_first, sink, gate, gate_row_stride, split_p, 0.f, nullptr, nullptr, 0, 0, nullptr, 0, 1.f, stream);
+                                          n_counters, keep_first, sink, gate, gate_row_stride, split_p, 0.f, nullptr, nullptr, 0, 0, nullptr, 0, 1.f, 0, NARROW, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

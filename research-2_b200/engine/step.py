@@ -39,6 +39,9 @@ class StepContext:
         t, r, w = counts or (host.n_tokens, host.n_entries, host.n_logit_rows)
         self.n_tokens, self.n_entries, self.n_logit_rows = t, r, w
         self.captured = counts is not None
+        # a step's first operation is the copy of its batch, an ordinary stream operation: what the steps before wrote into caches and states
+        # is complete when the step's first kernel starts, however early a kernel starts beside the one in front of it
+        self.cache_settled = True
         # (stream tensor, its rows in the compute dtype): a block whose last kernel wrote both leaves the pair here for the next one
         self.stream_rounded = None
         # shape facts that choose kernels: inside a graph every row is an entry of its own and

@@ -253,6 +253,23 @@ def decode_slices(n_rows: int, n_kv_heads: int, max_context: int, device="cuda:0
     return max(1, min(want, most, 32))
 
 
+def decode_plan(n_rows: int, n_kv_heads: int, head_dim: int, max_context: int, device="cuda:0") -> tuple[int, int]:
+    """(slices of the keys, warps of a CTA per (row, kv head) pair) of fused decode attention: wide CTAs, one to an SM, while all pairs find
+    room on the chip side by side (all of a CTA's 16 warps for a pair, 8 for head sizes above 64; half of them where there are more pairs than
+    SMs), with slices (a cluster) only for contexts of more than two tiles a warp and where SMs are left; else narrow ones (`decode_slices`). Measured in
+    steps of GPT-2 (20, 200, 500 and 1,000 keys a row, ms): 124M, 8 rows, narrow 0.245 / 0.272 / 0.285 / 0.338, wide 0.236 / 0.236 / 0.258 /
+    0.295; 16 rows 0.294 / 0.323 / 0.381 / 0.439 and 0.285 / 0.297 / 0.335 / 0.406; 355M, 16 rows (256 pairs) 0.579 / 0.654 / 0.764 / 0.974 and 0.577 /
+    0.602 / 0.679 / 0.825. With 32 rows (384 pairs) short rows are faster narrow (0.334 and 0.370), long ones wide (0.703 and 0.631).
+    One row: two slices cost 12 us of 406 (355M) where they are not needed and gain 33 of 496 at 1,000 keys."""
+    pairs, sms = max(1, n_rows * n_kv_heads), sm_count(device)
+    wide = 16 if head_dim <= 64 else 8 if head_dim <= 128 else 0
+    if wide and pairs <= sms:
+        return max(1, min(sms // pairs, -(-max_context // (64 * wide)), 8)), wide
+    if wide and pairs <= 2 * sms:
+        return 1, wide // 2
+    return decode_slices(n_rows, n_kv_heads, max_context, device), 4
+
+
 def _lib_for_head_dim(source: str, head_dim: int) -> C.CDLL:
     key = f"{source}:{head_dim}"
     lib = _libs.get(key)
@@ -1662,14 +1679,16 @@ def decode_attention_fused(q: torch.Tensor, k_new: torch.Tensor | None, v_new: t
                            gate: torch.Tensor | None = None, exact_weights: bool = False, softcap: float = 0.0,
                            sinks: torch.Tensor | None = None, head_gate: torch.Tensor | None = None, chunk: int = 0,
                            dist_bias: torch.Tensor | None = None, out_scale: float = 1.0,
-                           out: torch.Tensor | None = None) -> torch.Tensor | None:
+                           out: torch.Tensor | None = None, *, cache_settled: bool = False) -> torch.Tensor | None:
     """Decode attention in ONE launch for a batch in which every row is an entry of its own: the
     kernel writes the new keys and values to their cache slots, and the slice that finishes last
     merges all slices of its row. Returns None when it does not take the case (the caller then writes
     the cache and calls `paged_attention`). With `k_new` None nothing is written: the rows read a cache that already holds
     their own position (a layer that reads the keys and values another layer wrote in this step).
     `keep_first`, `sink`, `gate`, `softcap`, `sinks`, `head_gate`, `chunk`, `dist_bias` and `out_scale` as in `paged_attention`;
-    `exact_weights` carries the softmax's weights into the second product as two bfloat16 terms."""
+    `exact_weights` carries the softmax's weights into the second product as two bfloat16 terms. `cache_settled`: the caller says that no
+    launch of this package shortly before wrote cache rows that the batch reads (an ordinary stream operation, such as the copy of a step's batch,
+    lies between): they are then asked for while the previous kernel still runs."""
     group = n_heads // max(n_kv_heads, 1)
     if not (_fast_attention and _fused_decode and q.dtype == torch.bfloat16 and k_cache.dtype == torch.bfloat16
             and 1 <= group <= 8 and head_dim % 16 == 0):
@@ -1692,7 +1711,7 @@ def decode_attention_fused(q: torch.Tensor, k_new: torch.Tensor | None, v_new: t
     elif chunk > 0:
         max_context = min(max_context, chunk)
     bias_len = _bias_len(dist_bias, n_heads)
-    slices = decode_slices(n, n_kv_heads, max_context, q.device)
+    slices, pair_warps = decode_plan(n, n_kv_heads, head_dim, max_context, q.device)
     lib = _lib_for_head_dim("attention_decode", head_dim)
     ws = _workspace(q.device)
     if (lib.r2_attention_decode_scratch_floats(n, n_heads, slices) > ws.floats.numel()
@@ -1725,7 +1744,7 @@ def decode_attention_fused(q: torch.Tensor, k_new: torch.Tensor | None, v_new: t
         n_kv_heads, C.c_float(scale), window, slices, _p(k_new), _p(v_new), stride, _p(slot_mapping), _p(ws.floats),
         C.c_longlong(ws.floats.numel()), _p(ws.counters), ws.counters.numel(), keep_first, int(bool(sink)), _p(gate),
         gate_stride, int(bool(exact_weights)), C.c_float(softcap), _p(sinks), _p(head_gate), head_gate_stride, chunk, _p(dist_bias), bias_len,
-        C.c_float(out_scale), _stream())
+        C.c_float(out_scale), int(cache_settled), pair_warps, _stream())
     if status == -4:
         return None
     _check(status, "decode attention (fused)")

@@ -273,3 +273,28 @@ def test_norms_of_rows(width, dtype, gathered):
     want = read * torch.rsqrt((read * read).mean(-1, keepdim=True) + 1e-5) * gain.double()
     bound = 2.0 ** -20 * want.abs() + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0.0)
     assert ((o.rms_norm(x, gain, 1e-5, dtype, rows=rows).double() - want).abs() <= bound).all()
+
+
+# contexts (before the new token) around a tile, a CTA's tiles (16 and 24 warps' worth at head size 64, 8 and 12 at 128) and clusters' runs
+@pytest.mark.parametrize("h,hkv,hd", [(4, 4, 64), (8, 2, 64), (6, 1, 64), (2, 1, 128), (2, 2, 16)])
+@pytest.mark.parametrize("window", [0, 260])
+def test_decode_attention_of_every_plan(h, hkv, hd, window, monkeypatch):
+    o = ops()
+    contexts = [0, 1, 31, 32, 255, 256, 383, 511, 512, 513, 767, 768, 1100]
+    wide = 16 if hd <= 64 else 8
+    for plan in ((1, 4), (6, 4), (1, wide // 2), (1, wide), (2, wide), (3, wide)):
+        pc = PagedCase([(c, 1) for c in contexts], h, hkv, hd, 16, torch.bfloat16, seed=hd + window, garbage=1e4)
+        monkeypatch.setattr(o, "decode_plan", lambda *a, **k: plan)
+        got = o.decode_attention_fused(pc.q_rows, pc.k_new, pc.v_new, pc.slots, pc.k_cache, pc.v_cache, pc.page_stride, pc.page, pc.n_pages,
+                                       pc.tables, pc.row_entry, pc.positions, pc.seq_lens, h, hkv, hd, hd ** -0.5, window, 2048, cache_settled=True)
+        torch.testing.assert_close(got.float().cpu(), pc.plain(hd ** -0.5, window), atol=3e-2, rtol=3e-2, msg=lambda m: f"plan {plan}: {m}")
+        cached = o.paged_attention(pc.q_rows, pc.k_cache, pc.v_cache, pc.page_stride, pc.page, pc.n_pages, pc.tables, pc.row_entry, pc.positions,
+                                   pc.seq_lens, h, hkv, hd, hd ** -0.5, window)   # the new rows are in the cache
+        torch.testing.assert_close(cached.float(), got.float(), atol=2e-2, rtol=2e-2)
+
+
+def test_decode_plans():
+    o = ops()
+    assert o.decode_plan(8, 12, 64, 1024) == (1, 16) and o.decode_plan(1, 12, 64, 4096) == (4, 16) and o.decode_plan(1, 12, 64, 1024) == (1, 16)
+    assert o.decode_plan(16, 12, 64, 1024) == (1, 8) and o.decode_plan(64, 12, 64, 1024) == (1, 4)
+    assert o.decode_plan(1, 2, 128, 600) == (2, 8) and o.decode_plan(8, 12, 256, 1024) == (6, 4)   # (head sizes beyond 128 have narrow CTAs alone)
