@@ -30,9 +30,15 @@ __global__ void embed_kernel(const int32_t* __restrict__ ids, const int32_t* __r
 }
 
 extern "C" int r2_embed(const int32_t* ids, const int32_t* positions, const void* table, const void* pos_table,
-                        float* out, int n_rows, int width, int n_vocab, int n_positions, int wdtype, float scale,
+                        float* out, int n_rows, int width, int n_vocab, int n_positions, int wdtype, float scale, int plain_order,
                         cudaStream_t stream) {
   if (n_rows <= 0) return R2_OK;
+  // (plain_order: the launch waits for the whole kernel before, so that what that one wrote is there for every later kernel's prologue)
+  struct PlainOrder {
+    int before = t_r2_plain_order;
+    ~PlainOrder() { t_r2_plain_order = before; }
+  } restore;
+  if (plain_order) t_r2_plain_order = 1;
   if (width < 1 || n_vocab < 1) return R2_BAD_SHAPE;
   int threads = width >= 256 ? 256 : (width >= 128 ? 128 : 64);
   if (wdtype == R2_F32) {

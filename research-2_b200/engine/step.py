@@ -39,8 +39,8 @@ class StepContext:
         t, r, w = counts or (host.n_tokens, host.n_entries, host.n_logit_rows)
         self.n_tokens, self.n_entries, self.n_logit_rows = t, r, w
         self.captured = counts is not None
-        # a step's first operation is the copy of its batch, an ordinary stream operation: what the steps before wrote into caches and states
-        # is complete when the step's first kernel starts, however early a kernel starts beside the one in front of it
+        # a step's first operations, the copy of its batch (a graph: the kernel that fetches it) and the embedding behind it, run in plain order: what
+        # the steps before wrote into caches and states is complete when a later kernel starts, however early it starts beside the one in front
         self.cache_settled = True
         # (stream tensor, its rows in the compute dtype): a block whose last kernel wrote both leaves the pair here for the next one
         self.stream_rounded = None
@@ -93,27 +93,38 @@ def _bucket(n: int) -> int:
 class StepGraph:
     """Forward pass + sampling of a batch of up to `t_cap` rows in up to `r_cap` entries (one
     logit row per entry), as one CUDA graph. t_cap == r_cap is the decode-only form. The graph
-    begins with the copy of the pinned host batch to the device and ends with the copy of the
-    sampled tokens into pinned host memory, so that a step is one graph launch and one wait."""
+    begins with the pinned host batch's way to the device and ends with the sampled tokens' into
+    pinned host memory, so that a step is one graph launch and one wait. There are two host
+    batches, which replays read in turn: the next step's batch can be written while this one runs."""
 
     def __init__(self, step_fn: "StepFunction", t_cap: int, r_cap: int):
         self.cap = r_cap
-        self.device = step_fn.device
-        self.host = StepBatch(BatchLayout(t_cap, r_cap, r_cap, step_fn.table_widths), pinned=True)
-        self.host.max_context_bound = step_fn.max_seq_len
-        self.host.pad()
-        self.host.set_logit_rows([])
-        self.host.set_sampling([], [], [], [], [])
-        self.dev = torch.zeros(self.host.buf.shape[0], dtype=torch.int32, device=step_fn.device)
-        self.dev.copy_(self.host._pinned_tensor)
-        self.ctx = StepContext(self.host, self.dev, counts=(t_cap, r_cap, r_cap))
+        self.device, self.device_index = step_fn.device, step_fn._device_index
+        self.hosts = []
+        for _ in range(2):
+            host = StepBatch(BatchLayout(t_cap, r_cap, r_cap, step_fn.table_widths), pinned=True)
+            host.max_context_bound = step_fn.max_seq_len
+            host.pad()
+            host.set_logit_rows([])
+            host.set_sampling([], [], [], [], [])
+            host.copy_done = torch.cuda.Event()   # recorded after every replay that read it: it may be written again
+            self.hosts.append(host)
+        self.turn = 0                             # the host batch that the next replay reads
+        self.turn_device = torch.zeros(1, dtype=torch.int32, device=step_fn.device)
+        self.dev = torch.zeros(self.hosts[0].buf.shape[0], dtype=torch.int32, device=step_fn.device)
+        self.dev.copy_(self.hosts[0]._pinned_tensor)
+        self.ctx = StepContext(self.hosts[0], self.dev, counts=(t_cap, r_cap, r_cap))
         self.tokens_host = torch.zeros(r_cap, dtype=torch.int32).pin_memory()
         self.tokens_host_np = self.tokens_host.numpy()
         # the device's error word travels to the host with the tokens: a kernel's time-out is seen at no extra cost
         self.error_host = torch.zeros(4, dtype=torch.int32).pin_memory()
         self.error_host_np = self.error_host.numpy()
         self.error_word = ops.error_word(self.device)
-        self.done = torch.cuda.Event()   # recorded after every replay: the batch is consumed, the tokens are on the host
+        self.addresses = [ops.host_address(t) for t in (self.hosts[0]._pinned_tensor, self.hosts[1]._pinned_tensor, self.tokens_host, self.error_host)]
+        if any(a is None for a in self.addresses):
+            raise RuntimeError("the step's pinned host memory cannot be reached from the device")
+        self.done = self.hosts[1].copy_done   # of the last replay: the tokens are on the host
+        self.stream = None                    # the last replay's
         side = torch.cuda.Stream(device=step_fn.device)
         side.wait_stream(torch.cuda.current_stream(step_fn.device))
         with torch.cuda.stream(side):  # inert warm-up: every row is a pad row
@@ -139,17 +150,38 @@ class StepGraph:
         self.graph = torch.cuda.CUDAGraph()
         before = ops.launch_count()
         with torch.cuda.graph(self.graph, pool=step_fn.graph_pool()):
-            self.dev.copy_(self.host._pinned_tensor, non_blocking=True)
+            ops.fetch_batch(self.addresses[0], self.addresses[1], self.dev, self.turn_device)
             self.logits = step_fn.forward(self.ctx)
             self.tokens = step_fn.sample(self.logits, self.ctx)
-            self.tokens_host.copy_(self.tokens, non_blocking=True)
-            self.error_host.copy_(self.error_word, non_blocking=True)
+            ops.finish_step(self.tokens, self.addresses[2], self.error_word, self.addresses[3], self.turn_device)
         self.kernels = ops.launch_count() - before
 
-    def replay(self) -> None:
+    def __del__(self):
+        # a replay that still runs reads and writes the graph's pinned memory, which others may be given once it is let go
+        try:
+            for host in self.hosts:
+                host.copy_done.synchronize()
+        except Exception:  # noqa: BLE001  (an unfinished constructor, the interpreter's end)
+            pass
+
+    @property
+    def host(self) -> StepBatch:
+        """The host batch that the next replay reads."""
+        return self.hosts[self.turn]
+
+    def replay(self, batch: StepBatch) -> None:
+        """Runs one of the graph's host batches (the other one's numbers are copied where it is that one's turn)."""
+        if batch is not self.host:
+            self.host.copy_done.synchronize()
+            self.host.buf[:] = batch.buf
+        stream = torch._C._cuda_getCurrentRawStream(self.device_index)
+        if self.stream is not None and stream != self.stream:   # a replay waits for the one before, whose buffers it uses
+            torch.cuda.current_stream(self.device).wait_event(self.done)
+        self.stream = stream
         self.graph.replay()
+        self.done = self.host.copy_done
         self.done.record()
-        self.host.copy_done = self.done
+        self.turn ^= 1
         ops.count_launches(self.kernels)
 
     def tokens_on_host(self, n: int) -> np.ndarray:
@@ -243,7 +275,7 @@ class StepFunction:
 
     def _graph_of(self, batch: StepBatch) -> StepGraph | None:
         graph = self._graphs.get((batch.t_cap, batch.r_cap)) if self.capture else None
-        return graph if graph is not None and batch is graph.host else None
+        return graph if graph is not None and (batch is graph.hosts[0] or batch is graph.hosts[1]) else None
 
     def upload(self, batch: StepBatch) -> StepContext:
         if not batch.trusted:
@@ -289,7 +321,7 @@ class StepFunction:
             if graph is not None:
                 if not batch.trusted:
                     batch.pad()
-                graph.replay()
+                graph.replay(batch)
                 self.h2d_bytes += batch.buf.nbytes
                 return graph.logits[: batch.n_logit_rows]
             return self.forward(self.upload(batch))
@@ -306,9 +338,9 @@ class StepFunction:
             return None
         if torch.cuda.current_device() != self._device_index:
             with torch.cuda.device(self.device):
-                graph.replay()
+                graph.replay(batch)
         else:
-            graph.replay()
+            graph.replay(batch)
         self.h2d_bytes += batch.buf.nbytes
         return graph
 
@@ -321,7 +353,7 @@ class StepFunction:
             if graph is not None:
                 if not batch.trusted:
                     batch.pad()
-                graph.replay()
+                graph.replay(batch)
                 self.h2d_bytes += batch.buf.nbytes
                 return graph.tokens[: batch.n_logit_rows]
             ctx = self.upload(batch)

@@ -137,6 +137,8 @@ def _lib(source: str) -> C.CDLL:
     if lib is None:
         lib = kernel_library(source)
         lib.r2_set_pdl(int(_pdl))
+        if source == "step_io":
+            lib.r2_host_address.restype = C.c_void_p
         _libs[source] = lib
     return lib
 
@@ -144,7 +146,7 @@ def _lib(source: str) -> C.CDLL:
 def build_all(head_dims=()) -> None:
     """Compile every kernel library that does not depend on a model, and the attention kernels
     for the given head sizes (a model compiles its own head size at first use otherwise)."""
-    for source in ("rowwise", "recurrent", "state_scan", "decay_chunks", "streams", "routing", "gemm_simt", "gemm_tc", "few_rows", "attention_simt", "attention_prefill_tc", "latent_attention",
+    for source in ("rowwise", "recurrent", "state_scan", "decay_chunks", "streams", "routing", "gemm_simt", "gemm_tc", "few_rows", "step_io", "attention_simt", "attention_prefill_tc", "latent_attention",
                    "sampling", "wait_selftest"):
         _lib(source)
     kernel_library("sfu_probe")  # (profiling/sfu_probe.py: a measurement, no part of a step)
@@ -405,9 +407,30 @@ def wait_selftest(device="cuda:0", polls: int = 64, code: int = 99) -> None:
 # ---------------------------------------------------------------------------------------------
 
 
+def host_address(pinned: torch.Tensor) -> int | None:
+    """The device's address of a pinned host tensor; None where the device cannot reach it."""
+    return _lib("step_io").r2_host_address(C.c_void_p(pinned.data_ptr()))
+
+
+def fetch_batch(even: int, odd: int, dev: torch.Tensor, turn: torch.Tensor) -> None:
+    """dev <- one of two pinned host arrays (device addresses), by `turn`'s lowest bit (int32 [1] on the device). The launch that follows
+    must be in plain order (`embed(plain_order=True)`)."""
+    _need(dev, "dev", torch.int32, 1)
+    _need(turn, "turn", torch.int32, 1)
+    _check(_lib("step_io").r2_fetch_batch(C.c_void_p(even), C.c_void_p(odd), _p(dev), dev.shape[0], _p(turn), _stream()), "fetch_batch")
+
+
+def finish_step(tokens: torch.Tensor, host_tokens: int, error: torch.Tensor, host_error: int, turn: torch.Tensor) -> None:
+    """tokens and the error word into pinned host memory (device addresses); `turn` counts one more."""
+    _need(tokens, "tokens", torch.int32, 1)
+    _check(_lib("step_io").r2_finish_step(_p(tokens), tokens.shape[0], C.c_void_p(host_tokens), _p(error), error.shape[0], C.c_void_p(host_error), _p(turn),
+                                          _stream()), "finish_step")
+
+
 def embed(ids: torch.Tensor, table: torch.Tensor, positions: torch.Tensor | None = None,
-          pos_table: torch.Tensor | None = None, out: torch.Tensor | None = None, scale: float = 1.0) -> torch.Tensor:
-    """out[t] = table[ids[t]] * scale (+ pos_table[positions[t]]) as float32 [T, width]."""
+          pos_table: torch.Tensor | None = None, out: torch.Tensor | None = None, scale: float = 1.0, *, plain_order: bool = False) -> torch.Tensor:
+    """out[t] = table[ids[t]] * scale (+ pos_table[positions[t]]) as float32 [T, width]. `plain_order`: not launched beside the kernel
+    before (`fetch_batch`, whose arrays later kernels read ahead of their own waits)."""
     _need(ids, "ids", torch.int32, 1)
     _need(table, "table", dim=2)
     n, width = ids.shape[0], table.shape[1]
@@ -423,7 +446,7 @@ def embed(ids: torch.Tensor, table: torch.Tensor, positions: torch.Tensor | None
     _need(out, "out", torch.float32, 2)
     fn = _lib("rowwise").r2_embed
     status = fn(_p(ids), _p(positions), _p(table), _p(pos_table), _p(out), n, width, table.shape[0],
-                0 if pos_table is None else pos_table.shape[0], dtype_code(table.dtype), C.c_float(scale), _stream())
+                0 if pos_table is None else pos_table.shape[0], dtype_code(table.dtype), C.c_float(scale), int(plain_order), _stream())
     _check(status, "embed")
     return out
 

@@ -94,7 +94,7 @@ class PagedAttention:
             mixed = ops.decode_attention_fused(
                 q, k, v, ctx.slot_mapping[cache.group], cache.k, cache.v, cache.page_stride, cache.page_size,
                 cache.n_pages, ctx.block_tables[cache.group], ctx.row_entry, ctx.positions, ctx.seq_lens, self.n_heads,
-                self.n_kv_heads, self.head_dim, self.scale, self.window, ctx.max_context, cache_settled=ctx.cache_settled)
+                self.n_kv_heads, self.head_dim, self.scale, self.window, ctx.max_context, cache_settled=getattr(ctx, "cache_settled", False))
             if mixed is not None:
                 return ops.linear(mixed, self.w_out, self.b_out, w_is_nk=self.w_is_nk, residual=residual)
         if writes_cache and not in_cache:
@@ -192,7 +192,7 @@ class QKNormAttention:
                 q, k, v, ctx.slot_mapping[cache.group], cache.k, cache.v, cache.page_stride, cache.page_size,
                 cache.n_pages, ctx.block_tables[cache.group], ctx.row_entry, ctx.positions, ctx.seq_lens, self.n_heads,
                 self.n_kv_heads, self.head_dim, self.scale, self.window, ctx.max_context, keep_first=self.keep_first,
-                sink=self.sink, gate=gate, exact_weights=ops.exact_weights(), cache_settled=ctx.cache_settled)
+                sink=self.sink, gate=gate, exact_weights=ops.exact_weights(), cache_settled=getattr(ctx, "cache_settled", False))
             if mixed is not None:
                 return ops.linear(mixed, self.w_out, None, w_is_nk=True, residual=residual)
             ops.kv_write(k, v, cache.k, cache.v, ctx.slot_mapping[cache.group], self.n_kv_heads, self.head_dim,
@@ -319,7 +319,7 @@ class RotaryWindowAttention:
                 q, k if writes_cache else None, v if writes_cache else None, ctx.slot_mapping[cache.group], cache.k, cache.v, cache.page_stride,
                 cache.page_size, cache.n_pages, ctx.block_tables[cache.group], ctx.row_entry, ctx.positions, ctx.seq_lens, self.n_heads,
                 self.n_kv_heads, self.head_dim, self.scale, self.window, ctx.max_context, exact_weights=ops.exact_weights(), softcap=self.softcap,
-                sinks=self.sinks, head_gate=gate, cache_settled=ctx.cache_settled)
+                sinks=self.sinks, head_gate=gate, cache_settled=getattr(ctx, "cache_settled", False))
             if mixed is not None:
                 return mixed
             if writes_cache:
@@ -579,7 +579,7 @@ class DistanceBiasAttention:
             mixed = ops.decode_attention_fused(
                 q, k, v, ctx.slot_mapping[cache.group], cache.k, cache.v, cache.page_stride, cache.page_size, cache.n_pages,
                 ctx.block_tables[cache.group], ctx.row_entry, ctx.positions, ctx.seq_lens, self.n_heads, self.n_kv_heads, self.head_dim,
-                self.scale, 0, ctx.max_context, exact_weights=ops.exact_weights(), cache_settled=ctx.cache_settled, **attend)
+                self.scale, 0, ctx.max_context, exact_weights=ops.exact_weights(), cache_settled=getattr(ctx, "cache_settled", False), **attend)
             if mixed is not None:
                 return mixed
             ops.kv_write(k, v, cache.k, cache.v, ctx.slot_mapping[cache.group], self.n_kv_heads, self.head_dim,

@@ -21,7 +21,8 @@ class TokenEmbedding:
         self.scale = float(scale)  # table rows are multiplied by it on their way into the stream
 
     def forward(self, ctx, additive_table=None):
-        return ops.embed(ctx.input_ids, self.table, ctx.positions, additive_table, scale=self.scale)
+        # (a captured step's batch comes from the kernel in front)
+        return ops.embed(ctx.input_ids, self.table, ctx.positions, additive_table, scale=self.scale, plain_order=getattr(ctx, "captured", False))
 
 
 class Head:
