@@ -1341,6 +1341,8 @@ def _linear_of_normed(a: NormedRows, w, bias, w_is_nk, act, residual, out_dtype,
     n = w.shape[0] if w_is_nk else w.shape[1]
     if not (_tensor_core_gemm and _fused_norm and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and m <= 16 and k <= 1024):
         return None
+    if n > 16384:
+        return None   # (a table of logits: every CTA of hundreds would normalise the rows again; a step of 16 rows of GPT-2 124M 270 us, with a kernel of its own 260)
     if (w.shape[1] if w_is_nk else w.shape[0]) != k:
         raise KernelError(f"linear: normed rows {a.shape} do not fit w {tuple(w.shape)} (w_is_nk={w_is_nk})")
     _need(a.x, "x", torch.float32, 2)
