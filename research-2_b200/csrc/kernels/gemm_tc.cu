@@ -41,7 +41,7 @@ namespace {
 constexpr int BM = 128;          // rows of the a side = UMMA M
 constexpr int BK = 64;           // one 128-byte swizzle span of bfloat16
 constexpr int UMMA_K = 16;
-constexpr int THREADS = 192;     // warp 0: TMA, warp 1: MMA + tensor memory, warps 2-5: epilogue
+constexpr int THREADS = 192;     // warp 0: TMA, warp 1: MMA + tensor memory, warps 2-5: epilogue (2-9 in the wide token-major form)
 constexpr int MAX_STAGES = 8;
 constexpr uint32_t SPIN_LIMIT = 1u << 22;
 
@@ -71,6 +71,7 @@ struct GemmParams {
   int a_total, b_total, k_total;  // extents of the a side, the b side and K
   int bn;                         // tile width on the b side = UMMA N (multiple of 16, <= 256)
   int n_kb, kb_per_split, splits, stages;
+  int epilogue_warps;             // token-major: 4 or 8 (launch picks the kernel by it)
   int n_tiles, col_tiles;         // the pair form: tiles in all, and per row of tiles (tile = row * col_tiles + column)
   const float* bias;
   const float* residual;
@@ -677,8 +678,11 @@ __device__ __forceinline__ void finish_tile_rows(const GemmParams& p, uint32_t l
 // TRANSPOSED: the a side is the features and the b side the tokens.
 // SHARED: the token-major form whose cluster shares a tile's K (a kernel of its own: as a branch of the plain form it cost that one
 // 1 to 2 % of a prompt's step).
-template <bool A_MN, bool B_MN, bool TRANSPOSED, bool FUSED_LN = false, bool ROUTED = false, bool SHARED = false>
-__global__ void __launch_bounds__(THREADS, (TRANSPOSED && !FUSED_LN) ? 1 : 2)  // token-major tiles run two CTAs to an SM, and so does the form with the norm inside (the logits' 393 CTAs)
+// EW: epilogue warps. Token-major tiles with an SM to themselves have eight, two to a quarter of the tile's rows that take half of its columns
+// each: the epilogue of four warps was 2.1 to 4 us of the 6.7 to 12 that a product of 528 rows takes after its wait (528 x 1,024 x 1,024 with a residual
+// 7.7 and now 6.8 us a launch, 2,046 x 1,024 x 1,024 10.9 and 9.0, 2,046 x 1,600 x 1,600 16.2 and 13.3).
+template <bool A_MN, bool B_MN, bool TRANSPOSED, bool FUSED_LN = false, bool ROUTED = false, bool SHARED = false, int EW = 4>
+__global__ void __launch_bounds__(64 + EW * 32, ((TRANSPOSED && !FUSED_LN) || EW == 8) ? 1 : 2)  // token-major tiles run two CTAs to an SM, and so does the form with the norm inside (the logits' 393 CTAs)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -909,10 +913,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       cta_stamp(p, 3);
     }
     const int q = warp & 3;  // tensor-memory lanes [32q, 32q + 32) belong to warps with id % 4 == q
+    const int side = EW == 8 ? (warp - 2) >> 2 : 0;   // which half of the columns (of a shared K's groups every other one)
     if constexpr (!TRANSPOSED) {
       // the tile's bias, once for the four epilogue warps, while the products run
-      for (int j = int(threadIdx.x) - 64; j < p.bn; j += 128) reduce[j] = (p.bias != nullptr && b0 + j < p.b_total) ? p.bias[b0 + j] : 0.f;
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      for (int j = int(threadIdx.x) - 64; j < p.bn; j += EW * 32) reduce[j] = (p.bias != nullptr && b0 + j < p.b_total) ? p.bias[b0 + j] : 0.f;
+      asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");
     }
     if constexpr (TRANSPOSED) {
       // what the epilogue adds does not depend on the products: it is fetched while they run
@@ -927,8 +932,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     if constexpr (!TRANSPOSED) {
       // the residual of the first 32 columns that this warp finishes, while the products run
-      const int c = SHARED ? int(rank) * SHARE_COLS : 0, last = SHARED ? c + SHARE_COLS : p.bn;
-      res_here = p.residual != nullptr && !p.out_is_bf16 && a0 + q * 32 + 32 <= p.a_total && b0 + last <= p.b_total && p.bn >= SHARE_COLS &&
+      const int c = SHARED ? (int(rank) + side * p.splits) * SHARE_COLS : side * (p.bn / 2), last = SHARED ? c + SHARE_COLS : p.bn;
+      res_here = p.residual != nullptr && c < p.bn && !p.out_is_bf16 && a0 + q * 32 + 32 <= p.a_total && b0 + last <= p.b_total && p.bn >= SHARE_COLS &&
                  (p.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 && (p.ldr & 3) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 15) == 0;
       if (res_here) {
         const float* src = p.residual + size_t(a0 + q * 32 + (lane >> 3)) * p.ldr + b0 + c + 4 * (lane & 7);
@@ -946,7 +951,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // This slice's partial sums of the groups that other CTAs finish, laid out over the operand tiles (every product of this
       // CTA has completed) as [group][column][row], so that a warp's stores and the receiver's loads are whole rows of banks; a
       // group travels as one bulk copy whose bytes the receiver's barrier counts.
-      for (int g = 0; g < p.bn / SHARE_COLS; ++g) {
+      for (int g = side; g < p.bn / SHARE_COLS; g += EW / 4) {
         if (g % p.splits == int(rank)) continue;
         uint32_t r[32];
         if (ok && n_kb > 0) {
@@ -960,7 +965,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int j = 0; j < 32; ++j) to[j * BM] = r[j];
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes, read by the bulk copies
-      asm volatile("bar.sync 1, 128;" ::: "memory");               // the four epilogue warps
+      asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");               // the four epilogue warps
       if (warp == 2 && lane < p.bn / SHARE_COLS && lane % p.splits != int(rank)) {
         const uint32_t to = uint32_t(lane % p.splits), owned = uint32_t((p.bn / SHARE_COLS - int(to) + p.splits - 1) / p.splits);
         const uint32_t sender = rank < to ? rank : rank - 1;
@@ -996,7 +1001,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes, read by the bulk copy
-      asm volatile("bar.sync 1, 128;" ::: "memory");               // the four epilogue warps
+      asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");               // the four epilogue warps
       if (threadIdx.x == 64) {
         uint32_t remote, remote_bar;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(reduce)), "r"(0u));
@@ -1010,7 +1015,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
   if constexpr (SHARED) {
     if (warp >= 2) {
-      const int q = warp & 3;
+      const int q = warp & 3, side = EW == 8 ? (warp - 2) >> 2 : 0;
       const uint32_t lane_addr = tmem_base + (uint32_t(q * 32) << 16);
       const bool landed = mbar_wait(partials_ready, 0);   // (also after an error: the others' copies must not outlive this CTA)
       if (!landed) atomicMax(p.error_flag, R2_ERR_TIMEOUT_ACC);
@@ -1018,7 +1023,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const int owned = (p.bn / SHARE_COLS - int(rank) + p.splits - 1) / p.splits;
       const uint32_t* got = reinterpret_cast<const uint32_t*>(reduce + BIAS_SLOTS) + q * 32 + lane;
       if (acc_ok) {
-        for (int i = 0; i < owned; ++i) {
+        for (int i = side; i < owned; i += EW / 4) {
           // own sums out of tensor memory, the slices' added in rank order (the same bits every run), the total back into it
           const uint32_t at = lane_addr + uint32_t((int(rank) + i * p.splits) * SHARE_COLS);
           uint32_t own[32];
@@ -1039,12 +1044,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           tmem_store32(at, v);
         }
       }
-      asm volatile("bar.sync 1, 128;" ::: "memory");   // the received sums have been read: their place serves as the warps' slabs
+      asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");   // the received sums have been read: their place serves as the warps' slabs
       if (acc_ok && a0 + q * 32 < p.a_total) {
-        const uint32_t slab = smem_u32(reduce + BIAS_SLOTS) + uint32_t(q * STAGING_WORDS) * 4u;
-        for (int i = 0; i < owned; ++i) {
+        const uint32_t slab = smem_u32(reduce + BIAS_SLOTS) + uint32_t((warp - 2) * STAGING_WORDS) * 4u;
+        for (int i = side; i < owned; i += EW / 4) {
           const int c = (int(rank) + i * p.splits) * SHARE_COLS;
-          finish_tile_rows<ROUTED>(p, lane_addr, slab, reduce, a0 + q * 32, b0, c, c + SHARE_COLS, lane, true, res_first, i == 0 && res_here);
+          finish_tile_rows<ROUTED>(p, lane_addr, slab, reduce, a0 + q * 32, b0, c, c + SHARE_COLS, lane, true, res_first, i == side && res_here);
         }
       }
     }
@@ -1064,7 +1069,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if constexpr (!TRANSPOSED) {
       // every product has completed: the first tiles' shared memory serves as the warps' slabs
       if (ok && a0 + q * 32 < p.a_total) {
-        finish_tile_rows<ROUTED>(p, lane_addr, smem_u32(a_tiles) + uint32_t(q * STAGING_WORDS) * 4u, reduce, a0 + q * 32, b0, 0, p.bn, lane, n_kb > 0,
+        const int half = EW == 8 ? p.bn / 2 : p.bn, c = EW == 8 ? ((warp - 2) >> 2) * half : 0;
+        finish_tile_rows<ROUTED>(p, lane_addr, smem_u32(a_tiles) + uint32_t((warp - 2) * STAGING_WORDS) * 4u, reduce, a0 + q * 32, b0, c, c + half, lane, n_kb > 0,
                                  res_first, res_here);
       }
     } else if (ok) {
@@ -1428,12 +1434,15 @@ bool make_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer
   return r2::encode_bf16_map(map, base, 2, dims, strides, box);
 }
 
-template <bool A_MN, bool B_MN, bool TRANSPOSED, bool FUSED_LN = false, bool ROUTED = false, bool SHARED = false>
+template <bool A_MN, bool B_MN, bool TRANSPOSED, bool FUSED_LN = false, bool ROUTED = false, bool SHARED = false, int EW = 4>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, dim3 grid, size_t smem, cudaStream_t stream) {
   if constexpr (!TRANSPOSED && !SHARED) {
-    if (p.splits > 1) return launch<A_MN, B_MN, TRANSPOSED, FUSED_LN, ROUTED, true>(ma, mb, p, grid, smem, stream);
+    if (p.splits > 1) return launch<A_MN, B_MN, TRANSPOSED, FUSED_LN, ROUTED, true, EW>(ma, mb, p, grid, smem, stream);
   }
-  auto kernel = gemm_tc_kernel<A_MN, B_MN, TRANSPOSED, FUSED_LN, ROUTED, SHARED>;
+  if constexpr (!TRANSPOSED && EW == 4) {
+    if (p.epilogue_warps == 8) return launch<A_MN, B_MN, TRANSPOSED, FUSED_LN, ROUTED, SHARED, 8>(ma, mb, p, grid, smem, stream);
+  }
+  auto kernel = gemm_tc_kernel<A_MN, B_MN, TRANSPOSED, FUSED_LN, ROUTED, SHARED, EW>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -1444,7 +1453,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, di
   }
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
-  config.blockDim = dim3(THREADS);
+  config.blockDim = dim3(64 + EW * 32);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -1470,7 +1479,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, di
 
 struct Plan {
   bool swapped;
-  int a_total, b_total, bn, n_kb, splits, kb_per_split, stages;
+  int a_total, b_total, bn, n_kb, splits, kb_per_split, stages, epilogue_warps;
   size_t smem;
 };
 
@@ -1583,8 +1592,10 @@ Plan make_plan(int m, int n, int k, int w_is_nk, bool fused_ln = false, bool who
   }
   if (!pl.swapped) pl.splits = shares;   // (the CTAs of a cluster share K and, afterwards, the tile's columns)
   pl.kb_per_split = (pl.n_kb + pl.splits - 1) / pl.splits;
+  pl.epilogue_warps = !pl.swapped && tiles * pl.splits <= n_sms() && pl.bn % 64 == 0 ? 8 : 4;
+  const size_t slabs = size_t(pl.epilogue_warps) * STAGING_WORDS * 4;
   size_t share = !pl.swapped && pl.splits > 1 ? size_t(pl.splits - 1) * ((pl.bn / SHARE_COLS + pl.splits - 1) / pl.splits) * SHARE_BYTES : 0;   // received
-  if (share > 0 && share < 4 * size_t(STAGING_WORDS) * 4) share = 4 * size_t(STAGING_WORDS) * 4;   // (its place serves as the epilogue's slabs)
+  if (share > 0 && share < slabs) share = slabs;   // (its place serves as the epilogue's slabs)
   const size_t a_bytes = BM * BK * 2, b_stride = (size_t(pl.bn) * BK * 2 + 1023) & ~size_t(1023);
   const size_t fixed = 1024 + (2 * MAX_STAGES + 3) * 8 + 32 +
                        (pl.swapped ? size_t(pl.splits - 1) * (pl.bn + 4) * BM * 4 : size_t(BIAS_SLOTS) * 4 + share);  // partial sums, or the bias and them
@@ -1604,9 +1615,9 @@ Plan make_plan(int m, int n, int k, int w_is_nk, bool fused_ln = false, bool who
   if (stages > MAX_STAGES) stages = MAX_STAGES;
   if (stages > pl.kb_per_split) stages = pl.kb_per_split;
   if (stages < 1) stages = 1;
-  // the token-major epilogue lays its four slabs over the tiles: a short K keeps stages it does not fill
+  // the token-major epilogue lays its warps' slabs over the tiles: a short K keeps stages it does not fill
   // (with a shared K: the groups to be sent)
-  while (!pl.swapped && size_t(stages) * (a_bytes + b_stride) < (share > 0 ? size_t(pl.bn / SHARE_COLS) * SHARE_BYTES : 4 * size_t(STAGING_WORDS) * 4)) ++stages;
+  while (!pl.swapped && size_t(stages) * (a_bytes + b_stride) < (share > 0 ? size_t(pl.bn / SHARE_COLS) * SHARE_BYTES : slabs)) ++stages;
   pl.stages = stages;
   pl.smem = fixed + size_t(stages) * (a_bytes + b_stride);
   return pl;
@@ -1837,6 +1848,7 @@ int gemm_tc_run(const void* x, int lda, const void* w, int ldw, int w_is_nk, con
   p.splits = pl.splits;
   p.kb_per_split = pl.kb_per_split;
   p.stages = pl.stages;
+  p.epilogue_warps = pl.epilogue_warps;
   p.bias = bias;
   p.residual = residual;
   p.ldr = ldr;

@@ -89,80 +89,158 @@ __global__ void layer_norm_kernel(const float* __restrict__ x, const int32_t* __
 }
 
 // Both norms of rows (LayerNorm; RMS norm with the gain offset + weight) for rows of up to 2,048 elements whose length is a multiple of 4:
-// a CTA a row, eight values a thread, so that the path from the last store of the kernel before is one round trip for the row and its gain
+// a CTA a row, eight or sixteen values a thread, so that the path from the last store of the kernel before is one round trip for the row and its gain
 // and shift together, ten shuffles and one barrier. A warp's sum and squares about its own mean join as one set's would (Chan, Golub and
 // LeVeque). The hand-over between kernels bounds it; the form before had a warp a row with up to 16 pieces a lane and asked for gain and
 // shift at the end. Inside a
 // decode step, us a launch, before and now: 4.2 and 1.9 for 32 rows of 768, 5.3 and 2.1 for 8 rows of 1,600; a step of 512 prompt rows of 355M takes 0.06 ms less
 // of 1.5.
-template <typename O, bool CENTRED>
+template <typename O, bool CENTRED, int PIECES>   // PIECES: pieces of eight values a thread
 __global__ void __launch_bounds__(256)
 norm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const float* __restrict__ gain, const float* __restrict__ shift,
                  O* __restrict__ out, int width, float eps, float offset) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float2 shares[8];   // of every warp: sum (then mean), squares
+  constexpr int SHARE = 256 * PIECES;   // values of a warp
+  __shared__ float2 shares[8];          // of every warp: mean, squares
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-  const int r = blockIdx.x, d = threadIdx.x * 8;
+  const int r = blockIdx.x, d0 = warp * SHARE + lane * 8;
   const int src = rows != nullptr ? rows[r] : r;
-  const bool lo = d < width, hi = d + 4 < width;
-  const float* xr = x + size_t(src) * width + d;
+  const float* xr = x + size_t(src) * width;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 u = lo ? *reinterpret_cast<const float4*>(xr) : zero, v = hi ? *reinterpret_cast<const float4*>(xr + 4) : zero;
-  const float4 g0 = lo ? *reinterpret_cast<const float4*>(gain + d) : zero, g1 = hi ? *reinterpret_cast<const float4*>(gain + d + 4) : zero;
-  float4 b0 = zero, b1 = zero;
-  if (CENTRED) {
-    if (lo) b0 = *reinterpret_cast<const float4*>(shift + d);
-    if (hi) b1 = *reinterpret_cast<const float4*>(shift + d + 4);
+  float4 v[2 * PIECES], g[2 * PIECES], b[2 * PIECES];
+#pragma unroll
+  for (int i = 0; i < 2 * PIECES; ++i) {
+    const int d = d0 + (i >> 1) * 256 + (i & 1) * 4;
+    v[i] = d < width ? *reinterpret_cast<const float4*>(xr + d) : zero;
+  }
+#pragma unroll
+  for (int i = 0; i < 2 * PIECES; ++i) {
+    const int d = d0 + (i >> 1) * 256 + (i & 1) * 4;
+    g[i] = d < width ? *reinterpret_cast<const float4*>(gain + d) : zero;
+    b[i] = CENTRED && d < width ? *reinterpret_cast<const float4*>(shift + d) : zero;
   }
   float mean = 0.f;
   if (CENTRED) {
-    const int count = max(0, min(256, width - warp * 256));
-    const float sum = warp_sum(((u.x + u.y) + (u.z + u.w)) + ((v.x + v.y) + (v.z + v.w)));
+    const int count = max(0, min(SHARE, width - warp * SHARE));
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2 * PIECES; ++i) sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+    sum = warp_sum(sum);
     mean = count > 0 ? sum / float(count) : 0.f;
   }
-  auto squares = [&](const float4& f) { return ((f.x - mean) * (f.x - mean) + (f.y - mean) * (f.y - mean)) + ((f.z - mean) * (f.z - mean) + (f.w - mean) * (f.w - mean)); };
-  float sq = warp_sum((lo ? squares(u) : 0.f) + (hi ? squares(v) : 0.f));
+  float sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < 2 * PIECES; ++i) {
+    const float e = ((v[i].x - mean) * (v[i].x - mean) + (v[i].y - mean) * (v[i].y - mean)) + ((v[i].z - mean) * (v[i].z - mean) + (v[i].w - mean) * (v[i].w - mean));
+    if (d0 + (i >> 1) * 256 + (i & 1) * 4 < width) sq += e;
+  }
+  sq = warp_sum(sq);
   if (n_warps > 1) {
     if (lane == 0) shares[warp] = make_float2(mean, sq);
     __syncthreads();
     float total = 0.f;
     sq = 0.f;
     if (CENTRED) {
-      for (int i = 0; i < n_warps; ++i) total += shares[i].x * float(max(0, min(256, width - i * 256)));
+      for (int i = 0; i < n_warps; ++i) total += shares[i].x * float(max(0, min(SHARE, width - i * SHARE)));
       mean = total / float(width);
     }
     for (int i = 0; i < n_warps; ++i) {
       const float2 s = shares[i];
       const float c = s.x - mean;
-      sq += CENTRED ? fmaf(float(max(0, min(256, width - i * 256))), c * c, s.y) : s.y;
+      sq += CENTRED ? fmaf(float(max(0, min(SHARE, width - i * SHARE))), c * c, s.y) : s.y;
     }
   }
   const float inv = 1.f / sqrtf(sq / float(width) + eps);
-  auto value = [&](float f, float g, float b) { return CENTRED ? (f - mean) * inv * g + b : f * inv * (offset + g); };
-  u = make_float4(value(u.x, g0.x, b0.x), value(u.y, g0.y, b0.y), value(u.z, g0.z, b0.z), value(u.w, g0.w, b0.w));
-  v = make_float4(value(v.x, g1.x, b1.x), value(v.y, g1.y, b1.y), value(v.z, g1.z, b1.z), value(v.w, g1.w, b1.w));
-  O* o = out + size_t(r) * width + d;
-  if constexpr (sizeof(O) == 2) {
-    const __nv_bfloat162 p0 = __floats2bfloat162_rn(u.x, u.y), p1 = __floats2bfloat162_rn(u.z, u.w), p2 = __floats2bfloat162_rn(v.x, v.y), p3 = __floats2bfloat162_rn(v.z, v.w);
-    const uint2 first = make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
-    const uint2 second = make_uint2(*reinterpret_cast<const uint32_t*>(&p2), *reinterpret_cast<const uint32_t*>(&p3));
-    if (width % 8 == 0) {   // (else rows begin on multiples of 8 bytes)
-      if (lo) *reinterpret_cast<uint4*>(o) = make_uint4(first.x, first.y, second.x, second.y);
+  auto value = [&](float f, float gf, float bf) { return CENTRED ? (f - mean) * inv * gf + bf : f * inv * (offset + gf); };
+  O* o = out + size_t(r) * width;
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const int d = d0 + i * 256;
+    const bool lo = d < width, hi = d + 4 < width;
+    const float4 u = make_float4(value(v[2 * i].x, g[2 * i].x, b[2 * i].x), value(v[2 * i].y, g[2 * i].y, b[2 * i].y),
+                                 value(v[2 * i].z, g[2 * i].z, b[2 * i].z), value(v[2 * i].w, g[2 * i].w, b[2 * i].w));
+    const float4 w = make_float4(value(v[2 * i + 1].x, g[2 * i + 1].x, b[2 * i + 1].x), value(v[2 * i + 1].y, g[2 * i + 1].y, b[2 * i + 1].y),
+                                 value(v[2 * i + 1].z, g[2 * i + 1].z, b[2 * i + 1].z), value(v[2 * i + 1].w, g[2 * i + 1].w, b[2 * i + 1].w));
+    if constexpr (sizeof(O) == 2) {
+      const __nv_bfloat162 p0 = __floats2bfloat162_rn(u.x, u.y), p1 = __floats2bfloat162_rn(u.z, u.w), p2 = __floats2bfloat162_rn(w.x, w.y), p3 = __floats2bfloat162_rn(w.z, w.w);
+      const uint2 first = make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
+      const uint2 second = make_uint2(*reinterpret_cast<const uint32_t*>(&p2), *reinterpret_cast<const uint32_t*>(&p3));
+      if (width % 8 == 0) {   // (else rows begin on multiples of 8 bytes)
+        if (lo) *reinterpret_cast<uint4*>(o + d) = make_uint4(first.x, first.y, second.x, second.y);
+      } else {
+        if (lo) *reinterpret_cast<uint2*>(o + d) = first;
+        if (hi) *reinterpret_cast<uint2*>(o + d + 4) = second;
+      }
     } else {
-      if (lo) *reinterpret_cast<uint2*>(o) = first;
-      if (hi) *reinterpret_cast<uint2*>(o + 4) = second;
+      if (lo) *reinterpret_cast<float4*>(o + d) = u;
+      if (hi) *reinterpret_cast<float4*>(o + d + 4) = w;
     }
-  } else {
-    if (lo) *reinterpret_cast<float4*>(o) = u;
-    if (hi) *reinterpret_cast<float4*>(o + 4) = v;
   }
 }
 
+// The same with a warp a row and four rows a CTA, for thousands of rows: fewer warps wait for the kernel before.
+template <typename O, bool CENTRED>
+__global__ void __launch_bounds__(128)
+norm_many_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const float* __restrict__ gain, const float* __restrict__ shift,
+                      O* __restrict__ out, int n_rows, int width, float eps, float offset) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (r >= n_rows) return;
+  const int src = rows != nullptr ? rows[r] : r;
+  const float4* xr = reinterpret_cast<const float4*>(x + size_t(src) * width);
+  constexpr int CHUNKS = 2048 / 128;
+  float4 v[CHUNKS];
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < CHUNKS; ++i) {
+    v[i] = (lane + 32 * i) * 4 < width ? xr[lane + 32 * i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+  }
+  const float mean = CENTRED ? warp_sum(sum) / float(width) : 0.f;
+  float sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < CHUNKS; ++i) {
+    const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
+    if ((lane + 32 * i) * 4 < width) sq += (a * a + b * b) + (c * c + d * d);
+  }
+  const float inv = 1.f / sqrtf(warp_sum(sq) / float(width) + eps);
+  O* o = out + size_t(r) * width;
+#pragma unroll
+  for (int i = 0; i < CHUNKS; ++i) {
+    const int k = (lane + 32 * i) * 4;
+    if (k < width) {
+      const float4 g = *reinterpret_cast<const float4*>(gain + k);
+      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (CENTRED) b = *reinterpret_cast<const float4*>(shift + k);
+      auto value = [&](float f, float gf, float bf) { return CENTRED ? (f - mean) * inv * gf + bf : f * inv * (offset + gf); };
+      const float y0 = value(v[i].x, g.x, b.x), y1 = value(v[i].y, g.y, b.y), y2 = value(v[i].z, g.z, b.z), y3 = value(v[i].w, g.w, b.w);
+      if constexpr (sizeof(O) == 2) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(y0, y1), hi = __floats2bfloat162_rn(y2, y3);
+        *reinterpret_cast<uint2*>(o + k) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+      } else {
+        *reinterpret_cast<float4*>(o + k) = make_float4(y0, y1, y2, y3);
+      }
+    }
+  }
+}
+
+// What each form adds to a step in front of a product, us (rows of 768, 1,024 and 1,600): 264 rows 2.1, 2.1 and 3.6 with eight values a thread,
+// 2.1, 2.3 and 3.3 with sixteen, 3.1, 3.1 and 3.5 with a warp a row; 528 rows 2.6, 3.5, 3.8 / 2.5, 2.9, 3.7 / 3.3, 3.3, 3.8; 1,000 rows 3.6, 3.9, 5.1 / 3.6,
+// 3.9, 4.1 / 3.6, 3.9, 4.6; 2,046 rows 4.1, 5.5, 8.0 / 3.6, 4.9, 6.4 / 3.4, 4.4, 5.0. (Warps that wait for the kernel before keep the next one's out.)
 template <typename O, bool CENTRED>
 static int launch_norm_rows(const float* x, const int32_t* rows, const float* gain, const float* shift, void* out, int n_rows, int width, float eps, float offset,
                             cudaStream_t stream) {
-  r2_launch(norm_rows_kernel<O, CENTRED>, dim3(n_rows), dim3((width + 255) / 256 * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
+  const int warps = (width + 255) / 256;
+  if (n_rows > 1500) {
+    r2_launch(norm_many_rows_kernel<O, CENTRED>, dim3((n_rows + 3) / 4), dim3(128), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), n_rows, width, eps, offset);
+  } else if (n_rows * warps > 1200) {
+    r2_launch(norm_rows_kernel<O, CENTRED, 2>, dim3(n_rows), dim3((width + 511) / 512 * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
+  } else {
+    r2_launch(norm_rows_kernel<O, CENTRED, 1>, dim3(n_rows), dim3(warps * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
+  }
   return launch_status();
 }
 

@@ -259,10 +259,10 @@ def test_products_of_few_rows_side_by_side(t, groups, per, k):
 @pytest.mark.parametrize("width", [4, 36, 256, 260, 768, 1600, 2048, 2052])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("gathered", [False, True])
-def test_norms_of_rows(width, dtype, gathered):
+def test_norms_of_rows(width, dtype, gathered, n_rows=37):
     o = ops()
     gen = torch.Generator(device=DEV).manual_seed(width)
-    x = torch.randn(37, width, generator=gen, device=DEV) + 20.0   # (a mean far beyond the spread)
+    x = torch.randn(n_rows, width, generator=gen, device=DEV) + 20.0   # (a mean far beyond the spread)
     gain, shift = torch.randn(width, generator=gen, device=DEV), torch.randn(width, generator=gen, device=DEV)
     rows = torch.tensor([36, 0, 5, 5], dtype=torch.int32, device=DEV) if gathered else None
     read = x[rows.long()].double() if gathered else x.double()
@@ -298,3 +298,10 @@ def test_decode_plans():
     assert o.decode_plan(8, 12, 64, 1024) == (1, 16) and o.decode_plan(1, 12, 64, 4096) == (4, 16) and o.decode_plan(1, 12, 64, 1024) == (1, 16)
     assert o.decode_plan(16, 12, 64, 1024) == (1, 8) and o.decode_plan(64, 12, 64, 1024) == (1, 4)
     assert o.decode_plan(1, 2, 128, 600) == (2, 8) and o.decode_plan(8, 12, 256, 1024) == (6, 4)   # (head sizes beyond 128 have narrow CTAs alone)
+
+
+@pytest.mark.parametrize("n_rows", [401, 1500, 1501])   # sixteen values a thread; the most rows of a CTA each, and a warp a row beyond
+@pytest.mark.parametrize("width", [260, 1028, 2048])
+def test_norms_of_many_rows(n_rows, width):
+    for dtype in (torch.float32, torch.bfloat16):
+        test_norms_of_rows(width, dtype, False, n_rows)
