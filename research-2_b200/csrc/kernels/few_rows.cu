@@ -325,6 +325,7 @@ int by_form(const FewRows& p, cudaStream_t stream) {
   if (p.n <= 2368) return launch<MH, 2, 16, 0>(p, stream);
   if constexpr (MH <= 4) {
     if (p.n <= 4736 && p.k <= 1024) return launch<MH, 4, 16, 0>(p, stream);
+    if (p.n > 7104 && p.k <= 1024) return launch<MH, 4, 8, 0>(p, stream);   // (9,216 x 768, 8 rows: 4.0 us, 16 features 4.5, tcgen05 6.4; 6,144: 3.4 and 3.3)
     return launch<MH, 2, 8, 0>(p, stream);
   }
   return launch<MH, 2, 16, 0>(p, stream);
@@ -335,10 +336,11 @@ int by_form(const FewRows& p, cudaStream_t stream) {
 // a [m, k] bfloat16 (row stride lda), or x [m, k] float with gain [k] and, centred, shift [k] (a is then ignored); w [n, k] bfloat16 (row
 // stride ldw); bias [n] float or null; residual [m, n] float or null, added after the activation; out [m, n] bfloat16 or float. With
 // group_n > 0 the rows are [m, n / group_n * k] wide and features s * group_n .. read the columns from s * k on.
-// R2_UNSUPPORTED where the tcgen05 kernel is the faster one or must decide: more than 64 rows; more than 8,192 features (a table of
+// R2_UNSUPPORTED where the tcgen05 kernel is the faster one or must decide: more than 64 rows; more than 12,288 features (a table of
 // logits is a matter of bandwidth: 10.9 us there, 12.4 here); many weights for many rows, where every CTA's reading of all rows outweighs
-// the shorter path (1,600 x 6,400: 16 rows 9.4 us there and 9.7 here, 32 rows of 1,600 x 4,800 8.1 and 10.2; 64 rows of 1,024 x 4,096 9.0
-// and 9.1, of 768 x 3,072 8.4 and 6.0); norms beyond 16 rows or 1,024 numbers; rows that are no multiples of 16 bytes.
+// the shorter path (K x N 6,400 x 1,600: 16 rows 9.4 us there and 9.7 here; 6,144 x 1,024: 16 rows 8.2 and 8.6, 32 rows 9.4 and 7.6; 768 x 9,216, 24
+// rows: 7.3 and 7.6; 1,600 x 4,800, 32 rows: 8.1 and 10.2; 64 rows of 4,608 x 768 8.9 and 8.9, of 6,144 x 768 9.9 and 10.9, of 768 x 3,072 8.4 and
+// 6.0); norms beyond 16 rows or 1,024 numbers; rows that are no multiples of 16 bytes.
 extern "C" int r2_few_rows(const void* a, int lda, const float* x, int ldx, const float* gain, const float* shift, float eps, int centred,
                            const void* w, int ldw, const float* bias, const float* residual, int ldr, void* out, int ldo, int out_dtype,
                            int m, int n, int k, int act, int group_n, cudaStream_t stream) {
@@ -352,7 +354,8 @@ extern "C" int r2_few_rows(const void* a, int lda, const float* x, int ldx, cons
     return R2_UNSUPPORTED;
   }
   const long long weights = (long long)n * k;
-  if (m > 64 || n > 8192 || weights > (m > 32 ? 2400000LL : m > 16 ? 4500000LL : m > 8 && k > 4096 ? 8000000LL : 12000000LL)) return R2_UNSUPPORTED;
+  const long long most = m > 32 ? (k >= 2048 ? 4000000LL : 2400000LL) : m > 16 ? (k >= 2048 ? 6500000LL : 4500000LL) : m > 8 ? (k > 4096 ? 5000000LL : 8000000LL) : 12000000LL;
+  if (m > 64 || n > 12288 || weights > most) return R2_UNSUPPORTED;
   if (group_n > 0 && (n % group_n != 0 || group_n % 32 != 0)) return R2_UNSUPPORTED;   // (a CTA's features lie in one group)
   const FewRows p{static_cast<const bf16*>(a), lda, x, ldx, gain, shift, eps, centred, static_cast<const bf16*>(w), ldw, bias, residual, ldr, out, ldo,
                   out_dtype == R2_BF16, m, n, k, act, group_n};
