@@ -215,14 +215,87 @@ __device__ __forceinline__ RouteRow route_row(float* at, const RouteArgs& a) {
 }
 
 // a logit: what becomes of it
-__device__ __forceinline__ void put_logit(const RouteArgs& a, const RouteRow& r, int t, int n, float z) {
+__device__ __forceinline__ void put_logit(const RouteArgs& a, const RouteRow& r, int t, int n, float z, float correction) {
   if (n < a.n_experts) {
     const float s = a.softmax_scores ? z : 1.f / (1.f + expf(-z));   // (the softmax follows once all logits are there)
     r.score[n] = s;
-    r.choice[n] = s + (a.correction != nullptr ? a.correction[n] : 0.f);
+    r.choice[n] = s + correction;
   } else {
     a.extra[size_t(t) * a.n_extra + (n - a.n_experts)] = z;
   }
+}
+
+// A number whose order among its like is that of the floats, for the warp's maximum in one instruction; 0 (below all) for -inf and NaN.
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t u = __float_as_uint(v + 0.f);   // (-0 is 0)
+  return v > -INFINITY ? (u >> 31 ? ~u : u | 0x80000000u) : 0u;
+}
+
+// choose_experts for up to 32 outputs, one a lane: the same choices and weights. The largest of a warp's numbers is one instruction and a
+// ballot finds the lowest lane that has it, where a reduction of (value, index) pairs is ten exchanges. `correction`: the lane's output's.
+__device__ __forceinline__ float choose_among_32(const RouteArgs& a, const RouteRow& r, int t, int lane, float correction) {
+  const bool there = lane < a.n_experts;
+  float s = there ? r.score[lane] : 0.f, choice = there ? r.choice[lane] : -INFINITY;
+  if (a.softmax_scores) {
+    float top_z = there ? s : -INFINITY;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top_z = fmaxf(top_z, __shfl_xor_sync(0xffffffffu, top_z, o));
+    const float e = there ? expf(s - top_z) : 0.f;
+    s = e * (1.f / warp_sum(e));
+    choice = there ? s + correction : -INFINITY;
+  }
+  if (a.keep < a.n_groups) {
+    const int size = a.n_experts / a.n_groups;
+    __syncwarp();
+    if (there) r.choice[lane] = choice;
+    __syncwarp();
+    float mark = -INFINITY;
+    if (lane < a.n_groups) {
+      float best = -INFINITY, second = -INFINITY;   // the group's largest and second largest
+      for (int n = lane * size; n < (lane + 1) * size; ++n) {
+        const float c = r.choice[n];
+        if (c > best) { second = best; best = c; }
+        else if (c > second) second = c;
+      }
+      mark = (size > 1 && !a.mark_best_only) ? best + second : best;
+    }
+    bool kept = mark == INFINITY;   // (a mark of +inf is a kept group's)
+    for (int c = 0; c < a.keep; ++c) {
+      // (1: a group without a finite mark, taken when no other is left)
+      const uint32_t key = lane < a.n_groups && !kept ? max(order_key(mark), 1u) : 0u, best = __reduce_max_sync(0xffffffffu, key);
+      const int at = __ffs(__ballot_sync(0xffffffffu, key == best && key != 0u)) - 1;
+      if (lane == at) kept = true;
+    }
+    const uint32_t kept_groups = __ballot_sync(0xffffffffu, kept);
+    if (there && !((kept_groups >> (lane / size)) & 1u)) choice = -INFINITY;
+  }
+  float sum = 0.f, given = 0.f;
+  for (int c = 0; c < a.top; ++c) {
+    const uint32_t key = order_key(choice), best = __reduce_max_sync(0xffffffffu, key);
+    // scores that are not numbers: no index may leave the row
+    const uint32_t holders = __ballot_sync(0xffffffffu, key == best);
+    const int at = best == 0u ? c : __ffs(holders) - 1;
+    sum += __shfl_sync(0xffffffffu, s, at);
+    if (lane == at) {
+      choice = -INFINITY;
+      r.pick[c] = at;
+      r.pick_weight[c] = s;
+    }
+  }
+  __syncwarp();
+  const float inv = (a.normalise ? 1.f / (sum + 1e-20f) : 1.f) * a.weight_scale;
+  for (int c = 0; c < a.top; ++c) {
+    const int at = r.pick[c];
+    const float p = r.pick_weight[c] * inv;
+    if (lane == at) given = p;
+    if (lane == 0) {
+      a.chosen[size_t(t) * a.top + c] = at;
+      a.chosen_weight[size_t(t) * a.top + c] = p;
+    }
+  }
+  if (there) r.given[lane] = given;
+  __syncwarp();
+  return warp_sum(there && lane >= a.n_experts - a.n_identity ? given : 0.f);
 }
 
 // One warp: scores, groups, picks and weights of row t, from its logits. -> the identity outputs' weights' sum
@@ -332,6 +405,8 @@ route_scored_kernel(const RouteArgs a) {
   }
   for (int n = threadIdx.x; n < a.n_experts; n += blockDim.x) r.given[n] = 0.f;
   pdl_wait();
+  auto correction_of = [&](int n) { return a.correction != nullptr && n < a.n_experts ? a.correction[n] : 0.f; };
+  const float lane_correction = correction_of(lane), warp_correction = correction_of(warp);
   const T* hr = static_cast<const T*>(a.h) + size_t(t) * a.h_stride;
   for (int k = threadIdx.x; k < width; k += blockDim.x) r.row[k] = to_float(hr[k]);
   __syncthreads();
@@ -354,11 +429,11 @@ route_scored_kernel(const RouteArgs a) {
       for (int k = lane; k < width; k += 32) acc = fmaf(r.row[k], wr[k], acc);
     }
     acc = warp_sum(acc);
-    if (lane == 0) put_logit(a, r, t, n, acc);
+    if (lane == 0) put_logit(a, r, t, n, acc, n == warp ? warp_correction : correction_of(n));
   }
   __syncthreads();
   if (warp == 0) {
-    const float share = choose_experts(a, r, t, lane);
+    const float share = a.n_experts <= 32 ? choose_among_32(a, r, t, lane, lane_correction) : choose_experts(a, r, t, lane);
     if (lane == 0) identity_weight = share;
   }
   __syncthreads();
@@ -382,6 +457,7 @@ route_scored_rows_kernel(const RouteArgs a, int n_rows) {
   for (int i = threadIdx.x; i < outputs * width / 4; i += blockDim.x) reinterpret_cast<float4*>(ws)[i] = reinterpret_cast<const float4*>(a.w)[i];
   __syncthreads();
   pdl_wait();
+  const float lane_correction = a.correction != nullptr && lane < a.n_experts ? a.correction[lane] : 0.f;
   for (int t = blockIdx.x * ROUTE_ROWS + warp; t < n_rows; t += gridDim.x * ROUTE_ROWS) {
     const T* hr = static_cast<const T*>(a.h) + size_t(t) * a.h_stride;
     for (int k = lane; k < width; k += 32) r.row[k] = to_float(hr[k]);
@@ -401,11 +477,12 @@ route_scored_rows_kernel(const RouteArgs a, int n_rows) {
 #pragma unroll
       for (int o = 0; o < 4; ++o) {
         const float acc = warp_sum((sum[o][0] + sum[o][1]) + (sum[o][2] + sum[o][3]));
-        if (lane == 0 && n0 + o < outputs) put_logit(a, r, t, n0 + o, acc);
+        const float correction = __shfl_sync(0xffffffffu, lane_correction, (n0 + o) & 31);
+        if (lane == 0 && n0 + o < outputs) put_logit(a, r, t, n0 + o, acc, n0 + o < 32 ? correction : n0 + o < a.n_experts && a.correction != nullptr ? a.correction[n0 + o] : 0.f);
       }
     }
     __syncwarp();
-    const float share = choose_experts(a, r, t, lane);
+    const float share = a.n_experts <= 32 ? choose_among_32(a, r, t, lane, lane_correction) : choose_experts(a, r, t, lane);
     for (int n = lane; n < a.n_experts; n += 32) a.dense[size_t(t) * a.n_experts + n] = r.given[n];
     if (a.n_identity > 0) {
       for (int k = 4 * lane; k < width; k += 128) {
