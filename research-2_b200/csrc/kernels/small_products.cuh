@@ -49,7 +49,7 @@ __device__ __forceinline__ void rows_times_matrix(const float* rows, int kpad, c
     for (int o = 0; o < OUTS; ++o)
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) acc[o][r] = 0.f;
-#pragma unroll 2
+#pragma unroll (OUTS * ROWS == 1 ? 8 : 2)
     for (int k = lane * 4; k < kpad; k += 128) {
       float4 v[OUTS];
 #pragma unroll

@@ -557,6 +557,94 @@ delta_prepare_kernel(const DeltaPrepareArgs a) {
   }
 }
 
+// The same for few rows of up to four taps: a CTA a row and group, so that a row's channels, gates and norms are one column, one output or
+// one vector a thread or warp, and their loads one round trip (a CTA a row made three passes over its channels with eight dependent loads
+// each: 10 us for 6 rows of 12 heads of 64). Every sum is made in the other kernel's order. Rows of h and w_gates are pieces of four.
+constexpr int PREP_FEW_THREADS = 256, PREP_FEW_TAPS = 4;
+template <typename T>
+__global__ void __launch_bounds__(PREP_FEW_THREADS)
+delta_prepare_few_kernel(const DeltaPrepareArgs a) {
+  pdl_launch_dependents();
+  extern __shared__ __align__(16) float prep_smem[];
+  __shared__ float product;
+  const int grp = blockIdx.x, t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per = a.heads / a.groups, qk_width = 2 * a.groups * a.dim, channels = qk_width + a.heads * a.vdim, own = 2 * a.dim + per * a.vdim;
+  float* row_h = prep_smem;            // [width]
+  float* conv = row_h + a.width;       // [2 dim]: the group's query and key
+  float* gates = conv + 2 * a.dim;     // [2 per]: the group's heads' gates, then their steps
+  const int e = a.row_entry[t];
+  const int entry_row = e >= 0 ? t - a.q_start[e] : -1;
+  const float* kept = (e >= 0 && a.fresh[e] == 0) ? a.state + size_t(a.state_slot[e]) * a.slot_stride + a.conv_off : nullptr;
+  pdl_wait();
+  const T* in = static_cast<const T*>(a.in);
+  const T* h = static_cast<const T*>(a.h) + size_t(t) * a.h_stride;
+  for (int i = 4 * threadIdx.x; i < a.width; i += 4 * PREP_FEW_THREADS)
+    *reinterpret_cast<float4*>(row_h + i) = entry_row >= 0 ? load4(h + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i = threadIdx.x; i < own; i += PREP_FEW_THREADS) {
+    const int c = i < a.dim ? grp * a.dim + i : i < 2 * a.dim ? (a.groups + grp) * a.dim + (i - a.dim) : qk_width + grp * per * a.vdim + (i - 2 * a.dim);
+    float tap[PREP_FEW_TAPS], val[PREP_FEW_TAPS];
+#pragma unroll
+    for (int d = 0; d < PREP_FEW_TAPS; ++d) {
+      tap[d] = val[d] = 0.f;
+      if (d < a.n_taps) {
+        const int back = a.n_taps - 1 - d, src = entry_row - back;
+        tap[d] = a.taps[size_t(c) * a.n_taps + d];
+        if (entry_row >= 0) {
+          if (src >= 0) val[d] = to_float(in[size_t(t - back) * a.in_stride + c]);
+          else if (kept != nullptr) val[d] = kept[size_t(a.n_taps - 1 + src) * channels + c];
+        }
+      }
+    }
+    float acc = 0.f;
+#pragma unroll
+    for (int d = 0; d < PREP_FEW_TAPS; ++d)
+      if (d < a.n_taps) acc = fmaf(tap[d], val[d], acc);
+    const float y = silu(acc);
+    if (i < 2 * a.dim) conv[i] = y;
+    else a.v_out[size_t(t) * (channels - qk_width) + (c - qk_width)] = y;
+  }
+  __syncthreads();
+  for (int n = warp; n < 2 * per + 1; n += PREP_FEW_THREADS / 32) {
+    if (n == 2 * per) {   // the group's query and key
+      const float* q = conv;
+      const float* k = conv + a.dim;
+      const int dim4 = (a.dim + 3) & ~3;
+      float qq = 0.f, kk = 0.f, kq = 0.f;
+      for (int i = lane; i < a.dim; i += 32) {
+        qq = fmaf(q[i], q[i], qq);
+        kk = fmaf(k[i], k[i], kk);
+        kq = fmaf(k[i], q[i], kq);
+      }
+      qq = warp_sum(qq);
+      kk = warp_sum(kk);
+      kq = warp_sum(kq);
+      const float qn = a.q_scale / sqrtf(qq + a.unit_eps), kn = 1.f / sqrtf(kk + a.unit_eps);
+      float* o = a.qk + (size_t(t) * a.groups + grp) * 2 * dim4;
+      for (int i = lane; i < dim4; i += 32) {
+        o[i] = i < a.dim ? q[i] * qn : 0.f;
+        o[dim4 + i] = i < a.dim ? k[i] * kn : 0.f;
+      }
+      if (lane == 0) product = kq * kn * qn;
+    } else {              // a gate or a step
+      const T* w = static_cast<const T*>(a.w_gates) + size_t(n < per ? grp * per + n : a.heads + grp * per + (n - per)) * a.width;
+      float acc = 0.f;
+#pragma unroll 8
+      for (int k = lane * 4; k < a.width; k += 128) {
+        const float4 m = *reinterpret_cast<const float4*>(row_h + k), v = load4(w + k);
+        acc = fmaf(m.w, v.w, fmaf(m.z, v.z, fmaf(m.y, v.y, fmaf(m.x, v.x, acc))));
+      }
+      acc = warp_sum(acc);
+      if (lane == 0) gates[n] = acc;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < per; i += PREP_FEW_THREADS) {
+    const int hd = grp * per + i;
+    const float step = softplus(gates[per + i] + a.step_bias[hd]);
+    a.numbers[size_t(t) * a.heads + hd] = make_float4(expf(-expf(a.log_rate[hd]) * step), 1.f / (1.f + expf(-gates[i])), product, 0.f);
+  }
+}
+
 // ---- what time mixing walks over -----------------------------------------------------------------
 // Mix s of row t: h + (h' - h) * mu[s], h' the row before it in its sequence: the row above inside the entry, the slot's row for
 // an entry's first (zeros for a sequence's first). Mixes 0 .. n_mixes - 1 go to out [T][n_mixes][width] in the rows' dtype. One
@@ -598,7 +686,30 @@ time_mix_prepare_kernel(const TimeMixPrepareArgs a) {
   T* out = static_cast<T*>(a.out);
   // (with few rows several CTAs share them: each makes the whole inner row, and its share of the mixes and of the columns)
   const int share = blockIdx.y, n_shares = gridDim.y;
-  for (int c = threadIdx.x; c < wpad; c += PREP_THREADS) {
+  if constexpr (ROWS == 1) {
+    // one row: two columns a thread at a time, everything they need asked for before anything is stored
+    for (int c0 = threadIdx.x; c0 < wpad; c0 += 2 * PREP_THREADS) {
+      float now[2], before[2], m_last[2], m_first[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int c = c0 + u * PREP_THREADS;
+        const bool inside = c < width;
+        now[u] = inside && kind[0] != 0 ? to_float(h[size_t(t0) * a.h_stride + c]) : 0.f;
+        before[u] = inside && kind[0] == 1 ? to_float(h[size_t(t0 - 1) * a.h_stride + c]) : inside && kind[0] == 3 ? kept_row[0][c] : 0.f;
+        m_last[u] = inside ? a.mu[size_t(a.n_mixes) * width + c] : 0.f;
+        m_first[u] = inside && share < a.n_mixes ? a.mu[size_t(share) * width + c] : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int c = c0 + u * PREP_THREADS;
+        if (c >= wpad) break;
+        const float step = before[u] - now[u];
+        for (int s = share; s < a.n_mixes && c < width; s += n_shares)
+          out[(size_t(t0) * a.n_mixes + s) * width + c] = from_float<T>(fmaf(step, s == share ? m_first[u] : a.mu[size_t(s) * width + c], now[u]));
+        mix[c] = fmaf(step, m_last[u], now[u]);
+      }
+    }
+  } else for (int c = threadIdx.x; c < wpad; c += PREP_THREADS) {
     const bool inside = c < width;
     float now[ROWS + 1], step[ROWS];   // now[r + 1]: row t0 + r; now[0]: the row above the first
     now[0] = (inside && kind[0] == 1) ? to_float(h[size_t(t0 - 1) * a.h_stride + c]) : 0.f;
@@ -617,7 +728,7 @@ time_mix_prepare_kernel(const TimeMixPrepareArgs a) {
     for (int r = 0; r < ROWS; ++r) mix[r * wpad + c] = fmaf(step[r], m, now[r + 1]);
   }
   __syncthreads();
-  rows_times_matrix<ROWS, 4>(mix, wpad, static_cast<const T*>(a.w1), width, a.rank, [&](int r, int n, float sum) { low[r * rpad + n] = tanhf(sum); });
+  rows_times_matrix<ROWS, (ROWS > 1 ? 4 : 1)>(mix, wpad, static_cast<const T*>(a.w1), width, a.rank, [&](int r, int n, float sum) { low[r * rpad + n] = tanhf(sum); });
   __syncthreads();
   for (int n = share * PREP_THREADS + threadIdx.x; n < a.n_out; n += n_shares * PREP_THREADS) {
     float acc[ROWS];
@@ -680,6 +791,14 @@ extern "C" int r2_delta_prepare(const void* in, int in_stride, const void* h, in
   a.row_entry = row_entry; a.q_start = q_start; a.state_slot = state_slot; a.fresh = fresh;
   const size_t per_row = sizeof(float) * (size_t((width + 3) & ~3) + size_t(2) * n_groups * dim + 2 * n_heads + n_groups);
   const int rows = rows_per_cta(n_rows, n_sms, per_row), shares = 1;
+  const size_t piece = dtype == R2_F32 ? 16 : 8, few_smem = sizeof(float) * (size_t(width) + 2 * dim + 2 * (n_heads / n_groups));
+  const bool pieces = width % 4 == 0 && h_stride % 4 == 0 && reinterpret_cast<uintptr_t>(h) % piece == 0 && reinterpret_cast<uintptr_t>(w_gates) % piece == 0;
+  // a CTA a row and group while a wave of four to an SM holds them all
+  if (rows == 1 && n_taps <= PREP_FEW_TAPS && pieces && few_smem <= 40 * 1024 && (long long)n_rows * n_groups <= 4LL * n_sms && (dtype == R2_F32 || dtype == R2_BF16)) {
+    if (dtype == R2_F32) r2_launch(delta_prepare_few_kernel<float>, dim3(n_groups, n_rows), dim3(PREP_FEW_THREADS), few_smem, stream, a);
+    else r2_launch(delta_prepare_few_kernel<bf16>, dim3(n_groups, n_rows), dim3(PREP_FEW_THREADS), few_smem, stream, a);
+    return launch_status();
+  }
   if (dtype == R2_F32) R2_PREPARE_ROWS(delta_prepare_kernel, float);
   else if (dtype == R2_BF16) R2_PREPARE_ROWS(delta_prepare_kernel, bf16);
   else return R2_BAD_DTYPE;

@@ -305,3 +305,52 @@ def test_decode_plans():
 def test_norms_of_many_rows(n_rows, width):
     for dtype in (torch.float32, torch.bfloat16):
         test_norms_of_rows(width, dtype, False, n_rows)
+
+
+# a CTA a row and group beside four rows a CTA: taps up to four (five take the other kernel), vectors that are no multiples of four or of a warp
+@pytest.mark.parametrize("heads,groups,dim,vdim,taps_n,width", [(4, 2, 24, 16, 4, 52), (6, 6, 7, 5, 3, 768), (12, 6, 64, 64, 4, 768), (3, 1, 40, 90, 1, 1028), (2, 2, 8, 8, 5, 64)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_what_the_delta_rule_walks_over_for_few_rows(heads, groups, dim, vdim, taps_n, width, dtype):
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(width + dim)
+    channels, n = 2 * groups * dim + heads * vdim, 400
+    raw, h = torch.randn(n, channels, generator=gen, device=DEV).to(dtype), torch.randn(n, width, generator=gen, device=DEV).to(dtype)
+    weights = (torch.randn(channels, taps_n, generator=gen, device=DEV), (0.1 * torch.randn(2 * heads, width, generator=gen, device=DEV)).to(dtype),
+               torch.randn(heads, generator=gen, device=DEV), torch.randn(heads, generator=gen, device=DEV))
+    state = torch.randn(2, 8 + (taps_n - 1) * channels + 8, generator=gen, device=DEV)
+
+    def prepared(rows, entry_of, starts, fresh):
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+        return o.delta_prepare(raw[:rows], h[:rows], *weights, 0.2, 1e-6, heads, groups, dim, vdim, state, 8, i32(entry_of), i32(starts), i32([1, 0]), i32(fresh))
+
+    for fresh in (0, 1):
+        many, few = prepared(n, [0] * n, [0, n, n], [fresh, 0]), prepared(7, [0] * 6 + [-1], [0, 6, 6], [fresh, 0])   # (the last a pad row)
+        for a, b in zip(many, few):
+            assert torch.equal(a[:6], b[:6])
+            assert torch.isfinite(b).all()
+
+
+@pytest.mark.parametrize("experts,groups,keep,top", [(8, 4, 2, 2), (10, 2, 1, 3), (31, 1, 1, 31), (32, 8, 3, 5), (33, 3, 2, 4), (1, 1, 1, 1)])
+@pytest.mark.parametrize("scoring", ["sigmoid", "softmax"])
+@pytest.mark.parametrize("rows", [5, 700])
+def test_routers_around_a_warp_of_outputs(experts, groups, keep, top, scoring, rows):
+    """Scores of a few values only, so that ties are common: the lower index wins, among groups and among experts."""
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(experts)
+    h = torch.zeros(rows, 64, device=DEV)
+    h[:, :experts] = torch.randint(-2, 3, (rows, experts), generator=gen, device=DEV).float()
+    w = torch.eye(64, device=DEV)[:experts].contiguous()
+    dense, chosen, weight, _ = o.route_scored(h, w, None, top, groups, keep, scoring=scoring, group_mark="best", normalise=False)
+    z = h[:, :experts].double()
+    score = torch.sigmoid(z) if scoring == "sigmoid" else torch.softmax(z, dim=1)
+    mark = z.view(rows, groups, -1).amax(-1)
+    kept = torch.sort(mark, dim=1, descending=True, stable=True).indices[:, :keep]
+    allowed = torch.zeros(rows, groups, dtype=torch.bool, device=DEV).scatter_(1, kept, True).repeat_interleave(experts // groups, dim=1)
+    want = torch.sort(z.masked_fill(~allowed, -float("inf")), dim=1, descending=True, stable=True).indices[:, :top]
+    assert torch.equal(chosen.long(), want)
+    torch.testing.assert_close(weight.double(), score.gather(1, want), atol=1e-6, rtol=1e-6)
+    assert torch.equal(dense.gather(1, want), weight) and torch.equal((dense != 0).sum(1), torch.full((rows,), top, device=DEV))
+    # rows that are not numbers: indices stay inside
+    h[0], h[1, :1], h[2] = float("nan"), float("nan"), float("inf")
+    _, chosen, _, _ = o.route_scored(h, w, None, top, groups, keep, scoring=scoring, group_mark="two_best")
+    assert int(chosen.min()) >= 0 and int(chosen.max()) < experts
