@@ -152,6 +152,7 @@ class DeviceLoopGraph:
         self.dev = torch.zeros(self.host.buf.shape[0], dtype=torch.int32, device=step_fn.device)
         self.dev.copy_(self.host._pinned_tensor)
         ctx = StepContext(self.host, self.dev, counts=(batch, batch, batch))
+        ctx.cache_settled = True   # (`run` copies the batch into `dev` in front of every replay)
         side = torch.cuda.Stream(device=step_fn.device)
         side.wait_stream(torch.cuda.current_stream(step_fn.device))
         with torch.cuda.stream(side):

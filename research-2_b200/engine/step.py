@@ -39,9 +39,10 @@ class StepContext:
         t, r, w = counts or (host.n_tokens, host.n_entries, host.n_logit_rows)
         self.n_tokens, self.n_entries, self.n_logit_rows = t, r, w
         self.captured = counts is not None
-        # a step's first operations, the copy of its batch (a graph: the kernel that fetches it) and the embedding behind it, run in plain order: what
-        # the steps before wrote into caches and states is complete when a later kernel starts, however early it starts beside the one in front
-        self.cache_settled = True
+        # Whether what earlier passes wrote into the caches is complete before this pass's first kernel starts, however early later ones start beside
+        # the one in front: whoever puts a plain operation (the copy of the batch, the kernel that fetches it) directly in front of the pass sets it. A
+        # context that was uploaded some time ago may follow another pass whose kernels still run.
+        self.cache_settled = False
         # (stream tensor, its rows in the compute dtype): a block whose last kernel wrote both leaves the pair here for the next one
         self.stream_rounded = None
         # shape facts that choose kernels: inside a graph every row is an entry of its own and
@@ -114,6 +115,7 @@ class StepGraph:
         self.dev = torch.zeros(self.hosts[0].buf.shape[0], dtype=torch.int32, device=step_fn.device)
         self.dev.copy_(self.hosts[0]._pinned_tensor)
         self.ctx = StepContext(self.hosts[0], self.dev, counts=(t_cap, r_cap, r_cap))
+        self.ctx.cache_settled = True             # (the graph's first kernel fetches the batch, in plain order)
         self.tokens_host = torch.zeros(r_cap, dtype=torch.int32).pin_memory()
         self.tokens_host_np = self.tokens_host.numpy()
         # the device's error word travels to the host with the tokens: a kernel's time-out is seen at no extra cost
@@ -287,6 +289,12 @@ class StepFunction:
         self.h2d_bytes += batch.buf.nbytes
         return StepContext(batch, dev)
 
+    def _uploaded_in_front(self, batch: StepBatch) -> StepContext:
+        """`upload` for a forward pass that follows at once, with nothing launched between."""
+        ctx = self.upload(batch)
+        ctx.cache_settled = True
+        return ctx
+
     def validate(self, batch: StepBatch) -> None:
         """Host-side bounds checks of a batch that the caller filled. A batch that the scheduler
         filled natively is inside the pool by construction and is not checked again."""
@@ -324,7 +332,7 @@ class StepFunction:
                 graph.replay(batch)
                 self.h2d_bytes += batch.buf.nbytes
                 return graph.logits[: batch.n_logit_rows]
-            return self.forward(self.upload(batch))
+            return self.forward(self._uploaded_in_front(batch))
 
     def launch_graph(self, batch: StepBatch) -> StepGraph | None:
         """Launches the step as its CUDA graph, if the batch is one that the scheduler filled and
@@ -356,7 +364,7 @@ class StepFunction:
                 graph.replay(batch)
                 self.h2d_bytes += batch.buf.nbytes
                 return graph.tokens[: batch.n_logit_rows]
-            ctx = self.upload(batch)
+            ctx = self._uploaded_in_front(batch)
             return self.sample(self.forward(ctx), ctx)
 
 

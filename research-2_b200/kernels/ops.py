@@ -414,7 +414,7 @@ def host_address(pinned: torch.Tensor) -> int | None:
 
 def fetch_batch(even: int, odd: int, dev: torch.Tensor, turn: torch.Tensor) -> None:
     """dev <- one of two pinned host arrays (device addresses), by `turn`'s lowest bit (int32 [1] on the device). The launch that follows
-    must be in plain order (`embed(plain_order=True)`)."""
+    must be in plain order (`embed(plain_order=True)`, as the embedding part launches it)."""
     _need(dev, "dev", torch.int32, 1)
     _need(turn, "turn", torch.int32, 1)
     _check(_lib("step_io").r2_fetch_batch(C.c_void_p(even), C.c_void_p(odd), _p(dev), dev.shape[0], _p(turn), _stream()), "fetch_batch")

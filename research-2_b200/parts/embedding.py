@@ -21,8 +21,9 @@ class TokenEmbedding:
         self.scale = float(scale)  # table rows are multiplied by it on their way into the stream
 
     def forward(self, ctx, additive_table=None):
-        # (a captured step's batch comes from the kernel in front)
-        return ops.embed(ctx.input_ids, self.table, ctx.positions, additive_table, scale=self.scale, plain_order=getattr(ctx, "captured", False))
+        # a pass's first kernel: in plain order, so that whatever lies in front (a kernel that fetches the batch, the last kernels of another
+        # pass) has ended before later kernels read index arrays ahead of their waits; behind a copy it is so anyway
+        return ops.embed(ctx.input_ids, self.table, ctx.positions, additive_table, scale=self.scale, plain_order=True)
 
 
 class Head:

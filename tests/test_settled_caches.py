@@ -1,0 +1,93 @@
+"""Which passes may read the cache ahead of a kernel's wait: those behind a copy of their own batch, and no others."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from research_2_b200.engine import step
+from research_2_b200.engine.batch import batch_for
+
+
+def one_row_batch():
+    batch = batch_for((4,), 1, 1, 1)
+    batch.set_entries([0], [0], [[3]])
+    batch.set_logit_rows([0])
+    batch.trusted = True
+    return batch
+
+
+def context(batch):
+    return step.StepContext(batch, torch.from_numpy(batch.buf.copy()))
+
+
+def test_a_context_that_was_uploaded_earlier_is_not_settled():
+    assert context(one_row_batch()).cache_settled is False
+
+
+@pytest.mark.parametrize("entry", ["__call__", "step_and_sample"])
+def test_the_step_function_settles_the_pass_behind_its_own_copy(entry, monkeypatch):
+    monkeypatch.setattr(step.torch.cuda, "device", lambda d: torch.no_grad())
+    fn, seen = step.StepFunction.__new__(step.StepFunction), []
+    fn.capture, fn._graphs, fn.device, fn._device_index = False, {}, "cpu", 0
+    fn.upload, fn.sample = context, lambda logits, ctx: logits
+    fn.forward = lambda ctx: seen.append(ctx.cache_settled)
+    batch = one_row_batch()
+    getattr(fn, entry)(batch)
+    assert seen == [True]
+    assert fn.upload(batch).cache_settled is False   # (what a caller uploads)
+
+
+def test_the_embedding_is_launched_in_plain_order(monkeypatch):
+    from research_2_b200.parts import Runtime, embedding
+
+    orders = []
+    monkeypatch.setattr(embedding.ops, "embed", lambda *a, plain_order=False, **k: orders.append(plain_order))
+    embedding.TokenEmbedding(torch.zeros(10, 4), Runtime(torch.device("cpu"), torch.float32)).forward(context(one_row_batch()))
+    assert orders == [True]
+
+
+@pytest.mark.gpu
+def test_two_contexts_uploaded_before_either_pass():
+    """The second pass reads the key and value that the first one writes; neither copy lies between them."""
+    from research_2_b200.cache.manager import CacheManager
+    from research_2_b200.parts import PartSpec, Runtime, build_part
+
+    dev, heads, hd, width, steps = torch.device("cuda:0"), 4, 64, 256, 12
+    gen = torch.Generator().manual_seed(0)
+    tensors = {"w": torch.randn(width, 3 * heads * hd, generator=gen) * width ** -0.5, "b": torch.randn(3 * heads * hd, generator=gen) * 0.1,
+               "o": torch.randn(heads * hd, width, generator=gen) * width ** -0.5, "ob": torch.zeros(width)}
+    part = build_part("mixer", PartSpec("attention", {"n_heads": heads, "n_kv_heads": heads, "head_dim": hd, "scale": hd ** -0.5, "window": 0},
+                                        {"w_qkv": "w", "b_qkv": "b", "w_out": "o", "b_out": "ob"}), tensors, Runtime(dev, torch.bfloat16))
+
+    class Shell:
+        rt, cache_members, state_members, max_seq_len, vocab_size, blocks = Runtime(dev, torch.bfloat16), [part.cache_spec], [], 128, 10, []
+
+    def logits(ahead: bool):
+        fn = step.StepFunction(Shell, 16, 16, 1)
+        cache = CacheManager(fn.cache_groups(), 1, 128)
+        fn.arena.fill_(64.0)   # (a row that is read before it is written shows)
+        cache.open(0)
+        cache.reserve(0, 0, steps)
+        contexts = []
+        for i in range(steps):
+            batch = fn.new_batch(1, 1, 1)
+            batch.set_entries([0], [i], [[0]])
+            cache.fill(batch)
+            batch.set_logit_rows([0])
+            contexts.append(fn.upload(batch))
+        h = torch.randn(steps, width, generator=torch.Generator().manual_seed(1)).to(dev)
+        rows, residual = h.bfloat16(), h.clone()
+        torch.cuda.synchronize()   # from here on nothing is launched but the passes' own kernels
+        out = []
+        for i, ctx in enumerate(contexts):
+            out.append(part.forward(rows[i: i + 1], residual[i: i + 1], ctx, fn.arena.members[0]))
+            if not ahead:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return torch.cat(out)
+
+    want = logits(False)
+    assert torch.isfinite(want).all() and np.isfinite(float(want.abs().max()))
+    assert torch.equal(logits(True), want)
