@@ -230,17 +230,23 @@ norm_many_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ r
 // What each form adds to a step in front of a product, us (rows of 768, 1,024 and 1,600): 264 rows 2.1, 2.1 and 3.6 with eight values a thread,
 // 2.1, 2.3 and 3.3 with sixteen, 3.1, 3.1 and 3.5 with a warp a row; 528 rows 2.6, 3.5, 3.8 / 2.5, 2.9, 3.7 / 3.3, 3.3, 3.8; 1,000 rows 3.6, 3.9, 5.1 / 3.6,
 // 3.9, 4.1 / 3.6, 3.9, 4.6; 2,046 rows 4.1, 5.5, 8.0 / 3.6, 4.9, 6.4 / 3.4, 4.4, 5.0. (Warps that wait for the kernel before keep the next one's out.)
+// Each form adds a row in an order of its own, so the choice by the number of rows is bfloat16's alone: float32 rows have the same bits whatever shares
+// their step, and take the first form at any number (its 3 us more at 2,046 rows of 1,600 stand beside products of milliseconds).
 template <typename O, bool CENTRED>
 static int launch_norm_rows(const float* x, const int32_t* rows, const float* gain, const float* shift, void* out, int n_rows, int width, float eps, float offset,
                             cudaStream_t stream) {
   const int warps = (width + 255) / 256;
-  if (n_rows > 1500) {
-    r2_launch(norm_many_rows_kernel<O, CENTRED>, dim3((n_rows + 3) / 4), dim3(128), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), n_rows, width, eps, offset);
-  } else if (n_rows * warps > 1200) {
-    r2_launch(norm_rows_kernel<O, CENTRED, 2>, dim3(n_rows), dim3((width + 511) / 512 * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
-  } else {
-    r2_launch(norm_rows_kernel<O, CENTRED, 1>, dim3(n_rows), dim3(warps * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
+  if constexpr (sizeof(O) == 2) {
+    if (n_rows > 1500) {
+      r2_launch(norm_many_rows_kernel<O, CENTRED>, dim3((n_rows + 3) / 4), dim3(128), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), n_rows, width, eps, offset);
+      return launch_status();
+    }
+    if (n_rows * warps > 1200) {
+      r2_launch(norm_rows_kernel<O, CENTRED, 2>, dim3(n_rows), dim3((width + 511) / 512 * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
+      return launch_status();
+    }
   }
+  r2_launch(norm_rows_kernel<O, CENTRED, 1>, dim3(n_rows), dim3(warps * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
   return launch_status();
 }
 

@@ -354,3 +354,20 @@ def test_routers_around_a_warp_of_outputs(experts, groups, keep, top, scoring, r
     h[0], h[1, :1], h[2] = float("nan"), float("nan"), float("inf")
     _, chosen, _, _ = o.route_scored(h, w, None, top, groups, keep, scoring=scoring, group_mark="two_best")
     assert int(chosen.min()) >= 0 and int(chosen.max()) < experts
+
+
+@pytest.mark.parametrize("width", [256, 768, 1600, 2048])
+@pytest.mark.parametrize("gathered", [False, True])
+def test_float32_norms_have_the_same_bits_beside_any_number_of_rows(width, gathered):
+    o = ops()
+    gen = torch.Generator(device=DEV).manual_seed(width)
+    x = torch.randn(1700, width, generator=gen, device=DEV) + 3.0
+    gain, shift = torch.randn(width, generator=gen, device=DEV), torch.randn(width, generator=gen, device=DEV)
+    order = torch.randperm(1700, generator=gen, device=DEV).to(torch.int32) if gathered else torch.arange(1700, dtype=torch.int32, device=DEV)
+    read = x if gathered else x[order.long()]
+    whole = [o.layer_norm(x, gain, shift, 1e-5, torch.float32, rows=order), o.rms_norm(x, gain, 1e-5, torch.float32, rows=order)]
+    for n in (1, 2, 150, 151, 400, 401, 1500, 1501, 1700):
+        rows = order[:n] if gathered else None
+        few = read if gathered else read[:n]
+        assert torch.equal(o.layer_norm(few, gain, shift, 1e-5, torch.float32, rows=rows), whole[0][:n]), n
+        assert torch.equal(o.rms_norm(few, gain, 1e-5, torch.float32, rows=rows), whole[1][:n]), n
