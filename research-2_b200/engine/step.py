@@ -91,6 +91,25 @@ def _bucket(n: int) -> int:
     return b if n <= 8 else -(-n // 8) * 8
 
 
+class PassOrder:
+    """All passes of a step function, graphs and single launches, use the same caches, states, workspaces and (graphs) activations: a
+    pass on another stream than the one before it waits for that one's end."""
+
+    def __init__(self, device, device_index: int):
+        self.device, self.device_index = device, device_index
+        self.stream = self.done = None   # the last pass': its stream, the event behind it
+
+    def begin(self) -> None:
+        stream = torch._C._cuda_getCurrentRawStream(self.device_index)
+        if self.done is not None and stream != self.stream:
+            torch.cuda.current_stream(self.device).wait_event(self.done)
+        self.stream = stream
+
+    def end(self, event: torch.cuda.Event) -> None:
+        event.record()
+        self.done = event
+
+
 class StepGraph:
     """Forward pass + sampling of a batch of up to `t_cap` rows in up to `r_cap` entries (one
     logit row per entry), as one CUDA graph. t_cap == r_cap is the decode-only form. The graph
@@ -100,7 +119,7 @@ class StepGraph:
 
     def __init__(self, step_fn: "StepFunction", t_cap: int, r_cap: int):
         self.cap = r_cap
-        self.device, self.device_index = step_fn.device, step_fn._device_index
+        self.device, self.order = step_fn.device, step_fn.order
         self.hosts = []
         for _ in range(2):
             host = StepBatch(BatchLayout(t_cap, r_cap, r_cap, step_fn.table_widths), pinned=True)
@@ -126,7 +145,6 @@ class StepGraph:
         if any(a is None for a in self.addresses):
             raise RuntimeError("the step's pinned host memory cannot be reached from the device")
         self.done = self.hosts[1].copy_done   # of the last replay: the tokens are on the host
-        self.stream = None                    # the last replay's
         side = torch.cuda.Stream(device=step_fn.device)
         side.wait_stream(torch.cuda.current_stream(step_fn.device))
         with torch.cuda.stream(side):  # inert warm-up: every row is a pad row
@@ -176,13 +194,10 @@ class StepGraph:
         if batch is not self.host:
             self.host.copy_done.synchronize()
             self.host.buf[:] = batch.buf
-        stream = torch._C._cuda_getCurrentRawStream(self.device_index)
-        if self.stream is not None and stream != self.stream:   # a replay waits for the one before, whose buffers it uses
-            torch.cuda.current_stream(self.device).wait_event(self.done)
-        self.stream = stream
+        self.order.begin()
         self.graph.replay()
         self.done = self.host.copy_done
-        self.done.record()
+        self.order.end(self.done)
         self.turn ^= 1
         ops.count_launches(self.kernels)
 
@@ -211,6 +226,8 @@ class StepFunction:
         self.device = model.rt.device
         # the device's number, for the launch path that skips torch's device guard when it is the current one
         self._device_index = self.device.index if self.device.index is not None else (torch.cuda.current_device() if torch.cuda.is_available() else 0)
+        self.order = PassOrder(self.device, self._device_index)
+        self._pass_done = None   # the event behind passes that are no graphs
         self.groups, self.member_group = derive_groups(model.cache_members, page_size, num_pages)
         self.arena = KVArena(model.cache_members, self.groups, self.member_group, model.rt.dtype, self.device)
         self.state_tensors = [
@@ -289,11 +306,19 @@ class StepFunction:
         self.h2d_bytes += batch.buf.nbytes
         return StepContext(batch, dev)
 
-    def _uploaded_in_front(self, batch: StepBatch) -> StepContext:
-        """`upload` for a forward pass that follows at once, with nothing launched between."""
+    def _launch_by_launch(self, batch: StepBatch, sampled: bool) -> torch.Tensor:
+        """The pass of a batch that is no graph: logits, or with `sampled` the tokens."""
+        self.order.begin()
         ctx = self.upload(batch)
-        ctx.cache_settled = True
-        return ctx
+        ctx.cache_settled = True   # (the copy lies directly in front of the pass)
+        out = self.forward(ctx)
+        if sampled:
+            out = self.sample(out, ctx)
+        if not torch.cuda.is_current_stream_capturing():   # (a caller's own graph orders its replays itself)
+            if self._pass_done is None:
+                self._pass_done = torch.cuda.Event()
+            self.order.end(self._pass_done)
+        return out
 
     def validate(self, batch: StepBatch) -> None:
         """Host-side bounds checks of a batch that the caller filled. A batch that the scheduler
@@ -332,7 +357,7 @@ class StepFunction:
                 graph.replay(batch)
                 self.h2d_bytes += batch.buf.nbytes
                 return graph.logits[: batch.n_logit_rows]
-            return self.forward(self._uploaded_in_front(batch))
+            return self._launch_by_launch(batch, sampled=False)
 
     def launch_graph(self, batch: StepBatch) -> StepGraph | None:
         """Launches the step as its CUDA graph, if the batch is one that the scheduler filled and
@@ -364,8 +389,7 @@ class StepFunction:
                 graph.replay(batch)
                 self.h2d_bytes += batch.buf.nbytes
                 return graph.tokens[: batch.n_logit_rows]
-            ctx = self._uploaded_in_front(batch)
-            return self.sample(self.forward(ctx), ctx)
+            return self._launch_by_launch(batch, sampled=True)
 
 
 def logit_rows_of_last(batch: StepBatch) -> np.ndarray:

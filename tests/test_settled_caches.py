@@ -10,6 +10,18 @@ from research_2_b200.engine import step
 from research_2_b200.engine.batch import batch_for
 
 
+class Event:
+    def __init__(self, name):
+        self.name, self.recorded = name, 0
+
+    def record(self):
+        self.recorded += 1
+
+
+class Order:
+    begin = end = staticmethod(lambda *a: None)
+
+
 def one_row_batch():
     batch = batch_for((4,), 1, 1, 1)
     batch.set_entries([0], [0], [[3]])
@@ -29,14 +41,52 @@ def test_a_context_that_was_uploaded_earlier_is_not_settled():
 @pytest.mark.parametrize("entry", ["__call__", "step_and_sample"])
 def test_the_step_function_settles_the_pass_behind_its_own_copy(entry, monkeypatch):
     monkeypatch.setattr(step.torch.cuda, "device", lambda d: torch.no_grad())
+    monkeypatch.setattr(step.torch.cuda, "is_current_stream_capturing", lambda: False)
     fn, seen = step.StepFunction.__new__(step.StepFunction), []
-    fn.capture, fn._graphs, fn.device, fn._device_index = False, {}, "cpu", 0
+    fn.capture, fn._graphs, fn.device, fn._device_index, fn._pass_done = False, {}, "cpu", 0, Event("pass")
+    fn.order = Order()
     fn.upload, fn.sample = context, lambda logits, ctx: logits
     fn.forward = lambda ctx: seen.append(ctx.cache_settled)
     batch = one_row_batch()
     getattr(fn, entry)(batch)
     assert seen == [True]
     assert fn.upload(batch).cache_settled is False   # (what a caller uploads)
+
+
+def test_a_pass_on_another_stream_waits_for_the_one_before(monkeypatch):
+    """Whichever graph the one before was, and where it was none."""
+    current, waits = [7], []
+
+    class Stream:
+        wait_event = staticmethod(lambda event: waits.append((current[0], event.name)))
+
+    monkeypatch.setattr(step.torch._C, "_cuda_getCurrentRawStream", lambda i: current[0])
+    monkeypatch.setattr(step.torch.cuda, "current_stream", lambda d=None: Stream)
+    monkeypatch.setattr(step.torch.cuda, "device", lambda d: torch.no_grad())
+    monkeypatch.setattr(step.torch.cuda, "is_current_stream_capturing", lambda: False)
+    fn = step.StepFunction.__new__(step.StepFunction)
+    fn.capture, fn._graphs, fn.device, fn._device_index, fn._pass_done = False, {}, "cpu", 0, Event("eager")
+    fn.order = step.PassOrder("cpu", 0)
+    fn.upload, fn.forward = context, lambda ctx: None
+
+    def graph(name):
+        g = step.StepGraph.__new__(step.StepGraph)
+        g.order, g.turn, g.kernels, g.done = fn.order, 0, 0, None
+        g.hosts = [one_row_batch(), one_row_batch()]
+        for i, host in enumerate(g.hosts):
+            host.copy_done = Event(f"{name} {i}")
+            host.copy_done.synchronize = lambda: None
+        g.graph = type("Graph", (), {"replay": staticmethod(lambda: None)})
+        return g
+
+    prompt, decode = graph("prompt"), graph("decode")
+    for launch, stream in [(prompt, 7), (decode, 7), (prompt, 7), (decode, 9), (decode, 9), (prompt, 7), (None, 9), (None, 9), (decode, 7), (None, 7)]:
+        current[0] = stream
+        if launch is None:
+            fn(one_row_batch())
+        else:
+            launch.replay(launch.host)
+    assert waits == [(9, "prompt 1"), (7, "decode 0"), (9, "prompt 0"), (7, "eager")]
 
 
 def test_the_embedding_is_launched_in_plain_order(monkeypatch):

@@ -52,3 +52,31 @@ def test_graph_steps_launched_ahead_give_the_logits_of_eager_ones(tmp_path, dtyp
         else:   # (padded steps may choose other kernels: two roundings of the logits' size apart)
             torch.testing.assert_close(a, b, atol=2.0 ** -5 * float(a.abs().max()), rtol=0.0)
     assert torch.equal(graphs[-1], graphs[-2])
+
+
+@pytest.mark.parametrize("capture", [False, True])
+def test_steps_on_two_streams_in_turn(tmp_path, capture):
+    """Every pass, whichever graph or single launches it takes, waits for the one before, whose caches and buffers it uses: nobody else orders the streams."""
+    import research_2_b200 as r2
+
+    folder = make_model_dir(tmp_path / "tiny", TINY_B, std=0.2)
+    prompts = [random_tokens(60 + i, n, 512) for i, n in enumerate((70, 9, 33))]
+
+    def logits(streams):
+        out = []
+        with r2.run(folder, dtype="bfloat16", block_size=16, max_requests=3, max_batch_tokens=64, capture=capture) as engine:
+            engine.step_fn.capture_after = 0
+            for p in prompts:
+                engine.submit(p, 20)
+            torch.cuda.synchronize()
+            while (plan := engine.plan()) is not None:
+                batch = engine.build_batch(plan)
+                with torch.cuda.stream(streams[len(out) % len(streams)]):
+                    out.append(engine.step_fn(batch).clone())
+                engine.commit(np.full(plan.n_entries, len(out) % 512, dtype=np.int32))
+            torch.cuda.synchronize()
+        return out
+
+    one, two = logits([torch.cuda.current_stream()]), logits([torch.cuda.Stream(), torch.cuda.Stream()])
+    assert len(one) == len(two) > 20
+    assert all(torch.equal(a, b) for a, b in zip(one, two))
