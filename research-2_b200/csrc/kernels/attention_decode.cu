@@ -145,8 +145,11 @@ bool g_decode_mma = true;              // r2_attention_decode_set_mma (tests com
 // between CTAs: clusters cost a launch 0.5 to 0.8 us even where a row is too short for their merge and 1 to 2.7 us where it is not. Inside a
 // step of 8 rows of GPT-2 124M (12 layers; 200 and 500 keys a row) CTAs of four warps in clusters of six take 272 and 285 us, wide ones 236 and 258.
 // NARROW CTAs, several to an SM, are for more pairs than that.
+// CTAs to an SM of the narrow form: five up to head size 64 is what the tiles' shared memory allows; three up to 80 is what the compiler needs a bound
+// for (170 registers without: two CTAs, and 320 pairs of 4,000 keys take 127 us instead of 84); above, two of up to 221 registers (with three
+// of 168, 320 pairs of 128 take 120 us instead of 164 but 512 pairs 217 instead of 182).
 template <int G, bool MMA, int X, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, (MMA && HD <= 64 && WARPS == NARROW) ? 5 : 1)  // five narrow CTAs to an SM is what the tiles' shared memory allows
+__global__ void __launch_bounds__(WARPS * 32, MMA && WARPS == NARROW ? (HD <= 64 ? 5 : HD <= 80 ? 3 : 1) : 1)
 decode_kernel(const DecodeParams p) {
   pdl_launch_dependents();  // the next kernel may begin its prologue
   // The wait on the previous kernel comes further down: positions, context lengths and block
@@ -219,8 +222,9 @@ decode_kernel(const DecodeParams p) {
   // Tiles of 32 keys go through shared memory: every lane copies its own key's K row and V row
   // with 16-byte asynchronous copies, so a tile's 2 x 32 rows are all in flight at once, and
   // (for head sizes up to 128) the next tile is on its way while this one is used. The newest
-  // key's row comes from the projection's output (k_new, v_new), not from the cache: it is left out of the copies and put in its place
-  // once the tile has landed.
+  // key's row comes from the projection's output (k_new, v_new), not from the cache: it is put over what the cache has in its place
+  // once the tile has landed (leaving that row out of the copies is a branch for each of them: 4,000 keys a row, 512 pairs, one CTA each, head
+  // sizes 64, 96 and 128: 94, 171 and 206 us a launch, and 91, 154 and 182 without).
   extern __shared__ __align__(16) uint8_t tile_smem[];
   // this warp's places for tiles: its own and, in the first half of a wide CTA's pair, one behind all warps'
   const int depth = WARPS != NARROW && warp < pair_warps / 2 ? 2 : 1;
@@ -245,7 +249,6 @@ decode_kernel(const DecodeParams p) {
   // then consecutive lanes copy consecutive 16-byte pieces of a row, then the next row: whole
   // lines per request
   auto copy = [&](int tile, uint8_t* to, long long my_row) {
-    const int new_row = tile == tile_of_new ? v_of_pos - tile * 32 : -1;
     const uint32_t kd = smem_u32(to), vd = smem_u32(to + 32 * ROW_BYTES);
 #pragma unroll
     for (int i = 0; i < VECS; ++i) {
@@ -255,10 +258,8 @@ decode_kernel(const DecodeParams p) {
       const int bytes = from >= 0 ? 16 : 0;  // 0 source bytes: zeros
       const bf16* ksrc = from >= 0 ? p.k_cache + from + c * 8 : p.k_cache;
       const bf16* vsrc = from >= 0 ? p.v_cache + from + c * 8 : p.v_cache;
-      if (row != new_row) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kd + row * ROW_BYTES + c * 16), "l"(ksrc), "r"(bytes) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vd + row * ROW_BYTES + c * 16), "l"(vsrc), "r"(bytes) : "memory");
-      }
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kd + row * ROW_BYTES + c * 16), "l"(ksrc), "r"(bytes) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vd + row * ROW_BYTES + c * 16), "l"(vsrc), "r"(bytes) : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -319,6 +320,7 @@ decode_kernel(const DecodeParams p) {
     uint8_t* k_tile = place(it);
     uint8_t* v_tile = k_tile + 32 * ROW_BYTES;
     if (tile == tile_of_new) {
+      __syncwarp();   // (every lane's copies have landed: what the cache has in the newest key's place is overwritten)
 #pragma unroll
       for (int i = 0; i < FRESH; ++i) {
         const int f = lane + 32 * i;
@@ -808,7 +810,7 @@ extern "C" int r2_attention_decode_fused_biased(const void* q, int q_row_stride,
   p.counters = n_slices > 1 ? counters : nullptr;
   p.clustered = n_slices > 1 && n_slices <= MAX_CLUSTER;
   p.n_rows = n_rows;
-  // the caller's plan (r2_attention_decode_plan); the scalar form has narrow CTAs alone
+  // the caller's plan (`decode_plan` in kernels/ops.py); the scalar form has narrow CTAs alone
   p.wide = MMA_FITS && g_decode_mma && pair_warps > NARROW;
   p.pair_warps = p.wide ? pair_warps : NARROW;
   if (p.wide && (pair_warps > WIDE || (pair_warps & (pair_warps - 1)) != 0 || (n_slices > 1 && (pair_warps != WIDE || !p.clustered)))) return R2_BAD_SHAPE;
