@@ -256,20 +256,36 @@ def decode_slices(n_rows: int, n_kv_heads: int, max_context: int, device="cuda:0
 
 
 def decode_plan(n_rows: int, n_kv_heads: int, head_dim: int, max_context: int, device="cuda:0") -> tuple[int, int]:
-    """(slices of the keys, warps of a CTA per (row, kv head) pair) of fused decode attention: wide CTAs, one to an SM, while all pairs find
-    room on the chip side by side (all of a CTA's 16 warps for a pair, 8 for head sizes above 64; half of them where there are more pairs than
-    SMs), with slices (a cluster) only for contexts of more than two tiles a warp and where SMs are left; else narrow ones (`decode_slices`). Measured in
-    steps of GPT-2 (20, 200, 500 and 1,000 keys a row, ms): 124M, 8 rows, narrow 0.245 / 0.272 / 0.285 / 0.338, wide 0.236 / 0.236 / 0.258 /
-    0.295; 16 rows 0.294 / 0.323 / 0.381 / 0.439 and 0.285 / 0.297 / 0.335 / 0.406; 355M, 16 rows (256 pairs) 0.579 / 0.654 / 0.764 / 0.974 and 0.577 /
-    0.602 / 0.679 / 0.825. With 32 rows (384 pairs) short rows are faster narrow (0.334 and 0.370), long ones wide (0.703 and 0.631).
-    One row: two slices cost 12 us of 406 (355M) where they are not needed and gain 33 of 496 at 1,000 keys."""
+    """(slices of the keys, warps of a CTA per (row, kv head) pair) of fused decode attention.
+
+    Pairs up to the SMs: wide CTAs, one to an SM, all of whose warps (16; 8 for head sizes above 64) have one pair, with slices (a cluster)
+    only for contexts of more than two tiles a warp and where SMs are left. Measured in steps of GPT-2, head size 64 (20, 200, 500 and 1,000
+    keys a row, ms): 124M, 8 rows, narrow 0.245 / 0.272 / 0.285 / 0.338, wide 0.236 / 0.236 / 0.258 / 0.295; 16 rows 0.294 / 0.323 / 0.381 /
+    0.439 and 0.285 / 0.297 / 0.335 / 0.406. One row: two slices cost 12 us of 406 (355M) where they are not needed and gain 33 of 496 at 1,000
+    keys. Head sizes above 64 with few pairs take a slice for each tile a warp beyond 640 keys, which costs short rows nothing there (8 pairs of
+    128, us a launch at 20 / 200 / 1,000 keys: two slices 3.2 / 3.7 / 7.2, four 3.2 / 3.7 / 5.1, narrow 3.3 / 5.3 / 5.0).
+
+    Up to two pairs an SM: head sizes up to 64 half a wide CTA each (355M, 16 rows, 256 pairs: narrow 0.579 / 0.654 / 0.764 / 0.974, so 0.577 /
+    0.602 / 0.679 / 0.825; with 384 pairs short rows are faster narrow, 0.334 and 0.370, long ones wide, 0.703 and 0.631), above narrow CTAs in
+    as many slices as an SM's registers hold (three CTAs up to 80, two beyond; 160 pairs of 128 at 200 / 1,000 keys: one slice 7.2 / 24.6, the three
+    of `decode_slices` 13.9 / 27.0 in two waves). Where contexts may be long and there are few more pairs than SMs, either leaves SMs idle that
+    more slices fill (160 pairs at 4,000 keys: of 64 43.3 and 34.2, of 128 90.9 and 71.9; 200 pairs of 128 94.3 and 96.1).
+
+    More pairs: `decode_slices`."""
     pairs, sms = max(1, n_rows * n_kv_heads), sm_count(device)
     wide = 16 if head_dim <= 64 else 8 if head_dim <= 128 else 0
+    narrow = decode_slices(n_rows, n_kv_heads, max_context, device)
     if wide and pairs <= sms:
-        return max(1, min(sms // pairs, -(-max_context // (64 * wide)), 8)), wide
+        slices, tiles = -(-max_context // (64 * wide)), min(-(-max_context // (32 * wide)), 8)
+        if head_dim > 64 and max_context > 80 * wide and pairs * tiles <= 64:
+            slices = tiles
+        return max(1, min(sms // pairs, slices, 8)), wide
     if wide and pairs <= 2 * sms:
-        return 1, wide // 2
-    return decode_slices(n_rows, n_kv_heads, max_context, device), 4
+        held = 2 * sms if head_dim <= 64 else (3 if head_dim <= 80 else 2) * sms
+        if max_context > 2048 and narrow >= 3 and held // pairs == 1:
+            return narrow, 4
+        return (1, 8) if head_dim <= 64 else (max(1, min(held // pairs, narrow)), 4)
+    return narrow, 4
 
 
 def _lib_for_head_dim(source: str, head_dim: int) -> C.CDLL:
