@@ -325,22 +325,48 @@ int by_form(const FewRows& p, cudaStream_t stream) {
   if (p.n <= 2368) return launch<MH, 2, 16, 0>(p, stream);
   if constexpr (MH <= 4) {
     if (p.n <= 4736 && p.k <= 1024) return launch<MH, 4, 16, 0>(p, stream);
-    if (p.n > 7104 && p.k <= 1024) return launch<MH, 4, 8, 0>(p, stream);   // (9,216 x 768, 8 rows: 4.0 us, 16 features 4.5, tcgen05 6.4; 6,144: 3.4 and 3.3)
+    if constexpr (MH <= 2) {
+      if (p.n > 7104 && p.k <= 1024) return launch<MH, 4, 8, 0>(p, stream);   // (9,216 x 768, 8 rows: 4.0 us, 16 features 4.5, tcgen05 6.4; 6,144: 3.4 and 3.3)
+    }
     return launch<MH, 2, 8, 0>(p, stream);
   }
   return launch<MH, 2, 16, 0>(p, stream);
 }
 
+// The most features for which this kernel is no slower than the tcgen05 one, beside the bounds on all weights below. Both measured with 24
+// launches one behind the other, and with a norm of the rows between them, over rows of 1 to 64, K of 64 to 12,288 and 8 to 12,288 features; the line
+// lies where this kernel is more than about 1 us slower in both (an activation adds up to 3 us to the other one: 64 rows of 3,072 x 768
+// take 8.0 / 7.4 us bare, and a step of GPT-2 124M, whose 12 have one, 0.722 / 0.737 ms). This kernel / the other one, us, one behind the other:
+//   * every CTA reads all rows: with many features and a short K that is most of its work (64 rows of 64: 2,560 features 4.8 / 3.1, 6,144
+//     7.0 / 3.2; 24 rows of 256: 8,192 features 5.0 / 4.4, 10,240 7.4 / 3.4). A LayerNorm inside is made anew by every CTA (8 rows of 768: 8,192 features
+//     6.9 / 8.1, 10,240, a second wave, 10.2 / 7.3).
+//   * long K: eight features to a CTA, so the CTAs are many (one row of 2,048: 3,072 features 6.0 / 6.5, 3,584 7.7 / 6.5; of 4,096: 2,560 8.6 / 7.7;
+//     of 8,192: 1,280 9.9 / 8.2; 16 rows of 2,560: 2,560 9.4 / 7.4; 24 of 2,048: 2,560 9.0 / 7.8), and with more than 16 rows one to an SM:
+//     160 of them are two waves (24 rows of 4,096: 1,280 features 9.0 / 7.5; 64 of 3,072: 1,280 12.3 / 9.0).
+int most_features(int m, int k, int norm) {   // norm: 0 none, 1 RMS, 2 LayerNorm
+  if (norm == 2) return 9472;
+  if (m <= 8) return k < 2048 ? 12288 : k <= 3072 ? 3072 : k < 7000 ? 2368 : 1184;
+  if (m <= 16) return k < 2048 ? 9472 : 2368;
+  if (m <= 32) return k < 128 ? 4736 : k < 2048 ? 7104 : k <= 3072 ? 2368 : 1184;
+  return k < 128 ? 2368 : k < 2048 ? 4608 : k <= 4608 ? 1184 : 0;
+}
+
 }  // namespace
+
+// Whether the kernel is the choice for these sizes (`norm`: 0 none, 1 RMS norm, 2 LayerNorm). Bounds on all weights: many weights for many
+// rows, where every CTA's reading of all rows outweighs the shorter path (K x N 6,400 x 1,600: 16 rows 9.4 us there and 9.7 here; 768 x 9,216, 24 rows: 7.3
+// and 7.6; 1,600 x 4,800, 32 rows: 8.1 and 10.2; 64 rows of 4,608 x 768 8.9 and 8.9, of 6,144 x 768 9.9 and 10.9).
+extern "C" int r2_few_rows_takes(int m, int n, int k, int norm) {
+  const long long weights = (long long)n * k;
+  const long long most = m > 32 ? (k >= 2048 ? 4000000LL : 2400000LL) : m > 16 ? (k >= 2048 ? 6500000LL : 4500000LL) : m > 8 ? (k > 4096 ? 5000000LL : 8000000LL) : 12000000LL;
+  return m <= 64 && weights <= most && n <= most_features(m, k, norm);
+}
 
 // a [m, k] bfloat16 (row stride lda), or x [m, k] float with gain [k] and, centred, shift [k] (a is then ignored); w [n, k] bfloat16 (row
 // stride ldw); bias [n] float or null; residual [m, n] float or null, added after the activation; out [m, n] bfloat16 or float. With
 // group_n > 0 the rows are [m, n / group_n * k] wide and features s * group_n .. read the columns from s * k on.
-// R2_UNSUPPORTED where the tcgen05 kernel is the faster one or must decide: more than 64 rows; more than 12,288 features (a table of
-// logits is a matter of bandwidth: 10.9 us there, 12.4 here); many weights for many rows, where every CTA's reading of all rows outweighs
-// the shorter path (K x N 6,400 x 1,600: 16 rows 9.4 us there and 9.7 here; 6,144 x 1,024: 16 rows 8.2 and 8.6, 32 rows 9.4 and 7.6; 768 x 9,216, 24
-// rows: 7.3 and 7.6; 1,600 x 4,800, 32 rows: 8.1 and 10.2; 64 rows of 4,608 x 768 8.9 and 8.9, of 6,144 x 768 9.9 and 10.9, of 768 x 3,072 8.4 and
-// 6.0); norms beyond 16 rows or 1,024 numbers; rows that are no multiples of 16 bytes.
+// R2_UNSUPPORTED where the tcgen05 kernel must decide (more than 64 rows, norms beyond 16 rows or 1,024 numbers, rows that are no multiples of
+// 16 bytes) or is the faster one (`most_features`).
 extern "C" int r2_few_rows(const void* a, int lda, const float* x, int ldx, const float* gain, const float* shift, float eps, int centred,
                            const void* w, int ldw, const float* bias, const float* residual, int ldr, void* out, int ldo, int out_dtype,
                            int m, int n, int k, int act, int group_n, cudaStream_t stream) {
@@ -353,9 +379,7 @@ extern "C" int r2_few_rows(const void* a, int lda, const float* x, int ldx, cons
   } else if (lda % 8 != 0 || (reinterpret_cast<uintptr_t>(a) & 15)) {
     return R2_UNSUPPORTED;
   }
-  const long long weights = (long long)n * k;
-  const long long most = m > 32 ? (k >= 2048 ? 4000000LL : 2400000LL) : m > 16 ? (k >= 2048 ? 6500000LL : 4500000LL) : m > 8 ? (k > 4096 ? 5000000LL : 8000000LL) : 12000000LL;
-  if (m > 64 || n > 12288 || weights > most) return R2_UNSUPPORTED;
+  if (!r2_few_rows_takes(m, n, k, x == nullptr ? 0 : centred ? 2 : 1)) return R2_UNSUPPORTED;
   if (group_n > 0 && (n % group_n != 0 || group_n % 32 != 0)) return R2_UNSUPPORTED;   // (a CTA's features lie in one group)
   const FewRows p{static_cast<const bf16*>(a), lda, x, ldx, gain, shift, eps, centred, static_cast<const bf16*>(w), ldw, bias, residual, ldr, out, ldo,
                   out_dtype == R2_BF16, m, n, k, act, group_n};
