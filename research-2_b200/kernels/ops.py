@@ -62,7 +62,7 @@ _uses: dict[str, int] = {}
 
 
 def kernel_uses() -> dict[str, int]:
-    """How often each attention kernel has been chosen (tests check the choice by it)."""
+    """How often a kernel has been chosen where there is a choice: attention, linear attention, products of few rows (tests check by it)."""
     return dict(_uses)
 
 
@@ -1375,6 +1375,7 @@ def _linear_of_normed(a: NormedRows, w, bias, w_is_nk, act, residual, out_dtype,
             _p(residual), ldr, _p(out), _rows(out, "out"), dtype_code(out.dtype), m, n, k, ACTIVATIONS[act], 0, _stream())
         if status != -4:
             _check(status, "linear (few rows, norm inside)")
+            _used("few_rows")
             return out
     ws = _workspace(a.device)
     status = _lib("gemm_tc").r2_gemm_tc(
@@ -1471,6 +1472,7 @@ def linear(a, w: torch.Tensor, bias: torch.Tensor | None = None, *, w_is_nk: boo
                 dtype_code(out.dtype), m, n, k, ACTIVATIONS[act], 0, _stream())
             if status != -4:
                 _check(status, "linear (few rows)")
+                _used("few_rows")
                 return out
         ws = _workspace(a.device)
         status = _lib("gemm_tc").r2_gemm_tc(
@@ -1504,6 +1506,7 @@ def grouped_linear(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
                                                   BF16, t, n * per, k, ACT_NONE, per, _stream())
             if status != -4:
                 _check(status, "grouped_linear (few rows)")
+                _used("few_rows")
                 return out
         status = _lib("gemm_tc").r2_gemm_tc_grouped(_p(flat), n * k, _p(w), _rows(w, "w"), _p(out), n * per, t, per, k, n, BF16,
                                                     _p(_workspace(a.device).error), _stream())
