@@ -681,8 +681,10 @@ __device__ __forceinline__ void finish_tile_rows(const GemmParams& p, uint32_t l
 // EW: epilogue warps. Token-major tiles with an SM to themselves have eight, two to a quarter of the tile's rows that take half of its columns
 // each: the epilogue of four warps was 2.1 to 4 us of the 6.7 to 12 that a product of 528 rows takes after its wait (528 x 1,024 x 1,024 with a residual
 // 7.7 and now 6.8 us a launch, 2,046 x 1,024 x 1,024 10.9 and 9.0, 2,046 x 1,600 x 1,600 16.2 and 13.3).
+// Token-major tiles of four epilogue warps run two CTAs to an SM. So does the form with the norm inside: its bound is that of a table of logits (393 CTAs),
+// which has its norm made apart since; what still comes here has up to 128 tiles and was not measured with one CTA to an SM.
 template <bool A_MN, bool B_MN, bool TRANSPOSED, bool FUSED_LN = false, bool ROUTED = false, bool SHARED = false, int EW = 4>
-__global__ void __launch_bounds__(64 + EW * 32, ((TRANSPOSED && !FUSED_LN) || EW == 8) ? 1 : 2)  // token-major tiles run two CTAs to an SM, and so does the form with the norm inside (the logits' 393 CTAs)
+__global__ void __launch_bounds__(64 + EW * 32, ((TRANSPOSED && !FUSED_LN) || EW == 8) ? 1 : 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -915,7 +917,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int q = warp & 3;  // tensor-memory lanes [32q, 32q + 32) belong to warps with id % 4 == q
     const int side = EW == 8 ? (warp - 2) >> 2 : 0;   // which half of the columns (of a shared K's groups every other one)
     if constexpr (!TRANSPOSED) {
-      // the tile's bias, once for the four epilogue warps, while the products run
+      // the tile's bias, once for all epilogue warps, while the products run
       for (int j = int(threadIdx.x) - 64; j < p.bn; j += EW * 32) reduce[j] = (p.bias != nullptr && b0 + j < p.b_total) ? p.bias[b0 + j] : 0.f;
       asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");
     }
@@ -965,7 +967,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int j = 0; j < 32; ++j) to[j * BM] = r[j];
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes, read by the bulk copies
-      asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");               // the four epilogue warps
+      asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");               // all epilogue warps
       if (warp == 2 && lane < p.bn / SHARE_COLS && lane % p.splits != int(rank)) {
         const uint32_t to = uint32_t(lane % p.splits), owned = uint32_t((p.bn / SHARE_COLS - int(to) + p.splits - 1) / p.splits);
         const uint32_t sender = rank < to ? rank : rank - 1;
@@ -1001,7 +1003,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes, read by the bulk copy
-      asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");               // the four epilogue warps
+      asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");               // all epilogue warps
       if (threadIdx.x == 64) {
         uint32_t remote, remote_bar;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(reduce)), "r"(0u));
@@ -1519,7 +1521,8 @@ int g_pair_form = 1;
 
 // Tile width and shares of K of a token-major product, by a model of its time in nanoseconds. A k-block of 64 is bound by the SM's
 // shared memory (TMA writes it, the tensor core reads it: 48, 64 and 80 KB at 64, 128 and 192 columns): measured 200, 225 and
-// 252 ns with one CTA on an SM, 140 and 175 a CTA with two; what no k-block hides (launch, first loads, epilogue) 4.3, 5.2 and 6.5 us. Sharing
+// 252 ns with one CTA on an SM, 140 and 175 a CTA with two; what no k-block hides (launch, first loads, epilogue) 4.3, 5.2 and 6.5 us. (Both, and the
+// price of sharing, were measured with four epilogue warps; with eight, where a tile has an SM to itself, they are 0.9 to 2.9 us less, which the model leaves out.) Sharing
 // K over a cluster costs 3.8 us (3.0 with 64 columns). Measured against a 128-column tile a CTA, which was the only form (us): 512 x 1,024 x 1,024
 // 8.7 and now 6.9, 512 x 4,096 x 1,024 19.8 and 12.2, 1,024 x 768 x 768 7.8 and 6.4, 200 x 768 x 2,304 6.7 and 5.4, 512 x 6,400 x 1,600 29.6 and
 // 19.1, 2,048 x 6,400 x 1,600 (144 tiles of 192 columns in one wave instead of 208) 48.6 and 38.7. (Tiles of 256 columns are never the best.)

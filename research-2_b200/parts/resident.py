@@ -95,8 +95,8 @@ class ResidentLayers:
         n = x.shape[0]
         most = min(self.max_rows, ops.resident_decode_rows())
         if self.width > 1024 and n > 8:
-            # measured at width 1,600 (GPT-2 1.5B): 3.39 against 3.12 ms a step at 12 rows, 3.56 against 3.24 at 16; at
-            # width 1,024 the resident kernel is still the faster one there (1.16 against 1.24 ms at 16 rows)
+            # measured at width 1,600 (GPT-2 1.5B) against the chain when its products ran on tcgen05: 3.39 and 3.12 ms a step at 12
+            # rows, 3.56 and 3.24 at 16. (With csrc/kernels/few_rows.cu the chain is the faster form at every width: `set_resident_decode_rows`.)
             most = min(most, 8)
         if not (ctx.decode_only and 0 < n <= most and x.is_contiguous()):
             return None

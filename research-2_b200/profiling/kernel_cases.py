@@ -45,10 +45,11 @@ def cases(rows: int = 8):
     torch.manual_seed(0)
     Q = H * HD
     x = torch.randn(2048, D, device=dev).bfloat16()
-    wqkv = (torch.randn(D, 3 * Q, device=dev) * 0.02).bfloat16()
-    wfc = (torch.randn(D, F, device=dev) * 0.02).bfloat16()
-    wproj = (torch.randn(Q, D, device=dev) * 0.02).bfloat16()
-    wproj2 = (torch.randn(F, D, device=dev) * 0.02).bfloat16()
+    # (matrices stored [out, in], as a bfloat16 step keeps them)
+    wqkv = (torch.randn(3 * Q, D, device=dev) * 0.02).bfloat16()
+    wfc = (torch.randn(F, D, device=dev) * 0.02).bfloat16()
+    wproj = (torch.randn(D, Q, device=dev) * 0.02).bfloat16()
+    wproj2 = (torch.randn(D, F, device=dev) * 0.02).bfloat16()
     wte = (torch.randn(V, D, device=dev) * 0.02).bfloat16()
     bf, bqkv, bd = torch.zeros(F, device=dev), torch.zeros(3 * Q, device=dev), torch.zeros(D, device=dev)
     x8k = torch.randn(8192, D, device=dev).bfloat16()
@@ -57,22 +58,22 @@ def cases(rows: int = 8):
     out = []
     for t, xt in ((2048, x), (8192, x8k)):
         out += [
-            (f"prefill: qkv product, {t:,} x {D:,} x {3 * Q:,}", lambda xt=xt: ops.linear(xt, wqkv, bqkv), 0, 2 * t * D * 3 * Q),
-            (f"prefill: fc product with gelu, {t:,} x {D:,} x {F:,}", lambda xt=xt: ops.linear(xt, wfc, bf, act="gelu_new"), 0, 2 * t * D * F),
+            (f"prefill: qkv product, {t:,} x {D:,} x {3 * Q:,}", lambda xt=xt: ops.linear(xt, wqkv, bqkv, w_is_nk=True), 0, 2 * t * D * 3 * Q),
+            (f"prefill: fc product with gelu, {t:,} x {D:,} x {F:,}", lambda xt=xt: ops.linear(xt, wfc, bf, w_is_nk=True, act="gelu_new"), 0, 2 * t * D * F),
         ]
     # the same q/k/v product with the keys and values going straight into the rows' cache slots (2 x 1,024 tokens)
     kc2, vc2, _, stride2, pages2 = paged(2)
     slots2 = torch.arange(PS, PS + 2048, dtype=torch.int32, device=dev)
     scatter = ops.kv_scatter(slots2, kc2, vc2, stride2, PS, pages2, Q, Q, HD)
     q_out = torch.empty(2048, 3 * Q, device=dev, dtype=torch.bfloat16)
-    out.append((f"prefill: qkv product with cache write, 2,048 x {D:,} x {3 * Q:,}", lambda: ops.linear(x, wqkv, bqkv, out=q_out, kv=scatter), 0, 2 * 2048 * D * 3 * Q))
+    out.append((f"prefill: qkv product with cache write, 2,048 x {D:,} x {3 * Q:,}", lambda: ops.linear(x, wqkv, bqkv, w_is_nk=True, out=q_out, kv=scatter), 0, 2 * 2048 * D * 3 * Q))
     out += [
-        (f"prefill: attention output product + residual, 2,048 x {Q:,} x {D:,}", lambda: ops.linear(x[:, :Q].contiguous() if Q != D else x, wproj, bd, residual=r2k), 0, 2 * 2048 * Q * D),
-        (f"prefill: mlp output product + residual, 2,048 x {F:,} x {D:,}", lambda: ops.linear(h2k, wproj2, bd, residual=r2k), 0, 2 * 2048 * F * D),
+        (f"prefill: attention output product + residual, 2,048 x {Q:,} x {D:,}", lambda: ops.linear(x[:, :Q].contiguous() if Q != D else x, wproj, bd, w_is_nk=True, residual=r2k), 0, 2 * 2048 * Q * D),
+        (f"prefill: mlp output product + residual, 2,048 x {F:,} x {D:,}", lambda: ops.linear(h2k, wproj2, bd, w_is_nk=True, residual=r2k), 0, 2 * 2048 * F * D),
     ]
     h128, r128 = h2k[:128].contiguous(), r2k[:128].contiguous()
     out.append((f"prefill: mlp output product + residual, 128 x {F:,} x {D:,} (6 tiles: what one SM takes in)",
-                lambda: ops.linear(h128, wproj2, bd, residual=r128), 0, 2 * 128 * F * D))
+                lambda: ops.linear(h128, wproj2, bd, w_is_nk=True, residual=r128), 0, 2 * 128 * F * D))
     ln_out, ln_g, ln_b = torch.empty(2048, D, device=dev, dtype=torch.bfloat16), torch.ones(D, device=dev), torch.zeros(D, device=dev)
     out.append((f"prefill: LayerNorm, 2,048 x {D:,}", lambda: ops.layer_norm(r2k, ln_g, ln_b, 1e-5, torch.bfloat16, out=ln_out), 2048 * D * 6, 0))
     for r in sorted({8, 64, rows}):
@@ -86,10 +87,10 @@ def cases(rows: int = 8):
     fr = torch.randn(rows, F, device=dev).bfloat16()
     normed = lambda: ops.NormedRows(hr, gamma, beta, 1e-5, torch.bfloat16)
     out += [
-        (f"decode: LayerNorm + qkv product, {rows} x {D:,} x {3 * Q:,}", lambda: ops.linear(normed(), wqkv, bqkv), wqkv.numel() * 2, 2 * rows * D * 3 * Q),
-        (f"decode: attention output product + residual, {rows} x {Q:,} x {D:,}", lambda: ops.linear(ar, wproj, bd, residual=hr), wproj.numel() * 2, 2 * rows * Q * D),
-        (f"decode: LayerNorm + fc product with gelu, {rows} x {D:,} x {F:,}", lambda: ops.linear(normed(), wfc, bf, act="gelu_new"), wfc.numel() * 2, 2 * rows * D * F),
-        (f"decode: mlp output product + residual, {rows} x {F:,} x {D:,}", lambda: ops.linear(fr, wproj2, bd, residual=hr), wproj2.numel() * 2, 2 * rows * F * D),
+        (f"decode: LayerNorm + qkv product, {rows} x {D:,} x {3 * Q:,}", lambda: ops.linear(normed(), wqkv, bqkv, w_is_nk=True), wqkv.numel() * 2, 2 * rows * D * 3 * Q),
+        (f"decode: attention output product + residual, {rows} x {Q:,} x {D:,}", lambda: ops.linear(ar, wproj, bd, w_is_nk=True, residual=hr), wproj.numel() * 2, 2 * rows * Q * D),
+        (f"decode: LayerNorm + fc product with gelu, {rows} x {D:,} x {F:,}", lambda: ops.linear(normed(), wfc, bf, w_is_nk=True, act="gelu_new"), wfc.numel() * 2, 2 * rows * D * F),
+        (f"decode: mlp output product + residual, {rows} x {F:,} x {D:,}", lambda: ops.linear(fr, wproj2, bd, w_is_nk=True, residual=hr), wproj2.numel() * 2, 2 * rows * F * D),
     ]
     logits = torch.randn(rows, V, device=dev)
     zeros_i = torch.zeros(rows, dtype=torch.int32, device=dev)
@@ -110,7 +111,7 @@ def cases(rows: int = 8):
         out.append((f"decode: attention with cache write, {batch} rows x {H} heads, context {ctx_len}",
                     lambda qkv=qkv, slots=slots, kc=kc, vc=vc, page_stride=page_stride, n_pages=n_pages, tables=tables, row_ids=row_ids,
                     pos=pos, lens=lens: ops.decode_attention_fused(qkv[:, :Q], qkv[:, Q: 2 * Q], qkv[:, 2 * Q:], slots, kc, vc, page_stride,
-                                                                   PS, n_pages, tables, row_ids, pos, lens, H, H, HD, HD**-0.5, 0, 1024),
+                                                                   PS, n_pages, tables, row_ids, pos, lens, H, H, HD, HD**-0.5, 0, 1024, cache_settled=True),
                     batch * ctx_len * 2 * Q * 2, 4 * batch * ctx_len * Q))
     # prefill attention: the tcgen05 kernel, then the mma.sync one. 2 and 8 prompts of 1,024 tokens; one prompt of 128 to
     # 1,024 tokens (every CTA alone on an SM: the time of a key tile and what a CTA costs besides); a length that is no
@@ -200,7 +201,7 @@ def gated_cases(rows: int = 8, kv_heads: int | None = None, window: int = 256, k
                         pos=pos, lens=lens, win=win, keep=keep: ops.decode_attention_fused(
                             qkvg[:, :Q], qkvg[:, Q: Q + KV], qkvg[:, Q + KV: Q + 2 * KV], slots, kc, vc, page_stride, PS, n_pages, tables,
                             row_ids, pos, lens, H, G, HD, HD**-0.5, win, 1024, keep_first=keep, sink=True, gate=qkvg[:, Q + 2 * KV:],
-                            exact_weights=True),
+                            exact_weights=True, cache_settled=True),
                         batch * seen * 2 * KV * 2, 4 * batch * seen * Q))
 
     def attention_case(name, entries, win, keep):
