@@ -774,6 +774,13 @@ int rows_per_cta(int n_rows, int n_sms, size_t per_row) {
 
 }  // namespace
 
+// Whether few rows take a CTA a row and group: while a wave of four to an SM holds them all, and with groups to share a row's work. One group of all heads
+// has a CTA a row either way, and eight warps for its gates instead of sixteen (6 rows of 768, head size 64, one group of 4 / 12 / 24 heads: 5.4 / 9.7 /
+// 16.2 us, the other kernel 4.9 / 6.7 / 9.4; two groups of 6 heads 0.5 to 1.0 of its time, of 16 heads 0.6 to 1.1).
+extern "C" int r2_delta_prepare_by_group(int n_rows, int n_heads, int n_groups, int n_sms) {
+  return n_groups > 1 && n_heads / n_groups <= 16 && (long long)n_rows * n_groups <= 4LL * n_sms;
+}
+
 // in [T, 2 groups dim + heads vdim], h [T, width], w_gates [2 heads, width] (dtype); everything else float: see DeltaPrepareArgs.
 extern "C" int r2_delta_prepare(const void* in, int in_stride, const void* h, int h_stride, int width, const float* taps, int n_taps,
                                 const void* w_gates, const float* step_bias, const float* log_rate, float q_scale, float unit_eps, int n_heads,
@@ -793,8 +800,7 @@ extern "C" int r2_delta_prepare(const void* in, int in_stride, const void* h, in
   const int rows = rows_per_cta(n_rows, n_sms, per_row), shares = 1;
   const size_t piece = dtype == R2_F32 ? 16 : 8, few_smem = sizeof(float) * (size_t(width) + 2 * dim + 2 * (n_heads / n_groups));
   const bool pieces = width % 4 == 0 && h_stride % 4 == 0 && reinterpret_cast<uintptr_t>(h) % piece == 0 && reinterpret_cast<uintptr_t>(w_gates) % piece == 0;
-  // a CTA a row and group while a wave of four to an SM holds them all
-  if (rows == 1 && n_taps <= PREP_FEW_TAPS && pieces && few_smem <= 40 * 1024 && (long long)n_rows * n_groups <= 4LL * n_sms && (dtype == R2_F32 || dtype == R2_BF16)) {
+  if (rows == 1 && n_taps <= PREP_FEW_TAPS && pieces && few_smem <= 40 * 1024 && r2_delta_prepare_by_group(n_rows, n_heads, n_groups, n_sms) && (dtype == R2_F32 || dtype == R2_BF16)) {
     if (dtype == R2_F32) r2_launch(delta_prepare_few_kernel<float>, dim3(n_groups, n_rows), dim3(PREP_FEW_THREADS), few_smem, stream, a);
     else r2_launch(delta_prepare_few_kernel<bf16>, dim3(n_groups, n_rows), dim3(PREP_FEW_THREADS), few_smem, stream, a);
     return launch_status();

@@ -1,5 +1,5 @@
-"""Which products of few rows their own kernel takes: the sizes at which it was measured to be slower go to the tcgen05 kernel, as they did
-before there was another."""
+"""Which kernels for few rows are taken: the sizes at which they were measured to be slower go to the general kernel, as they did before there was
+another."""
 
 from __future__ import annotations
 
@@ -34,3 +34,11 @@ def test_sizes_that_the_other_kernel_does_faster(m, n, k, norm):
 ])
 def test_sizes_that_it_takes(m, n, k, norm):
     assert takes(m, n, k, norm)
+
+
+@pytest.mark.parametrize("rows,heads,groups,by_group", [(6, 12, 6, True), (1, 12, 2, True), (148, 16, 4, True), (149, 16, 4, False), (6, 12, 1, False), (1, 32, 1, False), (6, 34, 2, False)])
+def test_what_the_delta_rule_walks_over_by_row_and_group(rows, heads, groups, by_group):
+    try:
+        assert bool(kernel_library("state_scan").r2_delta_prepare_by_group(rows, heads, groups, 148)) is by_group
+    except BuildError as err:
+        pytest.skip(str(err))
