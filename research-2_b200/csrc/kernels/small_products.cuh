@@ -36,6 +36,33 @@ __device__ __forceinline__ int warp_sums(float (&v)[N], int lane) {
   return index;
 }
 
+// A lane's share of row . w: pieces of four, 128 apart, eight asked for at a time. All eight are asked for under a condition each and not in a loop
+// unrolled by eight, whose rest, all six pieces of a row of 768, would be one round trip after the other.
+template <typename W>
+__device__ __forceinline__ float lane_product(const float* row, int kpad, const W* __restrict__ w, int K, bool pieces, int lane) {
+  constexpr int AHEAD = 8;
+  float acc = 0.f;
+  for (int k0 = lane * 4; k0 < kpad; k0 += 128 * AHEAD) {
+    float4 v[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int k = k0 + 128 * u;
+      if (k >= kpad) v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      else if (pieces) v[u] = load4(w + k);
+      else v[u] = make_float4(to_float(w[k]), k + 1 < K ? to_float(w[k + 1]) : 0.f, k + 2 < K ? to_float(w[k + 2]) : 0.f, k + 3 < K ? to_float(w[k + 3]) : 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int k = k0 + 128 * u;
+      if (k < kpad) {
+        const float4 m = *reinterpret_cast<const float4*>(row + k);
+        acc = fmaf(m.w, v[u].w, fmaf(m.z, v[u].z, fmaf(m.y, v[u].y, fmaf(m.x, v[u].x, acc))));
+      }
+    }
+  }
+  return acc;
+}
+
 // rows[r] . w[n] for ROWS rows in shared memory ([ROWS][kpad] float, kpad a multiple of 4, zeros from K on) and every row n of
 // w [N][K] (float or bfloat16): a warp has OUTS outputs of all rows at a time, lanes over K in pieces of four, so the matrix comes out of L2 once for all
 // rows. emit(r, n, sum) is called by one lane, the lanes of a warp side by side. A sum is made in the same order whatever ROWS and OUTS are.
@@ -49,7 +76,9 @@ __device__ __forceinline__ void rows_times_matrix(const float* rows, int kpad, c
     for (int o = 0; o < OUTS; ++o)
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) acc[o][r] = 0.f;
-#pragma unroll (OUTS * ROWS == 1 ? 8 : 2)
+    if constexpr (OUTS * ROWS == 1) acc[0][0] = lane_product(rows, kpad, w + size_t(n0) * K, K, pieces, lane);
+    else
+#pragma unroll 2
     for (int k = lane * 4; k < kpad; k += 128) {
       float4 v[OUTS];
 #pragma unroll

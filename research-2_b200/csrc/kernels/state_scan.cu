@@ -627,13 +627,7 @@ delta_prepare_few_kernel(const DeltaPrepareArgs a) {
       if (lane == 0) product = kq * kn * qn;
     } else {              // a gate or a step
       const T* w = static_cast<const T*>(a.w_gates) + size_t(n < per ? grp * per + n : a.heads + grp * per + (n - per)) * a.width;
-      float acc = 0.f;
-#pragma unroll 8
-      for (int k = lane * 4; k < a.width; k += 128) {
-        const float4 m = *reinterpret_cast<const float4*>(row_h + k), v = load4(w + k);
-        acc = fmaf(m.w, v.w, fmaf(m.z, v.z, fmaf(m.y, v.y, fmaf(m.x, v.x, acc))));
-      }
-      acc = warp_sum(acc);
+      const float acc = warp_sum(lane_product(row_h, a.width, w, a.width, true, lane));
       if (lane == 0) gates[n] = acc;
     }
   }
