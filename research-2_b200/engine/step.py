@@ -308,13 +308,16 @@ class StepFunction:
 
     def _launch_by_launch(self, batch: StepBatch, sampled: bool) -> torch.Tensor:
         """The pass of a batch that is no graph: logits, or with `sampled` the tokens."""
-        self.order.begin()
+        # in a caller's own graph nothing can wait for what lies outside it: the caller orders its replays
+        ordered = not torch.cuda.is_current_stream_capturing()
+        if ordered:
+            self.order.begin()
         ctx = self.upload(batch)
         ctx.cache_settled = True   # (the copy lies directly in front of the pass)
         out = self.forward(ctx)
         if sampled:
             out = self.sample(out, ctx)
-        if not torch.cuda.is_current_stream_capturing():   # (a caller's own graph orders its replays itself)
+        if ordered:
             if self._pass_done is None:
                 self._pass_done = torch.cuda.Event()
             self.order.end(self._pass_done)

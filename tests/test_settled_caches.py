@@ -89,6 +89,24 @@ def test_a_pass_on_another_stream_waits_for_the_one_before(monkeypatch):
     assert waits == [(9, "prompt 1"), (7, "decode 0"), (9, "prompt 0"), (7, "eager")]
 
 
+def test_a_pass_in_a_callers_own_graph_waits_for_nothing_outside_it(monkeypatch):
+    """(An event recorded outside a capture ends the capture with an error.)"""
+    calls = []
+
+    class Recorder:
+        begin = staticmethod(lambda: calls.append("begin"))
+        end = staticmethod(lambda event: calls.append("end"))
+
+    monkeypatch.setattr(step.torch.cuda, "device", lambda d: torch.no_grad())
+    fn = step.StepFunction.__new__(step.StepFunction)
+    fn.capture, fn._graphs, fn.device, fn._device_index, fn._pass_done = False, {}, "cpu", 0, Event("eager")
+    fn.order, fn.upload, fn.forward = Recorder(), context, lambda ctx: None
+    for capturing in (True, False):
+        monkeypatch.setattr(step.torch.cuda, "is_current_stream_capturing", lambda: capturing)
+        fn(one_row_batch())
+        assert calls == ([] if capturing else ["begin", "end"])
+
+
 def test_the_embedding_is_launched_in_plain_order(monkeypatch):
     from research_2_b200.parts import Runtime, embedding
 
@@ -141,3 +159,23 @@ def test_two_contexts_uploaded_before_either_pass():
     want = logits(False)
     assert torch.isfinite(want).all() and np.isfinite(float(want.abs().max()))
     assert torch.equal(logits(True), want)
+
+
+@pytest.mark.gpu
+def test_a_pass_in_a_callers_own_graph(tmp_path):
+    import research_2_b200 as r2
+    from tests.helpers import TINY_B, make_model_dir, random_tokens
+
+    folder = make_model_dir(tmp_path / "tiny", TINY_B, std=0.2)
+    with r2.run(folder, dtype="bfloat16", block_size=16, max_requests=1, max_batch_tokens=64, capture=False) as engine:
+        engine.submit(random_tokens(5, 40, 512), 4)
+        batch = engine.build_batch(engine.plan())
+        want = engine.step_fn(batch).clone()   # on the current stream; a capture has one of its own
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = engine.step_fn(batch)
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
