@@ -288,6 +288,7 @@ class StepFunction:
         graph = self._graphs.get((t_cap, r_cap))
         if graph is None:
             with torch.cuda.device(self.device):
+                self.order.begin()   # (its warm-up uses what a pass on another stream may still use)
                 graph = StepGraph(self, t_cap, r_cap)
             self._graphs[(t_cap, r_cap)] = graph
         return graph

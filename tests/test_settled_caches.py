@@ -107,6 +107,21 @@ def test_a_pass_in_a_callers_own_graph_waits_for_nothing_outside_it(monkeypatch)
         assert calls == ([] if capturing else ["begin", "end"])
 
 
+def test_a_graph_made_on_another_stream_waits_for_the_pass_before(monkeypatch):
+    """Its warm-up passes write the same workspaces and pad pages."""
+    calls = []
+
+    class Recorder:
+        begin = staticmethod(lambda: calls.append("begin"))
+
+    monkeypatch.setattr(step.torch.cuda, "device", lambda d: torch.no_grad())
+    monkeypatch.setattr(step, "StepGraph", lambda *a: calls.append("warm-up"))
+    fn = step.StepFunction.__new__(step.StepFunction)
+    fn._graphs, fn.device, fn.order = {}, "cpu", Recorder()
+    fn._graph(4, 4)
+    assert calls == ["begin", "warm-up"]
+
+
 def test_the_embedding_is_launched_in_plain_order(monkeypatch):
     from research_2_b200.parts import Runtime, embedding
 
