@@ -88,103 +88,165 @@ __global__ void layer_norm_kernel(const float* __restrict__ x, const int32_t* __
   }
 }
 
-// Both norms of rows (LayerNorm; RMS norm with the gain offset + weight) for rows of up to 2,048 elements whose length is a multiple of 4. A row is
-// a run of chunks of 128 elements, four to a lane. A lane adds its values four chunks at a time, then the fours one after the other, and the lanes' sums
-// are joined by the warp's exchanges. Whether every warp of a CTA has four chunks of one row (ROWS 1) and takes the others' sums from shared memory, or
-// a warp has a row of its own (ROWS of them to a CTA), changes no bit: a row's result does not depend on how many rows share its step.
-//
-// What bounds it up to some thousand rows is the path from the last store of the kernel before: a CTA a row asks for the row and its gain and shift in one
-// round trip. Beyond, it is the bytes and the warps that an SM holds: a warp a row, as many chunks as the width has, gains asked for at the end.
-template <typename O, bool CENTRED, int CHUNKS, int ROWS>
-__global__ void __launch_bounds__(ROWS > 1 ? 32 * ROWS : 128, ROWS > 1 ? (CHUNKS > 12 || (CENTRED && CHUNKS > 8) ? 16 : 20) / ROWS : 1)
+// Both norms of rows (LayerNorm; RMS norm with the gain offset + weight) for rows of up to 2,048 elements whose length is a multiple of 4:
+// a CTA a row, eight or sixteen values a thread, so that the path from the last store of the kernel before is one round trip for the row and its gain
+// and shift together, ten shuffles and one barrier. A warp's sum and squares about its own mean join as one set's would (Chan, Golub and
+// LeVeque). The hand-over between kernels bounds it; the form before had a warp a row with up to 16 pieces a lane and asked for gain and
+// shift at the end. Inside a
+// decode step, us a launch, before and now: 4.2 and 1.9 for 32 rows of 768, 5.3 and 2.1 for 8 rows of 1,600; a step of 512 prompt rows of 355M takes 0.06 ms less
+// of 1.5.
+template <typename O, bool CENTRED, int PIECES>   // PIECES: pieces of eight values a thread
+__global__ void __launch_bounds__(256)
 norm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const float* __restrict__ gain, const float* __restrict__ shift,
-                 O* __restrict__ out, int n_rows, int width, float eps, float offset) {
+                 O* __restrict__ out, int width, float eps, float offset) {
   pdl_launch_dependents();
   pdl_wait();
-  static_assert(ROWS > 1 || CHUNKS == 4, "the warps that share a row have four chunks each");
-  __shared__ float parts[2][ROWS > 1 ? 1 : 4][32];   // (a row's warps) the lanes' sums, squares
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, first = ROWS > 1 ? 0 : warp * CHUNKS;
-  const int r = ROWS > 1 ? blockIdx.x * ROWS + warp : blockIdx.x;
-  if (ROWS > 1 && r >= n_rows) return;
-  const int n_warps = blockDim.x >> 5;
-  const bool shared = ROWS == 1 && n_warps > 1;
+  constexpr int SHARE = 256 * PIECES;   // values of a warp
+  __shared__ float2 shares[8];          // of every warp: mean, squares
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+  const int r = blockIdx.x, d0 = warp * SHARE + lane * 8;
   const int src = rows != nullptr ? rows[r] : r;
   const float* xr = x + size_t(src) * width;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto place = [&](int i) { return (first + i) * 128 + lane * 4; };
-  float4 v[CHUNKS], g[CHUNKS], b[CHUNKS];
+  float4 v[2 * PIECES], g[2 * PIECES], b[2 * PIECES];
 #pragma unroll
-  for (int i = 0; i < CHUNKS; ++i) v[i] = place(i) < width ? *reinterpret_cast<const float4*>(xr + place(i)) : zero;
-  if (ROWS == 1) {   // few rows: gain and shift in the same round trip
+  for (int i = 0; i < 2 * PIECES; ++i) {
+    const int d = d0 + (i >> 1) * 256 + (i & 1) * 4;
+    v[i] = d < width ? *reinterpret_cast<const float4*>(xr + d) : zero;
+  }
 #pragma unroll
-    for (int i = 0; i < CHUNKS; ++i) {
-      g[i] = place(i) < width ? *reinterpret_cast<const float4*>(gain + place(i)) : zero;
-      b[i] = CENTRED && place(i) < width ? *reinterpret_cast<const float4*>(shift + place(i)) : zero;
+  for (int i = 0; i < 2 * PIECES; ++i) {
+    const int d = d0 + (i >> 1) * 256 + (i & 1) * 4;
+    g[i] = d < width ? *reinterpret_cast<const float4*>(gain + d) : zero;
+    b[i] = CENTRED && d < width ? *reinterpret_cast<const float4*>(shift + d) : zero;
+  }
+  float mean = 0.f;
+  if (CENTRED) {
+    const int count = max(0, min(SHARE, width - warp * SHARE));
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2 * PIECES; ++i) sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+    sum = warp_sum(sum);
+    mean = count > 0 ? sum / float(count) : 0.f;
+  }
+  float sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < 2 * PIECES; ++i) {
+    const float e = ((v[i].x - mean) * (v[i].x - mean) + (v[i].y - mean) * (v[i].y - mean)) + ((v[i].z - mean) * (v[i].z - mean) + (v[i].w - mean) * (v[i].w - mean));
+    if (d0 + (i >> 1) * 256 + (i & 1) * 4 < width) sq += e;
+  }
+  sq = warp_sum(sq);
+  if (n_warps > 1) {
+    if (lane == 0) shares[warp] = make_float2(mean, sq);
+    __syncthreads();
+    float total = 0.f;
+    sq = 0.f;
+    if (CENTRED) {
+      for (int i = 0; i < n_warps; ++i) total += shares[i].x * float(max(0, min(SHARE, width - i * SHARE)));
+      mean = total / float(width);
+    }
+    for (int i = 0; i < n_warps; ++i) {
+      const float2 s = shares[i];
+      const float c = s.x - mean;
+      sq += CENTRED ? fmaf(float(max(0, min(SHARE, width - i * SHARE))), c * c, s.y) : s.y;
     }
   }
-  // the row's sum of every lane's values of the chunks: four chunks, then the fours one after the other, then the lanes
-  auto total = [&](int which, auto chunk) {
-    auto four = [&](int i) { return (chunk(i) + (i + 1 < CHUNKS ? chunk(i + 1) : 0.f)) + ((i + 2 < CHUNKS ? chunk(i + 2) : 0.f) + (i + 3 < CHUNKS ? chunk(i + 3) : 0.f)); };
-    float sum = 0.f;
-    if (shared) {
-      parts[which][warp][lane] = four(0);
-      __syncthreads();
+  const float inv = 1.f / sqrtf(sq / float(width) + eps);
+  auto value = [&](float f, float gf, float bf) { return CENTRED ? (f - mean) * inv * gf + bf : f * inv * (offset + gf); };
+  O* o = out + size_t(r) * width;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (i < n_warps) sum += parts[which][i][lane];
+  for (int i = 0; i < PIECES; ++i) {
+    const int d = d0 + i * 256;
+    const bool lo = d < width, hi = d + 4 < width;
+    const float4 u = make_float4(value(v[2 * i].x, g[2 * i].x, b[2 * i].x), value(v[2 * i].y, g[2 * i].y, b[2 * i].y),
+                                 value(v[2 * i].z, g[2 * i].z, b[2 * i].z), value(v[2 * i].w, g[2 * i].w, b[2 * i].w));
+    const float4 w = make_float4(value(v[2 * i + 1].x, g[2 * i + 1].x, b[2 * i + 1].x), value(v[2 * i + 1].y, g[2 * i + 1].y, b[2 * i + 1].y),
+                                 value(v[2 * i + 1].z, g[2 * i + 1].z, b[2 * i + 1].z), value(v[2 * i + 1].w, g[2 * i + 1].w, b[2 * i + 1].w));
+    if constexpr (sizeof(O) == 2) {
+      const __nv_bfloat162 p0 = __floats2bfloat162_rn(u.x, u.y), p1 = __floats2bfloat162_rn(u.z, u.w), p2 = __floats2bfloat162_rn(w.x, w.y), p3 = __floats2bfloat162_rn(w.z, w.w);
+      const uint2 first = make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
+      const uint2 second = make_uint2(*reinterpret_cast<const uint32_t*>(&p2), *reinterpret_cast<const uint32_t*>(&p3));
+      if (width % 8 == 0) {   // (else rows begin on multiples of 8 bytes)
+        if (lo) *reinterpret_cast<uint4*>(o + d) = make_uint4(first.x, first.y, second.x, second.y);
+      } else {
+        if (lo) *reinterpret_cast<uint2*>(o + d) = first;
+        if (hi) *reinterpret_cast<uint2*>(o + d + 4) = second;
+      }
     } else {
-#pragma unroll
-      for (int i = 0; i < CHUNKS; i += 4) sum += four(i);   // (past the row: zeros, which change no bit)
+      if (lo) *reinterpret_cast<float4*>(o + d) = u;
+      if (hi) *reinterpret_cast<float4*>(o + d + 4) = w;
     }
-    return warp_sum(sum);
-  };
-  float mean = 0.f;
-  if (CENTRED) mean = total(0, [&](int i) { return (v[i].x + v[i].y) + (v[i].z + v[i].w); }) / float(width);
-  const float squares = total(1, [&](int i) {
-    const float p = v[i].x - mean, q = v[i].y - mean, s = v[i].z - mean, t = v[i].w - mean;
-    return place(i) < width ? fmaf(p, p, q * q) + fmaf(s, s, t * t) : 0.f;
-  });
-  const float inv = 1.f / sqrtf(squares / float(width) + eps);
-  auto value = [&](float f, float gf, float bf) { return CENTRED ? fmaf((f - mean) * inv, gf, bf) : f * inv * (offset + gf); };
+  }
+}
+
+// The same with a warp a row and four rows a CTA, for thousands of rows: fewer warps wait for the kernel before.
+template <typename O, bool CENTRED>
+__global__ void __launch_bounds__(128)
+norm_many_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const float* __restrict__ gain, const float* __restrict__ shift,
+                      O* __restrict__ out, int n_rows, int width, float eps, float offset) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (r >= n_rows) return;
+  const int src = rows != nullptr ? rows[r] : r;
+  const float4* xr = reinterpret_cast<const float4*>(x + size_t(src) * width);
+  constexpr int CHUNKS = 2048 / 128;
+  float4 v[CHUNKS];
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < CHUNKS; ++i) {
+    v[i] = (lane + 32 * i) * 4 < width ? xr[lane + 32 * i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+  }
+  const float mean = CENTRED ? warp_sum(sum) / float(width) : 0.f;
+  float sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < CHUNKS; ++i) {
+    const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
+    if ((lane + 32 * i) * 4 < width) sq += (a * a + b * b) + (c * c + d * d);
+  }
+  const float inv = 1.f / sqrtf(warp_sum(sq) / float(width) + eps);
   O* o = out + size_t(r) * width;
 #pragma unroll
   for (int i = 0; i < CHUNKS; ++i) {
-    const int d = place(i);
-    if (d < width) {
-      if (ROWS > 1) {
-        g[i] = *reinterpret_cast<const float4*>(gain + d);
-        b[i] = CENTRED ? *reinterpret_cast<const float4*>(shift + d) : zero;
-      }
-      const float y0 = value(v[i].x, g[i].x, b[i].x), y1 = value(v[i].y, g[i].y, b[i].y), y2 = value(v[i].z, g[i].z, b[i].z), y3 = value(v[i].w, g[i].w, b[i].w);
+    const int k = (lane + 32 * i) * 4;
+    if (k < width) {
+      const float4 g = *reinterpret_cast<const float4*>(gain + k);
+      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (CENTRED) b = *reinterpret_cast<const float4*>(shift + k);
+      auto value = [&](float f, float gf, float bf) { return CENTRED ? (f - mean) * inv * gf + bf : f * inv * (offset + gf); };
+      const float y0 = value(v[i].x, g.x, b.x), y1 = value(v[i].y, g.y, b.y), y2 = value(v[i].z, g.z, b.z), y3 = value(v[i].w, g.w, b.w);
       if constexpr (sizeof(O) == 2) {
         const __nv_bfloat162 lo = __floats2bfloat162_rn(y0, y1), hi = __floats2bfloat162_rn(y2, y3);
-        *reinterpret_cast<uint2*>(o + d) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        *reinterpret_cast<uint2*>(o + k) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
       } else {
-        *reinterpret_cast<float4*>(o + d) = make_float4(y0, y1, y2, y3);
+        *reinterpret_cast<float4*>(o + k) = make_float4(y0, y1, y2, y3);
       }
     }
   }
 }
 
-// A CTA a row and a warp a row, us a launch one behind the other (LayerNorm into bfloat16; rows of 768, 1,024, 1,600): 1 row 1.6, 1.6, 1.6 and 1.8, 1.8, 2.2;
-// 528 rows 2.0, 2.1, 2.6 and 2.1, 2.3, 3.1; 1,500 rows 2.8, 2.9, 4.0 and 3.0, 3.2, 3.9; 2,046 rows 3.6, 3.8, 4.6 and 3.2, 3.3, 3.8. RMS norm: 1.4, 1.4, 1.4 and
-// 1.6, 1.7, 2.2; 1.7, 1.8, 2.4 and 1.9, 2.0, 2.7; 2.2, 2.3, 3.5 and 2.7, 3.0, 3.4; 2.6, 2.7, 3.8 and 2.8, 2.9, 3.3 (4,096 rows 4.8, 5.0, 6.8 and 3.2, 3.4, 5.5).
+// What each form adds to a step in front of a product, us (rows of 768, 1,024 and 1,600): 264 rows 2.1, 2.1 and 3.6 with eight values a thread,
+// 2.1, 2.3 and 3.3 with sixteen, 3.1, 3.1 and 3.5 with a warp a row; 528 rows 2.6, 3.5, 3.8 / 2.5, 2.9, 3.7 / 3.3, 3.3, 3.8; 1,000 rows 3.6, 3.9, 5.1 / 3.6,
+// 3.9, 4.1 / 3.6, 3.9, 4.6; 2,046 rows 4.1, 5.5, 8.0 / 3.6, 4.9, 6.4 / 3.4, 4.4, 5.0. (Warps that wait for the kernel before keep the next one's out.)
+// Each form adds a row in an order of its own, so the choice by the number of rows is bfloat16's alone: float32 rows have the same bits whatever shares
+// their step, and take the first form at any number (its 3 us more at 2,046 rows of 1,600 stand beside products of milliseconds).
 template <typename O, bool CENTRED>
 static int launch_norm_rows(const float* x, const int32_t* rows, const float* gain, const float* shift, void* out, int n_rows, int width, float eps, float offset,
                             cudaStream_t stream) {
-  const int chunks = (width + 127) / 128;
-  constexpr int MANY = 4;
-  auto go = [&](auto kernel, int ctas, int warps) {
-    r2_launch(kernel, dim3(ctas), dim3(warps * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), n_rows, width, eps, offset);
-  };
-  const int ctas = (n_rows + MANY - 1) / MANY;
-  if (n_rows <= 1800) go(norm_rows_kernel<O, CENTRED, 4, 1>, n_rows, (chunks + 3) / 4);
-  else if (chunks <= 2) go(norm_rows_kernel<O, CENTRED, 2, MANY>, ctas, MANY);
-  else if (chunks <= 4) go(norm_rows_kernel<O, CENTRED, 4, MANY>, ctas, MANY);
-  else if (chunks <= 6) go(norm_rows_kernel<O, CENTRED, 6, MANY>, ctas, MANY);
-  else if (chunks <= 8) go(norm_rows_kernel<O, CENTRED, 8, MANY>, ctas, MANY);
-  else if (chunks <= 12) go(norm_rows_kernel<O, CENTRED, 12, MANY>, ctas, MANY);
-  else go(norm_rows_kernel<O, CENTRED, 16, MANY>, ctas, MANY);
+  const int warps = (width + 255) / 256;
+  if constexpr (sizeof(O) == 2) {
+    if (n_rows > 1500) {
+      r2_launch(norm_many_rows_kernel<O, CENTRED>, dim3((n_rows + 3) / 4), dim3(128), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), n_rows, width, eps, offset);
+      return launch_status();
+    }
+    if (n_rows * warps > 1200) {
+      r2_launch(norm_rows_kernel<O, CENTRED, 2>, dim3(n_rows), dim3((width + 511) / 512 * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
+      return launch_status();
+    }
+  }
+  r2_launch(norm_rows_kernel<O, CENTRED, 1>, dim3(n_rows), dim3(warps * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
   return launch_status();
 }
 
