@@ -179,74 +179,120 @@ norm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, 
   }
 }
 
-// The same with a warp a row and four rows a CTA, for thousands of rows: fewer warps wait for the kernel before.
-template <typename O, bool CENTRED>
-__global__ void __launch_bounds__(128)
+// The same norms for rows by the thousand (a warp a row, ROWS of them to a CTA), and for float32, whose rows have one order of summation, at any number
+// (ROWS 1: every warp of a CTA has four chunks of one row and takes the others' sums from shared memory, which changes no bit). A row is a run of
+// chunks of 128 elements, four to a lane. A lane adds its chunks one after the other, in float32 four at a time and then the fours (fewer sums to
+// exchange: 8 rows of 768 1.8 us with all of them); the lanes' sums are joined by the warp's exchanges.
+// What bounds rows by the thousand is the bytes and the warps that an SM holds (AT_ONCE CTAs): as many chunks as the width has, gains asked for at the end. Up to
+// 12 rows an SM, which find room side by side with registers for 2,048 elements, those are faster.
+template <typename O, bool CENTRED, int CHUNKS, int ROWS, int AT_ONCE>
+__global__ void __launch_bounds__(ROWS > 1 ? 32 * ROWS : 128, AT_ONCE)
 norm_many_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const float* __restrict__ gain, const float* __restrict__ shift,
                       O* __restrict__ out, int n_rows, int width, float eps, float offset) {
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (r >= n_rows) return;
+  static_assert(ROWS > 1 || CHUNKS == 4, "the warps that share a row have four chunks each");
+  constexpr bool FOURS = sizeof(O) == 4;
+  static_assert(ROWS > 1 || FOURS, "the warps that share a row exchange fours");
+  __shared__ float parts[2][ROWS > 1 ? 1 : 4][32];   // (a row's warps) the lanes' sums, squares
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, first = ROWS > 1 ? 0 : warp * CHUNKS;
+  const int r = ROWS > 1 ? blockIdx.x * ROWS + warp : blockIdx.x;
+  if (ROWS > 1 && r >= n_rows) return;
+  const int n_warps = blockDim.x >> 5;
+  const bool shared = ROWS == 1 && n_warps > 1;
   const int src = rows != nullptr ? rows[r] : r;
-  const float4* xr = reinterpret_cast<const float4*>(x + size_t(src) * width);
-  constexpr int CHUNKS = 2048 / 128;
-  float4 v[CHUNKS];
-  float sum = 0.f;
+  const float* xr = x + size_t(src) * width;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto place = [&](int i) { return (first + i) * 128 + lane * 4; };
+  float4 v[CHUNKS], g[CHUNKS], b[CHUNKS];
 #pragma unroll
-  for (int i = 0; i < CHUNKS; ++i) {
-    v[i] = (lane + 32 * i) * 4 < width ? xr[lane + 32 * i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
-  }
-  const float mean = CENTRED ? warp_sum(sum) / float(width) : 0.f;
-  float sq = 0.f;
+  for (int i = 0; i < CHUNKS; ++i) v[i] = place(i) < width ? *reinterpret_cast<const float4*>(xr + place(i)) : zero;
+  if (ROWS == 1) {   // few rows: gain and shift in the same round trip
 #pragma unroll
-  for (int i = 0; i < CHUNKS; ++i) {
-    const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
-    if ((lane + 32 * i) * 4 < width) sq += (a * a + b * b) + (c * c + d * d);
+    for (int i = 0; i < CHUNKS; ++i) {
+      g[i] = place(i) < width ? *reinterpret_cast<const float4*>(gain + place(i)) : zero;
+      b[i] = CENTRED && place(i) < width ? *reinterpret_cast<const float4*>(shift + place(i)) : zero;
+    }
   }
-  const float inv = 1.f / sqrtf(warp_sum(sq) / float(width) + eps);
+  // the row's sum of every lane's values of the chunks (past the row: zeros, which change no bit)
+  auto total = [&](int which, auto chunk) {
+    auto four = [&](int i) { return (chunk(i) + (i + 1 < CHUNKS ? chunk(i + 1) : 0.f)) + ((i + 2 < CHUNKS ? chunk(i + 2) : 0.f) + (i + 3 < CHUNKS ? chunk(i + 3) : 0.f)); };
+    float sum = 0.f;
+    if (shared) {
+      parts[which][warp][lane] = four(0);
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < n_warps) sum += parts[which][i][lane];
+    } else if (FOURS) {
+#pragma unroll
+      for (int i = 0; i < CHUNKS; i += 4) sum += four(i);
+    } else {
+#pragma unroll
+      for (int i = 0; i < CHUNKS; ++i) sum += chunk(i);
+    }
+    return warp_sum(sum);
+  };
+  float mean = 0.f;
+  if (CENTRED) mean = total(0, [&](int i) { return (v[i].x + v[i].y) + (v[i].z + v[i].w); }) / float(width);
+  const float squares = total(1, [&](int i) {
+    const float p = v[i].x - mean, q = v[i].y - mean, s = v[i].z - mean, t = v[i].w - mean;
+    if (!CENTRED && !FOURS) return place(i) < width ? (p * p + q * q) + (s * s + t * t) : 0.f;
+    return place(i) < width ? fmaf(p, p, q * q) + fmaf(s, s, t * t) : 0.f;
+  });
+  const float inv = 1.f / sqrtf(squares / float(width) + eps);
+  auto value = [&](float f, float gf, float bf) { return CENTRED ? fmaf((f - mean) * inv, gf, bf) : f * inv * (offset + gf); };
   O* o = out + size_t(r) * width;
 #pragma unroll
   for (int i = 0; i < CHUNKS; ++i) {
-    const int k = (lane + 32 * i) * 4;
-    if (k < width) {
-      const float4 g = *reinterpret_cast<const float4*>(gain + k);
-      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (CENTRED) b = *reinterpret_cast<const float4*>(shift + k);
-      auto value = [&](float f, float gf, float bf) { return CENTRED ? (f - mean) * inv * gf + bf : f * inv * (offset + gf); };
-      const float y0 = value(v[i].x, g.x, b.x), y1 = value(v[i].y, g.y, b.y), y2 = value(v[i].z, g.z, b.z), y3 = value(v[i].w, g.w, b.w);
+    const int d = place(i);
+    if (d < width) {
+      if (ROWS > 1) {
+        g[i] = *reinterpret_cast<const float4*>(gain + d);
+        b[i] = CENTRED ? *reinterpret_cast<const float4*>(shift + d) : zero;
+      }
+      const float y0 = value(v[i].x, g[i].x, b[i].x), y1 = value(v[i].y, g[i].y, b[i].y), y2 = value(v[i].z, g[i].z, b[i].z), y3 = value(v[i].w, g[i].w, b[i].w);
       if constexpr (sizeof(O) == 2) {
         const __nv_bfloat162 lo = __floats2bfloat162_rn(y0, y1), hi = __floats2bfloat162_rn(y2, y3);
-        *reinterpret_cast<uint2*>(o + k) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        *reinterpret_cast<uint2*>(o + d) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
       } else {
-        *reinterpret_cast<float4*>(o + k) = make_float4(y0, y1, y2, y3);
+        *reinterpret_cast<float4*>(o + d) = make_float4(y0, y1, y2, y3);
       }
     }
   }
 }
 
-// What each form adds to a step in front of a product, us (rows of 768, 1,024 and 1,600): 264 rows 2.1, 2.1 and 3.6 with eight values a thread,
+// Bfloat16: what each form adds to a step in front of a product, us (rows of 768, 1,024 and 1,600): 264 rows 2.1, 2.1 and 3.6 with eight values a thread,
 // 2.1, 2.3 and 3.3 with sixteen, 3.1, 3.1 and 3.5 with a warp a row; 528 rows 2.6, 3.5, 3.8 / 2.5, 2.9, 3.7 / 3.3, 3.3, 3.8; 1,000 rows 3.6, 3.9, 5.1 / 3.6,
-// 3.9, 4.1 / 3.6, 3.9, 4.6; 2,046 rows 4.1, 5.5, 8.0 / 3.6, 4.9, 6.4 / 3.4, 4.4, 5.0. (Warps that wait for the kernel before keep the next one's out.)
-// Each form adds a row in an order of its own, so the choice by the number of rows is bfloat16's alone: float32 rows have the same bits whatever shares
-// their step, and take the first form at any number (its 3 us more at 2,046 rows of 1,600 stand beside products of milliseconds).
+// 3.9, 4.1 / 3.6, 3.9, 4.6; 2,046 rows 4.1, 5.5, 8.0 / 3.6, 4.9, 6.4 / 3.4, 4.4, 5.0. (Warps that wait for the kernel before keep the next one's out.) The forms
+// add a row in orders of their own, so a row's last bit depends on how many rows share its step.
+// Float32 rows have the same bits whatever shares their step, so they take one order: a CTA a row up to 1,500 rows, a warp a row beyond.
+// A warp a row with registers for 2,048 elements and for the row's alone, LayerNorm into bfloat16, us one behind the other (768, 1,024, 1,600): 1,501 rows 2.8, 3.0,
+// 3.4 and 3.0, 3.2, 3.9; 2,046 rows 4.5, 4.8, 5.4 and 3.2, 3.2, 3.8; 4,096 rows 6.2, 6.6, 7.4 and 4.1, 4.9, 6.5.
 template <typename O, bool CENTRED>
 static int launch_norm_rows(const float* x, const int32_t* rows, const float* gain, const float* shift, void* out, int n_rows, int width, float eps, float offset,
                             cudaStream_t stream) {
-  const int warps = (width + 255) / 256;
-  if constexpr (sizeof(O) == 2) {
-    if (n_rows > 1500) {
-      r2_launch(norm_many_rows_kernel<O, CENTRED>, dim3((n_rows + 3) / 4), dim3(128), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), n_rows, width, eps, offset);
-      return launch_status();
-    }
-    if (n_rows * warps > 1200) {
-      r2_launch(norm_rows_kernel<O, CENTRED, 2>, dim3(n_rows), dim3((width + 511) / 512 * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
-      return launch_status();
-    }
+  const int warps = (width + 255) / 256, chunks = (width + 127) / 128;
+  constexpr int MANY = 4;
+  const int ctas = (n_rows + MANY - 1) / MANY;
+  auto go = [&](auto kernel, int n_ctas, int n_warps) {
+    r2_launch(kernel, dim3(n_ctas), dim3(n_warps * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), n_rows, width, eps, offset);
+  };
+  if (n_rows > 1500) {
+    if (n_rows <= 12 * 148) go(norm_many_rows_kernel<O, CENTRED, 16, MANY, 1>, ctas, MANY);
+    else if (chunks <= 2) go(norm_many_rows_kernel<O, CENTRED, 2, MANY, 5>, ctas, MANY);
+    else if (chunks <= 4) go(norm_many_rows_kernel<O, CENTRED, 4, MANY, 5>, ctas, MANY);
+    else if (chunks <= 6) go(norm_many_rows_kernel<O, CENTRED, 6, MANY, 5>, ctas, MANY);
+    else if (chunks <= 8) go(norm_many_rows_kernel<O, CENTRED, 8, MANY, 5>, ctas, MANY);
+    else if (chunks <= 12) go(norm_many_rows_kernel<O, CENTRED, 12, MANY, CENTRED ? 4 : 5>, ctas, MANY);
+    else go(norm_many_rows_kernel<O, CENTRED, 16, MANY, 4>, ctas, MANY);
+  } else if constexpr (sizeof(O) == 4) {
+    go(norm_many_rows_kernel<O, CENTRED, 4, 1, 1>, n_rows, (chunks + 3) / 4);
+  } else if (n_rows * warps > 1200) {
+    r2_launch(norm_rows_kernel<O, CENTRED, 2>, dim3(n_rows), dim3((width + 511) / 512 * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
+  } else {
+    r2_launch(norm_rows_kernel<O, CENTRED, 1>, dim3(n_rows), dim3(warps * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
   }
-  r2_launch(norm_rows_kernel<O, CENTRED, 1>, dim3(n_rows), dim3(warps * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
   return launch_status();
 }
 

@@ -356,17 +356,18 @@ def test_routers_around_a_warp_of_outputs(experts, groups, keep, top, scoring, r
     assert int(chosen.min()) >= 0 and int(chosen.max()) < experts
 
 
-@pytest.mark.parametrize("width", [256, 768, 1600, 2048])
+# widths around every number of chunks that a warp may have; the last number of rows of a CTA each, and beyond
+@pytest.mark.parametrize("width", [4, 128, 132, 256, 260, 512, 768, 772, 1024, 1028, 1600, 2048])
 @pytest.mark.parametrize("gathered", [False, True])
 def test_float32_norms_have_the_same_bits_beside_any_number_of_rows(width, gathered):
     o = ops()
     gen = torch.Generator(device=DEV).manual_seed(width)
-    x = torch.randn(1700, width, generator=gen, device=DEV) + 3.0
+    x = torch.randn(2100, width, generator=gen, device=DEV) + 3.0
     gain, shift = torch.randn(width, generator=gen, device=DEV), torch.randn(width, generator=gen, device=DEV)
-    order = torch.randperm(1700, generator=gen, device=DEV).to(torch.int32) if gathered else torch.arange(1700, dtype=torch.int32, device=DEV)
+    order = torch.randperm(2100, generator=gen, device=DEV).to(torch.int32) if gathered else torch.arange(2100, dtype=torch.int32, device=DEV)
     read = x if gathered else x[order.long()]
     whole = [o.layer_norm(x, gain, shift, 1e-5, torch.float32, rows=order), o.rms_norm(x, gain, 1e-5, torch.float32, rows=order)]
-    for n in (1, 2, 150, 151, 400, 401, 1500, 1501, 1700):
+    for n in (1, 2, 150, 151, 401, 1500, 1501, 1776, 1777, 2099):
         rows = order[:n] if gathered else None
         few = read if gathered else read[:n]
         assert torch.equal(o.layer_norm(few, gain, shift, 1e-5, torch.float32, rows=rows), whole[0][:n]), n
