@@ -88,17 +88,17 @@ __global__ void layer_norm_kernel(const float* __restrict__ x, const int32_t* __
   }
 }
 
-// Both norms of rows (LayerNorm; RMS norm with the gain offset + weight) for rows of up to 2,048 elements whose length is a multiple of 4:
+// Both norms of rows (LayerNorm; RMS norm with the gain offset + weight) into bfloat16, for rows of up to 2,048 elements whose length is a multiple of 4:
 // a CTA a row, eight or sixteen values a thread, so that the path from the last store of the kernel before is one round trip for the row and its gain
 // and shift together, ten shuffles and one barrier. A warp's sum and squares about its own mean join as one set's would (Chan, Golub and
 // LeVeque). The hand-over between kernels bounds it; the form before had a warp a row with up to 16 pieces a lane and asked for gain and
 // shift at the end. Inside a
 // decode step, us a launch, before and now: 4.2 and 1.9 for 32 rows of 768, 5.3 and 2.1 for 8 rows of 1,600; a step of 512 prompt rows of 355M takes 0.06 ms less
 // of 1.5.
-template <typename O, bool CENTRED, int PIECES>   // PIECES: pieces of eight values a thread
+template <bool CENTRED, int PIECES>   // PIECES: pieces of eight values a thread
 __global__ void __launch_bounds__(256)
 norm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const float* __restrict__ gain, const float* __restrict__ shift,
-                 O* __restrict__ out, int width, float eps, float offset) {
+                 bf16* __restrict__ out, int width, float eps, float offset) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr int SHARE = 256 * PIECES;   // values of a warp
@@ -153,7 +153,7 @@ norm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, 
   }
   const float inv = 1.f / sqrtf(sq / float(width) + eps);
   auto value = [&](float f, float gf, float bf) { return CENTRED ? (f - mean) * inv * gf + bf : f * inv * (offset + gf); };
-  O* o = out + size_t(r) * width;
+  bf16* o = out + size_t(r) * width;
 #pragma unroll
   for (int i = 0; i < PIECES; ++i) {
     const int d = d0 + i * 256;
@@ -162,19 +162,14 @@ norm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, 
                                  value(v[2 * i].z, g[2 * i].z, b[2 * i].z), value(v[2 * i].w, g[2 * i].w, b[2 * i].w));
     const float4 w = make_float4(value(v[2 * i + 1].x, g[2 * i + 1].x, b[2 * i + 1].x), value(v[2 * i + 1].y, g[2 * i + 1].y, b[2 * i + 1].y),
                                  value(v[2 * i + 1].z, g[2 * i + 1].z, b[2 * i + 1].z), value(v[2 * i + 1].w, g[2 * i + 1].w, b[2 * i + 1].w));
-    if constexpr (sizeof(O) == 2) {
-      const __nv_bfloat162 p0 = __floats2bfloat162_rn(u.x, u.y), p1 = __floats2bfloat162_rn(u.z, u.w), p2 = __floats2bfloat162_rn(w.x, w.y), p3 = __floats2bfloat162_rn(w.z, w.w);
-      const uint2 first = make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
-      const uint2 second = make_uint2(*reinterpret_cast<const uint32_t*>(&p2), *reinterpret_cast<const uint32_t*>(&p3));
-      if (width % 8 == 0) {   // (else rows begin on multiples of 8 bytes)
-        if (lo) *reinterpret_cast<uint4*>(o + d) = make_uint4(first.x, first.y, second.x, second.y);
-      } else {
-        if (lo) *reinterpret_cast<uint2*>(o + d) = first;
-        if (hi) *reinterpret_cast<uint2*>(o + d + 4) = second;
-      }
+    const __nv_bfloat162 p0 = __floats2bfloat162_rn(u.x, u.y), p1 = __floats2bfloat162_rn(u.z, u.w), p2 = __floats2bfloat162_rn(w.x, w.y), p3 = __floats2bfloat162_rn(w.z, w.w);
+    const uint2 first = make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
+    const uint2 second = make_uint2(*reinterpret_cast<const uint32_t*>(&p2), *reinterpret_cast<const uint32_t*>(&p3));
+    if (width % 8 == 0) {   // (else rows begin on multiples of 8 bytes)
+      if (lo) *reinterpret_cast<uint4*>(o + d) = make_uint4(first.x, first.y, second.x, second.y);
     } else {
-      if (lo) *reinterpret_cast<float4*>(o + d) = u;
-      if (hi) *reinterpret_cast<float4*>(o + d + 4) = w;
+      if (lo) *reinterpret_cast<uint2*>(o + d) = first;
+      if (hi) *reinterpret_cast<uint2*>(o + d + 4) = second;
     }
   }
 }
@@ -289,9 +284,9 @@ static int launch_norm_rows(const float* x, const int32_t* rows, const float* ga
   } else if constexpr (sizeof(O) == 4) {
     go(norm_many_rows_kernel<O, CENTRED, 4, 1, 1>, n_rows, (chunks + 3) / 4);
   } else if (n_rows * warps > 1200) {
-    r2_launch(norm_rows_kernel<O, CENTRED, 2>, dim3(n_rows), dim3((width + 511) / 512 * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
+    r2_launch(norm_rows_kernel<CENTRED, 2>, dim3(n_rows), dim3((width + 511) / 512 * 32), size_t(0), stream, x, rows, gain, shift, static_cast<bf16*>(out), width, eps, offset);
   } else {
-    r2_launch(norm_rows_kernel<O, CENTRED, 1>, dim3(n_rows), dim3(warps * 32), size_t(0), stream, x, rows, gain, shift, static_cast<O*>(out), width, eps, offset);
+    r2_launch(norm_rows_kernel<CENTRED, 1>, dim3(n_rows), dim3(warps * 32), size_t(0), stream, x, rows, gain, shift, static_cast<bf16*>(out), width, eps, offset);
   }
   return launch_status();
 }
