@@ -271,7 +271,11 @@ def decode_plan(n_rows: int, n_kv_heads: int, head_dim: int, max_context: int, d
     of `decode_slices` 13.9 / 27.0 in two waves). Where contexts may be long and there are few more pairs than SMs, either leaves SMs idle that
     more slices fill (160 pairs at 4,000 keys: of 64 43.3 and 34.2, of 128 90.9 and 71.9; 200 pairs of 128 94.3 and 96.1).
 
-    More pairs: `decode_slices`."""
+    More pairs: `decode_slices`.
+
+    A captured step's plan goes by the longest context that it may meet, so the plan is for the rows that such a step has most of the time. Rows of 8,000
+    keys and more that few pairs have are faster narrow (8 pairs of 128, wide and narrow, us: 4,000 keys 7.3 and 8.0, 8,000 11.8 and 10.9, 16,000 20.7 and
+    16.2, 32,000 45 and 31; 16 pairs in groups of four 16.2 and 24.9, 25 and 31, 51 and 47, 90 and 68), rows of 4,000 and less slower, up to 3.5 times."""
     pairs, sms = max(1, n_rows * n_kv_heads), sm_count(device)
     wide = 16 if head_dim <= 64 else 8 if head_dim <= 128 else 0
     narrow = decode_slices(n_rows, n_kv_heads, max_context, device)
